@@ -77,6 +77,7 @@ struct sayram_batch_s {
   int* d_tile = nullptr;
   double *d_xe = nullptr, *d_ye = nullptr, *d_wx = nullptr, *d_wy = nullptr, *d_dirv = nullptr;
   double* d_part = nullptr;
+  long long pstride = 0;       // reduction segments the partial-sum arrays hold per quantity
   double* d_stage = nullptr;   // 6 * max instance cells (setup) / packed field (get/set)
   long long ycap_ = 0;         // y-edge table length
   double* d_tab = nullptr;     // D table (3 * n_alpha * n_energy), grown on demand
@@ -201,6 +202,10 @@ struct sayram_batch_s {
   int nchunks_of(int nx, int ny) const {
     const long long cells = round_up((long long)ny * round_up(nx, 4), 4);
     return (int)((cells + chunk - 1) / chunk);
+  }
+  int nsegs_of(const InstDev& I) const {  // reduction segments of an instance
+    const int s = sg::seg_cells(chunk);
+    return (int)(((long long)I.ny * I.pitch + s - 1) / s);
   }
   // dynamic shared memory of the SpMV kernels: the chunk plus one row above and below
   template <typename T>
@@ -472,7 +477,8 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
   SG_ALLOC(d_wx, 2 * xcap);
   SG_ALLOC(d_wy, 2 * ycap);
   SG_ALLOC(d_dirv, std::max<long long>(dcap, 1));
-  SG_ALLOC(d_part, 4LL * chunks_cap);
+  pstride = 8LL * chunks_cap;  // a chunk of 1024 cells holds 8 segments, the most of any chunk size
+  SG_ALLOC(d_part, sg::kPartQ * pstride);
   SG_ALLOC(d_stage, stage_cap);
   cell_arrays.clear();
   double** geos[10] = {&geo.aAx, &geo.aBx, &geo.Sx, &geo.aAy, &geo.aBy, &geo.Sy, &geo.ukk, &geo.sdiag, &geo.G,
@@ -492,7 +498,7 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
       SG_ALLOC(*c, cells);
       cell_arrays.push_back({*c, 4});
     }
-    float** ks[8] = {&k32.r, &k32.rh, &k32.t, &k32.x, &k32.p[0], &k32.p[1], &k32.v[0], &k32.v[1]};
+    float** ks[9] = {&k32.rh, &k32.t, &k32.x, &k32.r[0], &k32.r[1], &k32.p[0], &k32.p[1], &k32.v[0], &k32.v[1]};
     for (auto k : ks) {
       SG_ALLOC(*k, cells);
       cell_arrays.push_back({*k, 4});
@@ -503,7 +509,7 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
       SG_ALLOC(*c, cells);
       cell_arrays.push_back({*c, 8});
     }
-    double** ks[8] = {&k64.r, &k64.rh, &k64.t, &k64.x, &k64.p[0], &k64.p[1], &k64.v[0], &k64.v[1]};
+    double** ks[9] = {&k64.rh, &k64.t, &k64.x, &k64.r[0], &k64.r[1], &k64.p[0], &k64.p[1], &k64.v[0], &k64.v[1]};
     for (auto k : ks) {
       SG_ALLOC(*k, cells);
       cell_arrays.push_back({*k, 8});
@@ -523,6 +529,7 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
   cm.wy = d_wy;
   cm.dirv = d_dirv;
   cm.part = d_part;
+  cm.pstride = pstride;
   cm.dyn = d_dyn;
   cm.hist_cap = sg::kOrder;
   cm.precond = opt.precond;
@@ -595,7 +602,7 @@ int sayram_batch_s::place(int b, const sayram_problem& p, long long base, int xe
 int sayram_batch_s::rebuild_lists() {
   h_chunk.clear();
   h_tile.clear();
-  int ninst = 0;
+  int ninst = 0, nseg = 0;
   for (int b = 0; b < cap_slots; ++b) {
     InstDev& I = hinst[b];
     if (!I.enabled) continue;
@@ -603,6 +610,9 @@ int sayram_batch_s::rebuild_lists() {
     I.nchunks = nchunks_of(I.nx, I.ny);
     I.chunk0 = (int)h_chunk.size();
     for (int k = 0; k < I.nchunks; ++k) h_chunk.push_back(b);
+    I.seg0 = nseg;
+    I.nseg = nsegs_of(I);
+    nseg += I.nseg;
     I.tile0 = (int)h_tile.size();
     for (int k = 0; k < I.ntx * I.nty; ++k) h_tile.push_back(b);
   }
@@ -753,8 +763,8 @@ int sayram_batch_s::step_once(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, c
       }
       launch(tail ? "krylov_tail10" : "krylov_rest", [&] {
         launch("bicg1", [&] { k_bicg1<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr); });
-        launch("bicg2", [&] { k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr); });
-        launch("bicg3", [&] { k_bicg3<T, CH><<<gs, kThreads, 0, stream>>>(cm, kr, opt.max_iters); });
+        launch("bicg2", [&] { k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr, opt.max_iters); });
+        launch("bicg3", [&] { k_bicg3<T, CH><<<gs, kThreads, 0, stream>>>(cm, kr); });
       });
       SG_CUDA(cudaGetLastError());
       if (!timing && (it < 4 || (it & 3) == 3)) {
@@ -869,8 +879,8 @@ int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck,
   cudaGraph_t ibody = ip.conditional.phGraph_out[0];
   SG_CUDA(cudaStreamBeginCaptureToGraph(stream, ibody, nullptr, nullptr, 0, mode));
   k_bicg1<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(c2, ck, kr);
-  k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(c2, ck, kr);
-  k_bicg3<T, CH><<<gs, kThreads, 0, stream>>>(c2, kr, opt.max_iters);
+  k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(c2, ck, kr, opt.max_iters);
+  k_bicg3<T, CH><<<gs, kThreads, 0, stream>>>(c2, kr);
   SG_CUDA(cudaStreamEndCapture(stream, &ibody));
   // suffix (the solve-only graph leaves the polish to its caller)
   if (prefix) {
@@ -1546,7 +1556,7 @@ void sayram_batch_destroy(sayram_batch b) { delete b; }
 size_t sayram_instance_bytes(int nx, int ny, int precision) {
   const long long pitch = round_up(nx, 4);
   const long long cells = round_up((long long)(ny + 2) * pitch, 32);
-  const long long per = 19 * 8 + (precision != SAYRAM_FP64 ? 8 * 4 + 8 * 4 : 4 * 8 + 8 * 8) + 8;
+  const long long per = 19 * 8 + (precision != SAYRAM_FP64 ? 8 * 4 + 9 * 4 : 4 * 8 + 9 * 8) + 8;
   return (size_t)(cells * per + 4096);
 }
 
@@ -1846,7 +1856,9 @@ struct ServerLane {
     const double per_cell = (double)sayram_instance_bytes(64, 64, e.opt.precision) /
                             (double)region_cells(64, 64);  // bytes per arena cell (all arrays)
     const double avail = c.hbm_budget_bytes - table_bytes - stage_bytes - 64.0 * 1048576.0;
-    const long long cells = (long long)(avail / (per_cell + 4.0 / 1024 * 2 + 8.0 * 4 / 1024));
+    // work lists and partial sums beside the cells: a chunk index, a tile index and kPartQ * 8 sums of
+    // 8 bytes per 1024 cells
+    const long long cells = (long long)(avail / (per_cell + 4.0 / 1024 * 2 + 8.0 * 8 * sg::kPartQ / 1024));
     if (cells < region_cells(1, 1) + 64) return fail(SAYRAM_ERR_BUDGET, "HBM budget too small for any instance");
     const long long side_tiles = (long long)c.max_slots * (c.max_side / sg::kTX + c.max_side / sg::kTY + 2);
     const int chunks_cap = (int)std::min<long long>(cells / 1024 + c.max_slots + 1, 1LL << 30);
@@ -2053,7 +2065,7 @@ constexpr int kNoAllocChunk = 1024;  // cells per chunk of the streaming kernels
 constexpr int kNoAllocMaxChunks = (int)(kNoAllocCells / kNoAllocChunk) + 2;
 constexpr int kNoAllocMaxTiles = 8192;
 constexpr size_t kNoAllocTableBytes = 1u << 20;
-constexpr size_t kNoAllocBytes = kNoAllocTableBytes + (size_t)kNoAllocCells * 27 * sizeof(double);
+constexpr size_t kNoAllocBytes = kNoAllocTableBytes + (size_t)kNoAllocCells * 28 * sizeof(double);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -2156,6 +2168,8 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   I.hoff = 0;
   I.chunk0 = 0;
   I.nchunks = (int)((round_up((long long)ny * pitch, 4) + kNoAllocChunk - 1) / kNoAllocChunk);
+  I.seg0 = 0;
+  I.nseg = (int)(((long long)ny * pitch + seg_cells(kNoAllocChunk) - 1) / seg_cells(kNoAllocChunk));
   I.tile0 = 0;
   I.ntx = (nx + kTX - 1) / kTX;
   I.nty = (ny + kTY - 1) / kTY;
@@ -2183,7 +2197,8 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   double* d_wx = lay.take<double>(2 * (nx + 1));
   double* d_wy = lay.take<double>(2 * (ny + 1));
   double* d_dirv = lay.take<double>(doff > 0 ? doff : 1);
-  double* d_part = lay.take<double>(4LL * kNoAllocMaxChunks);
+  const long long pstride = 8LL * kNoAllocMaxChunks;
+  double* d_part = lay.take<double>(kPartQ * pstride);
   unsigned char* tables_end = lay.cur;
   if (!d_part || tables_end > base + kNoAllocTableBytes) return fail(SAYRAM_ERR_ARG, "tables exceed the scratch");
   lay.cur = base + kNoAllocTableBytes;
@@ -2191,10 +2206,10 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   Fields fl{};
   Coef<double> co{};
   Kry<double> kr{};
-  double** cellarrs[27] = {&geo.aAx, &geo.aBx, &geo.Sx, &geo.aAy, &geo.aBy, &geo.Sy, &geo.ukk, &geo.sdiag,
+  double** cellarrs[28] = {&geo.aAx, &geo.aBx, &geo.Sx, &geo.aAy, &geo.aBy, &geo.Sy, &geo.ukk, &geo.sdiag,
                            &fl.f, &fl.fh[0], &fl.invD, &fl.R, &fl.colsum, &fl.y64[0], &fl.y64[1],
                            &co.cw, &co.ce, &co.cs, &co.cn,
-                           &kr.r, &kr.rh, &kr.t, &kr.x, &kr.p[0], &kr.p[1], &kr.v[0], &kr.v[1]};
+                           &kr.rh, &kr.t, &kr.x, &kr.r[0], &kr.r[1], &kr.p[0], &kr.p[1], &kr.v[0], &kr.v[1]};
   for (auto a : cellarrs) {
     *a = lay.take<double>(kNoAllocCells);
     if (!*a) return fail(SAYRAM_ERR_ARG, "cell arrays exceed the scratch");
@@ -2249,6 +2264,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   cm.wy = d_wy;
   cm.dirv = d_dirv;
   cm.part = d_part;
+  cm.pstride = pstride;
   // the caller's edges are read directly by the setup kernel
   const long long ncell = (long long)nx * ny;
   const int sblocks = (int)std::min<long long>((ncell + 255) / 256, (long long)nsm * 8);
@@ -2278,8 +2294,8 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
       if (hctl.n_outer == 0) break;
       for (int it = 0; it < o.max_iters; ++it) {
         k_bicg1<double, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, co, kr);
-        k_bicg2<double, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, co, kr);
-        k_bicg3<double, kNoAllocChunk><<<gs, kThreads, 0, stream>>>(cm, kr, o.max_iters);
+        k_bicg2<double, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, co, kr, o.max_iters);
+        k_bicg3<double, kNoAllocChunk><<<gs, kThreads, 0, stream>>>(cm, kr);
         SG_CUDA(cudaGetLastError());
         if (it < 4 || (it & 3) == 3) {
           SG_CUDA(cudaMemcpyAsync(&hctl, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));

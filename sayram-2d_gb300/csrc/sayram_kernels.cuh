@@ -15,14 +15,19 @@
 //   column-diagonally-dominant M-matrix), which keeps FP32 storage well scaled and makes the
 //   positivity polish y' = R + (I - A~) max(y, 0) a 1-norm contraction.
 //
-// Reductions are deterministic: every chunk (1024, 2048 or 4096 cells, chosen per batch) writes
-// its partial sums, and the last block to finish an instance's chunks (counted with one atomic
-// per chunk) adds them in chunk order and updates that instance's Krylov scalars.  No kernel waits on another block.
+// Reductions are deterministic and have one order, whichever kernel runs them: the cells of an
+// instance are cut into segments (Seg<chunk>: 128, 1024 or 4096 cells, by the batch's chunk size),
+// every segment's sum is a fixed tree over its cells, and an instance's total is a fixed tree over
+// its segments (seg_total). In the per-pass kernels the last block to finish an instance's
+// chunks (counted with one atomic per chunk) forms the totals and updates that instance's Krylov
+// scalars; no block waits on another.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
+
+#include "dword.cuh"
 
 namespace sg {
 
@@ -37,7 +42,7 @@ constexpr double kEps = DBL_EPSILON;  // gEPS, source/common.h:38
 enum { XMIN = 0, XMAX = 1, YMIN = 2, YMAX = 3 };
 enum { DIRICHLET = 0, ZEROFLUX = 1 };
 enum { ST_OK = 0, ST_NOT_CONVERGED = 3, ST_NEGATIVE = 4 };
-enum { PH_K1 = 0, PH_K2 = 1, PH_K3 = 2, PH_RESID = 3, PH_POLISH = 4, PH_COUNT = 8 };
+enum { PH_K1 = 0, PH_K2 = 1, PH_RESID = 3, PH_POLISH = 4, PH_COUNT = 8 };
 
 // Per-instance constants.
 struct InstDev {
@@ -46,7 +51,8 @@ struct InstDev {
   long long base;  // index of cell (0,0) in the padded storage
   long long hoff;  // offset of the instance in the packed alpha-major host layout
   int chunk0, nchunks;
-  int tile0, ntx, nty, pad0;
+  int tile0, ntx, nty;
+  int seg0, nseg;  // its reduction segments in the partial-sum arrays
   int xe, ye;     // offsets into the per-vertex-column / per-vertex-row arrays (nx+1 / ny+1)
   int dir[4];     // offsets into the Dirichlet vertex value array (-1 for zero-flux sides)
   double dt;
@@ -59,8 +65,10 @@ struct InstState {
   double rel, mass_drift, min_f, pad_d;
   long long clamped, steps;
   long long cum_iters, cum_refines;  // totals since creation (work accounting)
-  int ycur, pcur, outer_active, inner_active;
-  int restart, fresh, has_x, iters;
+  int ycur, outer_active, inner_active;
+  int restart, has_x;
+  int iters;               // Krylov iterations of this solve finished so far
+  unsigned int fin_seq;    // Ctl::seq of the iteration its last solve converged in (k_bicg3)
   int iters_total, refines, status;
   int nhist;               // earlier states held in the history buffers (extrapolated start)
   int hslot;               // history buffer holding f^(n-1); f^(n-2), ... are in the ones before it
@@ -77,6 +85,7 @@ struct Ctl {
   unsigned int outer_loops;     // residual evaluations run by the device-side loop this step
   unsigned int inner_loops;     // Krylov iterations run by the device-side loop this solve
   int go_outer, go_inner;       // the loop decisions of the cooperative solve (k_solve_coop)
+  unsigned int seq;             // Krylov iterations launched on this batch (one per k_bicg2)
 };
 
 template <typename T>
@@ -117,81 +126,172 @@ __device__ __forceinline__ void count_launch(Ctl* ctl) {
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctl->launches, 1ull);
 }
 
-// Sum of NQ values over the block (result valid in thread 0). T is the warp-level type.
-template <int NQ, typename T>
-__device__ __forceinline__ void block_sum(T (&v)[NQ], double (&out)[NQ]) {
-  __shared__ double sm[NQ][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// ------------------------------------------------------------------------------ reductions
+// Sums are carried in R: IEEE double, or a double word where the terms are FP32 (the FP64 pipe is
+// far too slow for the trees: 2 lanes per SM and cycle).
+__device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ dw radd(dw a, dw b) { return dw_add_same(a, b); }
+__device__ __forceinline__ double rshfl(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ dw rshfl(dw a, int o) {
+  return dw{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
+}
+__device__ __forceinline__ double rdbl(double a) { return a; }
+__device__ __forceinline__ double rdbl(dw a) { return dw_to_double(a); }
+template <typename R>
+__device__ __forceinline__ R rfrom(double a);
+template <>
+__device__ __forceinline__ double rfrom<double>(double a) { return a; }
+template <>
+__device__ __forceinline__ dw rfrom<dw>(double a) { return dw_from_double(a); }
+template <typename R>
+__device__ __forceinline__ R rfrom(float a);
+template <>
+__device__ __forceinline__ double rfrom<double>(float a) { return (double)a; }
+template <>
+__device__ __forceinline__ dw rfrom<dw>(float a) { return dw{a, 0.0f}; }
+template <typename S>
+__device__ __forceinline__ S rconv(double a) { return (S)a; }
+template <typename S>
+__device__ __forceinline__ S rconv(dw a);
+template <>
+__device__ __forceinline__ dw rconv<dw>(dw a) { return a; }
+template <>
+__device__ __forceinline__ double rconv<double>(dw a) { return dw_to_double(a); }
+// the type a pass's sums are carried in: by the precision T of its terms
+template <typename T>
+struct RedOf;
+template <>
+struct RedOf<double> { using R = double; };
+template <>
+struct RedOf<float> { using R = dw; };
+
+template <int NQ>
+__host__ __device__ constexpr int red_pow2() { return NQ <= 1 ? 1 : NQ <= 2 ? 2 : NQ <= 4 ? 4 : 8; }
+
+// Sums of NQ quantities over a warp, the transposed way: at each of the first steps a lane hands
+// half of its quantities to its partner and keeps the other half, so NQ = 5 takes 9 additions
+// instead of 25. Quantity q ends in the lanes with lane / (32 / P) = q (P: NQ rounded up to a power
+// of two); the value returned is this lane's.
+template <int NQ, typename R>
+__device__ __forceinline__ R warp_totals(const R (&in)[NQ]) {
+  constexpr int P = red_pow2<NQ>();
+  R v[P];
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    T x = v[q];
+  for (int q = 0; q < P; ++q) v[q] = q < NQ ? in[q] : rfrom<R>(0.0f);
+  const int lane = threadIdx.x & 31;
+  int off = 16;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) sm[q][warp] = (double)x;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
+  for (int n = P; n > 1; n >>= 1) {
+    const bool up = (lane & off) != 0;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      double x = lane < nw ? sm[q][lane] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      out[q] = x;
+    for (int q = 0; q < n / 2; ++q) {
+      const R send = up ? v[q] : v[q + n / 2];
+      const R keep = up ? v[q + n / 2] : v[q];
+      v[q] = radd(keep, rshfl(send, off));
     }
+    off >>= 1;
+  }
+#pragma unroll
+  for (; off > 0; off >>= 1) v[0] = radd(v[0], rshfl(v[0], off));
+  return v[0];
+}
+// the quantity this lane's warp_totals value belongs to, and whether it is the lane that hands it on
+template <int NQ>
+__device__ __forceinline__ int red_q() { return (threadIdx.x & 31) / (32 / red_pow2<NQ>()); }
+template <int NQ>
+__device__ __forceinline__ bool red_writes() {
+  return (threadIdx.x & (32 / red_pow2<NQ>() - 1)) == 0 && red_q<NQ>() < NQ;
+}
+
+// Cells of a reduction segment, by the chunk size of the batch. 128 cells (one warp's 4-cell
+// groups) where the chunks are smallest, so that a small instance can be spread over many SMs;
+// 4096 where it is largest, so that a thread sums four groups before the warp's tree.
+template <int CH>
+struct Seg { static constexpr int cells = CH; };
+template <>
+struct Seg<1024> { static constexpr int cells = 128; };
+template <>
+struct Seg<2048> { static constexpr int cells = 1024; };
+__host__ __device__ inline int seg_cells(int chunk) { return chunk == 1024 ? 128 : chunk == 2048 ? 1024 : 4096; }
+
+// eight warp sums -> one segment sum, as a fixed tree
+template <typename R>
+__device__ __forceinline__ R tree8(const R* a) {
+  return radd(radd(radd(a[0], a[1]), radd(a[2], a[3])), radd(radd(a[4], a[5]), radd(a[6], a[7])));
+}
+
+// The totals of NQ quantities over nseg segment sums part[q * stride + seg0 ...]: task (q, h) is one
+// warp adding every second run of 32 segments, lane by lane, then its tree; a total is the sum of
+// its two tasks. Valid for every thread after the call (sm holds 2 * NQ entries).
+template <int NQ, typename R>
+__device__ __forceinline__ void seg_total(const R* part, long long stride, int seg0, int nseg, R* sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int k = warp; k < 2 * NQ; k += nw) {
+    const int q = k >> 1, h = k & 1;
+    const double* src = reinterpret_cast<const double*>(part) + (size_t)q * stride + seg0;
+    R a = rfrom<R>(0.0f);
+    for (int s = h * 32 + lane; s < nseg; s += 64) {
+      const double w = __ldcg(src + s);
+      a = radd(a, *reinterpret_cast<const R*>(&w));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = radd(a, rshfl(a, o));
+    if (lane == 0) sm[k] = a;
   }
   __syncthreads();
 }
 
-// Sum over the block of per-warp totals held in lane 0 of each warp (result in thread 0).
-template <int NQ>
-__device__ __forceinline__ void block_sum_lane0(const double (&w)[NQ], double (&out)[NQ]) {
-  __shared__ double sm0[NQ][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) sm0[q][warp] = w[q];
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      double x = lane < nw ? sm0[q][lane] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      out[q] = x;
-    }
-  }
-  __syncthreads();
-}
-
-// Chunk-partial bookkeeping: thread 0 stores this chunk's partials, then the block learns whether
-// it is the last of the instance's chunks for this phase. If so, totals (in chunk order) are
-// returned in tot (valid in thread 0) and the phase counter is reset.
-template <int NQ>
-__device__ __forceinline__ bool chunk_finish(InstState& st, int phase, int chunk0, int nchunks,
-                                             int chunk, double* part, const double (&mine)[NQ],
-                                             double (&tot)[NQ]) {
+// Segment-partial bookkeeping of the per-pass kernels: after the block has stored the segment sums
+// of one chunk, it learns whether it is the last of the instance's chunks for this phase; if so
+// the totals are returned in tot (valid in thread 0) and the phase counter is reset.
+template <int NQ, typename R>
+__device__ __forceinline__ bool chunk_finish(InstState& st, int phase, const InstDev& I, const R* part,
+                                             long long stride, double (&tot)[NQ]) {
   __shared__ int s_last;
+  __shared__ double s_tot[2 * NQ];
+  __syncthreads();
   if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) part[(size_t)chunk * 4 + q] = mine[q];
     __threadfence();
     const unsigned prev = atomicAdd(&st.cnt[phase], 1u);
-    s_last = (prev == (unsigned)(nchunks - 1));
+    s_last = (prev == (unsigned)(I.nchunks - 1));
   }
   __syncthreads();
   if (!s_last) return false;
   __threadfence();
-  double acc[NQ];
+  R* sm = reinterpret_cast<R*>(s_tot);
+  seg_total<NQ, R>(part, stride, I.seg0, I.nseg, sm);
+  if (threadIdx.x == 0) {
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
-  for (int k = threadIdx.x; k < nchunks; k += blockDim.x)
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) acc[q] += __ldcg(&part[(size_t)(chunk0 + k) * 4 + q]);
-  block_sum<NQ, double>(acc, tot);
-  if (threadIdx.x == 0) st.cnt[phase] = 0;
+    for (int q = 0; q < NQ; ++q) tot[q] = rdbl(radd(sm[2 * q], sm[2 * q + 1]));
+    st.cnt[phase] = 0;
+  }
   return true;
 }
+
+// One block's sums of one chunk. add() takes the lane's terms of one 1024-cell row of the chunk and
+// closes the segments that end with it; store() writes the chunk's segment sums to the partials.
+template <int CH, int NQ, typename R>
+struct ChunkSums {
+  static constexpr int SEG = Seg<CH>::cells;
+  static constexpr int kParts = SEG == 4096 ? 8 : CH / 128;  // warp sums of a chunk
+  R (*sm)[kParts];  // [NQ][kParts] in shared memory
+  __device__ __forceinline__ void put(int row, const R (&v)[NQ]) {
+    const R t = warp_totals<NQ, R>(v);
+    if (red_writes<NQ>()) sm[red_q<NQ>()][(SEG == 4096 ? 0 : row * 8) + (threadIdx.x >> 5)] = t;
+  }
+  // seg: the chunk's first segment in the partials; nseg: how many of them the instance has; S: what
+  // a segment's sum is stored as (R, or double)
+  template <typename S = R>
+  __device__ __forceinline__ void store(S* part, long long stride, int seg, int nseg) {
+    __syncthreads();
+    constexpr int kSegs = CH / SEG;
+    for (int k = threadIdx.x; k < NQ * kSegs; k += blockDim.x) {
+      const int q = k / kSegs, s = k % kSegs;
+      if (s >= nseg) continue;
+      const R v = SEG == 128 ? sm[q][s] : tree8(&sm[q][s * 8]);
+      part[(size_t)q * stride + seg + s] = rconv<S>(v);
+    }
+  }
+};
 
 }  // namespace sg

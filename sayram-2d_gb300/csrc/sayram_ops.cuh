@@ -7,6 +7,7 @@
 //   k_resid      outer residual r = R - A~ y (adds the last Krylov correction first)
 //   k_bicg1/2/3  one BiCGSTAB iteration in T precision (FP64 or FP32) with fused SpMV + dots
 //   k_polish     positivity polish y' = R + (I - A~) y+, f = y'/D, min / clamp / mass checks
+//                (these four in sayram_solve.cuh)
 //   k_field_*    alpha-major FP64 <-> padded system order transposes for the host-buffer step
 //
 // The assembly, residual, polish and state are written once over an arithmetic policy A:
@@ -42,7 +43,8 @@ struct Common {
   const double* wx;    // per vertex column: (wL, wR) bilinear weights (Solver.cc:333-336)
   const double* wy;    // per vertex row: (wB, wT)
   const double* dirv;  // Dirichlet vertex values
-  double* part;        // 4 doubles per chunk
+  double* part;        // kPartQ segment sums of 8 bytes per reduction segment, quantity by quantity
+  long long pstride;   // segments per quantity
   // when set, [nchunks, ntiles, ninst] are read from device memory (lists that change between
   // steps, as in the server) instead of the by-value counts above
   const int* dyn;
@@ -115,11 +117,14 @@ struct Fields {
   double* y64[2];  // scaled solution y = D f (ping-pong)
 };
 
+// Krylov vectors. The residual a solve starts from is left in rh (the shadow residual); r and p
+// of the first iteration are that same array, so it writes neither.
 template <typename T>
 struct Kry {
-  T *r, *rh, *t, *x;
-  T *p[2], *v[2];
+  T *rh, *t, *x;
+  T *r[2], *p[2], *v[2];  // iteration i uses [i & 1]
 };
+constexpr int kPartQ = 5;  // most sums any pass forms at once
 
 // ------------------------------------------------------------------------------ arithmetic
 struct F64A {
@@ -131,19 +136,21 @@ struct F64A {
   __device__ static void st(double* p, Ix i, V v) { p[i] = v; }
   __device__ static Q4<V> ld4(const double* p) { return sg::ld4(p); }
   __device__ static void st4(double* p, const Q4<V>& q) { sg::st4(p, q); }
-  __device__ static V add(V a, V b) { return a + b; }
-  __device__ static V sub(V a, V b) { return a - b; }
-  __device__ static V mul(V a, V b) { return a * b; }
-  __device__ static V fma(V a, V b, V c) { return a * b + c; }
+  // every operation is fused or rounded explicitly, so that all kernels sharing a formula give the
+  // same bits whatever the compiler would contract
+  __device__ static V add(V a, V b) { return __dadd_rn(a, b); }
+  __device__ static V sub(V a, V b) { return __dadd_rn(a, -b); }
+  __device__ static V mul(V a, V b) { return __dmul_rn(a, b); }
+  __device__ static V fma(V a, V b, V c) { return __fma_rn(a, b, c); }
   // a*x + b*y and a*x - b*y (the same expression trees as fma(a, x, mul(b, y)) and
   // sub(mul(a, x), mul(b, y)))
-  __device__ static V dot2(V a, V x, V b, V y) { return a * x + b * y; }
-  __device__ static V fma0(V a, V b) { return a * b; }  // fma(a, b, 0)
-  __device__ static V dot2s(V a, V x, V b, V y) { return a * x - b * y; }
+  __device__ static V dot2(V a, V x, V b, V y) { return __fma_rn(a, x, __dmul_rn(b, y)); }
+  __device__ static V fma0(V a, V b) { return __dmul_rn(a, b); }  // fma(a, b, 0)
+  __device__ static V dot2s(V a, V x, V b, V y) { return __fma_rn(a, x, -__dmul_rn(b, y)); }
   // sums whose terms all have the same sign (cheaper in double-word form)
-  __device__ static V addp(V a, V b) { return a + b; }
-  __device__ static V fmap(V a, V b, V c) { return a * b + c; }
-  __device__ static V addf(V a, float b) { return a + (double)b; }
+  __device__ static V addp(V a, V b) { return __dadd_rn(a, b); }
+  __device__ static V fmap(V a, V b, V c) { return __fma_rn(a, b, c); }
+  __device__ static V addf(V a, float b) { return __dadd_rn(a, (double)b); }
   __device__ static V rcp(V a) { return 1.0 / a; }
   __device__ static V div(V a, V b) { return a / b; }
   __device__ static V abs(V a) { return fabs(a); }
@@ -154,21 +161,19 @@ struct F64A {
   // r (c0 + 4 (d1 + d3) - 6 d2 - d4) with d_m = c_(m-1) - c_m, c0 = f. Exact for pure loss;
   // r = 1 gives the plain polynomial. The next solve starts from y0 = D g.
   __device__ static V extrap(V f, V h1, V h2, V h3, V h4, int n, V r) {
-    const double c1 = h1 * r;
-    const double d1 = f - c1;
-    double c = d1;
-    if (n >= 2) {
-      const double r2 = r * r, c2 = h2 * r2;
-      const double d2 = c1 - c2;
-      if (n == 2) {
-        c = 2.0 * d1 - d2;
-      } else {
-        const double r3 = r2 * r, c3 = h3 * r3;
-        const double d3 = c2 - c3;
-        c = n == 3 ? 3.0 * (d1 - d2) + d3 : 4.0 * (d1 + d3) - 6.0 * d2 - (c3 - h4 * (r3 * r));
-      }
-    }
-    return r * (f + c);
+    // the closed forms 2 c0 - c1, 3 (c0 - c1) + c2, 4 (c0 + c2) - 6 c1 - c3 and
+    // 5 (c0 - c3) - 10 (c1 - c2) + c4, by Horner in r: at most 9 FP64 operations
+    double a;
+    if (n >= 4)
+      a = __fma_rn(r, __fma_rn(r, __fma_rn(r, __fma_rn(r, h4, __dmul_rn(-5.0, h3)), __dmul_rn(10.0, h2)),
+                               __dmul_rn(-10.0, h1)), __dmul_rn(5.0, f));
+    else if (n == 3)
+      a = __fma_rn(r, __fma_rn(r, __fma_rn(-r, h3, __dmul_rn(4.0, h2)), __dmul_rn(-6.0, h1)), __dmul_rn(4.0, f));
+    else if (n == 2)
+      a = __fma_rn(r, __fma_rn(r, h2, __dmul_rn(-3.0, h1)), __dmul_rn(3.0, f));
+    else
+      a = __fma_rn(-r, h1, __dadd_rn(f, f));
+    return __dmul_rn(r, a);
   }
   __device__ static V rsub1(V a) { return 1.0 - a; }
   __device__ static V max0(V a) { return fmax(a, 0.0); }
@@ -189,18 +194,16 @@ struct F64A {
   __device__ static V hilo(float hi, float lo) { return (double)hi + (double)lo; }
   // r * s for a power-of-two s, in the Krylov precision T
   template <typename T>
-  __device__ static T scaled(V a, float s) { return (T)(a * (double)s); }
+  __device__ static T scaled(V a, float s) { return (T)__dmul_rn(a, (double)s); }
   // y + x*s for the FP32/FP64 Krylov correction x in scaled units
   template <typename T>
-  __device__ static V add_scaled(V y, T x, float s) { return y + (double)x * (double)s; }
+  __device__ static V add_scaled(V y, T x, float s) { return __fma_rn((double)x, (double)s, y); }
   using Acc = double;  // per-thread accumulator of scaled squares
-  __device__ static Acc sq_scaled(V a, float s) { const double t = a * (double)s; return t * t; }
-  __device__ static double warp_total(Acc a) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    return a;
+  __device__ static Acc sq_scaled(V a, float s, Acc q) {
+    const double t = __dmul_rn(a, (double)s);
+    return __fma_rn(t, t, q);
   }
-  __device__ static double warp_total_v(V a) { return warp_total(a); }
+  using R = double;  // what the residual's sums are carried in
 };
 
 struct DWA {
@@ -281,24 +284,15 @@ struct DWA {
   }
   __device__ static V hilo(float hi, float lo) { return dw{hi, lo}; }
   template <typename T>
-  __device__ static T scaled(V a, float s) { return (T)(a.hi * s); }
+  __device__ static T scaled(V a, float s) { return (T)__fmul_rn(a.hi, s); }
   template <typename T>
-  __device__ static V add_scaled(V y, T x, float s) { return dw_add_f(y, (float)x * s); }
+  __device__ static V add_scaled(V y, T x, float s) { return dw_add_f(y, __fmul_rn((float)x, s)); }
   using Acc = float;
-  __device__ static Acc sq_scaled(V a, float s) { const float t = a.hi * s; return t * t; }
-  __device__ static double warp_total(Acc a) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    return (double)a;
+  __device__ static Acc sq_scaled(V a, float s, Acc q) {
+    const float t = __fmul_rn(a.hi, s);
+    return __fmaf_rn(t, t, q);
   }
-  __device__ static double warp_total_v(V a) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const dw b{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-      a = dw_add(a, b);
-    }
-    return dw_to_double(a);
-  }
+  using R = dw;
 };
 
 // Power-of-two scale of an instance's refinement system: 2^-e with max|R| = m * 2^e, m in
@@ -556,9 +550,9 @@ __global__ void k_begin(Common cm) {
     s.outer_active = on ? 1 : 0;
     s.inner_active = 0;
     s.restart = 0;
-    s.fresh = 0;
     s.has_x = 0;
     s.iters = 0;
+    s.fin_seq = 0u;
     s.iters_total = 0;
     s.refines = 0;
     s.clamped = 0;
@@ -570,6 +564,7 @@ __global__ void k_begin(Common cm) {
     cm.ctl->inner_loops = 0u;
     cm.ctl->kdone[0] = 0u;
     cm.ctl->kdone[1] = 0u;
+    cm.ctl->seq = 0u;
   }
 }
 
@@ -855,675 +850,6 @@ __global__ void __launch_bounds__(kAsmThreads, A::kAsmBlocks) k_assemble(Common 
   }
 }
 
-// ------------------------------------------------------------------------------ streaming helpers
-// Resident blocks per SM the Krylov kernels are compiled for: in FP32, 6 (registers capped at
-// 40; their shared memory allows 6, and the extra blocks in flight raised their bandwidth by
-// 8-14 %); in FP64, 4 (a cap of 40 registers spills).
-template <typename T>
-constexpr int krylov_blocks() { return sizeof(T) == 4 ? 6 : 4; }
-
-// Locates 4-cell group g (0 .. CH/(4*kThreads) - 1) of this thread in chunk c (CH cells) of
-// instance I.
-struct Slot {
-  long long K;
-  bool valid;
-};
-template <int CH>
-__device__ __forceinline__ long long chunk_start(int c, const InstDev& I) {
-  return I.base + (long long)(c - I.chunk0) * CH;
-}
-__device__ __forceinline__ long long inst_end(const InstDev& I) { return I.base + (long long)I.ny * I.pitch; }
-template <int CH>
-__device__ __forceinline__ Slot slot_of(int c, const InstDev& I, int g) {
-  Slot s;
-  s.K = chunk_start<CH>(c, I) + 4 * (threadIdx.x + g * kThreads);
-  s.valid = s.K < inst_end(I);
-  return s;
-}
-
-// Runs body(c) for every chunk c of this block (c = blockIdx.x + k*gridDim.x) whose instance
-// passes want(instance). The instance checks run in parallel, one chunk per thread, and the
-// passing chunks are compacted in shared memory: a launch in which most instances have finished
-// costs one round of checks per block instead of two dependent loads per chunk. Chunks are
-// independent, so the order in which a block takes them does not change any result.
-// Chunks [c0, c1) of the list only (c1 < 0: to the end).
-template <typename W, typename Body>
-__device__ __forceinline__ void for_active_chunks(const Common& cm, W&& want, Body&& body, int c0 = 0, int c1 = -1) {
-  __shared__ int s_list[kThreads];
-  __shared__ int s_cnt;
-  const int nc = (c1 < 0 ? n_chunks(cm) : c1) - c0;
-  const int per = (int)blockIdx.x < nc ? (nc - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  for (int r0 = 0; r0 < per; r0 += kThreads) {
-    if (threadIdx.x == 0) s_cnt = 0;
-    __syncthreads();
-    const int k = r0 + (int)threadIdx.x;
-    if (k < per) {
-      const int c = c0 + (int)blockIdx.x + k * (int)gridDim.x;
-      if (want(cm.chunk_inst[c])) s_list[atomicAdd(&s_cnt, 1)] = c;
-    }
-    __syncthreads();
-    const int m = s_cnt;
-    for (int q = 0; q < m; ++q) body(s_list[q]);
-    __syncthreads();
-  }
-}
-
-// Fills smem[0 .. n) with a 4-aligned stretch [e0, e0 + n) of a vector computed cell-wise by
-// f(k) -> Q4<T> (k a multiple of 4): the chunk plus one row above and below, so that the stencil
-// of every cell in the chunk reads shared memory only.
-template <typename T, typename F>
-__device__ __forceinline__ void stage_rows(T* sm, long long e0, long long n, F&& f) {
-#pragma unroll 2
-  for (long long q = 4LL * threadIdx.x; q < n; q += 4LL * blockDim.x) {
-    const Q4<T> v = f(e0 + q);
-    *reinterpret_cast<Q4<T>*>(sm + q) = v;
-  }
-}
-
-// A~ x over a 4-cell group from a staged vector (sm holds x at global index e0 + offset)
-template <typename T>
-__device__ __forceinline__ Q4<T> stencil_sm(const T* sm, long long o, int P, const Q4<T>& cw,
-                                            const Q4<T>& ce, const Q4<T>& cs, const Q4<T>& cn) {
-  const Q4<T> c = *reinterpret_cast<const Q4<T>*>(sm + o);
-  const Q4<T> d = *reinterpret_cast<const Q4<T>*>(sm + o - P);
-  const Q4<T> u = *reinterpret_cast<const Q4<T>*>(sm + o + P);
-  const T w0 = sm[o - 1], e3 = sm[o + 4];
-  Q4<T> r;
-  const T wv[4] = {w0, c.a[0], c.a[1], c.a[2]};
-  const T ev[4] = {c.a[1], c.a[2], c.a[3], e3};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) r.a[k] = c.a[k] - (cw.a[k] * wv[k] + ce.a[k] * ev[k] + cs.a[k] * d.a[k] + cn.a[k] * u.a[k]);
-  return r;
-}
-
-// ------------------------------------------------------------------------------ preconditioner
-// Alpha-line block preconditioner. Every 4-cell group of the padded layout lies inside one row
-// (rows start at multiples of 4), and B is the tridiagonal of the group's own west/east couplings
-// -- unit diagonal, -cw below, -ce above -- with the couplings to the neighbouring groups dropped:
-// block Jacobi with 4-cell alpha-line blocks, the direction in which the scaled systems are
-// stiffest (Dxx/dalpha^2 against Dyy/dlogE^2). line4 returns B^-1 q by Thomas elimination
-// without pivoting (B is a column-diagonally-dominant M-matrix: every column of the outflow
-// fractions sums to < 1, so each pivot stays in (0, 1]). The factors are formed in FP32 with
-// separately rounded intrinsics whatever the vector precision, so every kernel that applies
-// B^-1 applies the same linear map; padding cells (q = cw = ce = 0) stay 0.
-__device__ __forceinline__ float fmaT(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mulT(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mulT(double a, double b) { return __dmul_rn(a, b); }
-
-template <typename T, typename CT>
-__device__ __forceinline__ Q4<T> line4(const Q4<T>& q, const Q4<CT>& cw, const Q4<CT>& ce) {
-  const float w1 = (float)cw.a[1], w2 = (float)cw.a[2], w3 = (float)cw.a[3];
-  const float c0 = (float)ce.a[0];
-  const float i1 = __frcp_rn(__fmaf_rn(-w1, c0, 1.0f));
-  const float c1 = __fmul_rn((float)ce.a[1], i1);
-  const float i2 = __frcp_rn(__fmaf_rn(-w2, c1, 1.0f));
-  const float c2 = __fmul_rn((float)ce.a[2], i2);
-  const float i3 = __frcp_rn(__fmaf_rn(-w3, c2, 1.0f));
-  // forward: d_j = (q_j + w_j d_(j-1)) / pivot_j; backward: z_j = d_j + c_j z_(j+1)
-  const T d0 = q.a[0];
-  const T d1 = mulT(fmaT((T)w1, d0, q.a[1]), (T)i1);
-  const T d2 = mulT(fmaT((T)w2, d1, q.a[2]), (T)i2);
-  const T d3 = mulT(fmaT((T)w3, d2, q.a[3]), (T)i3);
-  Q4<T> z;
-  z.a[3] = d3;
-  z.a[2] = fmaT((T)c2, d3, d2);
-  z.a[1] = fmaT((T)c1, z.a[2], d1);
-  z.a[0] = fmaT((T)c0, z.a[1], d0);
-  return z;
-}
-
-// Coefficients of a row in the wide arithmetic: from the FP64 arrays or the (hi, lo) split
-template <typename C, typename A>
-struct CoefW;
-template <typename A>
-struct CoefW<double, A> {
-  __device__ static Q4<typename A::V> row(const Coef<double>& c, int which, long long K) {
-    const double* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
-    const Q4<double> q = ld4(a + K);
-    Q4<typename A::V> o;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) o.a[k] = A::from_d(q.a[k]);
-    return o;
-  }
-};
-template <typename A>
-struct CoefW<float, A> {
-  __device__ static Q4<typename A::V> row(const Coef<float>& c, int which, long long K) {
-    const float* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
-    const float* l = which == 0 ? c.lw : which == 1 ? c.le : which == 2 ? c.ls : c.ln;
-    const Q4<float> h = ld4(a + K), lo = ld4(l + K);
-    Q4<typename A::V> o;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) o.a[k] = A::hilo(h.a[k], lo.a[k]);
-    return o;
-  }
-};
-
-// y = A~ x for a 4-cell group given the centre values, the west value of cell 0, the east value
-// of cell 3 and the rows below/above.
-template <typename T, typename CT>
-__device__ __forceinline__ Q4<T> stencil(const Q4<T>& c, T w0, T e3, const Q4<T>& dn, const Q4<T>& up,
-                                         const Q4<CT>& cw, const Q4<CT>& ce, const Q4<CT>& cs,
-                                         const Q4<CT>& cn) {
-  Q4<T> o;
-  const T wv[4] = {w0, c.a[0], c.a[1], c.a[2]};
-  const T ev[4] = {c.a[1], c.a[2], c.a[3], e3};
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    o.a[k] = c.a[k] - ((T)cw.a[k] * wv[k] + (T)ce.a[k] * ev[k] + (T)cs.a[k] * dn.a[k] + (T)cn.a[k] * up.a[k]);
-  return o;
-}
-
-// The same stencil in the wide arithmetic: A~ y = y - sum_nbr c * y_nbr
-template <typename A>
-__device__ __forceinline__ Q4<typename A::V> stencilW(const Q4<typename A::V>& c, typename A::V w0,
-                                                      typename A::V e3, const Q4<typename A::V>& dn,
-                                                      const Q4<typename A::V>& up,
-                                                      const Q4<typename A::V>& cw, const Q4<typename A::V>& ce,
-                                                      const Q4<typename A::V>& cs, const Q4<typename A::V>& cn) {
-  using V = typename A::V;
-  Q4<V> o;
-  const V wv[4] = {w0, c.a[0], c.a[1], c.a[2]};
-  const V ev[4] = {c.a[1], c.a[2], c.a[3], e3};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const V s = A::fma(cn.a[k], up.a[k], A::fma(cs.a[k], dn.a[k], A::fma(ce.a[k], ev[k], A::mul(cw.a[k], wv[k]))));
-    o.a[k] = A::sub(c.a[k], s);
-  }
-  return o;
-}
-
-// ------------------------------------------------------------------------------ outer residual
-// r = R - A~ (y + x) in the wide arithmetic; writes y + x to the other y buffer and the Krylov's
-// right-hand side B^-1 r (T precision, scaled). Partials: ||r||^2, ||R||^2, ||B^-1 r||^2.
-template <typename T, typename C, typename A, int CH>
-__device__ __forceinline__ void resid_body(Common cm, Fields fl, Coef<C> co, Kry<T> kr, double tol, double inner_tol,
-                                           int max_refine) {
-  using V = typename A::V;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* sm = reinterpret_cast<V*>(smraw);
-  for_active_chunks(cm, [&](int b_) { return cm.st[b_].outer_active != 0; }, [&](int c) {
-    const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
-    const double* yin = sel2(fl.y64, st.ycur);
-    double* yout = sel2(fl.y64, st.ycur ^ 1);
-    const bool hx = st.has_x != 0;
-    const float sc = rhs_scale(st.rmax_bits);  // r is handed over as r * sc
-    const float isc = 1.0f / sc;                // exact: sc is a power of two
-    const int P = I.pitch;
-    const long long c0 = chunk_start<CH>(c, I);
-    const long long c1 = min(c0 + (long long)CH, inst_end(I));
-    const long long e0 = c0 - P;
-    // y + x (the last Krylov correction, in scaled units) over the chunk and one row each side
-    stage_rows<V>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
-      Q4<V> y = A::ld4(yin + k);
-      if (hx) {
-        const Q4<T> x = ld4(kr.x + k);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) y.a[m] = A::template add_scaled<T>(y.a[m], x.a[m], isc);
-      }
-      return y;
-    });
-    __syncthreads();
-    typename A::Acc q0 = 0, q1 = 0;
-    T q2 = (T)0;
-#pragma unroll 1
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
-      if (K < c1) {
-        const long long o = K - e0;
-        const Q4<V> cw = CoefW<C, A>::row(co, 0, K), ce = CoefW<C, A>::row(co, 1, K);
-        const Q4<V> cs = CoefW<C, A>::row(co, 2, K), cn = CoefW<C, A>::row(co, 3, K);
-        const Q4<V> R = A::ld4(fl.R + K);
-        Q4<T> r;
-        Q4<V> yc;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const V yv = sm[o + m];
-          const V s1 = A::fma(cn.a[m], sm[o + m + P], A::fma(cs.a[m], sm[o + m - P],
-                              A::fma(ce.a[m], sm[o + m + 1], A::mul(cw.a[m], sm[o + m - 1]))));
-          const V rv = A::sub(R.a[m], A::sub(yv, s1));
-          yc.a[m] = yv;
-          r.a[m] = A::template scaled<T>(rv, sc);
-          q0 += A::sq_scaled(rv, sc);
-          q1 += A::sq_scaled(R.a[m], sc);
-        }
-        if (cm.precond) {  // the Krylov matrix's couplings (the hi parts in the FP32 modes)
-          r = line4<T, C>(r, ld4(co.cw + K), ld4(co.ce + K));
-#pragma unroll
-          for (int m = 0; m < 4; ++m) q2 += r.a[m] * r.a[m];
-        }
-        A::st4(yout + K, yc);
-        st4(kr.r + K, r);
-      }
-    }
-    double w3 = (double)q2;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w3 += __shfl_xor_sync(0xffffffffu, w3, o);
-    const double w[3] = {A::warp_total(q0), A::warp_total(q1), w3};
-    double tot[3], mine[3];
-    block_sum_lane0<3>(w, mine);
-    if (chunk_finish<3>(st, PH_RESID, I.chunk0, I.nchunks, c, cm.part, mine, tot) && threadIdx.x == 0) {
-      // tot holds ||r*sc||^2, ||R*sc||^2 and ||B^-1 r*sc||^2
-      st.ycur ^= 1;
-      st.has_x = 0;
-      if (st.refines == 0) st.bb = tot[1];
-      st.refines += 1;
-      st.cum_refines += 1;
-      st.rr64 = tot[0];
-      st.rel = st.bb > 0 ? sqrt(tot[0] / st.bb) : 0.0;
-      if (!(st.rel > tol)) {
-        st.outer_active = 0;
-        st.status = ST_OK;
-        atomicSub(&cm.ctl->n_outer, 1);
-      } else if (st.refines >= max_refine) {
-        st.outer_active = 0;
-        st.status = ST_NOT_CONVERGED;
-        atomicSub(&cm.ctl->n_outer, 1);
-      } else {
-        st.inner_active = 1;
-        st.fresh = 1;
-        st.restart = 1;
-        st.iters = 0;
-        // the Krylov's residual is B^-1 r: its target is the relative reduction asked, or the
-        // final tolerance carried into preconditioned units by this pass's norm ratio
-        const double rrk = cm.precond ? tot[2] : tot[0];
-        st.rr = rrk;
-        const double a = inner_tol * inner_tol * rrk;
-        const double bnd = 0.0625 * tol * tol * st.bb * (cm.precond && tot[0] > 0.0 ? rrk / tot[0] : 1.0);
-        st.rr_target = a > bnd ? a : bnd;
-        atomicAdd(&cm.ctl->n_inner, 1);
-      }
-    }
-  });
-}
-template <typename T, typename C, typename A, int CH>
-__global__ void __launch_bounds__(kThreads, 4) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
-                                                        double tol, double inner_tol, int max_refine) {
-  count_launch(cm.ctl);
-  resid_body<T, C, A, CH>(cm, fl, co, kr, tol, inner_tol, max_refine);
-  loop_epilogue(cm, 0);
-}
-
-// ------------------------------------------------------------------------------ BiCGSTAB
-// Left-preconditioned BiCGSTAB on B^-1 A~ x = B^-1 r (B = I without the preconditioner; the
-// residual r the kernels carry is the preconditioned one, and x is the correction itself).
-// k1: p = r + beta (p_old - omega v_old)  (p = r on a restart, which also sets r^ = r);
-//     v = B^-1 A~ p;  partial (r^, v). p is computed once per cell into shared memory (chunk plus
-//     one row above and below) and the stencil reads it there.
-template <typename T, int CH>
-__device__ __forceinline__ void bicg1_body(Common cm, Coef<T> co, Kry<T> kr) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
-    const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
-    const int pc = st.pcur;
-    const bool rs = st.restart != 0;
-    const T beta = (T)st.beta, omega = (T)st.omega;
-    const T* __restrict__ r = kr.r;
-    const T* __restrict__ po = sel2(kr.p, pc);
-    const T* __restrict__ vo = sel2(kr.v, pc);
-    T* __restrict__ pn = sel2(kr.p, pc ^ 1);
-    T* __restrict__ vn = sel2(kr.v, pc ^ 1);
-    const int P = I.pitch;
-    const long long c0 = chunk_start<CH>(c, I);
-    const long long c1 = min(c0 + (long long)CH, inst_end(I));
-    const long long e0 = c0 - P;
-    stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
-      Q4<T> x = ld4(r + k);
-      if (!rs) {
-        const Q4<T> a = ld4(po + k), v = ld4(vo + k);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) x.a[m] = x.a[m] + beta * (a.a[m] - omega * v.a[m]);
-      }
-      return x;
-    });
-    __syncthreads();
-    T q[1] = {(T)0};
-#pragma unroll 2
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
-      if (K < c1) {
-        const long long o = K - e0;
-        const Q4<T> pcv = *reinterpret_cast<const Q4<T>*>(sm + o);
-        const Q4<T> cwq = ld4(co.cw + K), ceq = ld4(co.ce + K);
-        Q4<T> v = stencil_sm<T>(sm, o, P, cwq, ceq, ld4(co.cs + K), ld4(co.cn + K));
-        if (cm.precond) v = line4<T, T>(v, cwq, ceq);  // v = B^-1 A~ p
-        st4(pn + K, pcv);
-        st4(vn + K, v);
-        Q4<T> rh;
-        if (rs) {
-          rh = ld4(r + K);
-          st4(kr.rh + K, rh);
-        } else {
-          rh = ld4(kr.rh + K);
-        }
-#pragma unroll
-        for (int m = 0; m < 4; ++m) q[0] += rh.a[m] * v.a[m];
-      }
-    }
-    double tot[1], mine[1];
-    block_sum<1, T>(q, mine);
-    if (chunk_finish<1>(st, PH_K1, I.chunk0, I.nchunks, c, cm.part, mine, tot) && threadIdx.x == 0) {
-      if (st.restart) {
-        st.rho = st.rr;  // (r^, r) with r^ = r
-        st.restart = 0;
-      }
-      st.pcur ^= 1;
-      const double den = tot[0];
-      if (den != 0.0 && isfinite(den) && st.rho != 0.0) {
-        st.alpha = st.rho / den;
-      } else {
-        st.alpha = 0.0;  // breakdown: this iteration degenerates to a minimal-residual step
-        st.restart = 1;
-      }
-    }
-  });
-}
-template <typename T, int CH>
-__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg1(Common cm, Coef<T> co, Kry<T> kr) {
-  count_launch(cm.ctl);
-  bicg1_body<T, CH>(cm, co, kr);
-}
-
-// k2: s = r - alpha v;  t = B^-1 A~ s;  partials (t, s), (t, t). s is staged like p in k1.
-template <typename T, int CH>
-__device__ __forceinline__ void bicg2_body(Common cm, Coef<T> co, Kry<T> kr) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
-    const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
-    const T alpha = (T)st.alpha;
-    const T* __restrict__ r = kr.r;
-    const T* __restrict__ vv = sel2(kr.v, st.pcur);
-    const int P = I.pitch;
-    const long long c0 = chunk_start<CH>(c, I);
-    const long long c1 = min(c0 + (long long)CH, inst_end(I));
-    const long long e0 = c0 - P;
-    stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
-      Q4<T> x = ld4(r + k);
-      const Q4<T> v = ld4(vv + k);
-#pragma unroll
-      for (int m = 0; m < 4; ++m) x.a[m] -= alpha * v.a[m];
-      return x;
-    });
-    __syncthreads();
-    T q[2] = {(T)0, (T)0};
-#pragma unroll 2
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
-      if (K < c1) {
-        const long long o = K - e0;
-        const Q4<T> sc = *reinterpret_cast<const Q4<T>*>(sm + o);
-        const Q4<T> cwq = ld4(co.cw + K), ceq = ld4(co.ce + K);
-        Q4<T> t = stencil_sm<T>(sm, o, P, cwq, ceq, ld4(co.cs + K), ld4(co.cn + K));
-        if (cm.precond) t = line4<T, T>(t, cwq, ceq);  // t = B^-1 A~ s
-        st4(kr.t + K, t);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          q[0] += t.a[m] * sc.a[m];
-          q[1] += t.a[m] * t.a[m];
-        }
-      }
-    }
-    double tot[2], mine[2];
-    block_sum<2, T>(q, mine);
-    if (chunk_finish<2>(st, PH_K2, I.chunk0, I.nchunks, c, cm.part, mine, tot) && threadIdx.x == 0) {
-      if (tot[1] > 0.0 && isfinite(tot[0])) {
-        st.omega = tot[0] / tot[1];
-      } else {
-        st.omega = 0.0;
-      }
-      if (st.omega == 0.0) st.restart = 1;
-    }
-  });
-}
-template <typename T, int CH>
-__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg2(Common cm, Coef<T> co, Kry<T> kr) {
-  count_launch(cm.ctl);
-  bicg2_body<T, CH>(cm, co, kr);
-}
-
-// k3: x += alpha p + omega s (x starts at 0 on the first iteration of a solve);
-//     r = s - omega t;  partials (r^, r), (r, r); convergence test.
-template <typename T, int CH>
-__device__ __forceinline__ void bicg3_body(Common cm, Kry<T> kr, int max_iters) {
-  for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
-    const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
-    const T alpha = (T)st.alpha, omega = (T)st.omega;
-    const bool fresh = st.fresh != 0;
-    const T* pp = sel2(kr.p, st.pcur);
-    const T* vv = sel2(kr.v, st.pcur);
-    T q[2] = {(T)0, (T)0};
-#pragma unroll 2
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-    const Slot s = slot_of<CH>(c, I, g);
-    if (s.valid) {
-      const long long K = s.K;
-      const Q4<T> r = ld4(kr.r + K), v = ld4(vv + K), p = ld4(pp + K), t = ld4(kr.t + K);
-      const Q4<T> rh = ld4(kr.rh + K);
-      Q4<T> x = fresh ? Q4<T>{{(T)0, (T)0, (T)0, (T)0}} : ld4(kr.x + K);
-      Q4<T> rn;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const T sv = r.a[m] - alpha * v.a[m];
-        x.a[m] += alpha * p.a[m] + omega * sv;
-        rn.a[m] = sv - omega * t.a[m];
-        q[0] += rh.a[m] * rn.a[m];
-        q[1] += rn.a[m] * rn.a[m];
-      }
-      st4(kr.x + K, x);
-      st4(kr.r + K, rn);
-    }
-    }
-    double tot[2], mine[2];
-    block_sum<2, T>(q, mine);
-    if (chunk_finish<2>(st, PH_K3, I.chunk0, I.nchunks, c, cm.part, mine, tot) && threadIdx.x == 0) {
-      st.fresh = 0;
-      st.has_x = 1;
-      st.iters += 1;
-      st.iters_total += 1;
-      st.cum_iters += 1;
-      const double rhoN = tot[0];
-      st.rr = tot[1];
-      if (!(tot[1] > st.rr_target) || st.iters >= max_iters || !isfinite(tot[1])) {
-        st.inner_active = 0;
-        atomicSub(&cm.ctl->n_inner, 1);
-      } else {
-        const double beta = (rhoN / st.rho) * (st.alpha / st.omega);
-        st.rho = rhoN;
-        if (!isfinite(beta) || rhoN == 0.0) {
-          st.restart = 1;
-          st.beta = 0.0;
-        } else {
-          st.beta = beta;
-        }
-      }
-    }
-  });
-}
-template <typename T, int CH>
-__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg3(Common cm, Kry<T> kr, int max_iters) {
-  count_launch(cm.ctl);
-  bicg3_body<T, CH>(cm, kr, max_iters);
-  loop_epilogue(cm, 1);
-}
-
-// The refinement loop of one step in one cooperative launch, for batches whose chunks fit in
-// one wave of co-resident blocks (one large instance: there the launch and ramp of each kernel
-// of the graph's loops cost more than its pass over the cells). The same chunk bodies as the
-// kernels above, separated by grid-wide barriers. The loop decisions are the graph's: the last
-// block of each deciding pass writes them (loop_epilogue, use_cond = 2) before the barrier,
-// every block reads them after it, and nothing rewrites them before every block has finished
-// the next pass -- so every block runs the same sequence of barriers, and the guards bound it.
-// Launch only cooperatively (cudaLaunchAttributeCooperative), with at most one block per chunk.
-// MINB resident blocks per SM: 2 (124 registers, no spill) when the chunks fit in 2 per SM,
-// else 4 (64 registers, some spilled); on one 1024 x 1024 instance in double-word mode the first
-// took 0.84 ms per step, the second 0.90, the separate kernels 0.98.
-template <typename T, typename C, typename A, int CH, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_solve_coop(Common cm, Fields fl, Coef<C> cfull, Coef<T> ck,
-                                                                Kry<T> kr, double tol, double inner_tol,
-                                                                int max_refine, int max_iters) {
-  count_launch(cm.ctl);
-  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  const volatile int* go_outer = &cm.ctl->go_outer;
-  const volatile int* go_inner = &cm.ctl->go_inner;
-  // the trip counts are capped here as well (the same in every block), so the loops end even if
-  // the decisions were never written
-  for (int o = 0; o < cm.guard_refine; ++o) {
-    resid_body<T, C, A, CH>(cm, fl, cfull, kr, tol, inner_tol, max_refine);
-    loop_epilogue(cm, 0);
-    grid.sync();
-    const bool more = *go_outer != 0;
-    bool inner = *go_inner != 0;
-    for (int it = 0; inner && it < cm.guard_iters; ++it) {
-      bicg1_body<T, CH>(cm, ck, kr);
-      grid.sync();
-      bicg2_body<T, CH>(cm, ck, kr);
-      grid.sync();
-      bicg3_body<T, CH>(cm, kr, max_iters);
-      loop_epilogue(cm, 1);
-      grid.sync();
-      inner = *go_inner != 0;
-    }
-    if (!more) break;
-  }
-}
-
-// ------------------------------------------------------------------------------ polish + checks
-// y' = R + (I - A~) max(y, 0) >= 0 (R >= 0, fractions >= 0), f = y' / D; partials: sum colsum*f,
-// sum R, clamped count; the chunk minimum of f travels in part slot 3. Chunks [c0, c1) of the
-// list (c1 < 0: all); a range must hold whole instances.
-// It also forms the next solve's start g (extrap over the new f, f^n and up to kOrder - 1 earlier
-// states from the history) into the idle y buffer, and moves f^n into the oldest history slot.
-// 4 resident blocks per SM (64 registers; measured on the 4096-instance batch: 2.55 ms per
-// launch against 2.81 ms with 3 blocks and 80 registers)
-template <typename C, typename A, int CH>
-__global__ void __launch_bounds__(kThreads, 4) k_polish(Common cm, Fields fl, Coef<C> co, int c0, int c1) {
-  using V = typename A::V;
-  count_launch(cm.ctl);
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* sm = reinterpret_cast<V*>(smraw);
-  __shared__ float smin[kThreads / 32];
-  for_active_chunks(cm, [&](int b_) { return cm.inst[b_].enabled != 0; }, [&](int c) {
-    const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
-    const double* y = sel2(fl.y64, st.ycur);
-    double* gout = sel2(fl.y64, st.ycur ^ 1);
-    // earlier states for the next start: f^n (the current f) and up to kOrder - 1 from the history
-    const int nh = min(min(st.nhist + 1, kOrder), cm.hist_cap), hs = st.hslot;
-    const double* h2p = sel3(fl.fh, hs);
-    const double* h3p = sel3(fl.fh, (hs + 2) % kHist);
-    const double* h4p = sel3(fl.fh, (hs + 1) % kHist);
-    double* hw = sel3(fl.fh, (hs + 1) % kHist);  // the oldest slot (f^(n-3)) takes f^n
-    const int P = I.pitch;
-    const long long c0 = chunk_start<CH>(c, I);
-    const long long c1 = min(c0 + (long long)CH, inst_end(I));
-    const long long e0 = c0 - P;
-    stage_rows<V>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
-      Q4<V> v = A::ld4(y + k);
-#pragma unroll
-      for (int m = 0; m < 4; ++m) v.a[m] = A::max0(v.a[m]);
-      return v;
-    });
-    __syncthreads();
-    V mass = A::k(0.0), rsum = A::k(0.0);
-    float clamp = 0.0f;
-    float mn = 3.0e38f;
-#pragma unroll 1
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
-      if (K < c1) {
-        const long long o = K - e0;
-        // y' = R + sum over the neighbours of the outflow fraction times max(y, 0): every term is
-        // >= 0, accumulated one direction at a time so that one coefficient row is live at once
-        const Q4<V> R = A::ld4(fl.R + K);
-        Q4<V> yp = R;
-#pragma unroll
-        for (int dir = 0; dir < 4; ++dir) {
-          const Q4<V> c = CoefW<C, A>::row(co, dir, K);
-          const long long on = o + (dir == 0 ? -1 : dir == 1 ? 1 : dir == 2 ? -P : P);
-#pragma unroll
-          for (int m = 0; m < 4; ++m) yp.a[m] = A::fmap(c.a[m], sm[on + m], yp.a[m]);
-        }
-        const Q4<V> inv = A::ld4(fl.invD + K), cols = A::ld4(fl.colsum + K);
-        const int row_i0 = (int)((K - I.base) % I.pitch);
-        Q4<V> fo;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const V fv = A::mul(yp.a[m], inv.a[m]);
-          fo.a[m] = fv;
-          mass = A::fmap(cols.a[m], fv, mass);
-          rsum = A::addp(rsum, R.a[m]);
-          if (row_i0 + m < I.nx) {
-            clamp += A::lt0(A::ld(y, K + m)) ? 1.0f : 0.0f;
-            mn = fminf(mn, A::f32(fv));
-          }
-        }
-        const Q4<V> fn = A::ld4(fl.f + K);
-        Q4<V> g;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          // the states read here (the oldest one included) are read before the slot is replaced
-          const V h2 = nh >= 2 ? A::ld(h2p, K + m) : fn.a[m];
-          const V h3 = nh >= 3 ? A::ld(h3p, K + m) : h2;
-          const V h4 = nh >= 4 ? A::ld(h4p, K + m) : h3;
-          g.a[m] = A::extrap(fo.a[m], fn.a[m], h2, h3, h4, nh, fl.decay ? A::ld(fl.decay, K + m) : A::k(1.0));
-        }
-        A::st4(gout + K, g);
-        A::st4(hw + K, fn);  // f^n into the oldest slot
-        A::st4(fl.f + K, fo);
-      }
-    }
-    // block minimum (separate from the sums)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = mn;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mn = fminf(mn, smin[w]);
-      smin[0] = mn;
-    }
-    __syncthreads();
-    float cl = clamp;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cl += __shfl_xor_sync(0xffffffffu, cl, o);
-    const double w[3] = {A::warp_total_v(mass), A::warp_total_v(rsum), (double)cl};
-    double tot[3], mine[3];
-    block_sum_lane0<3>(w, mine);
-    if (threadIdx.x == 0) cm.part[(size_t)c * 4 + 3] = (double)smin[0];
-    if (chunk_finish<3>(st, PH_POLISH, I.chunk0, I.nchunks, c, cm.part, mine, tot)) {
-      // the last block of the instance: minimum over its chunks, by the whole block
-      __shared__ double s_min[kThreads / 32];
-      double m = 1.0e300;
-      for (int k = threadIdx.x; k < I.nchunks; k += blockDim.x) m = fmin(m, __ldcg(&cm.part[(size_t)(I.chunk0 + k) * 4 + 3]));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = m;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double gmin = s_min[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) gmin = fmin(gmin, s_min[w]);
-        st.min_f = gmin;
-        st.clamped = (long long)tot[2];
-        st.mass_drift = tot[1] != 0.0 ? fabs(tot[0] - tot[1]) / fabs(tot[1]) : 0.0;
-        st.steps += 1;
-        st.hslot = (st.hslot + 1) % kHist;
-        st.nhist = min(st.nhist + 1, kOrder);
-        if (!(gmin >= 0.0)) st.status = ST_NEGATIVE;
-      }
-    }
-    __syncthreads();
-  }, c0, c1);
-}
-
 }  // namespace sg
+
+#include "sayram_solve.cuh"

@@ -1,0 +1,784 @@
+// sayram_solve.cuh -- the solve of one backward-Euler step: outer residual, BiCGSTAB, polish.
+#pragma once
+
+#include "sayram_ops.cuh"
+
+namespace sg {
+
+// ------------------------------------------------------------------------------ streaming helpers
+// Resident blocks per SM the Krylov kernels are compiled for: in FP32, 6 (registers capped at
+// 40; their shared memory allows 6, and the extra blocks in flight raised their bandwidth by
+// 8-14 %); in FP64, 4 (a cap of 40 registers spills).
+template <typename T>
+constexpr int krylov_blocks() { return sizeof(T) == 4 ? 6 : 4; }
+
+template <int CH>
+__device__ __forceinline__ long long chunk_start(int c, const InstDev& I) {
+  return I.base + (long long)(c - I.chunk0) * CH;
+}
+__device__ __forceinline__ long long inst_end(const InstDev& I) { return I.base + (long long)I.ny * I.pitch; }
+
+// Runs body(c) for every chunk c of this block (c = blockIdx.x + k*gridDim.x) whose instance
+// passes want(instance). The instance checks run in parallel, one chunk per thread, and the
+// passing chunks are compacted in shared memory: a launch in which most instances have finished
+// costs one round of checks per block instead of two dependent loads per chunk. Chunks are
+// independent, so the order in which a block takes them does not change any result.
+// Chunks [c0, c1) of the list only (c1 < 0: to the end).
+template <typename W, typename Body>
+__device__ __forceinline__ void for_active_chunks(const Common& cm, W&& want, Body&& body, int c0 = 0, int c1 = -1) {
+  __shared__ int s_list[kThreads];
+  __shared__ int s_cnt;
+  const int nc = (c1 < 0 ? n_chunks(cm) : c1) - c0;
+  const int per = (int)blockIdx.x < nc ? (nc - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  for (int r0 = 0; r0 < per; r0 += kThreads) {
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    const int k = r0 + (int)threadIdx.x;
+    if (k < per) {
+      const int c = c0 + (int)blockIdx.x + k * (int)gridDim.x;
+      if (want(cm.chunk_inst[c])) s_list[atomicAdd(&s_cnt, 1)] = c;
+    }
+    __syncthreads();
+    const int m = s_cnt;
+    for (int q = 0; q < m; ++q) body(s_list[q]);
+    __syncthreads();
+  }
+}
+
+// Fills smem[0 .. n) with a 4-aligned stretch [e0, e0 + n) of a vector computed cell-wise by
+// f(k) -> Q4<T> (k a multiple of 4): the chunk plus one row above and below, so that the stencil
+// of every cell in the chunk reads shared memory only.
+template <typename T, typename F>
+__device__ __forceinline__ void stage_rows(T* sm, long long e0, long long n, F&& f) {
+#pragma unroll 2
+  for (long long q = 4LL * threadIdx.x; q < n; q += 4LL * blockDim.x) {
+    const Q4<T> v = f(e0 + q);
+    *reinterpret_cast<Q4<T>*>(sm + q) = v;
+  }
+}
+
+// ------------------------------------------------------------------------------ Krylov arithmetic
+// Every operation fused or rounded explicitly, so that all kernels that run a formula give the
+// same bits.
+__device__ __forceinline__ float fmaT(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mulT(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulT(double a, double b) { return __dmul_rn(a, b); }
+
+// FP64 <-> FP32 of the preconditioner's factors (non-negative, at most a few units) by moving the
+// fields: conversions run at the FP64 rate, 1/64 of the integer rate. Truncated; below FP32's
+// normal range they become 0.
+__device__ __forceinline__ float narrow(float a) { return a; }
+__device__ __forceinline__ float narrow(double a) {
+  const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
+  return hi < 0x38100000u ? 0.0f : __uint_as_float(__funnelshift_l(lo, hi - 0x38000000u, 3));
+}
+template <typename T>
+__device__ __forceinline__ T widen(float a);
+template <>
+__device__ __forceinline__ float widen<float>(float a) { return a; }
+template <>
+__device__ __forceinline__ double widen<double>(float a) {
+  const unsigned b = __float_as_uint(a);
+  return b < 0x00800000u ? 0.0 : __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
+// Alpha-line block preconditioner. Every 4-cell group of the padded layout lies inside one row
+// (rows start at multiples of 4), and B is the tridiagonal of the group's own west/east couplings
+// -- unit diagonal, -cw below, -ce above -- with the couplings to the neighbouring groups dropped:
+// block Jacobi with 4-cell alpha-line blocks, the direction in which the scaled systems are
+// stiffest (Dxx/dalpha^2 against Dyy/dlogE^2). line4 returns B^-1 q by Thomas elimination
+// without pivoting (B is a column-diagonally-dominant M-matrix: every column of the outflow
+// fractions sums to < 1, so each pivot stays in (0, 1]). The pivots are inverted in FP32 whatever
+// the vector precision (any map close to B^-1 preconditions as well; every kernel applies the
+// same one); padding cells (q = cw = ce = 0) stay 0.
+template <typename T>
+struct Line {
+  T w1, w2, w3, c0, c1, c2, i1, i2, i3;
+};
+template <typename T>
+__device__ __forceinline__ Line<T> line_of(const Q4<T>& cw, const Q4<T>& ce) {
+  Line<T> L;
+  L.w1 = cw.a[1];
+  L.w2 = cw.a[2];
+  L.w3 = cw.a[3];
+  L.c0 = ce.a[0];
+  const float i1 = __frcp_rn(__fmaf_rn(-narrow(cw.a[1]), narrow(ce.a[0]), 1.0f));
+  const float c1 = __fmul_rn(narrow(ce.a[1]), i1);
+  const float i2 = __frcp_rn(__fmaf_rn(-narrow(cw.a[2]), c1, 1.0f));
+  const float c2 = __fmul_rn(narrow(ce.a[2]), i2);
+  const float i3 = __frcp_rn(__fmaf_rn(-narrow(cw.a[3]), c2, 1.0f));
+  L.i1 = widen<T>(i1);
+  L.i2 = widen<T>(i2);
+  L.i3 = widen<T>(i3);
+  L.c1 = widen<T>(c1);
+  L.c2 = widen<T>(c2);
+  return L;
+}
+template <typename T>
+__device__ __forceinline__ Q4<T> line4(const Q4<T>& q, const Line<T>& L) {
+  // forward: d_j = (q_j + w_j d_(j-1)) / pivot_j; backward: z_j = d_j + c_j z_(j+1)
+  const T d0 = q.a[0];
+  const T d1 = mulT(fmaT(L.w1, d0, q.a[1]), L.i1);
+  const T d2 = mulT(fmaT(L.w2, d1, q.a[2]), L.i2);
+  const T d3 = mulT(fmaT(L.w3, d2, q.a[3]), L.i3);
+  Q4<T> z;
+  z.a[3] = d3;
+  z.a[2] = fmaT(L.c2, d3, d2);
+  z.a[1] = fmaT(L.c1, z.a[2], d1);
+  z.a[0] = fmaT(L.c0, z.a[1], d0);
+  return z;
+}
+
+// A~ x over a 4-cell group from a staged vector (sm + o: the group's first cell; rows P apart):
+// four multiply-adds per cell
+template <typename T>
+__device__ __forceinline__ Q4<T> stencil_sm(const T* sm, int o, int P, const Q4<T>& cw, const Q4<T>& ce,
+                                            const Q4<T>& cs, const Q4<T>& cn) {
+  const Q4<T> c = *reinterpret_cast<const Q4<T>*>(sm + o);
+  const Q4<T> d = *reinterpret_cast<const Q4<T>*>(sm + o - P);
+  const Q4<T> u = *reinterpret_cast<const Q4<T>*>(sm + o + P);
+  const T w0 = sm[o - 1], e3 = sm[o + 4];
+  Q4<T> r;
+  const T wv[4] = {w0, c.a[0], c.a[1], c.a[2]};
+  const T ev[4] = {c.a[1], c.a[2], c.a[3], e3};
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    r.a[k] = fmaT(-cn.a[k], u.a[k], fmaT(-cs.a[k], d.a[k], fmaT(-ce.a[k], ev[k], fmaT(-cw.a[k], wv[k], c.a[k]))));
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ T dot4(const Q4<T>& a, const Q4<T>& b, T q) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) q = fmaT(a.a[m], b.a[m], q);
+  return q;
+}
+
+// ------------------------------------------------------------------------------ solver scalars
+// The decisions of one instance's solve, shared by every kernel that runs it. Sums are doubles.
+// after the residual: tot = ||r sc||^2, ||R sc||^2, ||B^-1 r sc||^2. Returns 0 when the step's
+// solve ends here, 1 when a Krylov solve starts.
+__device__ __forceinline__ int after_resid(InstState& st, const double (&tot)[3], double tol, double inner_tol,
+                                           int max_refine, int precond) {
+  st.ycur ^= 1;
+  st.has_x = 0;
+  if (st.refines == 0) st.bb = tot[1];
+  st.refines += 1;
+  st.cum_refines += 1;
+  st.rr64 = tot[0];
+  st.rel = st.bb > 0 ? sqrt(tot[0] / st.bb) : 0.0;
+  if (!(st.rel > tol)) {
+    st.outer_active = 0;
+    st.status = ST_OK;
+    return 0;
+  }
+  if (st.refines >= max_refine) {
+    st.outer_active = 0;
+    st.status = ST_NOT_CONVERGED;
+    return 0;
+  }
+  st.restart = 1;
+  st.iters = 0;
+  // the Krylov's residual is B^-1 r: its target is the relative reduction asked, or the final
+  // tolerance carried into preconditioned units by this pass's norm ratio
+  const double rrk = precond ? tot[2] : tot[0];
+  st.rr = rrk;
+  const double a = __dmul_rn(__dmul_rn(inner_tol, inner_tol), rrk);
+  const double bnd =
+      __dmul_rn(__dmul_rn(__dmul_rn(0.0625, __dmul_rn(tol, tol)), st.bb), precond && tot[0] > 0.0 ? rrk / tot[0] : 1.0);
+  st.rr_target = a > bnd ? a : bnd;
+  return 1;
+}
+// after v = B^-1 A~ p: tot = (r^, v), (r, r) (the latter only formed on a restart)
+__device__ __forceinline__ void after_v(InstState& st, const double (&tot)[2]) {
+  if (st.restart) {
+    st.rho = st.iters == 0 ? st.rr : tot[1];  // (r^, r) with r^ = r
+    st.restart = 0;
+  }
+  const double den = tot[0];
+  if (den != 0.0 && isfinite(den) && st.rho != 0.0) {
+    st.alpha = st.rho / den;
+  } else {
+    st.alpha = 0.0;  // breakdown: this iteration degenerates to a minimal-residual step
+    st.restart = 1;
+  }
+}
+// after t = B^-1 A~ s: tot = (t, s), (t, t), (s, s), (r^, s), (r^, t). The next residual is r = s -
+// omega t, so (r, r) and (r^, r) follow from these sums and the pass that would form them is not
+// needed. Returns 1 when this Krylov solve ends.
+__device__ __forceinline__ int after_t(InstState& st, const double (&tot)[5], int max_iters) {
+  const double ts = tot[0], tt = tot[1];
+  st.omega = tt > 0.0 && isfinite(ts) ? ts / tt : 0.0;
+  if (st.omega == 0.0) st.restart = 1;
+  const double om = st.omega;
+  st.rr = __fma_rn(om, __fma_rn(om, tt, -2.0 * ts), tot[2]);
+  const double rhoN = __fma_rn(-om, tot[4], tot[3]);
+  st.iters += 1;
+  st.iters_total += 1;
+  st.cum_iters += 1;
+  if (!(st.rr > st.rr_target) || st.iters >= max_iters || !isfinite(st.rr)) {
+    st.has_x = 1;
+    return 1;
+  }
+  const double beta = (rhoN / st.rho) * (st.alpha / om);
+  st.rho = rhoN;
+  if (!isfinite(beta) || rhoN == 0.0) {
+    st.restart = 1;
+    st.beta = 0.0;
+  } else {
+    st.beta = beta;
+  }
+  return 0;
+}
+
+// Coefficients of a row in the wide arithmetic: from the FP64 arrays or the (hi, lo) split
+template <typename C, typename A>
+struct CoefW;
+template <typename A>
+struct CoefW<double, A> {
+  __device__ static Q4<typename A::V> row(const Coef<double>& c, int which, long long K) {
+    const double* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
+    const Q4<double> q = ld4(a + K);
+    Q4<typename A::V> o;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o.a[k] = A::from_d(q.a[k]);
+    return o;
+  }
+};
+template <typename A>
+struct CoefW<float, A> {
+  __device__ static Q4<typename A::V> row(const Coef<float>& c, int which, long long K) {
+    const float* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
+    const float* l = which == 0 ? c.lw : which == 1 ? c.le : which == 2 ? c.ls : c.ln;
+    const Q4<float> h = ld4(a + K), lo = ld4(l + K);
+    Q4<typename A::V> o;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o.a[k] = A::hilo(h.a[k], lo.a[k]);
+    return o;
+  }
+};
+
+// ------------------------------------------------------------------------------ outer residual
+// One 4-cell group of r = R - A~ y in the wide arithmetic from the staged y (sm + o): y itself, the
+// scaled residual with the preconditioner applied, and the group's terms of ||r||^2, ||R||^2 and
+// ||B^-1 r||^2.
+template <typename T, typename C, typename A>
+__device__ __forceinline__ void resid_group(const typename A::V* sm, int o, int P, const Coef<C>& co, long long K,
+                                            const double* Rp, float sc, int precond, Q4<typename A::V>& yc, Q4<T>& r,
+                                            typename A::Acc& q0, typename A::Acc& q1, T& q2) {
+  using V = typename A::V;
+  const Q4<V> cw = CoefW<C, A>::row(co, 0, K), ce = CoefW<C, A>::row(co, 1, K);
+  const Q4<V> cs = CoefW<C, A>::row(co, 2, K), cn = CoefW<C, A>::row(co, 3, K);
+  const Q4<V> R = A::ld4(Rp + K);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const V yv = sm[o + m];
+    const V s1 = A::fma(cn.a[m], sm[o + m + P], A::fma(cs.a[m], sm[o + m - P],
+                        A::fma(ce.a[m], sm[o + m + 1], A::mul(cw.a[m], sm[o + m - 1]))));
+    const V rv = A::sub(R.a[m], A::sub(yv, s1));
+    yc.a[m] = yv;
+    r.a[m] = A::template scaled<T>(rv, sc);
+    q0 = A::sq_scaled(rv, sc, q0);
+    q1 = A::sq_scaled(R.a[m], sc, q1);
+  }
+  if (precond) {  // the Krylov matrix's couplings (the hi parts in the FP32 modes)
+    r = line4<T>(r, line_of<T>(ld4(co.cw + K), ld4(co.ce + K)));
+    q2 = dot4<T>(r, r, q2);
+  }
+}
+
+// r = R - A~ (y + x) in the wide arithmetic; writes y + x to the other y buffer and the Krylov's
+// right-hand side B^-1 r (T precision, scaled) to rh.
+template <typename T, typename C, typename A, int CH>
+__device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, const Coef<C>& co, const Kry<T>& kr,
+                                           double tol, double inner_tol, int max_refine) {
+  using V = typename A::V;
+  using R = typename A::R;
+  using Sums = ChunkSums<CH, 3, R>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double s_part[3 * Sums::kParts];
+  V* sm = reinterpret_cast<V*>(smraw);
+  for_active_chunks(cm, [&](int b_) { return cm.st[b_].outer_active != 0; }, [&](int c) {
+    const int b = cm.chunk_inst[c];
+    InstState& st = cm.st[b];
+    const InstDev I = cm.inst[b];
+    const double* yin = sel2(fl.y64, st.ycur);
+    double* yout = sel2(fl.y64, st.ycur ^ 1);
+    const bool hx = st.has_x != 0;
+    const float sc = rhs_scale(st.rmax_bits);  // r is handed over as r * sc
+    const float isc = 1.0f / sc;                // exact: sc is a power of two
+    const int P = I.pitch;
+    const long long c0 = chunk_start<CH>(c, I);
+    const long long c1 = min(c0 + (long long)CH, inst_end(I));
+    const long long e0 = c0 - P;
+    Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
+    // y + x (the last Krylov correction, in scaled units) over the chunk and one row each side
+    stage_rows<V>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+      Q4<V> y = A::ld4(yin + k);
+      if (hx) {
+        const Q4<T> x = ld4(kr.x + k);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) y.a[m] = A::template add_scaled<T>(y.a[m], x.a[m], isc);
+      }
+      return y;
+    });
+    __syncthreads();
+    typename A::Acc q0 = 0, q1 = 0;
+    T q2 = (T)0;
+#pragma unroll 1
+    for (int g = 0; g < CH / (4 * kThreads); ++g) {
+      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+      if (K < c1) {
+        Q4<V> yc;
+        Q4<T> r;
+        resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
+        A::st4(yout + K, yc);
+        st4(kr.rh + K, r);
+      }
+      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
+        const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
+        sums.put(g, w);
+        q0 = q1 = 0;
+        q2 = (T)0;
+      }
+    }
+    const int sl = (c - I.chunk0) * (CH / Sums::SEG);
+    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
+    double tot[3];
+    if (chunk_finish<3, R>(st, PH_RESID, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
+      if (after_resid(st, tot, tol, inner_tol, max_refine, cm.precond)) {
+        st.inner_active = 1;
+        atomicAdd(&cm.ctl->n_inner, 1);
+      } else {
+        atomicSub(&cm.ctl->n_outer, 1);
+      }
+    }
+  });
+}
+template <typename T, typename C, typename A, int CH>
+__global__ void __launch_bounds__(kThreads, 4) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
+                                                        double tol, double inner_tol, int max_refine) {
+  count_launch(cm.ctl);
+  resid_body<T, C, A, CH>(cm, fl, co, kr, tol, inner_tol, max_refine);
+  loop_epilogue(cm, 0);
+}
+
+// ------------------------------------------------------------------------------ BiCGSTAB
+// Left-preconditioned BiCGSTAB on B^-1 A~ x = B^-1 r (B = I without the preconditioner; the
+// residual r the kernels carry is the preconditioned one, and x is the correction itself), in
+// two passes per iteration:
+// k1: r = s - omega t and x += alpha p + omega s of the previous iteration, p = r + beta (p - omega
+//     v) (p = r on a restart, which also sets r^ = r), v = B^-1 A~ p; sums (r^, v). r and p are
+//     computed once per cell into shared memory (chunk plus one row above and below) and the
+//     stencil reads p there. The first iteration of a solve has p = r = r^ and writes only v.
+// k2: s = r - alpha v staged likewise, t = B^-1 A~ s; the five sums of after_t.
+// k3: x += alpha p + omega s of the instances whose solve ended in this iteration.
+// The residual's own dot products come from k2's sums (after_t), so no third pass over the vectors
+// separates r from p: 88 B per cell and iteration in FP32 (first iteration 52 B) against 100 B (88
+// B) for update, product and update as three passes, and one barrier or launch less. FP64 is bound
+// by its pipe (525 GFMA/s): 26 operations per cell and iteration against 39, with the stencil as
+// four multiply-adds and no FP64-rate conversions in the preconditioner. Measured, whole calls: 192
+// uneven FP64 instances, 4 steps, 19.2 -> 15.8 ms; 1024 in double-word 22.5 -> 20.2 ms; 24 in
+// double-word, 6 steps, 2.94 -> 2.47 ms; 192 mixed with Jacobi scaling 14.7 -> 14.0 ms.
+template <typename T, int CH>
+__device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, const Kry<T>& kr) {
+  using R = typename RedOf<T>::R;
+  using Sums = ChunkSums<CH, 2, R>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double s_part[2 * Sums::kParts];
+  T* sm = reinterpret_cast<T*>(smraw);
+  for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
+    const int b = cm.chunk_inst[c];
+    InstState& st = cm.st[b];
+    const InstDev I = cm.inst[b];
+    const int it = st.iters;  // iterations finished; this one is it + 1
+    const bool rs = st.restart != 0;
+    const T alpha = (T)st.alpha, beta = (T)st.beta, omega = (T)st.omega;
+    const T* ro = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
+    const T* po = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
+    const T* vo = sel2(kr.v, it & 1);
+    T* rn = sel2(kr.r, (it + 1) & 1);
+    T* pn = sel2(kr.p, (it + 1) & 1);
+    T* vn = sel2(kr.v, (it + 1) & 1);
+    const int P = I.pitch;
+    const long long c0 = chunk_start<CH>(c, I);
+    const long long c1 = min(c0 + (long long)CH, inst_end(I));
+    const long long e0 = c0 - P;
+    Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
+    if (it == 0) {
+      stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) { return ld4(kr.rh + k); });
+    } else {
+      stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+        const Q4<T> r = ld4(ro + k), v = ld4(vo + k), t = ld4(kr.t + k);
+        Q4<T> p = it > 1 ? ld4(po + k) : r;
+        const bool mine = k >= c0 && k < c1;
+        Q4<T> s, q;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          s.a[m] = fmaT(-alpha, v.a[m], r.a[m]);
+          q.a[m] = fmaT(-omega, t.a[m], s.a[m]);
+        }
+        if (mine) {
+          Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
+          if (it > 1) x = ld4(kr.x + k);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) x.a[m] = fmaT(alpha, p.a[m], fmaT(omega, s.a[m], x.a[m]));
+          st4(kr.x + k, x);
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) p.a[m] = rs ? q.a[m] : fmaT(beta, fmaT(-omega, v.a[m], p.a[m]), q.a[m]);
+        if (mine) {
+          st4(rn + k, q);
+          st4(pn + k, p);
+          if (rs) st4(kr.rh + k, q);
+        }
+        return p;
+      });
+    }
+    __syncthreads();
+    T q0 = (T)0, q1 = (T)0;
+#pragma unroll 2
+    for (int g = 0; g < CH / (4 * kThreads); ++g) {
+      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+      if (K < c1) {
+        const int o = (int)(K - e0);
+        const Q4<T> cw = ld4(co.cw + K), ce = ld4(co.ce + K);
+        Q4<T> v = stencil_sm<T>(sm, o, P, cw, ce, ld4(co.cs + K), ld4(co.cn + K));
+        if (cm.precond) v = line4<T>(v, line_of<T>(cw, ce));  // v = B^-1 A~ p
+        st4(vn + K, v);
+        // r^ (on a restart it is p itself)
+        const Q4<T> rh = rs ? *reinterpret_cast<const Q4<T>*>(sm + o) : ld4(kr.rh + K);
+        q0 = dot4<T>(rh, v, q0);
+        if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
+      }
+      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
+        const R w[2] = {rfrom<R>(q0), rfrom<R>(q1)};
+        sums.put(g, w);
+        q0 = q1 = (T)0;
+      }
+    }
+    const int sl = (c - I.chunk0) * (CH / Sums::SEG);
+    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
+    double tot[2];
+    if (chunk_finish<2, R>(st, PH_K1, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0)
+      after_v(st, tot);
+  });
+}
+template <typename T, int CH>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 5 : 4) k_bicg1(Common cm, Coef<T> co, Kry<T> kr) {
+  count_launch(cm.ctl);
+  if (blockIdx.x == 0 && threadIdx.x == 0) cm.ctl->seq += 1u;
+  bicg1_body<T, CH>(cm, co, kr);
+}
+
+template <typename T, int CH>
+__device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, const Kry<T>& kr, int max_iters,
+                                           unsigned seq) {
+  using R = typename RedOf<T>::R;
+  using Sums = ChunkSums<CH, 5, R>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double s_part[5 * Sums::kParts];
+  T* sm = reinterpret_cast<T*>(smraw);
+  for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
+    const int b = cm.chunk_inst[c];
+    InstState& st = cm.st[b];
+    const InstDev I = cm.inst[b];
+    const int it = st.iters;
+    const T alpha = (T)st.alpha;
+    const T* r = it > 0 ? sel2(kr.r, (it + 1) & 1) : kr.rh;
+    const T* vv = sel2(kr.v, (it + 1) & 1);
+    const int P = I.pitch;
+    const long long c0 = chunk_start<CH>(c, I);
+    const long long c1 = min(c0 + (long long)CH, inst_end(I));
+    const long long e0 = c0 - P;
+    Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
+    stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+      Q4<T> x = ld4(r + k);
+      const Q4<T> v = ld4(vv + k);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) x.a[m] = fmaT(-alpha, v.a[m], x.a[m]);
+      return x;
+    });
+    __syncthreads();
+    T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
+#pragma unroll 2
+    for (int g = 0; g < CH / (4 * kThreads); ++g) {
+      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+      if (K < c1) {
+        const int o = (int)(K - e0);
+        const Q4<T> s = *reinterpret_cast<const Q4<T>*>(sm + o);
+        const Q4<T> cw = ld4(co.cw + K), ce = ld4(co.ce + K);
+        Q4<T> t = stencil_sm<T>(sm, o, P, cw, ce, ld4(co.cs + K), ld4(co.cn + K));
+        if (cm.precond) t = line4<T>(t, line_of<T>(cw, ce));  // t = B^-1 A~ s
+        st4(kr.t + K, t);
+        const Q4<T> rh = ld4(kr.rh + K);
+        q[0] = dot4<T>(t, s, q[0]);
+        q[1] = dot4<T>(t, t, q[1]);
+        q[2] = dot4<T>(s, s, q[2]);
+        q[3] = dot4<T>(rh, s, q[3]);
+        q[4] = dot4<T>(rh, t, q[4]);
+      }
+      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
+        const R w[5] = {rfrom<R>(q[0]), rfrom<R>(q[1]), rfrom<R>(q[2]), rfrom<R>(q[3]), rfrom<R>(q[4])};
+        sums.put(g, w);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) q[k] = (T)0;
+      }
+    }
+    const int sl = (c - I.chunk0) * (CH / Sums::SEG);
+    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
+    double tot[5];
+    if (chunk_finish<5, R>(st, PH_K2, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
+      if (after_t(st, tot, max_iters)) {
+        st.fin_seq = seq;
+        st.inner_active = 0;
+        atomicSub(&cm.ctl->n_inner, 1);
+      }
+    }
+  });
+}
+template <typename T, int CH>
+__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg2(Common cm, Coef<T> co, Kry<T> kr,
+                                                                         int max_iters) {
+  count_launch(cm.ctl);
+  bicg2_body<T, CH>(cm, co, kr, max_iters, cm.ctl->seq);
+  loop_epilogue(cm, 1);
+}
+
+template <typename T, int CH>
+__device__ __forceinline__ void bicg3_body(const Common& cm, const Kry<T>& kr, unsigned seq) {
+  for_active_chunks(cm, [&](int b_) { return cm.st[b_].fin_seq == seq; }, [&](int c) {
+    const int b = cm.chunk_inst[c];
+    const InstState& st = cm.st[b];
+    const InstDev I = cm.inst[b];
+    const int it = st.iters;  // the solve's last iteration
+    const T alpha = (T)st.alpha, omega = (T)st.omega;
+    const T* rr = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
+    const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
+    const T* vv = sel2(kr.v, it & 1);
+    const long long c0 = chunk_start<CH>(c, I);
+    const long long c1 = min(c0 + (long long)CH, inst_end(I));
+#pragma unroll 2
+    for (int g = 0; g < CH / (4 * kThreads); ++g) {
+      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+      if (K >= c1) continue;
+      const Q4<T> r = ld4(rr + K), v = ld4(vv + K);
+      const Q4<T> p = it > 1 ? ld4(pp + K) : r;
+      Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
+      if (it > 1) x = ld4(kr.x + K);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const T s = fmaT(-alpha, v.a[m], r.a[m]);
+        x.a[m] = fmaT(alpha, p.a[m], fmaT(omega, s, x.a[m]));
+      }
+      st4(kr.x + K, x);
+    }
+  });
+}
+template <typename T, int CH>
+__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg3(Common cm, Kry<T> kr) {
+  count_launch(cm.ctl);
+  bicg3_body<T, CH>(cm, kr, cm.ctl->seq);
+}
+
+// The refinement loop of one step in one cooperative launch, for batches whose chunks fit in
+// one wave of co-resident blocks (one large instance: there the launch and ramp of each kernel
+// of the graph's loops cost more than its pass over the cells). The same chunk bodies as the
+// kernels above, separated by grid-wide barriers. The loop decisions are the graph's: the last
+// block of each deciding pass writes them (loop_epilogue, use_cond = 2) before the barrier,
+// every block reads them after it, and nothing rewrites them before every block has finished
+// the next pass -- so every block runs the same sequence of barriers, and the guards bound it.
+// Launch only cooperatively (cudaLaunchAttributeCooperative), with at most one block per chunk.
+// MINB resident blocks per SM: 2 (124 registers, no spill) when the chunks fit in 2 per SM,
+// else 4 (64 registers, some spilled); on one 1024 x 1024 instance in double-word mode the first
+// took 0.84 ms per step, the second 0.90, the separate kernels 0.98.
+template <typename T, typename C, typename A, int CH, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) k_solve_coop(Common cm, Fields fl, Coef<C> cfull, Coef<T> ck,
+                                                                Kry<T> kr, double tol, double inner_tol,
+                                                                int max_refine, int max_iters) {
+  count_launch(cm.ctl);
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const volatile int* go_outer = &cm.ctl->go_outer;
+  const volatile int* go_inner = &cm.ctl->go_inner;
+  // the trip counts are capped here as well (the same in every block), so the loops end even if
+  // the decisions were never written
+  unsigned seq = 0;
+  for (int o = 0; o < cm.guard_refine; ++o) {
+    resid_body<T, C, A, CH>(cm, fl, cfull, kr, tol, inner_tol, max_refine);
+    loop_epilogue(cm, 0);
+    grid.sync();
+    const bool more = *go_outer != 0;
+    bool inner = *go_inner != 0;
+    for (int it = 0; inner && it < cm.guard_iters; ++it) {
+      bicg1_body<T, CH>(cm, ck, kr);
+      grid.sync();
+      bicg2_body<T, CH>(cm, ck, kr, max_iters, ++seq);
+      loop_epilogue(cm, 1);
+      grid.sync();
+      inner = *go_inner != 0;
+      bicg3_body<T, CH>(cm, kr, seq);  // touches only instances that no pass works on until the next residual
+      if (!inner) grid.sync();
+    }
+    if (!more) break;
+  }
+}
+
+// ------------------------------------------------------------------------------ polish + checks
+// The polish's pointers for one instance: its solution y, the idle y buffer (which takes the next
+// start g) and the earlier states the start goes back to (f^n, the current f, and up to kOrder - 1
+// from the history).
+struct PolishAt {
+  const double* y;
+  double* gout;
+  const double *h2, *h3, *h4;
+  double* hw;  // the oldest slot (f^(n-3)) takes f^n
+  int nh;
+};
+__device__ __forceinline__ PolishAt polish_at(const Fields& fl, int ycur, int nhist, int hslot, int hist_cap) {
+  PolishAt a;
+  a.y = sel2(fl.y64, ycur);
+  a.gout = sel2(fl.y64, ycur ^ 1);
+  a.nh = min(min(nhist + 1, kOrder), hist_cap);
+  a.h2 = sel3(fl.fh, hslot);
+  a.h3 = sel3(fl.fh, (hslot + 2) % kHist);
+  a.h4 = sel3(fl.fh, (hslot + 1) % kHist);
+  a.hw = sel3(fl.fh, (hslot + 1) % kHist);
+  return a;
+}
+// One 4-cell group from the staged max(y, 0) (sm + o); real: cells of the group inside the grid
+template <typename C, typename A>
+__device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int P, const Coef<C>& co, long long K,
+                                             const Fields& fl, const PolishAt& at, int real, typename A::V& mass,
+                                             typename A::V& rsum, float& mn) {
+  using V = typename A::V;
+  // y' = R + sum over the neighbours of the outflow fraction times max(y, 0): every term is
+  // >= 0, accumulated one direction at a time so that one coefficient row is live at once
+  const Q4<V> R = A::ld4(fl.R + K);
+  Q4<V> yp = R;
+#pragma unroll
+  for (int dir = 0; dir < 4; ++dir) {
+    const Q4<V> c = CoefW<C, A>::row(co, dir, K);
+    const int on = o + (dir == 0 ? -1 : dir == 1 ? 1 : dir == 2 ? -P : P);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) yp.a[m] = A::fmap(c.a[m], sm[on + m], yp.a[m]);
+  }
+  const Q4<V> inv = A::ld4(fl.invD + K), cols = A::ld4(fl.colsum + K);
+  Q4<V> fo;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const V fv = A::mul(yp.a[m], inv.a[m]);
+    fo.a[m] = fv;
+    mass = A::fmap(cols.a[m], fv, mass);
+    rsum = A::addp(rsum, R.a[m]);
+    if (m < real) mn = fminf(mn, A::f32(fv));
+  }
+  const Q4<V> fn = A::ld4(fl.f + K);
+  Q4<V> g;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    // the states read here (the oldest one included) are read before the slot is replaced
+    const V h2 = at.nh >= 2 ? A::ld(at.h2, K + m) : fn.a[m];
+    const V h3 = at.nh >= 3 ? A::ld(at.h3, K + m) : h2;
+    const V h4 = at.nh >= 4 ? A::ld(at.h4, K + m) : h3;
+    g.a[m] = A::extrap(fo.a[m], fn.a[m], h2, h3, h4, at.nh, fl.decay ? A::ld(fl.decay, K + m) : A::k(1.0));
+  }
+  A::st4(at.gout + K, g);
+  A::st4(at.hw + K, fn);  // f^n into the oldest slot
+  A::st4(fl.f + K, fo);
+}
+// an instance's step is complete: sums of colsum f, R and the clamped count, and the minimum of f
+__device__ __forceinline__ void after_polish(InstState& st, double mass, double rsum, double clamped, double gmin) {
+  st.min_f = gmin;
+  st.clamped = (long long)clamped;
+  st.mass_drift = rsum != 0.0 ? fabs(mass - rsum) / fabs(rsum) : 0.0;
+  st.steps += 1;
+  st.hslot = (st.hslot + 1) % kHist;
+  st.nhist = min(st.nhist + 1, kOrder);
+  if (!(gmin >= 0.0)) st.status = ST_NEGATIVE;
+}
+
+// y' = R + (I - A~) max(y, 0) >= 0 (R >= 0, fractions >= 0), f = y' / D; sums of colsum*f, R and the
+// clamped count (carried in doubles above the segments); the minimum of f travels as a fourth
+// quantity. Chunks [c0, c1) of the list (c1 < 0: all); a range must hold whole instances.
+// It also forms the next solve's start g (extrap over the new f, f^n and up to kOrder - 1 earlier
+// states from the history) into the idle y buffer, and moves f^n into the oldest history slot.
+// 4 resident blocks per SM (64 registers; measured on the 4096-instance batch: 2.55 ms per
+// launch against 2.81 ms with 3 blocks and 80 registers)
+template <typename C, typename A, int CH>
+__global__ void __launch_bounds__(kThreads, 4) k_polish(Common cm, Fields fl, Coef<C> co, int c0, int c1) {
+  using V = typename A::V;
+  using R = typename A::R;
+  using Sums = ChunkSums<CH, 3, R>;
+  count_launch(cm.ctl);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double s_part[3 * Sums::kParts];
+  __shared__ float s_min[kThreads / 32];
+  V* sm = reinterpret_cast<V*>(smraw);
+  for_active_chunks(cm, [&](int b_) { return cm.inst[b_].enabled != 0; }, [&](int c) {
+    const int b = cm.chunk_inst[c];
+    InstState& st = cm.st[b];
+    const InstDev I = cm.inst[b];
+    const PolishAt at = polish_at(fl, st.ycur, st.nhist, st.hslot, cm.hist_cap);
+    const int P = I.pitch;
+    const long long c0 = chunk_start<CH>(c, I);
+    const long long c1 = min(c0 + (long long)CH, inst_end(I));
+    const long long e0 = c0 - P;
+    Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
+    float clamp = 0.0f;
+    stage_rows<V>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+      Q4<V> v = A::ld4(at.y + k);
+      const bool mine = k >= c0 && k < c1;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        if (mine && A::lt0(v.a[m])) clamp += 1.0f;  // padding cells are 0
+        v.a[m] = A::max0(v.a[m]);
+      }
+      return v;
+    });
+    __syncthreads();
+    V mass = A::k(0.0), rsum = A::k(0.0);
+    float mn = 3.0e38f;
+#pragma unroll 1
+    for (int g = 0; g < CH / (4 * kThreads); ++g) {
+      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+      if (K < c1)
+        polish_group<C, A>(sm, (int)(K - e0), P, co, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
+      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
+        const R w[3] = {mass, rsum, rfrom<R>(clamp)};
+        sums.put(g, w);
+        mass = rsum = A::k(0.0);
+        clamp = 0.0f;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = mn;
+    const int sl = (c - I.chunk0) * (CH / Sums::SEG), left = I.nseg - sl;
+    sums.template store<double>(cm.part, cm.pstride, I.seg0 + sl, left);
+    if (threadIdx.x < CH / Sums::SEG && (int)threadIdx.x < left) {  // the chunk's minimum, for each of its segments
+      float m = s_min[0];
+      for (int w = 1; w < kThreads / 32; ++w) m = fminf(m, s_min[w]);
+      cm.part[3 * (size_t)cm.pstride + I.seg0 + sl + threadIdx.x] = (double)m;
+    }
+    double tot[3];
+    if (chunk_finish<3, double>(st, PH_POLISH, I, cm.part, cm.pstride, tot)) {
+      // the last block of the instance: minimum over its segments, by the whole block
+      double m = 1.0e300;
+      for (int k = threadIdx.x; k < I.nseg; k += blockDim.x)
+        m = fmin(m, __ldcg(&cm.part[3 * (size_t)cm.pstride + I.seg0 + k]));
+      __shared__ double s_gmin[kThreads / 32];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if ((threadIdx.x & 31) == 0) s_gmin[threadIdx.x >> 5] = m;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double gmin = s_gmin[0];
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) gmin = fmin(gmin, s_gmin[w]);
+        after_polish(st, tot[0], tot[1], tot[2], gmin);
+      }
+    }
+    __syncthreads();
+  }, c0, c1);
+}
+
+}  // namespace sg
