@@ -10,8 +10,10 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OUT_DIR = os.path.join(PKG, "_build")
 LIB = os.path.join(OUT_DIR, "libsayram_gpu.so")
-SOURCES = ["sayram_engine.cu", "h5_writer.cc", "h5_reader.cc"]
-DEPS = ["sayram_kernels.cuh", "sayram_ops.cuh", "sayram_solve.cuh", "dword.cuh", "host_errors.h"]
+SOURCES = ["sayram_engine.cu", "sayram_team_f64.cu", "sayram_team_mixed.cu", "sayram_team_dw.cu", "h5_writer.cc",
+           "h5_reader.cc"]
+DEPS = ["sayram_kernels.cuh", "sayram_ops.cuh", "sayram_solve.cuh", "sayram_team.cuh", "sayram_team.h",
+        "dword.cuh", "host_errors.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -39,7 +41,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     tmp = LIB + ".tmp"
     # host code: no fused multiply-adds, so host-side values (grid weights, D-table row factors)
     # are the same separately rounded operations on x86-64 and aarch64
-    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off", "-shared",
+    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "--threads", "0", "-Xcompiler", "-fPIC,-ffp-contract=off", "-shared",
            "-I", os.path.join(ROOT, "include"), "-o", tmp] + [os.path.join(CSRC, s) for s in SOURCES]
     if verbose:
         print(" ".join(cmd))

@@ -20,6 +20,7 @@
 #include "host_errors.h"
 #include "sayram_gpu.h"
 #include "sayram_ops.cuh"
+#include "sayram_team.h"
 
 namespace {
 
@@ -220,60 +221,27 @@ struct sayram_batch_s {
     SG_CUDA(cudaFuncSetAttribute(sg::k_bicg2<T, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, b1));
     SG_CUDA(cudaFuncSetAttribute(sg::k_resid<T, C, A, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, b2));
     SG_CUDA(cudaFuncSetAttribute(sg::k_polish<C, A, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, b2));
-    SG_CUDA(cudaFuncSetAttribute(sg::k_solve_coop<T, C, A, CH, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b2));
-    SG_CUDA(cudaFuncSetAttribute(sg::k_solve_coop<T, C, A, CH, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, b2));
     return SAYRAM_OK;
   }
-  // The cooperative solve (k_solve_coop) replaces the graph's refinement loops when every chunk
-  // gets a block of its own in one wave of co-resident blocks (a fixed instance list; the server's
-  // lanes set coop = 0). Returns its grid (negative: the 4-blocks-per-SM form), or 0 when the
-  // loops of separate kernels are used.
+  // Whole steps as one cooperative launch (k_team), for batches that fit the chip: every instance gets
+  // a team of blocks, or, with more instances than SMs, every block whole instances. Re-planned
+  // whenever the lists change; team_grid 0: the batch runs as separate kernels.
   int coop = 1;
-  template <typename T, typename C, typename A, int CH>
-  int coop_grid() {
-    if (!coop || nchunks < 1) return 0;
-    int can = 0;
-    if (cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !can) {
-      cudaGetLastError();
-      return 0;
-    }
-    int per_sm2 = 0, per_sm4 = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, sg::k_solve_coop<T, C, A, CH, 2>, sg::kThreads,
-                                                      smem_wide()) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm4, sg::k_solve_coop<T, C, A, CH, 4>, sg::kThreads,
-                                                      smem_wide()) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    if ((long long)nchunks <= (long long)per_sm2 * nsm) return nchunks;
-    if ((long long)nchunks <= (long long)per_sm4 * nsm) return -nchunks;
-    return 0;
-  }
-  template <typename T, typename C, typename A, int CH>
-  int launch_coop(int sgrid, const sg::Coef<C>& cfull, const sg::Coef<T>& ck, const sg::Kry<T>& kr) {
-    const int grid = sgrid < 0 ? -sgrid : sgrid;
-    sg::Common c2 = cm;
-    c2.use_cond = 2;
-    c2.guard_refine = opt.max_refine + 1;
-    c2.guard_iters = opt.max_iters + 1;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(sg::kThreads);
-    cfg.dynamicSmemBytes = smem_wide();
-    cfg.stream = stream;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (sgrid > 0)
-      SG_CUDA(cudaLaunchKernelEx(&cfg, sg::k_solve_coop<T, C, A, CH, 2>, c2, fl, cfull, ck, kr, opt.tol,
-                                 opt.inner_tol, opt.max_refine, opt.max_iters));
-    else
-      SG_CUDA(cudaLaunchKernelEx(&cfg, sg::k_solve_coop<T, C, A, CH, 4>, c2, fl, cfull, ck, kr, opt.tol,
-                                 opt.inner_tol, opt.max_refine, opt.max_iters));
-    return SAYRAM_OK;
-  }
+  int team_sms = 0;    // blocks the plan may use (0: one per SM)
+  int team_grid = 0;
+  bool team_chip = false;
+  size_t team_smem = 0;
+  int team_pmax = 4;
+  long long team_own = 0;
+  size_t team_limit[2] = {0, 0};  // shared memory a block may use: streaming, on chip (0: not asked yet)
+  sg::TeamShare* d_share = nullptr;
+  int* d_first = nullptr;
+  unsigned* d_bar = nullptr;
+  float* d_tmax = nullptr;
+  int* d_err = nullptr;
+  static constexpr int kTeamSteps = 32;
+  int plan_team();
+  int launch_team(int nsteps, int phases);
   // dispatch of the per-step sequence on precision and chunk size (graph: build it; else: run it)
   template <typename T, typename C, typename A>
   int run_chunked(const sg::Coef<C>& cf, const sg::Coef<T>& ck, const sg::Kry<T>& kr, bool as_graph, bool prefix) {
@@ -377,6 +345,7 @@ struct sayram_batch_s {
   int run_steps(int nsteps);
   int launch_steps(int nsteps);  // queue steps on the stream (no status read-back)
   int read_ctl();
+  int check_team();
   int finish_status();
   template <typename T, typename C, typename A, int CH>
   int step_once(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, const sg::Kry<T>& kr);
@@ -478,7 +447,12 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
   SG_ALLOC(d_wy, 2 * ycap);
   SG_ALLOC(d_dirv, std::max<long long>(dcap, 1));
   pstride = 8LL * chunks_cap;  // a chunk of 1024 cells holds 8 segments, the most of any chunk size
-  SG_ALLOC(d_part, sg::kPartQ * pstride);
+  SG_ALLOC(d_part, (long long)sg::kPartSets * sg::kPartQ * pstride);
+  SG_ALLOC(d_share, std::max(slots, nsm));
+  SG_ALLOC(d_first, nsm + 1);
+  SG_ALLOC(d_bar, (long long)slots * sg::kTeamBarStride);
+  SG_ALLOC(d_tmax, nsm);
+  SG_ALLOC(d_err, 1);
   SG_ALLOC(d_stage, stage_cap);
   cell_arrays.clear();
   double** geos[10] = {&geo.aAx, &geo.aBx, &geo.Sx, &geo.aAy, &geo.aBy, &geo.Sy, &geo.ukk, &geo.sdiag, &geo.G,
@@ -631,6 +605,144 @@ int sayram_batch_s::rebuild_lists() {
   cm.nchunks = nchunks;
   cm.ntiles = ntiles;
   cm.ninst = cap_slots;
+  return plan_team();
+}
+
+// Splits the enabled instances' reduction segments over the blocks of one cooperative launch: the
+// smallest number of segments per block with which the teams fit (whole instances, largest first,
+// when there are more instances than blocks), then the form that fits the shared memory -- on
+// chip, or with the vectors in global memory. No plan (team_grid = 0) when neither fits, or for
+// chunks of 4096 cells, whose segments are too coarse to split.
+int sayram_batch_s::plan_team() {
+  team_grid = 0;
+  if (!coop || chunk == 4096) return SAYRAM_OK;
+  std::vector<int> on;
+  long long total = 0;
+  int most = 0;
+  for (int b = 0; b < cap_slots; ++b)
+    if (hinst[b].enabled) {
+      on.push_back(b);
+      total += hinst[b].nseg;
+      most = std::max(most, hinst[b].nseg);
+    }
+  const int blocks = team_sms > 0 ? std::min(team_sms, nsm) : nsm, ni = (int)on.size();
+  if (ni == 0) return SAYRAM_OK;
+  std::vector<sg::TeamShare> share;
+  std::vector<int> first;
+  const int seg = sg::seg_cells(chunk);
+  long long per = 0;  // segments of the largest share
+  int pm = 4;
+  for (int b : on) pm = std::max(pm, hinst[b].pitch);
+  // the assembly's tile height: the one with the fewest rows (halo included) per block
+  auto tile_rows = [&](const InstDev& I, int nb) {
+    int best = sg::kTY;
+    long long cost = -1;
+    for (int ty = sg::kTY; ty >= 2; ty /= 2) {
+      const long long nt = (long long)I.ntx * ((I.ny + ty - 1) / ty), c = (nt + nb - 1) / nb * (ty + 2);
+      if (cost < 0 || c < cost) {
+        cost = c;
+        best = ty;
+      }
+    }
+    return best;
+  };
+  if (ni <= blocks) {
+    long long lo = std::max<long long>(1, (total + blocks - 1) / blocks), hi = most;
+    auto need = [&](long long q) {
+      long long k = 0;
+      for (int b : on) k += (hinst[b].nseg + q - 1) / q;
+      return k;
+    };
+    while (lo < hi) {
+      const long long mid = (lo + hi) / 2;
+      if (need(mid) <= blocks) hi = mid;
+      else lo = mid + 1;
+    }
+    const long long q = std::max<long long>(lo, 1);
+    for (int b : on) {
+      const InstDev& I = hinst[b];
+      const int nb = (int)((I.nseg + q - 1) / q), ty = tile_rows(I, nb);
+      for (int r = 0; r < nb; ++r) {
+        const int s0 = (int)((long long)I.nseg * r / nb), s1 = (int)((long long)I.nseg * (r + 1) / nb);
+        first.push_back((int)share.size());
+        share.push_back({b, r, nb, s0, s1, ty});
+        per = std::max<long long>(per, s1 - s0);
+      }
+    }
+    first.push_back((int)share.size());
+  } else {
+    std::vector<int> order(on);
+    std::sort(order.begin(), order.end(), [&](int a, int b) {
+      return hinst[a].nseg != hinst[b].nseg ? hinst[a].nseg > hinst[b].nseg : a < b;
+    });
+    std::vector<std::vector<int>> bin(blocks);
+    std::vector<long long> load(blocks, 0);
+    for (int b : order) {
+      const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      bin[k].push_back(b);
+      load[k] += hinst[b].nseg;
+    }
+    for (auto& v : bin) {
+      first.push_back((int)share.size());
+      for (int b : v) share.push_back({b, 0, 1, 0, hinst[b].nseg, sg::kTY});
+    }
+    first.push_back((int)share.size());
+    per = most;
+  }
+  const size_t ts = mixed ? 4 : 8;
+  const size_t tile = dwm ? sizeof(sg::AsmTile<sg::DWA>) : sizeof(sg::AsmTile<sg::F64A>);
+  const long long own = per * seg;
+  if (!team_limit[1]) {
+    SG_CUDA(cudaSetDevice(dev));
+    int can = 0;
+    SG_CUDA(cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, dev));
+    if (!can) {
+      coop = 0;
+      return SAYRAM_OK;
+    }
+    for (int c = 0; c < 2; ++c)
+      team_limit[c] = dwm ? sg::team_smem_limit_dw(c) : mixed ? sg::team_smem_limit_mixed(c) : sg::team_smem_limit_f64(c);
+    if (!team_limit[0] || !team_limit[1]) {
+      coop = 0;
+      return SAYRAM_OK;
+    }
+  }
+  bool chip = own <= sg::team_chip_cells(ts) && sg::team_smem(ts, true, own, pm, tile) <= team_limit[1];
+  if (!chip && sg::team_smem(ts, false, own, pm, tile) > team_limit[0]) return SAYRAM_OK;
+  SG_CUDA(cudaMemcpyAsync(d_share, share.data(), sizeof(sg::TeamShare) * share.size(), cudaMemcpyHostToDevice, stream));
+  SG_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, stream));
+  SG_CUDA(cudaStreamSynchronize(stream));
+  team_grid = (int)first.size() - 1;
+  team_chip = chip;
+  team_own = own;
+  team_pmax = pm;
+  team_smem = sg::team_smem(ts, chip, own, pm, tile);
+  return SAYRAM_OK;
+}
+
+int sayram_batch_s::launch_team(int nsteps, int phases) {
+  sg::TeamArgs ta{};
+  ta.share = d_share;
+  ta.first = d_first;
+  ta.bar = d_bar;
+  ta.tmax = d_tmax;
+  ta.err = d_err;
+  ta.tol = opt.tol;
+  ta.inner_tol = opt.inner_tol;
+  ta.max_refine = opt.max_refine;
+  ta.max_iters = opt.max_iters;
+  ta.nsteps = nsteps;
+  ta.phases = phases;
+  ta.seg = sg::seg_cells(chunk);
+  ta.own_cap = (int)team_own;
+  ta.pmax = team_pmax;
+  sg::TeamLaunch l{team_grid, team_smem, team_chip, stream};
+  if (dwm)
+    SG_CUDA(sg::team_launch_dw(l, cm, geo, fl, c32, k32, ta));
+  else if (mixed)
+    SG_CUDA(sg::team_launch_mixed(l, cm, geo, fl, c32, k32, ta));
+  else
+    SG_CUDA(sg::team_launch_f64(l, cm, geo, fl, c64, k64, ta));
   return SAYRAM_OK;
 }
 
@@ -729,18 +841,7 @@ int sayram_batch_s::step_once(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, c
   SG_CUDA(cudaMemsetAsync(d_ctl, 0, 2 * sizeof(int), stream));
   launch("begin", [&] { k_begin<<<(n + 255) / 256, 256, 0, stream>>>(cm); });
   launch("assemble", [&] { k_assemble<C, A><<<gt, kAsmThreads, 0, stream>>>(cm, geo, fl, cfull, 0, -1); });
-  int cgrid = coop_grid<T, C, A, CH>();
-  if (cgrid != 0) {
-    int crc = SAYRAM_OK;
-    launch("solve_coop", [&] { crc = launch_coop<T, C, A, CH>(cgrid, cfull, ck, kr); });
-    if (crc) {  // refused: the loops of separate kernels from now on
-      cudaGetLastError();
-      g_err.clear();
-      coop = 0;
-      cgrid = 0;
-    }
-  }
-  for (int o = 0; cgrid == 0 && o < opt.max_refine; ++o) {
+  for (int o = 0; o < opt.max_refine; ++o) {
     launch("resid", [&] {
       k_resid<T, C, A, CH><<<gs, kThreads, smem_wide(), stream>>>(cm, fl, cfull, kr, opt.tol, opt.inner_tol, opt.max_refine);
     });
@@ -802,39 +903,6 @@ int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck,
   SG_CUDA(cudaGraphCreate(&g, 0));
   (prefix ? graph : graph_solve) = g;
   int rc;
-  const int cgrid = coop_grid<T, C, A, CH>();
-  if (cgrid != 0) {
-    // [memset, begin, assemble,] the cooperative solve[, polish]
-    SG_CUDA(cudaStreamBeginCaptureToGraph(stream, g, nullptr, nullptr, 0, mode));
-    if (prefix) {
-      cudaMemsetAsync(d_ctl, 0, 2 * sizeof(int), stream);
-      k_begin<<<(n + 255) / 256, 256, 0, stream>>>(cm);
-      k_assemble<C, A><<<gt, kAsmThreads, 0, stream>>>(cm, geo, fl, cfull, 0, -1);
-    }
-    // a capture that refuses the cooperative launch or does not keep it cooperative falls back
-    // to the loops of separate kernels
-    bool coop_node = launch_coop<T, C, A, CH>(cgrid, cfull, ck, kr) == SAYRAM_OK;
-    cudaGraphNode_t cnode = nullptr;
-    if (coop_node) coop_node = last_captured(&cnode) == SAYRAM_OK;
-    if (coop_node) {
-      cudaLaunchAttributeValue cv = {};
-      coop_node = cudaGraphKernelNodeGetAttribute(cnode, cudaLaunchAttributeCooperative, &cv) == cudaSuccess &&
-                  cv.cooperative;
-    }
-    if (coop_node && prefix) k_polish<C, A, CH><<<gs, kThreads, smem_wide(), stream>>>(cm, fl, cfull, 0, -1);
-    cudaGraph_t gc = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(stream, &gc);
-    if (!coop_node || ce != cudaSuccess) {
-      cudaGetLastError();
-      g_err.clear();
-      cudaGraphDestroy(g);
-      (prefix ? graph : graph_solve) = nullptr;
-      coop = 0;
-      return build_graph<T, C, A, CH>(cfull, ck, kr, prefix);
-    }
-    SG_CUDA(cudaGraphInstantiate(prefix ? &gexec : &gexec_solve, g, 0));
-    return SAYRAM_OK;
-  }
   cudaGraphConditionalHandle hout, hin;
   SG_CUDA(cudaGraphConditionalHandleCreate(&hout, g, 1, cudaGraphCondAssignDefault));
   Common c2 = cm;
@@ -903,6 +971,30 @@ int sayram_batch_s::run_steps(int nsteps) {
 int sayram_batch_s::launch_steps(int nsteps) {
   if (nsteps < 0) return fail(SAYRAM_ERR_ARG, "nsteps must be >= 0");
   SG_CUDA(cudaSetDevice(dev));
+  if (team_grid > 0) {
+    if (timing) {  // the phases of a step one by one
+      for (int s = 0; s < nsteps; ++s) {
+        int rc = SAYRAM_OK;
+        launch("begin", [&] { sg::k_begin<<<(n + 255) / 256, 256, 0, stream>>>(cm); });
+        const std::pair<const char*, int> ph[3] = {
+            {"assemble", sg::TEAM_ASSEMBLE}, {"solve_coop", sg::TEAM_SOLVE}, {"polish", sg::TEAM_POLISH}};
+        for (auto& p : ph) {
+          int r2 = SAYRAM_OK;
+          launch(p.first, [&] { r2 = launch_team(1, p.second); });
+          if (r2) rc = r2;
+        }
+        if (rc) return rc;
+      }
+      return SAYRAM_OK;
+    }
+    for (int s = 0; s < nsteps;) {  // a launch stays well below a second
+      const int k = std::min(nsteps - s, kTeamSteps);
+      int rc = launch_team(k, sg::TEAM_STEP);
+      if (rc) return rc;
+      s += k;
+    }
+    return SAYRAM_OK;
+  }
   const bool use_graph = opt.use_graph && !timing;
   if (use_graph && !gexec) {
     int rc = run_mode(true);
@@ -1092,10 +1184,24 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
   return SAYRAM_OK;
 }
 
+// Waits for the stream; an error when a barrier of k_team gave up (its counters are cleared, so the
+// batch stays usable, but the step is lost).
+int sayram_batch_s::check_team() {
+  int err = 0;
+  if (team_grid > 0) SG_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  SG_CUDA(cudaStreamSynchronize(stream));
+  if (!err) return SAYRAM_OK;
+  SG_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
+  SG_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(unsigned) * (size_t)cap_slots * sg::kTeamBarStride, stream));
+  SG_CUDA(cudaStreamSynchronize(stream));
+  return fail(SAYRAM_ERR_TIMEOUT, "a device barrier of the cooperative step gave up waiting");
+}
+
 int sayram_batch_s::finish_status() {
   std::vector<InstState> hs(n);
   SG_CUDA(cudaMemcpyAsync(hs.data(), d_st, sizeof(InstState) * n, cudaMemcpyDeviceToHost, stream));
-  SG_CUDA(cudaStreamSynchronize(stream));
+  int rc = check_team();
+  if (rc) return rc;
   int worst = SAYRAM_OK;
   for (int b = 0; b < n; ++b) {
     if (!hinst[b].enabled || hs[b].steps == 0) continue;
@@ -1246,7 +1352,7 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
   // An instance whose state changed restarts its extrapolation history; one given back its own
   // current state (a host round trip) keeps it (k_field_in compares bit for bit).
   int rc = SAYRAM_OK;
-  const bool split = b->opt.use_graph && !b->timing && nsteps >= 1 && np >= 2 && (f_in || f_out);
+  const bool split = b->team_grid == 0 && b->opt.use_graph && !b->timing && nsteps >= 1 && np >= 2 && (f_in || f_out);
   if (split) {
     // Graph stepping with host buffers: the first step's assembly runs piece by piece behind the
     // copies in (each piece's tiles as soon as its cells have landed), and the last step's
@@ -1509,7 +1615,7 @@ int sayram_batch_set_coop(sayram_batch b, int on) {
   SG_CUDA(cudaStreamSynchronize(b->stream));
   b->coop = on ? 1 : 0;
   b->drop_graph();
-  return SAYRAM_OK;
+  return b->plan_team();
 }
 
 int sayram_batch_set_launch_shape(sayram_batch b, int chunk, int blocks_per_sm) {
@@ -1801,7 +1907,8 @@ struct ServerLane {
                               cudaMemcpyDeviceToHost, eng.stream));
       SG_CUDA(cudaMemcpyAsync(&sts[q], eng.d_st + fin[q], sizeof(InstState), cudaMemcpyDeviceToHost, eng.stream));
     }
-    SG_CUDA(cudaStreamSynchronize(eng.stream));
+    int trc = eng.check_team();  // waits for the copies too
+    if (trc) return trc;
     const double t1 = now_seconds();
     info.busy_seconds += t1 - t_begin;
     info.collect_seconds += t1 - ts;
@@ -1843,9 +1950,6 @@ struct ServerLane {
   int create(const sayram_server_config& c, const sayram_options* opt) {
     cfg = c;
     sayram_batch_s& e = eng;
-    // the lane's step graph outlives changes of its instance list; the cooperative solve's grid
-    // is sized to the list it was built for
-    e.coop = 0;
     int rc = e.set_options(opt);
     if (!rc) rc = e.init_device();
     if (rc) return rc;
@@ -1856,9 +1960,9 @@ struct ServerLane {
     const double per_cell = (double)sayram_instance_bytes(64, 64, e.opt.precision) /
                             (double)region_cells(64, 64);  // bytes per arena cell (all arrays)
     const double avail = c.hbm_budget_bytes - table_bytes - stage_bytes - 64.0 * 1048576.0;
-    // work lists and partial sums beside the cells: a chunk index, a tile index and kPartQ * 8 sums of
-    // 8 bytes per 1024 cells
-    const long long cells = (long long)(avail / (per_cell + 4.0 / 1024 * 2 + 8.0 * 8 * sg::kPartQ / 1024));
+    // work lists and partial sums beside the cells: a chunk index, a tile index and two sets of kPartQ * 8
+    // sums of 8 bytes per 1024 cells
+    const long long cells = (long long)(avail / (per_cell + 4.0 / 1024 * 2 + 8.0 * 8 * sg::kPartSets * sg::kPartQ / 1024));
     if (cells < region_cells(1, 1) + 64) return fail(SAYRAM_ERR_BUDGET, "HBM budget too small for any instance");
     const long long side_tiles = (long long)c.max_slots * (c.max_side / sg::kTX + c.max_side / sg::kTY + 2);
     const int chunks_cap = (int)std::min<long long>(cells / 1024 + c.max_slots + 1, 1LL << 30);
@@ -1968,6 +2072,11 @@ int sayram_server_create(const sayram_server_config* cfg, const sayram_options* 
       L.reset();
       s.reset();
       return fail(rc, m);
+    }
+    // two lanes step side by side: each lane's cooperative steps take its share of the SMs
+    if (nl == 2) {
+      const int small = std::min(L->eng.nsm - 1, std::max(1, (int)std::lround(frac * L->eng.nsm)));
+      L->eng.team_sms = k == 0 ? small : L->eng.nsm - small;
     }
     s->lanes.push_back(std::move(L));
   }
@@ -2198,7 +2307,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   double* d_wy = lay.take<double>(2 * (ny + 1));
   double* d_dirv = lay.take<double>(doff > 0 ? doff : 1);
   const long long pstride = 8LL * kNoAllocMaxChunks;
-  double* d_part = lay.take<double>(kPartQ * pstride);
+  double* d_part = lay.take<double>(kPartSets * kPartQ * pstride);
   unsigned char* tables_end = lay.cur;
   if (!d_part || tables_end > base + kNoAllocTableBytes) return fail(SAYRAM_ERR_ARG, "tables exceed the scratch");
   lay.cur = base + kNoAllocTableBytes;

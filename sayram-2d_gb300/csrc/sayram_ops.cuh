@@ -17,8 +17,6 @@
 // values) hold 8 bytes per entry in both: one double, or one (hi, lo) float pair.
 #pragma once
 
-#include <cooperative_groups.h>
-
 #include "dword.cuh"
 #include "sayram_kernels.cuh"
 
@@ -50,7 +48,7 @@ struct Common {
   const int* dyn;
   int pmax;  // largest row pitch of any instance (shared-memory halo of the SpMV kernels)
   // device-side loops of the per-step CUDA graph (use_cond = 0: the host drives the loops; 1: the
-  // graph's WHILE nodes; 2: the cooperative solve kernel)
+  // graph's WHILE nodes)
   unsigned long long h_outer, h_inner;  // cudaGraphConditionalHandle of the two WHILE nodes
   int use_cond;
   int guard_refine, guard_iters;  // hard caps on loop trips, whatever the bookkeeping says
@@ -86,13 +84,8 @@ __device__ __forceinline__ void loop_epilogue(const Common& cm, int which) {
         const unsigned li = atomicAdd(&cm.ctl->inner_loops, 1u) + 1u;
         go_i = (nin > 0 && li < (unsigned)cm.guard_iters) ? 1u : 0u;
       }
-      if (cm.use_cond == 1) {
-        if (which == 0) cudaGraphSetConditional(cm.h_outer, go_o);
-        cudaGraphSetConditional(cm.h_inner, go_i);
-      } else {  // read by every block of the cooperative solve after its next grid barrier
-        if (which == 0) atomicExch(&cm.ctl->go_outer, (int)go_o);
-        atomicExch(&cm.ctl->go_inner, (int)go_i);
-      }
+      if (which == 0) cudaGraphSetConditional(cm.h_outer, go_o);
+      cudaGraphSetConditional(cm.h_inner, go_i);
       atomicExch(&cm.ctl->kdone[which], 0u);
     }
   }
@@ -124,7 +117,8 @@ struct Kry {
   T *rh, *t, *x;
   T *r[2], *p[2], *v[2];  // iteration i uses [i & 1]
 };
-constexpr int kPartQ = 5;  // most sums any pass forms at once
+constexpr int kPartQ = 5;     // most sums any pass forms at once
+constexpr int kPartSets = 2;  // sets of partial sums (k_team alternates; the per-pass kernels use the first)
 
 // ------------------------------------------------------------------------------ arithmetic
 struct F64A {
@@ -542,7 +536,7 @@ __global__ void k_field_out(Common cm, double* dst, const double* src, int t0, i
 }
 
 // ------------------------------------------------------------------------------ step control
-__global__ void k_begin(Common cm) {
+static __global__ void k_begin(Common cm) {
   count_launch(cm.ctl);
   for (int b = blockIdx.x * blockDim.x + threadIdx.x, ni_ = n_inst(cm); b < ni_; b += gridDim.x * blockDim.x) {
     InstState& s = cm.st[b];
@@ -622,229 +616,247 @@ __device__ __forceinline__ void dirichlet_face(typename A::V aK, typename A::V S
   *Bm = A::max0(aK);
 }
 
-// One tile of kTX x kTY cells per iteration; vertices and faces are computed once per tile
-// (plus a one-cell halo), in shared memory.
-// Tiles [t0, t1) of the tile list (t1 < 0: all of them).
+// Shared memory of one tile of kTX x (up to) kTY cells: vertices and faces are computed once per
+// tile, plus a one-cell halo.
+template <typename A>
+struct AsmTile {
+  using V = typename A::V;
+  static constexpr int HX = kTX + 2, HY = kTY + 2, VX = kTX + 1, VY = kTY + 1;
+  V fS[HY][HX];
+  V iS[HY][HX];
+  V vS[VY][VX];
+  // x-faces: outflow to the left / right cell; y-faces: to the cell below / above. On a Dirichlet
+  // side the slot of the missing outside cell holds the face's RHS part instead.
+  V xL[kTY][VX], xR[kTY][VX];
+  V yB[VY][kTX], yT[VY][kTX];
+  V hS[VY][2];  // the tile's vertex rows: bilinear weights (wB, wT), Solver.cc:333-336
+};
+
+// Assembles the tile of kTX x ty cells at (i0, j0) of instance I by a block of NT threads; returns
+// this thread's max of the right-hand side. yc: the current y buffer; has_g: the idle one holds the
+// extrapolated start.
+template <typename C, typename A, int NT>
+__device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const Geo& geo, const Fields& fl,
+                                          const Coef<C>& co, const InstDev& I, int i0, int j0, const int ty,
+                                          bool has_g, int yc) {
+  using V = typename A::V;
+  constexpr int HX = AsmTile<A>::HX, VX = AsmTile<A>::VX;
+  const int HY = ty + 2, VY = ty + 1;
+  // f interpolated along each halo row at each vertex column (steps 1-2 only: shares the x-face
+  // arrays' storage, which step 3 fills after a barrier)
+  static_assert(AsmTile<A>::HY * VX <= 2 * kTY * VX, "row interpolations must fit in the x-face arrays");
+  V(*const rS)[VX] = reinterpret_cast<V(*)[VX]>(&S.xL[0][0]);
+  // step 1's thread layout: kRowT threads own one vertex column each and walk its halo rows,
+  // kRowS rows apart
+  constexpr int kRowS = NT / VX, kRowT = VX * kRowS;
+  static_assert(kRowT < NT, "step 1 layout");
+  // the y-faces start at another warp than the x-faces, so that what is left over of each after whole
+  // rounds of the block falls on different warps
+  const int tid = threadIdx.x, tid2 = (threadIdx.x + NT / 2) & (NT - 1);
+  const V zero = A::k(0.0);
+  const int nx = I.nx, ny = I.ny, P = I.pitch;
+  // 32-bit cell indices: every batch holds fewer than 2^31 cells (checked at allocation), and an
+  // int index makes each address one wide multiply-add
+  const int base = (int)I.base;
+  const double* gp = sel2(fl.y64, yc ^ 1);
+  // the per-cell data of step 4 is only needed after three barriers: start its trip to L2 now
+#pragma unroll
+  for (int q = tid; q < kTX * ty; q += NT) {
+    const int i = i0 + (q % kTX), j = j0 + (q / kTX);
+    if (i < nx && j < ny) {
+      const int K = base + j * P + i;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(geo.sdiag + K));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(geo.ukk + K));
+      if (has_g) asm volatile("prefetch.global.L2 [%0];" ::"l"(gp + K));
+    }
+  }
+  // 1) per vertex column Iv (threads below kRowT) and halo row j: f and 1/(f+eps) of the cell left
+  //    of the column, and r = wL f_left + wR f_right, f interpolated along the row at the column
+  //    (Solver.cc:333-336; a boundary column takes its adjacent cell's f). The remaining threads
+  //    take the right halo column and the vertex-row weights.
+  if (tid < kRowT) {
+    const int vx = tid % VX, Iv = i0 + vx;
+    const bool xin = Iv > 0 && Iv < nx;
+    const V wL = xin ? A::ld(cm.wx, 2 * (I.xe + Iv)) : zero;
+    const V wR = xin ? A::ld(cm.wx, 2 * (I.xe + Iv) + 1) : zero;
+    for (int hy = tid / VX; hy < HY; hy += kRowS) {
+      const int j = j0 + hy - 1;
+      V fa = zero, ia = zero, r = zero;
+      if (j >= 0 && j < ny && Iv <= nx) {
+        const int K = base + j * P + Iv;  // the cell right of the column
+        V fb = zero;
+        if (Iv > 0) {
+          fa = A::ld(fl.f, K - 1);
+          ia = A::rcp(A::addp(fa, A::k(kEps)));
+        }
+        if (Iv < nx) fb = A::ld(fl.f, K);
+        r = xin ? A::fmap(wL, fa, A::mul(wR, fb)) : (Iv == 0 ? fb : fa);
+      }
+      S.fS[hy][vx] = fa;
+      S.iS[hy][vx] = ia;
+      rS[hy][vx] = r;
+    }
+  } else {
+    for (int q = tid - kRowT; q < HY + VY; q += NT - kRowT) {
+      if (q < HY) {
+        const int i = i0 + kTX, j = j0 + q - 1;
+        V fv = zero, iv = zero;
+        if (i < nx && j >= 0 && j < ny) {
+          fv = A::ld(fl.f, base + j * P + i);
+          iv = A::rcp(A::addp(fv, A::k(kEps)));
+        }
+        S.fS[q][HX - 1] = fv;
+        S.iS[q][HX - 1] = iv;
+      } else {
+        const int vy = q - HY, Jv = j0 + vy;
+        const bool in = Jv > 0 && Jv < ny;
+        S.hS[vy][0] = in ? A::ld(cm.wy, 2 * (I.ye + Jv)) : zero;
+        S.hS[vy][1] = in ? A::ld(cm.wy, 2 * (I.ye + Jv) + 1) : zero;
+      }
+    }
+  }
+  __syncthreads();
+  // 2) vertex values (Solver.cc:299-422): corners copy, interior bilinear, boundary edges
+  //    linear, then Dirichlet overrides with XMIN < XMAX < YMIN < YMAX precedence. The bilinear
+  //    value wB (wL f00 + wR f10) + wT (wL f01 + wR f11) is formed from the two row
+  //    interpolations of step 1 with the same operations in the same order.
+  for (int q = tid; q < VX * VY; q += NT) {
+    const int vx = q % VX, vy = q / VX;
+    const int Iv = i0 + vx, Jv = j0 + vy;
+    if (Iv > nx || Jv > ny) continue;
+    V val;
+    if (Jv == ny && I.bc[YMAX] == DIRICHLET) val = A::ld(cm.dirv, I.dir[YMAX] + Iv);
+    else if (Jv == 0 && I.bc[YMIN] == DIRICHLET) val = A::ld(cm.dirv, I.dir[YMIN] + Iv);
+    else if (Iv == nx && I.bc[XMAX] == DIRICHLET) val = A::ld(cm.dirv, I.dir[XMAX] + Jv);
+    else if (Iv == 0 && I.bc[XMIN] == DIRICHLET) val = A::ld(cm.dirv, I.dir[XMIN] + Jv);
+    else {
+      // cell rows below / above vertex row Jv, clamped to the domain at the edges
+      const int cj0 = Jv > 0 ? Jv - 1 : 0, cj1 = Jv < ny ? Jv : ny - 1;
+      const V r0 = rS[cj0 - j0 + 1][vx];
+      if (Jv > 0 && Jv < ny) {  // interior and vertical boundary edges: linear in y
+        const V r1 = rS[cj1 - j0 + 1][vx];
+        val = A::fmap(S.hS[vy][0], r0, A::mul(S.hS[vy][1], r1));
+      } else {
+        val = r0;  // horizontal boundary edges (linear in x) and corners
+      }
+    }
+    S.vS[vy][vx] = val;
+  }
+  __syncthreads();
+  // 3a) x-faces (vertex column Iv between cells Iv-1 and Iv)
+  for (int q = tid; q < ty * VX; q += NT) {
+    const int vx = q % VX, ry = q / VX;
+    const int Iv = i0 + vx, j = j0 + ry;
+    V aL = zero, aR = zero, bm = zero;
+    if (j < ny && Iv <= nx) {
+      const V vLo = S.vS[ry][vx], vHi = S.vS[ry + 1][vx];  // vertices (Iv, j), (Iv, j+1)
+      if (Iv > 0 && Iv < nx) {
+        const int K = base + j * P + Iv, L = K - 1;
+        // K's XNEG edge: A=(Iv, j+1), B=(Iv, j); L's XPOS edge: A=(Iv, j), B=(Iv, j+1)
+        const V aK = A::dot2(A::ld(geo.aAx, K), vHi, A::ld(geo.aBx, K), vLo);
+        const V aLs = A::dot2(A::ld(geo.aAx, L), vLo, A::ld(geo.aBx, L), vHi);
+        inner_face<A>(aK, A::ld(geo.Sx, K), S.iS[ry + 1][vx + 1], aLs, A::ld(geo.Sx, L), S.iS[ry + 1][vx], &aR, &aL);
+      } else if (Iv == 0 && I.bc[XMIN] == DIRICHLET) {
+        const int K = base + j * P;
+        dirichlet_face<A>(A::dot2(A::ld(geo.aAx, K), vHi, A::ld(geo.aBx, K), vLo), A::ld(geo.Sx, K),
+                          S.iS[ry + 1][vx + 1], &aR, &bm);
+      } else if (Iv == nx && I.bc[XMAX] == DIRICHLET) {
+        const int K = base + j * P + nx - 1;  // XPOS edge: A=(nx, j), B=(nx, j+1)
+        dirichlet_face<A>(A::dot2(A::ld(geo.aAx, K), vLo, A::ld(geo.aBx, K), vHi), A::ld(geo.Sx, K),
+                          S.iS[ry + 1][vx], &aL, &bm);
+      }
+    }
+    S.xL[ry][vx] = Iv == 0 ? bm : aL;
+    S.xR[ry][vx] = Iv == nx ? bm : aR;
+  }
+  // 3b) y-faces (vertex row Jv between cells Jv-1 and Jv)
+  for (int q = tid2; q < VY * kTX; q += NT) {
+    const int cx = q % kTX, vy = q / kTX;
+    const int i = i0 + cx, Jv = j0 + vy;
+    V aB = zero, aT = zero, bm = zero;
+    if (i < nx && Jv <= ny) {
+      const V vLe = S.vS[vy][cx], vRi = S.vS[vy][cx + 1];  // vertices (i, Jv), (i+1, Jv)
+      if (Jv > 0 && Jv < ny) {
+        const int K = base + Jv * P + i, L = K - P;
+        // K's YNEG edge: A=(i, Jv), B=(i+1, Jv); L's YPOS edge: A=(i+1, Jv), B=(i, Jv)
+        const V aK = A::dot2(A::ld(geo.aAy, K), vLe, A::ld(geo.aBy, K), vRi);
+        const V aLs = A::dot2(A::ld(geo.aAy, L), vRi, A::ld(geo.aBy, L), vLe);
+        inner_face<A>(aK, A::ld(geo.Sy, K), S.iS[vy + 1][cx + 1], aLs, A::ld(geo.Sy, L), S.iS[vy][cx + 1], &aT, &aB);
+      } else if (Jv == 0 && I.bc[YMIN] == DIRICHLET) {
+        const int K = base + i;
+        dirichlet_face<A>(A::dot2(A::ld(geo.aAy, K), vLe, A::ld(geo.aBy, K), vRi), A::ld(geo.Sy, K),
+                          S.iS[vy + 1][cx + 1], &aT, &bm);
+      } else if (Jv == ny && I.bc[YMAX] == DIRICHLET) {
+        const int K = base + (ny - 1) * P + i;  // YPOS edge: A=(i+1,ny), B=(i,ny)
+        dirichlet_face<A>(A::dot2(A::ld(geo.aAy, K), vRi, A::ld(geo.aBy, K), vLe), A::ld(geo.Sy, K),
+                          S.iS[vy][cx + 1], &aB, &bm);
+      }
+    }
+    S.yB[vy][cx] = Jv == 0 ? bm : aB;
+    S.yT[vy][cx] = Jv == ny ? bm : aT;
+  }
+  __syncthreads();
+  // 4) per cell: diagonal in the reference's triplet order, RHS, scaling, scatter
+  float rmax = 0.0f;
+#pragma unroll
+  for (int q = tid; q < kTX * ty; q += NT) {
+    const int cx = q % kTX, cy = q / kTX;
+    const int i = i0 + cx, j = j0 + cy;
+    if (i >= nx || j >= ny) continue;
+    const int K = base + j * P + i;
+    const V Aw = S.xR[cy][cx], Ae = S.xL[cy][cx + 1], As = S.yT[cy][cx], An = S.yB[cy + 1][cx];
+    const bool wIn = i > 0, eIn = i < nx - 1, sIn = j > 0, nIn = j < ny - 1;
+    // every term below is >= 0; a sum that is still zero takes its first term as it is (0 + x
+    // = x), which spares an interior cell three double-word additions
+    V D = wIn ? Aw : zero, Rv = zero, dir = zero;
+    bool has_dir = false;
+    if (eIn) D = A::addp(D, Ae);
+    if (sIn) D = A::addp(D, As);
+    if (nIn) D = A::addp(D, An);
+    if (!wIn && I.bc[XMIN] == DIRICHLET) { D = A::addp(D, Aw); dir = A::addp(dir, Aw); Rv = A::addp(Rv, S.xL[cy][cx]); has_dir = true; }
+    if (!eIn && I.bc[XMAX] == DIRICHLET) { D = A::addp(D, Ae); dir = A::addp(dir, Ae); Rv = A::addp(Rv, S.xR[cy][cx + 1]); has_dir = true; }
+    if (!sIn && I.bc[YMIN] == DIRICHLET) { D = A::addp(D, As); dir = A::addp(dir, As); Rv = A::addp(Rv, S.yB[cy][cx]); has_dir = true; }
+    if (!nIn && I.bc[YMAX] == DIRICHLET) { D = A::addp(D, An); dir = A::addp(dir, An); Rv = A::addp(Rv, S.yT[cy + 1][cx]); has_dir = true; }
+    const V sd = A::ld(geo.sdiag, K);
+    D = A::addp(D, sd);
+    const V fK = S.fS[cy + 1][cx + 1];
+    const V ukk = A::ld(geo.ukk, K);
+    Rv = has_dir ? A::fmap(ukk, fK, Rv) : A::fma0(ukk, fK);
+    rmax = fmaxf(rmax, fabsf(A::f32(Rv)));
+    const V inv = A::rcp(D);
+    A::st(fl.invD, K, inv);
+    A::st(fl.R, K, Rv);
+    A::st(fl.colsum, K, has_dir ? A::addp(sd, dir) : sd);
+    // start the solve from D g, g the loss-compensated polynomial extrapolation in time the
+    // last polish formed (only the starting point of the iteration; the converged answer does
+    // not depend on it)
+    A::st(sel2(fl.y64, yc), K, A::mul(D, has_g ? A::ld(gp, K) : fK));
+    if (wIn) AsmOut<C, A>::put(co, 1, K - 1, A::mul(Aw, inv));  // row K-1, east entry
+    if (eIn) AsmOut<C, A>::put(co, 0, K + 1, A::mul(Ae, inv));  // row K+1, west entry
+    if (sIn) AsmOut<C, A>::put(co, 3, K - P, A::mul(As, inv));  // row K-P, north entry
+    if (nIn) AsmOut<C, A>::put(co, 2, K + P, A::mul(An, inv));  // row K+P, south entry
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+  return rmax;
+}
+
+// One tile of kTX x kTY cells per iteration. Tiles [t0, t1) of the tile list (t1 < 0: all of them).
 template <typename C, typename A>
 __global__ void __launch_bounds__(kAsmThreads, A::kAsmBlocks) k_assemble(Common cm, Geo geo, Fields fl, Coef<C> co,
                                                                        int t0, int t1) {
-  using V = typename A::V;
   count_launch(cm.ctl);
-  constexpr int HX = kTX + 2, HY = kTY + 2, VX = kTX + 1, VY = kTY + 1;
-  __shared__ V fS[HY][HX];
-  __shared__ V iS[HY][HX];
-  __shared__ V vS[VY][VX];
-  // x-faces: outflow to the left / right cell; y-faces: to the cell below / above. On a Dirichlet
-  // side the slot of the missing outside cell holds the face's RHS part instead.
-  __shared__ V xLR[2][kTY][VX];
-  V(*const xL)[VX] = xLR[0];
-  V(*const xR)[VX] = xLR[1];
-  __shared__ V yB[VY][kTX], yT[VY][kTX];
-  __shared__ V hS[VY][2];  // the tile's vertex rows: bilinear weights (wB, wT), Solver.cc:333-336
-  // f interpolated along each halo row at each vertex column (steps 1-2 only: shares the face
-  // arrays' storage, which step 3 fills after a barrier)
-  static_assert(HY * VX <= 2 * kTY * VX, "row interpolations must fit in the x-face arrays");
-  V(*const rS)[VX] = reinterpret_cast<V(*)[VX]>(&xLR[0][0][0]);
-  // step 1's thread layout: kRowT threads own one vertex column each and walk its halo rows,
-  // kRowS rows apart
-  constexpr int kRowS = 7, kRowT = VX * kRowS;
-  static_assert(kRowT < kAsmThreads && 3 * kRowS >= HY, "step 1 layout");
-  const V zero = A::k(0.0);
+  __shared__ AsmTile<A> S;
   const int nt_ = t1 < 0 ? n_tiles(cm) : t1;
   for (int t = t0 + blockIdx.x; t < nt_; t += gridDim.x) {
     const int b = cm.tile_inst[t];
     const InstDev I = cm.inst[b];
     if (!I.enabled) continue;  // uniform in the block
     const int lt = t - I.tile0;
-    const int i0 = (lt % I.ntx) * kTX, j0 = (lt / I.ntx) * kTY;
-    const int nx = I.nx, ny = I.ny, P = I.pitch;
-    // 32-bit cell indices: every batch holds fewer than 2^31 cells (checked at allocation), and an
-    // int index makes each address one wide multiply-add
-    const int base = (int)I.base;
     // the extrapolated start g the last polish left in the idle y buffer (none before the first
     // step or after the state was replaced: then y0 = D f)
-    const bool has_g = cm.st[b].nhist > 0;
-    const int yc = cm.st[b].ycur;
-    const double* gp = sel2(fl.y64, yc ^ 1);
-    // the per-cell data of step 4 is only needed after three barriers: start its trip to L2 now
-#pragma unroll
-    for (int q = threadIdx.x; q < kTX * kTY; q += kAsmThreads) {
-      const int i = i0 + (q % kTX), j = j0 + (q / kTX);
-      if (i < nx && j < ny) {
-        const int K = base + j * P + i;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(geo.sdiag + K));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(geo.ukk + K));
-        if (has_g) asm volatile("prefetch.global.L2 [%0];" ::"l"(gp + K));
-      }
-    }
-    // 1) per vertex column Iv (threads below kRowT) and halo row j: f and 1/(f+eps) of the cell left
-    //    of the column, and r = wL f_left + wR f_right, f interpolated along the row at the column
-    //    (Solver.cc:333-336; a boundary column takes its adjacent cell's f). The remaining threads
-    //    take the right halo column and the vertex-row weights.
-    if (threadIdx.x < kRowT) {
-      const int vx = threadIdx.x % VX, Iv = i0 + vx;
-      const bool xin = Iv > 0 && Iv < nx;
-      const V wL = xin ? A::ld(cm.wx, 2 * (I.xe + Iv)) : zero;
-      const V wR = xin ? A::ld(cm.wx, 2 * (I.xe + Iv) + 1) : zero;
-      for (int hy = threadIdx.x / VX; hy < HY; hy += kRowS) {
-        const int j = j0 + hy - 1;
-        V fa = zero, ia = zero, r = zero;
-        if (j >= 0 && j < ny && Iv <= nx) {
-          const int K = base + j * P + Iv;  // the cell right of the column
-          V fb = zero;
-          if (Iv > 0) {
-            fa = A::ld(fl.f, K - 1);
-            ia = A::rcp(A::addp(fa, A::k(kEps)));
-          }
-          if (Iv < nx) fb = A::ld(fl.f, K);
-          r = xin ? A::fmap(wL, fa, A::mul(wR, fb)) : (Iv == 0 ? fb : fa);
-        }
-        fS[hy][vx] = fa;
-        iS[hy][vx] = ia;
-        rS[hy][vx] = r;
-      }
-    } else {
-      for (int q = threadIdx.x - kRowT; q < HY + VY; q += kAsmThreads - kRowT) {
-        if (q < HY) {
-          const int i = i0 + kTX, j = j0 + q - 1;
-          V fv = zero, iv = zero;
-          if (i < nx && j >= 0 && j < ny) {
-            fv = A::ld(fl.f, base + j * P + i);
-            iv = A::rcp(A::addp(fv, A::k(kEps)));
-          }
-          fS[q][HX - 1] = fv;
-          iS[q][HX - 1] = iv;
-        } else {
-          const int vy = q - HY, Jv = j0 + vy;
-          const bool in = Jv > 0 && Jv < ny;
-          hS[vy][0] = in ? A::ld(cm.wy, 2 * (I.ye + Jv)) : zero;
-          hS[vy][1] = in ? A::ld(cm.wy, 2 * (I.ye + Jv) + 1) : zero;
-        }
-      }
-    }
-    __syncthreads();
-    // 2) vertex values (Solver.cc:299-422): corners copy, interior bilinear, boundary edges
-    //    linear, then Dirichlet overrides with XMIN < XMAX < YMIN < YMAX precedence. The bilinear
-    //    value wB (wL f00 + wR f10) + wT (wL f01 + wR f11) is formed from the two row
-    //    interpolations of step 1 with the same operations in the same order.
-    for (int q = threadIdx.x; q < VX * VY; q += blockDim.x) {
-      const int vx = q % VX, vy = q / VX;
-      const int Iv = i0 + vx, Jv = j0 + vy;
-      if (Iv > nx || Jv > ny) continue;
-      V val;
-      if (Jv == ny && I.bc[YMAX] == DIRICHLET) val = A::ld(cm.dirv, I.dir[YMAX] + Iv);
-      else if (Jv == 0 && I.bc[YMIN] == DIRICHLET) val = A::ld(cm.dirv, I.dir[YMIN] + Iv);
-      else if (Iv == nx && I.bc[XMAX] == DIRICHLET) val = A::ld(cm.dirv, I.dir[XMAX] + Jv);
-      else if (Iv == 0 && I.bc[XMIN] == DIRICHLET) val = A::ld(cm.dirv, I.dir[XMIN] + Jv);
-      else {
-        // cell rows below / above vertex row Jv, clamped to the domain at the edges
-        const int cj0 = Jv > 0 ? Jv - 1 : 0, cj1 = Jv < ny ? Jv : ny - 1;
-        const V r0 = rS[cj0 - j0 + 1][vx];
-        if (Jv > 0 && Jv < ny) {  // interior and vertical boundary edges: linear in y
-          const V r1 = rS[cj1 - j0 + 1][vx];
-          val = A::fmap(hS[vy][0], r0, A::mul(hS[vy][1], r1));
-        } else {
-          val = r0;  // horizontal boundary edges (linear in x) and corners
-        }
-      }
-      vS[vy][vx] = val;
-    }
-    __syncthreads();
-    // 3a) x-faces (vertex column Iv between cells Iv-1 and Iv)
-    for (int q = threadIdx.x; q < kTY * VX; q += blockDim.x) {
-      const int vx = q % VX, ry = q / VX;
-      const int Iv = i0 + vx, j = j0 + ry;
-      V aL = zero, aR = zero, bm = zero;
-      if (j < ny && Iv <= nx) {
-        const V vLo = vS[ry][vx], vHi = vS[ry + 1][vx];  // vertices (Iv, j), (Iv, j+1)
-        if (Iv > 0 && Iv < nx) {
-          const int K = base + j * P + Iv, L = K - 1;
-          // K's XNEG edge: A=(Iv, j+1), B=(Iv, j); L's XPOS edge: A=(Iv, j), B=(Iv, j+1)
-          const V aK = A::dot2(A::ld(geo.aAx, K), vHi, A::ld(geo.aBx, K), vLo);
-          const V aLs = A::dot2(A::ld(geo.aAx, L), vLo, A::ld(geo.aBx, L), vHi);
-          inner_face<A>(aK, A::ld(geo.Sx, K), iS[ry + 1][vx + 1], aLs, A::ld(geo.Sx, L), iS[ry + 1][vx], &aR, &aL);
-        } else if (Iv == 0 && I.bc[XMIN] == DIRICHLET) {
-          const int K = base + j * P;
-          dirichlet_face<A>(A::dot2(A::ld(geo.aAx, K), vHi, A::ld(geo.aBx, K), vLo), A::ld(geo.Sx, K),
-                            iS[ry + 1][vx + 1], &aR, &bm);
-        } else if (Iv == nx && I.bc[XMAX] == DIRICHLET) {
-          const int K = base + j * P + nx - 1;  // XPOS edge: A=(nx, j), B=(nx, j+1)
-          dirichlet_face<A>(A::dot2(A::ld(geo.aAx, K), vLo, A::ld(geo.aBx, K), vHi), A::ld(geo.Sx, K),
-                            iS[ry + 1][vx], &aL, &bm);
-        }
-      }
-      xL[ry][vx] = Iv == 0 ? bm : aL;
-      xR[ry][vx] = Iv == nx ? bm : aR;
-    }
-    // 3b) y-faces (vertex row Jv between cells Jv-1 and Jv)
-    for (int q = threadIdx.x; q < VY * kTX; q += blockDim.x) {
-      const int cx = q % kTX, vy = q / kTX;
-      const int i = i0 + cx, Jv = j0 + vy;
-      V aB = zero, aT = zero, bm = zero;
-      if (i < nx && Jv <= ny) {
-        const V vLe = vS[vy][cx], vRi = vS[vy][cx + 1];  // vertices (i, Jv), (i+1, Jv)
-        if (Jv > 0 && Jv < ny) {
-          const int K = base + Jv * P + i, L = K - P;
-          // K's YNEG edge: A=(i, Jv), B=(i+1, Jv); L's YPOS edge: A=(i+1, Jv), B=(i, Jv)
-          const V aK = A::dot2(A::ld(geo.aAy, K), vLe, A::ld(geo.aBy, K), vRi);
-          const V aLs = A::dot2(A::ld(geo.aAy, L), vRi, A::ld(geo.aBy, L), vLe);
-          inner_face<A>(aK, A::ld(geo.Sy, K), iS[vy + 1][cx + 1], aLs, A::ld(geo.Sy, L), iS[vy][cx + 1], &aT, &aB);
-        } else if (Jv == 0 && I.bc[YMIN] == DIRICHLET) {
-          const int K = base + i;
-          dirichlet_face<A>(A::dot2(A::ld(geo.aAy, K), vLe, A::ld(geo.aBy, K), vRi), A::ld(geo.Sy, K),
-                            iS[vy + 1][cx + 1], &aT, &bm);
-        } else if (Jv == ny && I.bc[YMAX] == DIRICHLET) {
-          const int K = base + (ny - 1) * P + i;  // YPOS edge: A=(i+1,ny), B=(i,ny)
-          dirichlet_face<A>(A::dot2(A::ld(geo.aAy, K), vRi, A::ld(geo.aBy, K), vLe), A::ld(geo.Sy, K),
-                            iS[vy][cx + 1], &aB, &bm);
-        }
-      }
-      yB[vy][cx] = Jv == 0 ? bm : aB;
-      yT[vy][cx] = Jv == ny ? bm : aT;
-    }
-    __syncthreads();
-    // 4) per cell: diagonal in the reference's triplet order, RHS, scaling, scatter
-    float rmax = 0.0f;
-#pragma unroll
-    for (int q = threadIdx.x; q < kTX * kTY; q += kAsmThreads) {
-      const int cx = q % kTX, cy = q / kTX;
-      const int i = i0 + cx, j = j0 + cy;
-      if (i >= nx || j >= ny) continue;
-      const int K = base + j * P + i;
-      const V Aw = xR[cy][cx], Ae = xL[cy][cx + 1], As = yT[cy][cx], An = yB[cy + 1][cx];
-      const bool wIn = i > 0, eIn = i < nx - 1, sIn = j > 0, nIn = j < ny - 1;
-      // every term below is >= 0; a sum that is still zero takes its first term as it is (0 + x
-      // = x), which spares an interior cell three double-word additions
-      V D = wIn ? Aw : zero, Rv = zero, dir = zero;
-      bool has_dir = false;
-      if (eIn) D = A::addp(D, Ae);
-      if (sIn) D = A::addp(D, As);
-      if (nIn) D = A::addp(D, An);
-      if (!wIn && I.bc[XMIN] == DIRICHLET) { D = A::addp(D, Aw); dir = A::addp(dir, Aw); Rv = A::addp(Rv, xL[cy][cx]); has_dir = true; }
-      if (!eIn && I.bc[XMAX] == DIRICHLET) { D = A::addp(D, Ae); dir = A::addp(dir, Ae); Rv = A::addp(Rv, xR[cy][cx + 1]); has_dir = true; }
-      if (!sIn && I.bc[YMIN] == DIRICHLET) { D = A::addp(D, As); dir = A::addp(dir, As); Rv = A::addp(Rv, yB[cy][cx]); has_dir = true; }
-      if (!nIn && I.bc[YMAX] == DIRICHLET) { D = A::addp(D, An); dir = A::addp(dir, An); Rv = A::addp(Rv, yT[cy + 1][cx]); has_dir = true; }
-      const V sd = A::ld(geo.sdiag, K);
-      D = A::addp(D, sd);
-      const V fK = fS[cy + 1][cx + 1];
-      const V ukk = A::ld(geo.ukk, K);
-      Rv = has_dir ? A::fmap(ukk, fK, Rv) : A::fma0(ukk, fK);
-      rmax = fmaxf(rmax, fabsf(A::f32(Rv)));
-      const V inv = A::rcp(D);
-      A::st(fl.invD, K, inv);
-      A::st(fl.R, K, Rv);
-      A::st(fl.colsum, K, has_dir ? A::addp(sd, dir) : sd);
-      // start the solve from D g, g the loss-compensated polynomial extrapolation in time the
-      // last polish formed (only the starting point of the iteration; the converged answer does
-      // not depend on it)
-      A::st(sel2(fl.y64, yc), K, A::mul(D, has_g ? A::ld(gp, K) : fK));
-      if (wIn) AsmOut<C, A>::put(co, 1, K - 1, A::mul(Aw, inv));  // row K-1, east entry
-      if (eIn) AsmOut<C, A>::put(co, 0, K + 1, A::mul(Ae, inv));  // row K+1, west entry
-      if (sIn) AsmOut<C, A>::put(co, 3, K - P, A::mul(As, inv));  // row K-P, north entry
-      if (nIn) AsmOut<C, A>::put(co, 2, K + P, A::mul(An, inv));  // row K+P, south entry
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    const float rmax = asm_tile<C, A, kAsmThreads>(S, cm, geo, fl, co, I, (lt % I.ntx) * kTX, (lt / I.ntx) * kTY, kTY,
+                                                   cm.st[b].nhist > 0, cm.st[b].ycur);
     if ((threadIdx.x & 31) == 0 && rmax > 0.0f) atomicMax(&cm.st[b].rmax_bits, __float_as_uint(rmax));
     __syncthreads();
   }

@@ -581,48 +581,6 @@ __global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg3(Common c
   bicg3_body<T, CH>(cm, kr, cm.ctl->seq);
 }
 
-// The refinement loop of one step in one cooperative launch, for batches whose chunks fit in
-// one wave of co-resident blocks (one large instance: there the launch and ramp of each kernel
-// of the graph's loops cost more than its pass over the cells). The same chunk bodies as the
-// kernels above, separated by grid-wide barriers. The loop decisions are the graph's: the last
-// block of each deciding pass writes them (loop_epilogue, use_cond = 2) before the barrier,
-// every block reads them after it, and nothing rewrites them before every block has finished
-// the next pass -- so every block runs the same sequence of barriers, and the guards bound it.
-// Launch only cooperatively (cudaLaunchAttributeCooperative), with at most one block per chunk.
-// MINB resident blocks per SM: 2 (124 registers, no spill) when the chunks fit in 2 per SM,
-// else 4 (64 registers, some spilled); on one 1024 x 1024 instance in double-word mode the first
-// took 0.84 ms per step, the second 0.90, the separate kernels 0.98.
-template <typename T, typename C, typename A, int CH, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_solve_coop(Common cm, Fields fl, Coef<C> cfull, Coef<T> ck,
-                                                                Kry<T> kr, double tol, double inner_tol,
-                                                                int max_refine, int max_iters) {
-  count_launch(cm.ctl);
-  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  const volatile int* go_outer = &cm.ctl->go_outer;
-  const volatile int* go_inner = &cm.ctl->go_inner;
-  // the trip counts are capped here as well (the same in every block), so the loops end even if
-  // the decisions were never written
-  unsigned seq = 0;
-  for (int o = 0; o < cm.guard_refine; ++o) {
-    resid_body<T, C, A, CH>(cm, fl, cfull, kr, tol, inner_tol, max_refine);
-    loop_epilogue(cm, 0);
-    grid.sync();
-    const bool more = *go_outer != 0;
-    bool inner = *go_inner != 0;
-    for (int it = 0; inner && it < cm.guard_iters; ++it) {
-      bicg1_body<T, CH>(cm, ck, kr);
-      grid.sync();
-      bicg2_body<T, CH>(cm, ck, kr, max_iters, ++seq);
-      loop_epilogue(cm, 1);
-      grid.sync();
-      inner = *go_inner != 0;
-      bicg3_body<T, CH>(cm, kr, seq);  // touches only instances that no pass works on until the next residual
-      if (!inner) grid.sync();
-    }
-    if (!more) break;
-  }
-}
-
 // ------------------------------------------------------------------------------ polish + checks
 // The polish's pointers for one instance: its solution y, the idle y buffer (which takes the next
 // start g) and the earlier states the start goes back to (f^n, the current f, and up to kOrder - 1

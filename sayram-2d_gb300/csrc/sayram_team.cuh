@@ -1,0 +1,548 @@
+// sayram_team.cuh -- k_team: whole steps of a small batch in one cooperative launch.
+//
+// Every instance is advanced by a team of blocks (one block per SM, in all at most the chip), each
+// owning a run of the instance's reduction segments. A team runs assembly, refinement loop and
+// polish of one step after another by itself: its blocks meet at a barrier of their own after
+// each pass, and instances do not wait for one another. What such batches spend their time on
+// in separate kernels is not arithmetic but launches, the reload of every vector in every pass and
+// the ramp of each; here a share's Krylov vectors stay in shared memory and its coefficients in
+// registers for the whole solve, and a pass only exchanges the boundary rows of its product and
+// the sums (through L2).
+//
+// The arithmetic, the reduction segments and the order of the totals are those of the per-pass
+// kernels (sayram_solve.cuh), so both give the same bits.
+#pragma once
+
+#include "sayram_team.h"
+
+namespace sg {
+
+// Meets the team's other blocks: counts this block in and waits until nb blocks have arrived that
+// often. The wait is bounded (a launch is cooperative, so the others are running: milliseconds at
+// most); a block that gives up records it and leaves, and so do the others in their turn.
+struct TeamBar {
+  unsigned* cnt;
+  unsigned target;
+  int nb;
+};
+constexpr int kTeamSpin = 1 << 25;  // polls of ~0.7 us
+__device__ __forceinline__ bool team_sync(TeamBar& tb, int* err) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (tb.nb == 1) return true;
+  if (threadIdx.x == 0) {
+    tb.target += (unsigned)tb.nb;
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(tb.cnt) : "memory");
+    unsigned v;
+    int ok = 0;
+    for (int k = 0; k < kTeamSpin; ++k) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(tb.cnt) : "memory");
+      if ((int)(v - tb.target) >= 0) {
+        ok = 1;
+        break;
+      }
+    }
+    if (!ok) atomicExch(err, 1);
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+// after a block's last barrier: the last one to leave clears the counters for the next launch
+__device__ __forceinline__ void team_leave(const TeamBar& tb) {
+  if (tb.nb == 1 || threadIdx.x != 0) return;
+  if (atomicAdd(tb.cnt + 1, 1u) == (unsigned)tb.nb - 1u) {
+    tb.cnt[0] = 0u;
+    tb.cnt[1] = 0u;
+    __threadfence();
+  }
+}
+
+__device__ __forceinline__ Q4<float> ld4cg(const float* p) {
+  const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+  return Q4<float>{{v.x, v.y, v.z, v.w}};
+}
+__device__ __forceinline__ Q4<double> ld4cg(const double* p) {
+  const double2 u = __ldcg(reinterpret_cast<const double2*>(p));
+  const double2 w = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+  return Q4<double>{{u.x, u.y, w.x, w.y}};
+}
+
+// Warp sums of a share -> segment sums in the global partials. parts[q][k]: the sum over cells
+// [128 k, 128 (k + 1)) of the share.
+template <int NQ, typename R, typename S>
+__device__ __forceinline__ void team_store(const R* parts, int np, int seg, int nseg, S* part, long long stride,
+                                           int at) {
+  __syncthreads();
+  for (int k = threadIdx.x; k < NQ * nseg; k += kTeamThreads) {
+    const int q = k / nseg, s = k - q * nseg;
+    const R v = seg == 128 ? parts[q * np + s] : tree8(&parts[q * np + 8 * s]);
+    part[(size_t)q * stride + at + s] = rconv<S>(v);
+  }
+}
+
+// G: 4-cell groups per thread whose coefficients stay in registers with the Krylov vectors in
+// shared memory (the on-chip form); 0: any number of groups, with x, t, v and the shadow residual in
+// global memory (an instance too large for the chip: one 1024 x 1024 FP64 instance).
+template <typename T, typename C, typename A, int G>
+__global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fields fl, Coef<C> cf, Coef<T> ck,
+                                                           Kry<T> kr, TeamArgs ta) {
+  using V = typename A::V;
+  using R = typename A::R;             // sums of the residual and polish
+  using RK = typename RedOf<T>::R;     // sums of the Krylov passes
+  constexpr bool ON = G > 0;
+  constexpr int GN = ON ? G : 1;
+  count_launch(cm.ctl);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ InstState S;
+  __shared__ InstDev sI;
+  __shared__ double s_tot[2 * kPartQ];
+  __shared__ float s_w[kTeamThreads / 32];
+  __shared__ int s_go;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int np = ta.own_cap / 128;  // warp sums of the largest share
+  const size_t ext_cap = (size_t)ta.own_cap + 2 * (size_t)ta.pmax;
+  double* const parts = reinterpret_cast<double*>(smraw);
+  unsigned char* const mem = smraw + (((size_t)kPartQ * np * 8 + 15) & ~(size_t)15);
+
+  for (int e = ta.first[blockIdx.x]; e < ta.first[blockIdx.x + 1]; ++e) {
+    const TeamShare sh = ta.share[e];
+    __syncthreads();
+    if (tid == 0) {
+      sI = cm.inst[sh.inst];
+      S = cm.st[sh.inst];
+    }
+    __syncthreads();
+    const InstDev& I = sI;
+    const int P = I.pitch, SEG = ta.seg;
+    const long long c0 = I.base + (long long)sh.s0 * SEG;
+    const long long c1 = min(I.base + (long long)sh.s1 * SEG, inst_end(I));
+    const int own = (int)(c1 - c0), ext = own + 2 * P;
+    const int nseg = sh.s1 - sh.s0, seg0 = I.seg0 + sh.s0;
+    const int gend = nseg * SEG / 4;  // groups of whole segments: a multiple of a warp
+    const long long e0 = c0 - P;
+    TeamBar bar{ta.bar + (size_t)sh.inst * kTeamBarStride, 0u, sh.nb};
+    float* const tmax = ta.tmax + (blockIdx.x - sh.rank);
+    // shared memory: r and p with halos, then (on chip) v and x with halos, t and the shadow residual; the
+    // staged 8-byte solution lies over p (and v). In the other form the halos of v and x only.
+    T* const sr = reinterpret_cast<T*>(mem);
+    T* const sp = sr + ext_cap;
+    V* const sv = reinterpret_cast<V*>(sp);
+    T* const sv_ = ON ? sp + ext_cap : reinterpret_cast<T*>(sv + ext_cap);  // v: on chip own + halo, else halo
+    T* const sx = ON ? sv_ + ext_cap : sv_ + 2 * ta.pmax;
+    T* const st_ = sx + ext_cap;               // t of the share (on chip)
+    T* const srh = st_ + ta.own_cap;           // shadow residual of the share (on chip)
+    // a cell of the share that a neighbouring share reads
+    const auto edge = [&](int l) { return l < P || l >= own - P; };
+    // x, v of extended index l (0 .. ext): in shared memory, or own cells in global memory
+    const auto at_x = [&](int l) -> T* {
+      if (ON) return sx + l;
+      return l < P ? sx + l : l < P + own ? kr.x + e0 + l : sx + (l - own);
+    };
+    const auto at_v = [&](int l) -> T* {
+      if (ON) return sv_ + l;
+      return l < P ? sv_ + l : l < P + own ? kr.v[0] + e0 + l : sv_ + (l - own);
+    };
+
+    // the sums of a pass, in turn in one of two sets: a block may write the next pass's while another
+    // still reads this one's
+    int flip = 0;
+    const auto part = [&]() { return cm.part + (size_t)flip * kPartQ * cm.pstride; };
+    bool ok = true;
+    for (int step = 0; ok && step < ta.nsteps; ++step) {
+      // ---------------------------------------------------------------- assembly
+      if (ta.phases & TEAM_ASSEMBLE) {
+        AsmTile<A>& tile = *reinterpret_cast<AsmTile<A>*>(mem);
+        const int nty = (I.ny + sh.ty - 1) / sh.ty, nt = I.ntx * nty;
+        const bool has_g = S.nhist > 0;
+        float rmax = 0.0f;
+        for (int t = sh.rank; t < nt; t += sh.nb) {
+          rmax = fmaxf(rmax, asm_tile<C, A, kTeamThreads>(tile, cm, geo, fl, cf, I, (t % I.ntx) * kTX,
+                                                          (t / I.ntx) * sh.ty, sh.ty, has_g, S.ycur));
+          __syncthreads();
+        }
+        if ((tid & 31) == 0) s_w[warp] = rmax;
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+          for (int w = 1; w < kTeamThreads / 32; ++w) rmax = fmaxf(rmax, s_w[w]);
+          tmax[sh.rank] = rmax;
+        }
+        if (!(ok = team_sync(bar, ta.err))) break;
+        float m = 0.0f;
+        for (int k = tid; k < sh.nb; k += kTeamThreads) m = fmaxf(m, __ldcg(tmax + k));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((tid & 31) == 0) s_w[warp] = m;
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+          for (int w = 1; w < kTeamThreads / 32; ++w) m = fmaxf(m, s_w[w]);
+          S.rmax_bits = m > 0.0f ? __float_as_uint(m) : 0u;
+          S.restart = 0;
+          S.has_x = 0;
+          S.iters = 0;
+          S.iters_total = 0;
+          S.refines = 0;
+          S.clamped = 0;
+        }
+        __syncthreads();
+      }
+      // ---------------------------------------------------------------- refinement loop
+      if (ta.phases & TEAM_SOLVE) {
+        const float sc = rhs_scale(S.rmax_bits), isc = 1.0f / sc;
+        for (;;) {
+          const double* yin = sel2(fl.y64, S.ycur);
+          double* yout = sel2(fl.y64, S.ycur ^ 1);
+          const bool hx = S.has_x != 0;
+          for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
+            Q4<V> y = A::ld4(yin + e0 + l);
+            if (hx) {
+              const Q4<T> x = ld4(at_x(l));
+#pragma unroll
+              for (int m = 0; m < 4; ++m) y.a[m] = A::template add_scaled<T>(y.a[m], x.a[m], isc);
+            }
+            *reinterpret_cast<Q4<V>*>(sv + l) = y;
+          }
+          __syncthreads();
+          for (int g = tid; g < gend; g += kTeamThreads) {
+            typename A::Acc q0 = 0, q1 = 0;
+            T q2 = (T)0;
+            if (4 * g < own) {
+              const int l = 4 * g;
+              Q4<V> yc;
+              Q4<T> r;
+              resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
+              A::st4(yout + c0 + l, yc);
+              st4(sr + P + l, r);
+              if (ON) st4(srh + l, r);
+              if (!ON || edge(l)) st4(kr.rh + c0 + l, r);
+            }
+            const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
+            const R t = warp_totals<3, R>(w);
+            if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + (g >> 5)] = t;
+          }
+          team_store<3, R, R>(reinterpret_cast<const R*>(parts), np, SEG, nseg, reinterpret_cast<R*>(part()),
+                              cm.pstride, seg0);
+          if (!(ok = team_sync(bar, ta.err))) break;
+          seg_total<3, R>(reinterpret_cast<const R*>(part()), cm.pstride, I.seg0, I.nseg,
+                          reinterpret_cast<R*>(s_tot));
+          flip ^= 1;
+          if (tid == 0) {
+            const R* tt = reinterpret_cast<const R*>(s_tot);
+            const double tot[3] = {rdbl(radd(tt[0], tt[1])), rdbl(radd(tt[2], tt[3])), rdbl(radd(tt[4], tt[5]))};
+            s_go = after_resid(S, tot, ta.tol, ta.inner_tol, ta.max_refine, cm.precond);
+          }
+          __syncthreads();
+          if (!s_go) break;
+          // -------------------------------------------------------------- Krylov solve
+          Q4<T> cw[GN], ce[GN], cs[GN], cn[GN];
+          if (ON) {
+#pragma unroll
+            for (int k = 0; k < GN; ++k) {
+              const int g = tid + k * kTeamThreads;
+              if (4 * g < own) {
+                const long long K = c0 + 4 * g;
+                cw[k] = ld4(ck.cw + K);
+                ce[k] = ld4(ck.ce + K);
+                cs[k] = ld4(ck.cs + K);
+                cn[k] = ld4(ck.cn + K);
+              }
+            }
+          }
+          // p = r = r^; the neighbours' rows of r
+          for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
+            Q4<T> r;
+            if (l < P || l >= P + own) {
+              r = ld4cg(kr.rh + e0 + l);
+              st4(sr + l, r);
+            } else {
+              r = ld4(sr + l);
+            }
+            st4(sp + l, r);
+          }
+          for (;;) {
+            const int it = S.iters;
+            const bool rs = S.restart != 0;
+            if (it > 0) {  // update by the previous iteration's products; sr holds s
+              const T alpha = (T)S.alpha, beta = (T)S.beta, omega = (T)S.omega;
+              for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
+                const bool halo = l < P || l >= P + own;
+                const Q4<T> t = halo ? ld4cg(kr.t + e0 + l) : ON ? ld4(st_ + (l - P)) : ld4(kr.t + e0 + l);
+                const Q4<T> s = ld4(sr + l), v = ld4(at_v(l));
+                Q4<T> p = ld4(sp + l), q, x{{(T)0, (T)0, (T)0, (T)0}};
+                if (it > 1) x = ld4(at_x(l));
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                  q.a[m] = fmaT(-omega, t.a[m], s.a[m]);
+                  x.a[m] = fmaT(alpha, p.a[m], fmaT(omega, s.a[m], x.a[m]));
+                  p.a[m] = rs ? q.a[m] : fmaT(beta, fmaT(-omega, v.a[m], p.a[m]), q.a[m]);
+                }
+                st4(sr + l, q);
+                st4(sp + l, p);
+                st4(at_x(l), x);
+                if (rs && !halo) st4(ON ? srh + (l - P) : kr.rh + e0 + l, q);
+              }
+            }
+            __syncthreads();
+            // v = B^-1 A~ p
+            const auto product_v = [&](int g, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
+                                       T& q0, T& q1) {
+              const int l = 4 * g;
+              Q4<T> v = stencil_sm<T>(sp, P + l, P, w, ea, so, no);
+              if (cm.precond) v = line4<T>(v, line_of<T>(w, ea));
+              st4(at_v(P + l), v);
+              if (ON && edge(l)) st4(kr.v[0] + c0 + l, v);
+              const Q4<T> rh = rs ? ld4(sp + P + l) : ON ? ld4(srh + l) : ld4(kr.rh + c0 + l);
+              q0 = dot4<T>(rh, v, q0);
+              if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
+            };
+            const auto put2 = [&](int g, T q0, T q1) {
+              const RK w[2] = {rfrom<RK>(q0), rfrom<RK>(q1)};
+              const RK t = warp_totals<2, RK>(w);
+              if (red_writes<2>()) reinterpret_cast<RK*>(parts)[red_q<2>() * np + (g >> 5)] = t;
+            };
+            if (ON) {
+#pragma unroll
+              for (int k = 0; k < GN; ++k) {
+                const int g = tid + k * kTeamThreads;
+                if (g < gend) {
+                  T q0 = (T)0, q1 = (T)0;
+                  if (4 * g < own) product_v(g, cw[k], ce[k], cs[k], cn[k], q0, q1);
+                  put2(g, q0, q1);
+                }
+              }
+            } else {
+              for (int g = tid; g < gend; g += kTeamThreads) {
+                T q0 = (T)0, q1 = (T)0;
+                if (4 * g < own) {
+                  const long long K = c0 + 4 * g;
+                  product_v(g, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q0, q1);
+                }
+                put2(g, q0, q1);
+              }
+            }
+            team_store<2, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
+                                  cm.pstride, seg0);
+            if (!(ok = team_sync(bar, ta.err))) break;
+            seg_total<2, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
+                             reinterpret_cast<RK*>(s_tot));
+            flip ^= 1;
+            if (tid == 0) {
+              const RK* tt = reinterpret_cast<const RK*>(s_tot);
+              const double tot[2] = {rdbl(radd(tt[0], tt[1])), rdbl(radd(tt[2], tt[3]))};
+              after_v(S, tot);
+            }
+            __syncthreads();
+            // s = r - alpha v over the share and its halo
+            {
+              const T alpha = (T)S.alpha;
+              for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
+                Q4<T> v, s = ld4(sr + l);
+                if (l < P || l >= P + own) {
+                  v = ld4cg(kr.v[0] + e0 + l);
+                  st4(at_v(l), v);
+                } else {
+                  v = ld4(at_v(l));
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) s.a[m] = fmaT(-alpha, v.a[m], s.a[m]);
+                st4(sr + l, s);
+              }
+            }
+            __syncthreads();
+            // t = B^-1 A~ s
+            const auto product_t = [&](int g, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
+                                       T (&q)[5]) {
+              const int l = 4 * g;
+              Q4<T> t = stencil_sm<T>(sr, P + l, P, w, ea, so, no);
+              if (cm.precond) t = line4<T>(t, line_of<T>(w, ea));
+              if (ON) st4(st_ + l, t);
+              if (!ON || edge(l)) st4(kr.t + c0 + l, t);
+              const Q4<T> s = ld4(sr + P + l), rh = ON ? ld4(srh + l) : ld4(kr.rh + c0 + l);
+              q[0] = dot4<T>(t, s, q[0]);
+              q[1] = dot4<T>(t, t, q[1]);
+              q[2] = dot4<T>(s, s, q[2]);
+              q[3] = dot4<T>(rh, s, q[3]);
+              q[4] = dot4<T>(rh, t, q[4]);
+            };
+            const auto put5 = [&](int g, const T (&q)[5]) {
+              const RK w[5] = {rfrom<RK>(q[0]), rfrom<RK>(q[1]), rfrom<RK>(q[2]), rfrom<RK>(q[3]), rfrom<RK>(q[4])};
+              const RK t = warp_totals<5, RK>(w);
+              if (red_writes<5>()) reinterpret_cast<RK*>(parts)[red_q<5>() * np + (g >> 5)] = t;
+            };
+            if (ON) {
+#pragma unroll
+              for (int k = 0; k < GN; ++k) {
+                const int g = tid + k * kTeamThreads;
+                if (g < gend) {
+                  T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
+                  if (4 * g < own) product_t(g, cw[k], ce[k], cs[k], cn[k], q);
+                  put5(g, q);
+                }
+              }
+            } else {
+              for (int g = tid; g < gend; g += kTeamThreads) {
+                T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
+                if (4 * g < own) {
+                  const long long K = c0 + 4 * g;
+                  product_t(g, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q);
+                }
+                put5(g, q);
+              }
+            }
+            team_store<5, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
+                                  cm.pstride, seg0);
+            if (!(ok = team_sync(bar, ta.err))) break;
+            seg_total<5, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
+                             reinterpret_cast<RK*>(s_tot));
+            flip ^= 1;
+            if (tid == 0) {
+              const RK* tt = reinterpret_cast<const RK*>(s_tot);
+              double tot[5];
+#pragma unroll
+              for (int k = 0; k < 5; ++k) tot[k] = rdbl(radd(tt[2 * k], tt[2 * k + 1]));
+              s_go = !after_t(S, tot, ta.max_iters);
+            }
+            __syncthreads();
+            if (!s_go) break;
+          }
+          if (!ok) break;
+          // the solve's correction over the share and its halo
+          {
+            const bool one = S.iters == 1;
+            const T alpha = (T)S.alpha, omega = (T)S.omega;
+            for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
+              const Q4<T> s = ld4(sr + l), p = ld4(sp + l);
+              Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
+              if (!one) x = ld4(at_x(l));
+#pragma unroll
+              for (int m = 0; m < 4; ++m) x.a[m] = fmaT(alpha, p.a[m], fmaT(omega, s.a[m], x.a[m]));
+              st4(at_x(l), x);
+            }
+            __syncthreads();
+          }
+        }
+        if (!ok) break;
+      }
+      // ---------------------------------------------------------------- polish
+      if (ta.phases & TEAM_POLISH) {
+        const PolishAt at = polish_at(fl, S.ycur, S.nhist, S.hslot, cm.hist_cap);
+        const bool staged = (ta.phases & TEAM_SOLVE) != 0;  // the last residual's y is still there
+        const bool last = step == ta.nsteps - 1;
+        // max(y, 0), and the cells it changes, counted per thread and then as part of its first group
+        float clamp = 0.0f;
+        for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
+          Q4<V> y = staged ? *reinterpret_cast<const Q4<V>*>(sv + l) : A::ld4(at.y + e0 + l);
+          const bool mine = l >= P && l < P + own;
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            if (mine && A::lt0(y.a[m])) clamp += 1.0f;  // padding cells are 0
+            y.a[m] = A::max0(y.a[m]);
+          }
+          *reinterpret_cast<Q4<V>*>(sv + l) = y;
+        }
+        __syncthreads();
+        float mn = 3.0e38f;
+        for (int g = tid; g < gend; g += kTeamThreads) {
+          V mass = A::k(0.0), rsum = A::k(0.0);
+          if (4 * g < own) {
+            const long long K = c0 + 4 * g;
+            polish_group<C, A>(sv, P + 4 * g, P, cf, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
+          }
+          const R w[2] = {mass, rsum};
+          const R t = warp_totals<2, R>(w);
+          if (red_writes<2>()) reinterpret_cast<R*>(parts)[red_q<2>() * np + (g >> 5)] = t;
+        }
+        team_store<2, R, double>(reinterpret_cast<const R*>(parts), np, SEG, nseg, part(), cm.pstride, seg0);
+        // clamped cells (whole numbers) and the minimum: one entry per share, the rest of its segments 0
+        // and no minimum
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          clamp += __shfl_xor_sync(0xffffffffu, clamp, o);
+          mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        }
+        __shared__ float s_c[kTeamThreads / 32];
+        if ((tid & 31) == 0) {
+          s_w[warp] = mn;
+          s_c[warp] = clamp;
+        }
+        __syncthreads();
+        if (tid < nseg || tid == 0) {
+          float m = s_w[0], c = s_c[0];
+          for (int w = 1; w < kTeamThreads / 32; ++w) {
+            m = fminf(m, s_w[w]);
+            c += s_c[w];
+          }
+          for (int k = tid; k < nseg; k += kTeamThreads) {
+            part()[2 * (size_t)cm.pstride + seg0 + k] = k == 0 ? (double)c : 0.0;
+            part()[3 * (size_t)cm.pstride + seg0 + k] = (double)m;
+          }
+        }
+        if (!(ok = team_sync(bar, ta.err))) break;
+        double tot[3] = {0.0, 0.0, 0.0}, gmin = 0.0;
+        if (last && sh.rank == 0) {
+          seg_total<3, double>(part(), cm.pstride, I.seg0, I.nseg, s_tot);
+          double m = 1.0e300;
+          for (int k = tid; k < I.nseg; k += kTeamThreads) m = fmin(m, __ldcg(part() + 3 * (size_t)cm.pstride + I.seg0 + k));
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
+          if ((tid & 31) == 0) s_w[warp] = (float)m;  // the minima are FP32 values
+          __syncthreads();
+          gmin = s_w[0];
+          for (int w = 1; w < kTeamThreads / 32; ++w) gmin = fmin(gmin, (double)s_w[w]);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) tot[k] = radd(s_tot[2 * k], s_tot[2 * k + 1]);
+        }
+        flip ^= 1;
+        if (tid == 0) after_polish(S, tot[0], tot[1], tot[2], gmin);
+        __syncthreads();
+      }
+    }
+    // the instance's state goes back once, by the team's first block (the others only read it
+    // before their first barrier)
+    if (ok && sh.rank == 0 && tid == 0) {
+      S.outer_active = 0;
+      S.inner_active = 0;
+      cm.st[sh.inst] = S;
+    }
+    team_leave(bar);
+  }
+}
+
+template <typename T, typename C, typename A, int G>
+size_t team_limit() {
+  cudaFuncAttributes fa;
+  int dev = 0, optin = 0;
+  if (cudaFuncGetAttributes(&fa, k_team<T, C, A, G>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const size_t left = (size_t)optin > fa.sharedSizeBytes ? (size_t)optin - fa.sharedSizeBytes : 0;
+  if (cudaFuncSetAttribute(k_team<T, C, A, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)left) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return left;
+}
+
+template <typename T, typename C, typename A, int G>
+cudaError_t team_launch(const TeamLaunch& l, const Common& cm, const Geo& geo, const Fields& fl, const Coef<C>& cf,
+                        const Coef<T>& ck, const Kry<T>& kr, const TeamArgs& ta) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)l.grid);
+  cfg.blockDim = dim3(kTeamThreads);
+  cfg.dynamicSmemBytes = l.smem;
+  cfg.stream = l.stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_team<T, C, A, G>, cm, geo, fl, cf, ck, kr, ta);
+}
+
+}  // namespace sg
