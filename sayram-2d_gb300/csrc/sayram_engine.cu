@@ -124,6 +124,8 @@ struct sayram_batch_s {
     tab_cap = 0;
     if (h_ctl) cudaFreeHost(h_ctl);
     h_ctl = nullptr;
+    if (h_stat) cudaFreeHost(h_stat);
+    h_stat = nullptr;
     for (auto e : evpool) cudaEventDestroy(e);
     evpool.clear();
     for (auto& e : slots)
@@ -238,10 +240,10 @@ struct sayram_batch_s {
   int* d_first = nullptr;
   unsigned* d_bar = nullptr;
   float* d_tmax = nullptr;
-  int* d_err = nullptr;
+  int* h_stat = nullptr;  // pinned, written by k_team (TEAM_* flags)
   static constexpr int kTeamSteps = 32;
   int plan_team();
-  int launch_team(int nsteps, int phases);
+  int launch_team(int nsteps, int phases, bool last = true);
   // dispatch of the per-step sequence on precision and chunk size (graph: build it; else: run it)
   template <typename T, typename C, typename A>
   int run_chunked(const sg::Coef<C>& cf, const sg::Coef<T>& ck, const sg::Kry<T>& kr, bool as_graph, bool prefix) {
@@ -326,6 +328,22 @@ struct sayram_batch_s {
   // wave), 5.85 with 10, 5.60 with 20, 5.40 with 40, 5.27 with 64 and 5.32 with one block per
   // tile; with 6 resident, 5.22 with 48, 5.16 with 64 and 5.09 with 96.
   int grid_tiles() const { return std::max(1, std::min(cap_tiles, nsm * sg::kAsmGridPerSm)); }
+  // the layout transforms of tiles [t0, t1) between the device state and packed alpha-major doubles
+  int grid_layout(int tiles) const { return std::max(1, std::min(tiles, nsm * sg::kAsmGridPerSm)); }
+  void layout_in(int t0, int t1, const double* src, int restart, cudaStream_t s) {
+    const int g = grid_layout(t1 - t0);
+    if (dwm)
+      sg::k_field_in<sg::DWA><<<g, sg::kFieldThreads, 0, s>>>(cm, fl.f, src, restart, t0, t1);
+    else
+      sg::k_field_in<sg::F64A><<<g, sg::kFieldThreads, 0, s>>>(cm, fl.f, src, restart, t0, t1);
+  }
+  void layout_out(int t0, int t1, double* dst, cudaStream_t s) {
+    const int g = grid_layout(t1 - t0);
+    if (dwm)
+      sg::k_field_out<sg::DWA><<<g, 256, 0, s>>>(cm, dst, fl.f, t0, t1);
+    else
+      sg::k_field_out<sg::F64A><<<g, 256, 0, s>>>(cm, dst, fl.f, t0, t1);
+  }
   int n_enabled() const {
     int k = 0;
     for (int b = 0; b < n && b < (int)hinst.size(); ++b) k += hinst[b].enabled ? 1 : 0;
@@ -346,6 +364,7 @@ struct sayram_batch_s {
   int launch_steps(int nsteps);  // queue steps on the stream (no status read-back)
   int read_ctl();
   int check_team();
+  int status_of(bool negative, bool not_converged);
   int finish_status();
   template <typename T, typename C, typename A, int CH>
   int step_once(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, const sg::Kry<T>& kr);
@@ -360,6 +379,11 @@ struct sayram_batch_s {
     float pr[2] = {h, l};
     std::memcpy(&out, pr, sizeof(out));
     return out;
+  }
+  // the relative residual the last step's solve ended at
+  double rel_of(const InstState& s) const {
+    const double bb = unwide(s.bb), rr = unwide(s.rr64);
+    return bb > 0 ? std::sqrt(rr / bb) : 0.0;
   }
   double unwide(double w) const {
     if (!dwm) return w;
@@ -452,7 +476,8 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
   SG_ALLOC(d_first, nsm + 1);
   SG_ALLOC(d_bar, (long long)slots * sg::kTeamBarStride);
   SG_ALLOC(d_tmax, nsm);
-  SG_ALLOC(d_err, 1);
+  SG_CUDA(cudaMallocHost(&h_stat, sizeof(int) * sg::TEAM_FLAGS));
+  std::memset(h_stat, 0, sizeof(int) * sg::TEAM_FLAGS);
   SG_ALLOC(d_stage, stage_cap);
   cell_arrays.clear();
   double** geos[10] = {&geo.aAx, &geo.aBx, &geo.Sx, &geo.aAy, &geo.aBy, &geo.Sy, &geo.ukk, &geo.sdiag, &geo.G,
@@ -720,13 +745,14 @@ int sayram_batch_s::plan_team() {
   return SAYRAM_OK;
 }
 
-int sayram_batch_s::launch_team(int nsteps, int phases) {
+int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   sg::TeamArgs ta{};
   ta.share = d_share;
   ta.first = d_first;
   ta.bar = d_bar;
   ta.tmax = d_tmax;
-  ta.err = d_err;
+  ta.stat = h_stat;
+  ta.report = last ? 1 : 0;
   ta.tol = opt.tol;
   ta.inner_tol = opt.inner_tol;
   ta.max_refine = opt.max_refine;
@@ -963,6 +989,12 @@ int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck,
 int sayram_batch_s::run_steps(int nsteps) {
   int rc = launch_steps(nsteps);
   if (rc) return rc;
+  if (team_grid > 0 && nsteps > 0) {  // k_team has left the outcome in host memory
+    if ((rc = check_team())) return rc;
+    if (timing) collect_timing();
+    volatile int* f = h_stat;
+    return status_of(f[sg::TEAM_NEGATIVE] != 0, f[sg::TEAM_NOT_CONVERGED] != 0);
+  }
   SG_CUDA(cudaStreamSynchronize(stream));
   if (timing) collect_timing();
   return finish_status();
@@ -972,6 +1004,7 @@ int sayram_batch_s::launch_steps(int nsteps) {
   if (nsteps < 0) return fail(SAYRAM_ERR_ARG, "nsteps must be >= 0");
   SG_CUDA(cudaSetDevice(dev));
   if (team_grid > 0) {
+    h_stat[sg::TEAM_NEGATIVE] = h_stat[sg::TEAM_NOT_CONVERGED] = 0;  // nothing of this batch is running
     if (timing) {  // the phases of a step one by one
       for (int s = 0; s < nsteps; ++s) {
         int rc = SAYRAM_OK;
@@ -980,7 +1013,7 @@ int sayram_batch_s::launch_steps(int nsteps) {
             {"assemble", sg::TEAM_ASSEMBLE}, {"solve_coop", sg::TEAM_SOLVE}, {"polish", sg::TEAM_POLISH}};
         for (auto& p : ph) {
           int r2 = SAYRAM_OK;
-          launch(p.first, [&] { r2 = launch_team(1, p.second); });
+          launch(p.first, [&] { r2 = launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH); });
           if (r2) rc = r2;
         }
         if (rc) return rc;
@@ -989,7 +1022,7 @@ int sayram_batch_s::launch_steps(int nsteps) {
     }
     for (int s = 0; s < nsteps;) {  // a launch stays well below a second
       const int k = std::min(nsteps - s, kTeamSteps);
-      int rc = launch_team(k, sg::TEAM_STEP);
+      int rc = launch_team(k, sg::TEAM_STEP, s + k == nsteps);
       if (rc) return rc;
       s += k;
     }
@@ -1187,14 +1220,18 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
 // Waits for the stream; an error when a barrier of k_team gave up (its counters are cleared, so the
 // batch stays usable, but the step is lost).
 int sayram_batch_s::check_team() {
-  int err = 0;
-  if (team_grid > 0) SG_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
-  if (!err) return SAYRAM_OK;
-  SG_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
+  if (!*(volatile int*)(h_stat + sg::TEAM_GAVE_UP)) return SAYRAM_OK;
+  h_stat[sg::TEAM_GAVE_UP] = 0;
   SG_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(unsigned) * (size_t)cap_slots * sg::kTeamBarStride, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
   return fail(SAYRAM_ERR_TIMEOUT, "a device barrier of the cooperative step gave up waiting");
+}
+
+int sayram_batch_s::status_of(bool negative, bool not_converged) {
+  if (negative) return fail(SAYRAM_ERR_NEGATIVE, "a negative cell survived the positivity polish");
+  if (not_converged) return fail(SAYRAM_ERR_NOT_CONVERGED, "a step ended above the residual target");
+  return SAYRAM_OK;
 }
 
 int sayram_batch_s::finish_status() {
@@ -1208,9 +1245,7 @@ int sayram_batch_s::finish_status() {
     if (hs[b].status == sg::ST_NEGATIVE) worst = SAYRAM_ERR_NEGATIVE;
     else if (hs[b].status == sg::ST_NOT_CONVERGED && worst == SAYRAM_OK) worst = SAYRAM_ERR_NOT_CONVERGED;
   }
-  if (worst == SAYRAM_ERR_NEGATIVE) return fail(worst, "a negative cell survived the positivity polish");
-  if (worst == SAYRAM_ERR_NOT_CONVERGED) return fail(worst, "a step ended above the residual target");
-  return SAYRAM_OK;
+  return status_of(worst == SAYRAM_ERR_NEGATIVE, worst == SAYRAM_ERR_NOT_CONVERGED);
 }
 
 namespace sg {
@@ -1294,8 +1329,10 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
   {
     // the first run is small (a quarter of the others): its copy in is what the first assembly
     // waits for, and its polish is what the first copy out waits for; the rest are about equal
-    const long long target = (b->nreal + kPieces - 1) / kPieces;
-    const long long first = (b->nreal + 4 * kPieces - 1) / (4 * kPieces);
+    // (a batch stepped by k_team copies around whole steps: runs of at least 4 MB, which take 20 us)
+    const long long least = b->team_grid > 0 ? 1LL << 19 : 1;
+    const long long target = std::max(least, (b->nreal + kPieces - 1) / kPieces);
+    const long long first = std::max(least, (b->nreal + 4 * kPieces - 1) / (4 * kPieces));
     int a = 0;
     while (a < b->n) {
       long long len = 0;
@@ -1317,22 +1354,11 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
     SG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     b->piece_ev.push_back(e);
   }
-  const int gt = b->grid_tiles();
   auto field_in = [&](const Piece& pc, cudaStream_t s) {
-    b->launch("field_in", [&] {
-      if (b->dwm)
-        sg::k_field_in<sg::DWA><<<gt, sg::kFieldThreads, 0, s>>>(b->cm, b->fl.f, b->d_stage, 1, pc.t0, pc.t1);
-      else
-        sg::k_field_in<sg::F64A><<<gt, sg::kFieldThreads, 0, s>>>(b->cm, b->fl.f, b->d_stage, 1, pc.t0, pc.t1);
-    });
+    b->launch("field_in", [&] { b->layout_in(pc.t0, pc.t1, b->d_stage, 1, s); });
   };
   auto field_out = [&](const Piece& pc) {
-    b->launch("field_out", [&] {
-      if (b->dwm)
-        sg::k_field_out<sg::DWA><<<gt, 256, 0, b->stream>>>(b->cm, b->d_stage, b->fl.f, pc.t0, pc.t1);
-      else
-        sg::k_field_out<sg::F64A><<<gt, 256, 0, b->stream>>>(b->cm, b->d_stage, b->fl.f, pc.t0, pc.t1);
-    });
+    b->launch("field_out", [&] { b->layout_out(pc.t0, pc.t1, b->d_stage, b->stream); });
   };
   auto copy_in = [&](size_t k) -> int {  // H2D of piece k on the copy stream, then an event
     const Piece& pc = pieces[k];
@@ -1429,12 +1455,12 @@ int sayram_batch_get_f(sayram_batch b, int idx, double* f_out) {
   if (!b || !f_out || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
-  // rows of the padded layout -> alpha-major on the host
-  std::vector<double> rows((size_t)I.ny * I.pitch);
-  SG_CUDA(cudaMemcpyAsync(rows.data(), b->fl.f + I.base, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost, b->stream));
+  const int t0 = I.tile0, t1 = I.tile0 + I.ntx * I.nty;
+  // transposed (and, in double-word mode, converted) on the device into the staging buffer
+  b->layout_out(t0, t1, b->d_stage - I.hoff, b->stream);
+  SG_CUDA(cudaGetLastError());
+  SG_CUDA(cudaMemcpyAsync(f_out, b->d_stage, sizeof(double) * (size_t)I.nx * I.ny, cudaMemcpyDeviceToHost, b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
-  for (int i = 0; i < I.nx; ++i)
-    for (int j = 0; j < I.ny; ++j) f_out[(size_t)i * I.ny + j] = b->unwide(rows[(size_t)j * I.pitch + i]);
   return SAYRAM_OK;
 }
 
@@ -1442,10 +1468,9 @@ int sayram_batch_set_f(sayram_batch b, int idx, const double* f) {
   if (!b || !f || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
-  std::vector<double> rows((size_t)I.ny * I.pitch, 0.0);
-  for (int i = 0; i < I.nx; ++i)
-    for (int j = 0; j < I.ny; ++j) rows[(size_t)j * I.pitch + i] = b->wide(f[(size_t)i * I.ny + j]);
-  SG_CUDA(cudaMemcpyAsync(b->fl.f + I.base, rows.data(), sizeof(double) * rows.size(), cudaMemcpyHostToDevice, b->stream));
+  SG_CUDA(cudaMemcpyAsync(b->d_stage, f, sizeof(double) * (size_t)I.nx * I.ny, cudaMemcpyHostToDevice, b->stream));
+  b->layout_in(I.tile0, I.tile0 + I.ntx * I.nty, b->d_stage - I.hoff, 0, b->stream);
+  SG_CUDA(cudaGetLastError());
   SG_CUDA(cudaMemsetAsync((char*)(b->d_st + idx) + offsetof(InstState, nhist), 0, sizeof(int), b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
   return SAYRAM_OK;
@@ -1501,7 +1526,7 @@ int sayram_batch_stats(sayram_batch b, int idx, sayram_stats* out) {
                 : s.status == sg::ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED : SAYRAM_OK;
   out->refinements = s.refines;
   out->iterations = s.iters_total;
-  out->rel_residual = s.rel;
+  out->rel_residual = b->rel_of(s);
   out->min_f = s.min_f;
   out->clamped = s.clamped;
   out->mass_drift = s.mass_drift;
@@ -1926,7 +1951,7 @@ struct ServerLane {
                     : hs.status == sg::ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED : SAYRAM_OK;
       R.st.refinements = hs.refines;
       R.st.iterations = hs.iters_total;
-      R.st.rel_residual = hs.rel;
+      R.st.rel_residual = eng.rel_of(hs);
       R.st.min_f = hs.min_f;
       R.st.clamped = hs.clamped;
       R.st.mass_drift = hs.mass_drift;
@@ -2429,7 +2454,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
                         : hs.status == ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED : SAYRAM_OK;
     stats_out->refinements = hs.refines;
     stats_out->iterations = hs.iters_total;
-    stats_out->rel_residual = hs.rel;
+    stats_out->rel_residual = hs.bb > 0 ? std::sqrt(hs.rr64 / hs.bb) : 0.0;
     stats_out->min_f = hs.min_f;
     stats_out->clamped = hs.clamped;
     stats_out->mass_drift = hs.mass_drift;

@@ -60,9 +60,12 @@ struct InstDev {
 
 // Per-instance solver state (mutable, device resident).
 struct InstState {
+  // 8-byte scalars of the solve: IEEE doubles, or double words (bit patterns, see num/set_num) where
+  // the sums behind them are double words -- the Krylov scalars in both FP32 modes, bb and rr64
+  // in the double-word mode
   double rho, alpha, omega, beta;
   double rr, rr_target, bb, rr64;
-  double rel, mass_drift, min_f, pad_d;
+  double mass_drift, min_f;
   long long clamped, steps;
   long long cum_iters, cum_refines;  // totals since creation (work accounting)
   int ycur, outer_active, inner_active;
@@ -125,6 +128,31 @@ __device__ __forceinline__ void count_launch(Ctl* ctl) {
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctl->launches, 1ull);
 }
 
+// ------------------------------------------------------------------------------ FP64 reciprocals
+// 1/b and a/b in FP64 by Newton-Raphson from an FP32 reciprocal (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): the
+// seed's error of ~2^-22 squares twice, so the reciprocal is rounded correctly but for ties within
+// 2^-30 of an ulp, and one residual step rounds the quotient. Four (seven) operations on the FP64
+// pipe; the plain operators measured 4478 cycles for one dependent division of one warp, 68 times a
+// multiply-add. Zeros, subnormals, infinities, NaNs and the outermost exponents take the operators.
+__device__ __forceinline__ double rcp64(double b) {
+  const int hi = __double2hiint(b), lo = __double2loint(b), e = (hi >> 20) & 0x7ff;
+  if (e < 3 || e > 2042) return 1.0 / b;
+  const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, lo);  // |b| = m 2^(e - 1023)
+  // m to FP32 (truncated), its reciprocal and back, by moving the fields
+  const float f = __uint_as_float(__funnelshift_l((unsigned)lo, (unsigned)((hi & 0x000fffff) | 0x07f00000), 3));
+  const unsigned s = __float_as_uint(__fdividef(1.0f, f));
+  const double r0 = __hiloint2double((int)((s >> 3) + 0x38000000u), (int)(s << 29));
+  const double r1 = __fma_rn(r0, __fma_rn(-m, r0, 1.0), r0);
+  const double r2 = __fma_rn(r1, __fma_rn(-m, r1, 1.0), r1);
+  return __hiloint2double((__double2hiint(r2) + (1023 - e) * 0x100000) | (hi & 0x80000000), __double2loint(r2));
+}
+__device__ __forceinline__ double div64(double a, double b) {
+  const double r = rcp64(b), q = __dmul_rn(a, r);
+  const double t = __fma_rn(__fma_rn(-b, q, a), r, q);
+  return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : t;
+}
+
 // ------------------------------------------------------------------------------ reductions
 // Sums are carried in R: IEEE double, or a double word where the terms are FP32 (the FP64 pipe is
 // far too slow for the trees: 2 lanes per SM and cycle).
@@ -156,6 +184,32 @@ template <>
 __device__ __forceinline__ dw rconv<dw>(dw a) { return a; }
 template <>
 __device__ __forceinline__ double rconv<double>(dw a) { return dw_to_double(a); }
+// scalars of type R in 8-byte storage
+template <typename R>
+__device__ __forceinline__ R num(double s) {
+  return *reinterpret_cast<const R*>(&s);
+}
+template <>
+__device__ __forceinline__ dw num<dw>(double s) {
+  return dw{__int_as_float(__double2loint(s)), __int_as_float(__double2hiint(s))};
+}
+__device__ __forceinline__ double stored(double a) { return a; }
+__device__ __forceinline__ double stored(dw a) { return __hiloint2double(__float_as_int(a.lo), __float_as_int(a.hi)); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ dw rmul(dw a, dw b) { return dw_mul(a, b); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ dw rfma(dw a, dw b, dw c) { return dw_fma(a, b, c); }
+__device__ __forceinline__ double rneg(double a) { return -a; }
+__device__ __forceinline__ dw rneg(dw a) { return dw_neg(a); }
+__device__ __forceinline__ double rdiv(double a, double b) { return div64(a, b); }
+__device__ __forceinline__ dw rdiv(dw a, dw b) { return dw_div(a, b); }
+__device__ __forceinline__ bool rgt(double a, double b) { return a > b; }
+__device__ __forceinline__ bool rgt(dw a, dw b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
+__device__ __forceinline__ double rhead(double a) { return a; }
+__device__ __forceinline__ float rhead(dw a) { return a.hi; }
+__device__ __forceinline__ double rto(double a, double) { return a; }  // a in the second argument's type
+__device__ __forceinline__ dw rto(dw a, dw) { return a; }
+__device__ __forceinline__ dw rto(double a, dw) { return dw_from_double(a); }
 // the type a pass's sums are carried in: by the precision T of its terms
 template <typename T>
 struct RedOf;
@@ -231,7 +285,7 @@ __device__ __forceinline__ void seg_total(const R* part, long long stride, int s
     R a = rfrom<R>(0.0f);
     for (int s = h * 32 + lane; s < nseg; s += 64) {
       const double w = __ldcg(src + s);
-      a = radd(a, *reinterpret_cast<const R*>(&w));
+      a = radd(a, num<R>(w));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a = radd(a, rshfl(a, o));
@@ -245,7 +299,7 @@ __device__ __forceinline__ void seg_total(const R* part, long long stride, int s
 // the totals are returned in tot (valid in thread 0) and the phase counter is reset.
 template <int NQ, typename R>
 __device__ __forceinline__ bool chunk_finish(InstState& st, int phase, const InstDev& I, const R* part,
-                                             long long stride, double (&tot)[NQ]) {
+                                             long long stride, R (&tot)[NQ]) {
   __shared__ int s_last;
   __shared__ double s_tot[2 * NQ];
   __syncthreads();
@@ -261,7 +315,7 @@ __device__ __forceinline__ bool chunk_finish(InstState& st, int phase, const Ins
   seg_total<NQ, R>(part, stride, I.seg0, I.nseg, sm);
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) tot[q] = rdbl(radd(sm[2 * q], sm[2 * q + 1]));
+    for (int q = 0; q < NQ; ++q) tot[q] = radd(sm[2 * q], sm[2 * q + 1]);
     st.cnt[phase] = 0;
   }
   return true;

@@ -145,8 +145,8 @@ struct F64A {
   __device__ static V addp(V a, V b) { return __dadd_rn(a, b); }
   __device__ static V fmap(V a, V b, V c) { return __fma_rn(a, b, c); }
   __device__ static V addf(V a, float b) { return __dadd_rn(a, (double)b); }
-  __device__ static V rcp(V a) { return 1.0 / a; }
-  __device__ static V div(V a, V b) { return a / b; }
+  __device__ static V rcp(V a) { return rcp64(a); }
+  __device__ static V div(V a, V b) { return div64(a, b); }
   __device__ static V abs(V a) { return fabs(a); }
   __device__ static V neg(V a) { return -a; }
   // g, the polynomial extrapolation in time through f and n earlier states h1..h4 (n = 1..4) of

@@ -155,19 +155,23 @@ __device__ __forceinline__ T dot4(const Q4<T>& a, const Q4<T>& b, T q) {
 }
 
 // ------------------------------------------------------------------------------ solver scalars
-// The decisions of one instance's solve, shared by every kernel that runs it. Sums are doubles.
-// after the residual: tot = ||r sc||^2, ||R sc||^2, ||B^-1 r sc||^2. Returns 0 when the step's
-// solve ends here, 1 when a Krylov solve starts.
-__device__ __forceinline__ int after_resid(InstState& st, const double (&tot)[3], double tol, double inner_tol,
+// The decisions of one instance's solve, shared by every kernel that runs it, on the types of the
+// sums they follow from: one thread's FP64 divisions and conversions between two passes would cost
+// more than the passes.
+// after the residual: tot = ||r sc||^2, ||R sc||^2, ||B^-1 r sc||^2 (R: its sums' type, RK: the Krylov
+// scalars'). Returns 0 when the step's solve ends here, 1 when a Krylov solve starts.
+template <typename RK, typename R>
+__device__ __forceinline__ int after_resid(InstState& st, const R (&tot)[3], double tol, double inner_tol,
                                            int max_refine, int precond) {
   st.ycur ^= 1;
   st.has_x = 0;
-  if (st.refines == 0) st.bb = tot[1];
+  if (st.refines == 0) st.bb = stored(tot[1]);
   st.refines += 1;
   st.cum_refines += 1;
-  st.rr64 = tot[0];
-  st.rel = st.bb > 0 ? sqrt(tot[0] / st.bb) : 0.0;
-  if (!(st.rel > tol)) {
+  st.rr64 = stored(tot[0]);
+  const R bb = num<R>(st.bb);
+  const R bound = rmul(rfrom<R>(tol * tol), bb);  // ||r|| <= tol ||R||
+  if (!rgt(tot[0], bound)) {
     st.outer_active = 0;
     st.status = ST_OK;
     return 0;
@@ -181,23 +185,24 @@ __device__ __forceinline__ int after_resid(InstState& st, const double (&tot)[3]
   st.iters = 0;
   // the Krylov's residual is B^-1 r: its target is the relative reduction asked, or the final
   // tolerance carried into preconditioned units by this pass's norm ratio
-  const double rrk = precond ? tot[2] : tot[0];
-  st.rr = rrk;
-  const double a = __dmul_rn(__dmul_rn(inner_tol, inner_tol), rrk);
-  const double bnd =
-      __dmul_rn(__dmul_rn(__dmul_rn(0.0625, __dmul_rn(tol, tol)), st.bb), precond && tot[0] > 0.0 ? rrk / tot[0] : 1.0);
-  st.rr_target = a > bnd ? a : bnd;
+  const R rrk = precond ? tot[2] : tot[0];
+  st.rr = stored(rto(rrk, RK{}));
+  const R a = rmul(rfrom<R>(inner_tol * inner_tol), rrk);
+  R bnd = rmul(rfrom<R>(0.0625), bound);
+  if (precond && rgt(tot[0], rfrom<R>(0.0f))) bnd = rmul(bnd, rdiv(rrk, tot[0]));
+  st.rr_target = stored(rto(rgt(a, bnd) ? a : bnd, RK{}));
   return 1;
 }
 // after v = B^-1 A~ p: tot = (r^, v), (r, r) (the latter only formed on a restart)
-__device__ __forceinline__ void after_v(InstState& st, const double (&tot)[2]) {
+template <typename R>
+__device__ __forceinline__ void after_v(InstState& st, const R (&tot)[2]) {
   if (st.restart) {
-    st.rho = st.iters == 0 ? st.rr : tot[1];  // (r^, r) with r^ = r
+    st.rho = st.iters == 0 ? st.rr : stored(tot[1]);  // (r^, r) with r^ = r
     st.restart = 0;
   }
-  const double den = tot[0];
-  if (den != 0.0 && isfinite(den) && st.rho != 0.0) {
-    st.alpha = st.rho / den;
+  const R rho = num<R>(st.rho), alpha = rdiv(rho, tot[0]);
+  if (rhead(tot[0]) != 0 && isfinite(rhead(alpha)) && rhead(rho) != 0) {
+    st.alpha = stored(alpha);
   } else {
     st.alpha = 0.0;  // breakdown: this iteration degenerates to a minimal-residual step
     st.restart = 1;
@@ -206,27 +211,31 @@ __device__ __forceinline__ void after_v(InstState& st, const double (&tot)[2]) {
 // after t = B^-1 A~ s: tot = (t, s), (t, t), (s, s), (r^, s), (r^, t). The next residual is r = s -
 // omega t, so (r, r) and (r^, r) follow from these sums and the pass that would form them is not
 // needed. Returns 1 when this Krylov solve ends.
-__device__ __forceinline__ int after_t(InstState& st, const double (&tot)[5], int max_iters) {
-  const double ts = tot[0], tt = tot[1];
-  st.omega = tt > 0.0 && isfinite(ts) ? ts / tt : 0.0;
-  if (st.omega == 0.0) st.restart = 1;
-  const double om = st.omega;
-  st.rr = __fma_rn(om, __fma_rn(om, tt, -2.0 * ts), tot[2]);
-  const double rhoN = __fma_rn(-om, tot[4], tot[3]);
+template <typename R>
+__device__ __forceinline__ int after_t(InstState& st, const R (&tot)[5], int max_iters) {
+  const R ts = tot[0], tt = tot[1];
+  R om = rfrom<R>(0.0f);
+  if (rhead(tt) > 0 && isfinite(rhead(ts))) om = rdiv(ts, tt);
+  if (!isfinite(rhead(om))) om = rfrom<R>(0.0f);
+  st.omega = stored(om);
+  if (rhead(om) == 0) st.restart = 1;
+  const R rr = rfma(om, rfma(om, tt, rneg(radd(ts, ts))), tot[2]);
+  const R rhoN = rfma(rneg(om), tot[4], tot[3]);
+  st.rr = stored(rr);
   st.iters += 1;
   st.iters_total += 1;
   st.cum_iters += 1;
-  if (!(st.rr > st.rr_target) || st.iters >= max_iters || !isfinite(st.rr)) {
+  if (!rgt(rr, num<R>(st.rr_target)) || st.iters >= max_iters || !isfinite(rhead(rr))) {
     st.has_x = 1;
     return 1;
   }
-  const double beta = (rhoN / st.rho) * (st.alpha / om);
-  st.rho = rhoN;
-  if (!isfinite(beta) || rhoN == 0.0) {
+  const R beta = rmul(rdiv(rhoN, num<R>(st.rho)), rdiv(num<R>(st.alpha), om));
+  st.rho = stored(rhoN);
+  if (!isfinite(rhead(beta)) || rhead(rhoN) == 0) {
     st.restart = 1;
     st.beta = 0.0;
   } else {
-    st.beta = beta;
+    st.beta = stored(beta);
   }
   return 0;
 }
@@ -344,9 +353,9 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
     }
     const int sl = (c - I.chunk0) * (CH / Sums::SEG);
     sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
-    double tot[3];
+    R tot[3];
     if (chunk_finish<3, R>(st, PH_RESID, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
-      if (after_resid(st, tot, tol, inner_tol, max_refine, cm.precond)) {
+      if (after_resid<typename RedOf<T>::R, R>(st, tot, tol, inner_tol, max_refine, cm.precond)) {
         st.inner_active = 1;
         atomicAdd(&cm.ctl->n_inner, 1);
       } else {
@@ -393,7 +402,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     const InstDev I = cm.inst[b];
     const int it = st.iters;  // iterations finished; this one is it + 1
     const bool rs = st.restart != 0;
-    const T alpha = (T)st.alpha, beta = (T)st.beta, omega = (T)st.omega;
+    const T alpha = rhead(num<R>(st.alpha)), beta = rhead(num<R>(st.beta)), omega = rhead(num<R>(st.omega));
     const T* ro = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
     const T* po = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
     const T* vo = sel2(kr.v, it & 1);
@@ -459,7 +468,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     }
     const int sl = (c - I.chunk0) * (CH / Sums::SEG);
     sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
-    double tot[2];
+    R tot[2];
     if (chunk_finish<2, R>(st, PH_K1, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0)
       after_v(st, tot);
   });
@@ -484,7 +493,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     InstState& st = cm.st[b];
     const InstDev I = cm.inst[b];
     const int it = st.iters;
-    const T alpha = (T)st.alpha;
+    const T alpha = rhead(num<R>(st.alpha));
     const T* r = it > 0 ? sel2(kr.r, (it + 1) & 1) : kr.rh;
     const T* vv = sel2(kr.v, (it + 1) & 1);
     const int P = I.pitch;
@@ -527,7 +536,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     }
     const int sl = (c - I.chunk0) * (CH / Sums::SEG);
     sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
-    double tot[5];
+    R tot[5];
     if (chunk_finish<5, R>(st, PH_K2, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
       if (after_t(st, tot, max_iters)) {
         st.fin_seq = seq;
@@ -552,7 +561,8 @@ __device__ __forceinline__ void bicg3_body(const Common& cm, const Kry<T>& kr, u
     const InstState& st = cm.st[b];
     const InstDev I = cm.inst[b];
     const int it = st.iters;  // the solve's last iteration
-    const T alpha = (T)st.alpha, omega = (T)st.omega;
+    using R = typename RedOf<T>::R;
+    const T alpha = rhead(num<R>(st.alpha)), omega = rhead(num<R>(st.omega));
     const T* rr = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
     const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
     const T* vv = sel2(kr.v, it & 1);
@@ -648,7 +658,7 @@ __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int
 __device__ __forceinline__ void after_polish(InstState& st, double mass, double rsum, double clamped, double gmin) {
   st.min_f = gmin;
   st.clamped = (long long)clamped;
-  st.mass_drift = rsum != 0.0 ? fabs(mass - rsum) / fabs(rsum) : 0.0;
+  st.mass_drift = rsum != 0.0 ? div64(fabs(mass - rsum), fabs(rsum)) : 0.0;
   st.steps += 1;
   st.hslot = (st.hslot + 1) % kHist;
   st.nhist = min(st.nhist + 1, kOrder);

@@ -19,20 +19,22 @@ namespace sg {
 
 // Meets the team's other blocks: counts this block in and waits until nb blocks have arrived that
 // often. The wait is bounded (a launch is cooperative, so the others are running: milliseconds at
-// most); a block that gives up records it and leaves, and so do the others in their turn.
+// most); a block that gives up records it and leaves, and so do the others in their turn. The block
+// barriers around one thread's release and acquire order every thread's accesses. Measured with 512
+// bytes written before and read after it by every block: 1.42 us at 9 to 152 blocks; further
+// fences around the two cost 0.27 us, and a flag per block that every block polls 2.98 us at 152.
 struct TeamBar {
   unsigned* cnt;
   unsigned target;
   int nb;
 };
 constexpr int kTeamSpin = 1 << 25;  // polls of ~0.7 us
-__device__ __forceinline__ bool team_sync(TeamBar& tb, int* err) {
+__device__ __forceinline__ bool team_sync(TeamBar& tb, volatile int* stat) {
   __shared__ int s_ok;
   __syncthreads();
   if (tb.nb == 1) return true;
   if (threadIdx.x == 0) {
     tb.target += (unsigned)tb.nb;
-    __threadfence();
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(tb.cnt) : "memory");
     unsigned v;
     int ok = 0;
@@ -43,8 +45,7 @@ __device__ __forceinline__ bool team_sync(TeamBar& tb, int* err) {
         break;
       }
     }
-    if (!ok) atomicExch(err, 1);
-    __threadfence();
+    if (!ok) stat[TEAM_GAVE_UP] = 1;
     s_ok = ok;
   }
   __syncthreads();
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
           for (int w = 1; w < kTeamThreads / 32; ++w) rmax = fmaxf(rmax, s_w[w]);
           tmax[sh.rank] = rmax;
         }
-        if (!(ok = team_sync(bar, ta.err))) break;
+        if (!(ok = team_sync(bar, ta.stat))) break;
         float m = 0.0f;
         for (int k = tid; k < sh.nb; k += kTeamThreads) m = fmaxf(m, __ldcg(tmax + k));
 #pragma unroll
@@ -226,14 +227,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
           }
           team_store<3, R, R>(reinterpret_cast<const R*>(parts), np, SEG, nseg, reinterpret_cast<R*>(part()),
                               cm.pstride, seg0);
-          if (!(ok = team_sync(bar, ta.err))) break;
+          if (!(ok = team_sync(bar, ta.stat))) break;
           seg_total<3, R>(reinterpret_cast<const R*>(part()), cm.pstride, I.seg0, I.nseg,
                           reinterpret_cast<R*>(s_tot));
           flip ^= 1;
           if (tid == 0) {
             const R* tt = reinterpret_cast<const R*>(s_tot);
-            const double tot[3] = {rdbl(radd(tt[0], tt[1])), rdbl(radd(tt[2], tt[3])), rdbl(radd(tt[4], tt[5]))};
-            s_go = after_resid(S, tot, ta.tol, ta.inner_tol, ta.max_refine, cm.precond);
+            const R tot[3] = {radd(tt[0], tt[1]), radd(tt[2], tt[3]), radd(tt[4], tt[5])};
+            s_go = after_resid<RK, R>(S, tot, ta.tol, ta.inner_tol, ta.max_refine, cm.precond);
           }
           __syncthreads();
           if (!s_go) break;
@@ -267,7 +268,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             const int it = S.iters;
             const bool rs = S.restart != 0;
             if (it > 0) {  // update by the previous iteration's products; sr holds s
-              const T alpha = (T)S.alpha, beta = (T)S.beta, omega = (T)S.omega;
+              const T alpha = rhead(num<RK>(S.alpha)), beta = rhead(num<RK>(S.beta)),
+                      omega = rhead(num<RK>(S.omega));
               for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
                 const bool halo = l < P || l >= P + own;
                 const Q4<T> t = halo ? ld4cg(kr.t + e0 + l) : ON ? ld4(st_ + (l - P)) : ld4(kr.t + e0 + l);
@@ -326,19 +328,19 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             team_store<2, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
                                   cm.pstride, seg0);
-            if (!(ok = team_sync(bar, ta.err))) break;
+            if (!(ok = team_sync(bar, ta.stat))) break;
             seg_total<2, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
                              reinterpret_cast<RK*>(s_tot));
             flip ^= 1;
             if (tid == 0) {
               const RK* tt = reinterpret_cast<const RK*>(s_tot);
-              const double tot[2] = {rdbl(radd(tt[0], tt[1])), rdbl(radd(tt[2], tt[3]))};
+              const RK tot[2] = {radd(tt[0], tt[1]), radd(tt[2], tt[3])};
               after_v(S, tot);
             }
             __syncthreads();
             // s = r - alpha v over the share and its halo
             {
-              const T alpha = (T)S.alpha;
+              const T alpha = rhead(num<RK>(S.alpha));
               for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
                 Q4<T> v, s = ld4(sr + l);
                 if (l < P || l >= P + own) {
@@ -395,15 +397,15 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             team_store<5, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
                                   cm.pstride, seg0);
-            if (!(ok = team_sync(bar, ta.err))) break;
+            if (!(ok = team_sync(bar, ta.stat))) break;
             seg_total<5, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
                              reinterpret_cast<RK*>(s_tot));
             flip ^= 1;
             if (tid == 0) {
               const RK* tt = reinterpret_cast<const RK*>(s_tot);
-              double tot[5];
+              RK tot[5];
 #pragma unroll
-              for (int k = 0; k < 5; ++k) tot[k] = rdbl(radd(tt[2 * k], tt[2 * k + 1]));
+              for (int k = 0; k < 5; ++k) tot[k] = radd(tt[2 * k], tt[2 * k + 1]);
               s_go = !after_t(S, tot, ta.max_iters);
             }
             __syncthreads();
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
           // the solve's correction over the share and its halo
           {
             const bool one = S.iters == 1;
-            const T alpha = (T)S.alpha, omega = (T)S.omega;
+            const T alpha = rhead(num<RK>(S.alpha)), omega = rhead(num<RK>(S.omega));
             for (int l = 4 * tid; l < ext; l += 4 * kTeamThreads) {
               const Q4<T> s = ld4(sr + l), p = ld4(sp + l);
               Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
@@ -481,7 +483,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             part()[3 * (size_t)cm.pstride + seg0 + k] = (double)m;
           }
         }
-        if (!(ok = team_sync(bar, ta.err))) break;
+        if (!(ok = team_sync(bar, ta.stat))) break;
         double tot[3] = {0.0, 0.0, 0.0}, gmin = 0.0;
         if (last && sh.rank == 0) {
           seg_total<3, double>(part(), cm.pstride, I.seg0, I.nseg, s_tot);
@@ -507,6 +509,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
       S.outer_active = 0;
       S.inner_active = 0;
       cm.st[sh.inst] = S;
+      if (ta.report && S.status == ST_NEGATIVE) ta.stat[TEAM_NEGATIVE] = 1;
+      if (ta.report && S.status == ST_NOT_CONVERGED) ta.stat[TEAM_NOT_CONVERGED] = 1;
     }
     team_leave(bar);
   }

@@ -18,15 +18,18 @@ struct TeamShare {
 
 enum { TEAM_ASSEMBLE = 1, TEAM_SOLVE = 2, TEAM_POLISH = 4, TEAM_STEP = 7 };
 
+enum { TEAM_GAVE_UP = 0, TEAM_NEGATIVE = 1, TEAM_NOT_CONVERGED = 2, TEAM_FLAGS = 3 };
+
 struct TeamArgs {
   const TeamShare* share;
   const int* first;    // block k has shares [first[k], first[k + 1]); more than one only of teams of one
   unsigned* bar;       // kTeamBarStride counters per instance: arrivals, departures
   float* tmax;         // per block: max of the right-hand side over its tiles
-  int* err;            // set when a barrier gave up
+  volatile int* stat;  // TEAM_* flags in mapped host memory: what the launch's last step ended with
   double tol, inner_tol;
   int max_refine, max_iters;
   int nsteps, phases;
+  int report;          // 1: set the flags of the last step
   int seg;             // cells per reduction segment (128 or 1024)
   int own_cap;         // cells of the largest share, rounded up to whole segments
   int pmax;            // widest row pitch
