@@ -206,10 +206,6 @@ struct sayram_batch_s {
     const long long cells = round_up((long long)ny * round_up(nx, 4), 4);
     return (int)((cells + chunk - 1) / chunk);
   }
-  int nsegs_of(const InstDev& I) const {  // reduction segments of an instance
-    const int s = sg::seg_cells(chunk);
-    return (int)(((long long)I.ny * I.pitch + s - 1) / s);
-  }
   // dynamic shared memory of the SpMV kernels: the chunk plus one row above and below
   template <typename T>
   size_t smem_spmv() const { return (size_t)(chunk + 2 * pmax) * sizeof(T); }
@@ -232,6 +228,9 @@ struct sayram_batch_s {
   int team_sms = 0;    // blocks the plan may use (0: one per SM)
   int team_grid = 0;
   bool team_chip = false;
+  bool rmax_clear = false;  // every instance's rmax_bits is 0 (k_team leaves it so)
+  bool team_split = false;  // the assembly as a kernel of its own before each step's launch
+  bool team_bins = false;  // blocks with several whole instances each
   size_t team_smem = 0;
   int team_pmax = 4;
   long long team_own = 0;
@@ -242,6 +241,7 @@ struct sayram_batch_s {
   float* d_tmax = nullptr;
   int* h_stat = nullptr;  // pinned, written by k_team (TEAM_* flags)
   static constexpr int kTeamSteps = 32;
+  static constexpr long long kSplitCells = 2048;
   int plan_team();
   int launch_team(int nsteps, int phases, bool last = true);
   // dispatch of the per-step sequence on precision and chunk size (graph: build it; else: run it)
@@ -610,7 +610,8 @@ int sayram_batch_s::rebuild_lists() {
     I.chunk0 = (int)h_chunk.size();
     for (int k = 0; k < I.nchunks; ++k) h_chunk.push_back(b);
     I.seg0 = nseg;
-    I.nseg = nsegs_of(I);
+    I.seg = sg::seg_cells(chunk, (long long)I.ny * I.pitch);
+    I.nseg = (int)(((long long)I.ny * I.pitch + I.seg - 1) / I.seg);
     nseg += I.nseg;
     I.tile0 = (int)h_tile.size();
     for (int k = 0; k < I.ntx * I.nty; ++k) h_tile.push_back(b);
@@ -640,30 +641,33 @@ int sayram_batch_s::rebuild_lists() {
 // chunks of 4096 cells, whose segments are too coarse to split.
 int sayram_batch_s::plan_team() {
   team_grid = 0;
+  rmax_clear = false;
   if (!coop || chunk == 4096) return SAYRAM_OK;
   std::vector<int> on;
-  long long total = 0;
-  int most = 0;
+  long long total = 0, most = 0;
+  int pm = 4;
+  auto cells = [&](int b) { return (long long)hinst[b].nseg * hinst[b].seg; };
   for (int b = 0; b < cap_slots; ++b)
     if (hinst[b].enabled) {
       on.push_back(b);
-      total += hinst[b].nseg;
-      most = std::max(most, hinst[b].nseg);
+      total += cells(b);
+      most = std::max(most, cells(b));
+      pm = std::max(pm, hinst[b].pitch);
     }
   const int blocks = team_sms > 0 ? std::min(team_sms, nsm) : nsm, ni = (int)on.size();
   if (ni == 0) return SAYRAM_OK;
   std::vector<sg::TeamShare> share;
   std::vector<int> first;
-  const int seg = sg::seg_cells(chunk);
-  long long per = 0;  // segments of the largest share
-  int pm = 4;
-  for (int b : on) pm = std::max(pm, hinst[b].pitch);
-  // the assembly's tile height: the one with the fewest rows (halo included) per block
+  long long own = 0;  // cells of the largest share
+  // The assembly's tile height: the least rows (halo included) that a block goes through, four tiles
+  // at a time (their steps overlap, so a round of them counts as a few rows more).
+  auto tile_count = [](const InstDev& I, int ty) { return (long long)I.ntx * ((I.ny + ty - 1) / ty); };
   auto tile_rows = [&](const InstDev& I, int nb) {
     int best = sg::kTY;
     long long cost = -1;
     for (int ty = sg::kTY; ty >= 2; ty /= 2) {
-      const long long nt = (long long)I.ntx * ((I.ny + ty - 1) / ty), c = (nt + nb - 1) / nb * (ty + 2);
+      const long long per = (tile_count(I, ty) + nb - 1) / nb;
+      const long long c = per * (ty + 2) + (per + sg::kTeamParts - 1) / sg::kTeamParts * 8;
       if (cost < 0 || c < cost) {
         cost = c;
         best = ty;
@@ -672,51 +676,58 @@ int sayram_batch_s::plan_team() {
     return best;
   };
   if (ni <= blocks) {
-    long long lo = std::max<long long>(1, (total + blocks - 1) / blocks), hi = most;
+    // the fewest cells per block with which the teams fit
     auto need = [&](long long q) {
       long long k = 0;
-      for (int b : on) k += (hinst[b].nseg + q - 1) / q;
+      for (int b : on) {
+        const long long s = std::max<long long>(1, q / hinst[b].seg);
+        k += (hinst[b].nseg + s - 1) / s;
+      }
       return k;
     };
+    long long lo = 1, hi = (most + 127) / 128;  // in units of 128 cells
     while (lo < hi) {
       const long long mid = (lo + hi) / 2;
-      if (need(mid) <= blocks) hi = mid;
+      if (need(mid * 128) <= blocks) hi = mid;
       else lo = mid + 1;
     }
-    const long long q = std::max<long long>(lo, 1);
+    if (need(lo * 128) > blocks) return SAYRAM_OK;  // one segment each is already too many: not for teams
+    const long long left = blocks - need(lo * 128);
     for (int b : on) {
       const InstDev& I = hinst[b];
-      const int nb = (int)((I.nseg + q - 1) / q), ty = tile_rows(I, nb);
-      for (int r = 0; r < nb; ++r) {
-        const int s0 = (int)((long long)I.nseg * r / nb), s1 = (int)((long long)I.nseg * (r + 1) / nb);
-        first.push_back((int)share.size());
-        share.push_back({b, r, nb, s0, s1, ty});
-        per = std::max<long long>(per, s1 - s0);
+      const long long s = std::max<long long>(1, lo * 128 / I.seg);
+      const int nb = (int)((I.nseg + s - 1) / s);
+      // blocks that are left over help with the assembly, up to one per smallest tile
+      const long long help = std::min(left * cells(b) / total, std::max<long long>(0, tile_count(I, 2) - nb));
+      const int all = nb + (int)help, ty = tile_rows(I, all);
+      for (int r = 0; r < all; ++r) {
+        const int s0 = r < nb ? (int)((long long)I.nseg * r / nb) : I.nseg;
+        const int s1 = r < nb ? (int)((long long)I.nseg * (r + 1) / nb) : I.nseg;
+        share.push_back({b, r, all, s0, s1, ty});
+        own = std::max<long long>(own, (long long)(s1 - s0) * I.seg);
       }
     }
-    first.push_back((int)share.size());
   } else {
     std::vector<int> order(on);
     std::sort(order.begin(), order.end(), [&](int a, int b) {
-      return hinst[a].nseg != hinst[b].nseg ? hinst[a].nseg > hinst[b].nseg : a < b;
+      return cells(a) != cells(b) ? cells(a) > cells(b) : a < b;
     });
     std::vector<std::vector<int>> bin(blocks);
     std::vector<long long> load(blocks, 0);
     for (int b : order) {
       const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
       bin[k].push_back(b);
-      load[k] += hinst[b].nseg;
+      load[k] += cells(b);
     }
     for (auto& v : bin) {
       first.push_back((int)share.size());
-      for (int b : v) share.push_back({b, 0, 1, 0, hinst[b].nseg, sg::kTY});
+      for (int b : v) share.push_back({b, 0, 1, 0, hinst[b].nseg, tile_rows(hinst[b], 1)});
     }
     first.push_back((int)share.size());
-    per = most;
+    own = most;
   }
   const size_t ts = mixed ? 4 : 8;
   const size_t tile = dwm ? sizeof(sg::AsmTile<sg::DWA>) : sizeof(sg::AsmTile<sg::F64A>);
-  const long long own = per * seg;
   if (!team_limit[1]) {
     SG_CUDA(cudaSetDevice(dev));
     int can = 0;
@@ -735,9 +746,14 @@ int sayram_batch_s::plan_team() {
   bool chip = own <= sg::team_chip_cells(ts) && sg::team_smem(ts, true, own, pm, tile) <= team_limit[1];
   if (!chip && sg::team_smem(ts, false, own, pm, tile) > team_limit[0]) return SAYRAM_OK;
   SG_CUDA(cudaMemcpyAsync(d_share, share.data(), sizeof(sg::TeamShare) * share.size(), cudaMemcpyHostToDevice, stream));
-  SG_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, stream));
+  if (!first.empty())
+    SG_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
-  team_grid = (int)first.size() - 1;
+  team_grid = first.empty() ? (int)share.size() : (int)first.size() - 1;
+  team_bins = !first.empty();
+  // a block of k_team has 16 warps for its tiles, k_assemble up to 48 per SM: with many cells per block
+  // the launch it costs is less than it gains
+  team_split = own >= kSplitCells;
   team_chip = chip;
   team_own = own;
   team_pmax = pm;
@@ -748,7 +764,7 @@ int sayram_batch_s::plan_team() {
 int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   sg::TeamArgs ta{};
   ta.share = d_share;
-  ta.first = d_first;
+  ta.first = team_bins ? d_first : nullptr;
   ta.bar = d_bar;
   ta.tmax = d_tmax;
   ta.stat = h_stat;
@@ -759,7 +775,6 @@ int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   ta.max_iters = opt.max_iters;
   ta.nsteps = nsteps;
   ta.phases = phases;
-  ta.seg = sg::seg_cells(chunk);
   ta.own_cap = (int)team_own;
   ta.pmax = team_pmax;
   sg::TeamLaunch l{team_grid, team_smem, team_chip, stream};
@@ -1016,6 +1031,16 @@ int sayram_batch_s::launch_steps(int nsteps) {
           launch(p.first, [&] { r2 = launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH); });
           if (r2) rc = r2;
         }
+        if (rc) return rc;
+      }
+      return SAYRAM_OK;
+    }
+    if (team_split) {
+      for (int s = 0; s < nsteps; ++s) {
+        int rc = rmax_clear ? SAYRAM_OK : launch_begin();
+        rmax_clear = true;
+        if (!rc) rc = launch_assemble(0, -1);
+        if (!rc) rc = launch_team(1, sg::TEAM_SOLVE | sg::TEAM_POLISH, s == nsteps - 1);
         if (rc) return rc;
       }
       return SAYRAM_OK;
@@ -1539,13 +1564,9 @@ int sayram_batch_export_system(sayram_batch b, int idx, double* M5, double* R) {
   if (!b || !M5 || !R || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
-  if (b->dwm)
-    sg::k_assemble<float, sg::DWA><<<b->grid_tiles(), sg::kAsmThreads, 0, b->stream>>>(b->cm, b->geo, b->fl, b->c32, 0, -1);
-  else if (b->mixed)
-    sg::k_assemble<float, sg::F64A><<<b->grid_tiles(), sg::kAsmThreads, 0, b->stream>>>(b->cm, b->geo, b->fl, b->c32, 0, -1);
-  else
-    sg::k_assemble<double, sg::F64A><<<b->grid_tiles(), sg::kAsmThreads, 0, b->stream>>>(b->cm, b->geo, b->fl, b->c64, 0, -1);
-  SG_CUDA(cudaGetLastError());
+  b->rmax_clear = false;
+  int rc = b->launch_assemble(0, -1);
+  if (rc) return rc;
   const size_t rows = (size_t)I.ny * I.pitch;
   std::vector<double> invD(rows), Rr(rows), c[4];
   SG_CUDA(cudaMemcpyAsync(invD.data(), b->fl.invD + I.base, rows * 8, cudaMemcpyDeviceToHost, b->stream));
@@ -2303,7 +2324,8 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   I.chunk0 = 0;
   I.nchunks = (int)((round_up((long long)ny * pitch, 4) + kNoAllocChunk - 1) / kNoAllocChunk);
   I.seg0 = 0;
-  I.nseg = (int)(((long long)ny * pitch + seg_cells(kNoAllocChunk) - 1) / seg_cells(kNoAllocChunk));
+  I.seg = seg_cells(kNoAllocChunk, (long long)ny * pitch);
+  I.nseg = (int)(((long long)ny * pitch + I.seg - 1) / I.seg);
   I.tile0 = 0;
   I.ntx = (nx + kTX - 1) / kTX;
   I.nty = (ny + kTY - 1) / kTY;

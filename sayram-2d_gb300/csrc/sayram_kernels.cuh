@@ -16,7 +16,7 @@
 //   positivity polish y' = R + (I - A~) max(y, 0) a 1-norm contraction.
 //
 // Reductions are deterministic and have one order, whichever kernel runs them: the cells of an
-// instance are cut into segments (Seg<chunk>: 128, 1024 or 4096 cells, by the batch's chunk size),
+// instance are cut into segments (seg_cells: 128 to 4096, by its size and the batch's chunk size),
 // every segment's sum is a fixed tree over its cells, and an instance's total is a fixed tree over
 // its segments (seg_total). In the per-pass kernels the last block to finish an instance's
 // chunks (counted with one atomic per chunk) forms the totals and updates that instance's Krylov
@@ -53,6 +53,7 @@ struct InstDev {
   int chunk0, nchunks;
   int tile0, ntx, nty;
   int seg0, nseg;  // its reduction segments in the partial-sum arrays
+  int seg, pad0;   // cells of one of them
   int xe, ye;     // offsets into the per-vertex-column / per-vertex-row arrays (nx+1 / ny+1)
   int dir[4];     // offsets into the Dirichlet vertex value array (-1 for zero-flux sides)
   double dt;
@@ -256,42 +257,58 @@ __device__ __forceinline__ bool red_writes() {
   return (threadIdx.x & (32 / red_pow2<NQ>() - 1)) == 0 && red_q<NQ>() < NQ;
 }
 
-// Cells of a reduction segment, by the chunk size of the batch. 128 cells (one warp's 4-cell
-// groups) where the chunks are smallest, so that a small instance can be spread over many SMs;
-// 4096 where it is largest, so that a thread sums four groups before the warp's tree.
-template <int CH>
-struct Seg { static constexpr int cells = CH; };
-template <>
-struct Seg<1024> { static constexpr int cells = 128; };
-template <>
-struct Seg<2048> { static constexpr int cells = 1024; };
-__host__ __device__ inline int seg_cells(int chunk) { return chunk == 1024 ? 128 : chunk == 2048 ? 1024 : 4096; }
+// Cells of a reduction segment. 4096 in chunks of 4096, so that a thread sums four groups before the
+// warp's tree; else the fewest of 128 (one warp's 4-cell groups), 256, 512 or 1024 that leave at most
+// 512 segments: short segments let a small instance be spread over many SMs, and the totals are
+// one more chain over the segments in every pass (at 1577 segments of 128 cells, 389 x 517, that
+// took 3.1 us a pass, at 394 of 512 1 us).
+__host__ __device__ inline int seg_cells(int chunk, long long cells) {
+  if (chunk == 4096) return 4096;
+  int s = 128;
+  while (s < 1024 && cells > 512LL * s) s *= 2;
+  return s;
+}
 
-// eight warp sums -> one segment sum, as a fixed tree
+// Cells whose terms one warp adds up before its tree: two 4-cell groups per lane in the longest
+// segments, which halves the trees where they are most of a pass's instructions.
+__host__ __device__ inline int part_cells(int seg) { return seg == 1024 ? 256 : 128; }
+
+// n = 1, 2, 4 or 8 warp sums -> one segment sum, as a fixed tree
 template <typename R>
-__device__ __forceinline__ R tree8(const R* a) {
-  return radd(radd(radd(a[0], a[1]), radd(a[2], a[3])), radd(radd(a[4], a[5]), radd(a[6], a[7])));
+__device__ __forceinline__ R tree(const R* a, int n) {
+  if (n == 1) return a[0];
+  R x = radd(a[0], a[1]);
+  if (n >= 4) x = radd(x, radd(a[2], a[3]));
+  if (n == 8) x = radd(x, radd(radd(a[4], a[5]), radd(a[6], a[7])));
+  return x;
 }
 
 // The totals of NQ quantities over nseg segment sums part[q * stride + seg0 ...]: task (q, h) is one
-// warp adding every second run of 32 segments, lane by lane, then its tree; a total is the sum of
-// its two tasks. Valid for every thread after the call (sm holds 2 * NQ entries).
+// warp adding every eighth run of 32 segments, lane by lane, then its tree; a total is the tree over
+// its eight tasks. In sm[0 .. NQ) for the first warp after the call (sm holds 8 * NQ entries).
 template <int NQ, typename R>
 __device__ __forceinline__ void seg_total(const R* part, long long stride, int seg0, int nseg, R* sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = warp; k < 2 * NQ; k += nw) {
-    const int q = k >> 1, h = k & 1;
-    const double* src = reinterpret_cast<const double*>(part) + (size_t)q * stride + seg0;
+  for (int q = warp >> 3; q < NQ; q += nw >> 3) {
+    const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
     R a = rfrom<R>(0.0f);
-    for (int s = h * 32 + lane; s < nseg; s += 64) {
-      const double w = __ldcg(src + s);
-      a = radd(a, num<R>(w));
-    }
+    if (h * 32 < nseg) {
+      const double* src = reinterpret_cast<const double*>(part) + (size_t)q * stride + seg0;
+#pragma unroll 4
+      for (int s = h * 32 + lane; s < nseg; s += 256) a = radd(a, num<R>(__ldcg(src + s)));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a = radd(a, rshfl(a, o));
-    if (lane == 0) sm[k] = a;
+      for (int o = 16; o > 0; o >>= 1) a = radd(a, rshfl(a, o));
+    }
+    if (lane == 0) sm[8 * q + h] = a;
   }
   __syncthreads();
+  if (warp == 0) {
+    R t = rfrom<R>(0.0f);
+    if (lane < NQ) t = tree(sm + 8 * lane, 8);
+    __syncwarp();
+    if (lane < NQ) sm[lane] = t;
+    __syncwarp();
+  }
 }
 
 // Segment-partial bookkeeping of the per-pass kernels: after the block has stored the segment sums
@@ -301,7 +318,7 @@ template <int NQ, typename R>
 __device__ __forceinline__ bool chunk_finish(InstState& st, int phase, const InstDev& I, const R* part,
                                              long long stride, R (&tot)[NQ]) {
   __shared__ int s_last;
-  __shared__ double s_tot[2 * NQ];
+  __shared__ double s_tot[8 * NQ];
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -315,36 +332,57 @@ __device__ __forceinline__ bool chunk_finish(InstState& st, int phase, const Ins
   seg_total<NQ, R>(part, stride, I.seg0, I.nseg, sm);
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) tot[q] = radd(sm[2 * q], sm[2 * q + 1]);
+    for (int q = 0; q < NQ; ++q) tot[q] = sm[q];
     st.cnt[phase] = 0;
   }
   return true;
 }
 
-// One block's sums of one chunk. add() takes the lane's terms of one 1024-cell row of the chunk and
-// closes the segments that end with it; store() writes the chunk's segment sums to the partials.
+// One block's sums of one chunk: put() closes a part (a warp's sum; in chunks of 4096 cells a warp's
+// share of the whole chunk), store() writes the chunk's segment sums.
 template <int CH, int NQ, typename R>
 struct ChunkSums {
-  static constexpr int SEG = Seg<CH>::cells;
-  static constexpr int kParts = SEG == 4096 ? 8 : CH / 128;  // warp sums of a chunk
+  static constexpr bool kWhole = CH == 4096;              // one segment per chunk
+  static constexpr int kParts = kWhole ? 8 : CH / 128;    // most parts of a chunk
   R (*sm)[kParts];  // [NQ][kParts] in shared memory
-  __device__ __forceinline__ void put(int row, const R (&v)[NQ]) {
+  __device__ __forceinline__ void put(int p, const R (&v)[NQ]) {
     const R t = warp_totals<NQ, R>(v);
-    if (red_writes<NQ>()) sm[red_q<NQ>()][(SEG == 4096 ? 0 : row * 8) + (threadIdx.x >> 5)] = t;
+    if (red_writes<NQ>()) sm[red_q<NQ>()][p] = t;
   }
-  // seg: the chunk's first segment in the partials; nseg: how many of them the instance has; S: what
-  // a segment's sum is stored as (R, or double)
+  // seg: the chunk's first segment in the partials; nseg: how many of them the instance has from there
+  // on; cells: of a segment; S: what a segment's sum is stored as (R, or double)
   template <typename S = R>
-  __device__ __forceinline__ void store(S* part, long long stride, int seg, int nseg) {
+  __device__ __forceinline__ void store(S* part, long long stride, int seg, int nseg, int cells) {
     __syncthreads();
-    constexpr int kSegs = CH / SEG;
-    for (int k = threadIdx.x; k < NQ * kSegs; k += blockDim.x) {
-      const int q = k / kSegs, s = k % kSegs;
-      if (s >= nseg) continue;
-      const R v = SEG == 128 ? sm[q][s] : tree8(&sm[q][s * 8]);
-      part[(size_t)q * stride + seg + s] = rconv<S>(v);
+    if (kWhole) {
+      if (threadIdx.x < NQ) part[(size_t)threadIdx.x * stride + seg] = rconv<S>(tree(sm[threadIdx.x], 8));
+      return;
+    }
+    const int pp = cells / part_cells(cells), ns = min(CH / cells, nseg);
+    for (int k = threadIdx.x; k < NQ * kParts; k += blockDim.x) {
+      const int q = k / kParts, s = k % kParts;
+      if (s < ns) part[(size_t)q * stride + seg + s] = rconv<S>(tree(&sm[q][s * pp], pp));
     }
   }
 };
+
+// Runs group(g) for the 4-cell groups g of a chunk that this thread owns, part by part, and put(p) after
+// the last group of part p.
+template <int CH, typename F, typename P>
+__device__ __forceinline__ void for_parts(int seg, F&& group, P&& put) {
+  if (CH == 4096) {
+#pragma unroll 1
+    for (int k = 0; k < CH / (4 * kThreads); ++k) group((int)threadIdx.x + k * kThreads);
+    put((int)threadIdx.x >> 5);
+  } else {
+    const int part = part_cells(seg);
+#pragma unroll 1
+    for (int p = threadIdx.x >> 5; p < CH / part; p += kThreads / 32) {
+#pragma unroll 1
+      for (int k = 0; k < part / 4; k += 32) group(p * (part / 4) + k + (int)(threadIdx.x & 31));
+      put(p);
+    }
+  }
+}
 
 }  // namespace sg

@@ -632,13 +632,20 @@ struct AsmTile {
   V hS[VY][2];  // the tile's vertex rows: bilinear weights (wB, wT), Solver.cc:333-336
 };
 
-// Assembles the tile of kTX x ty cells at (i0, j0) of instance I by a block of NT threads; returns
-// this thread's max of the right-hand side. yc: the current y buffer; has_g: the idle one holds the
+// Barrier among the NT threads that share a tile: the whole block, or (bar > 0) one of its parts.
+template <int NT>
+__device__ __forceinline__ void tile_sync(int bar) {
+  if (bar == 0) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NT) : "memory");
+}
+
+// Assembles the tile of kTX x ty cells at (i0, j0) of instance I by NT threads (tid: 0 .. NT); returns
+// this warp's max of the right-hand side. yc: the current y buffer; has_g: the idle one holds the
 // extrapolated start.
 template <typename C, typename A, int NT>
 __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const Geo& geo, const Fields& fl,
                                           const Coef<C>& co, const InstDev& I, int i0, int j0, const int ty,
-                                          bool has_g, int yc) {
+                                          bool has_g, int yc, const int tid, const int bar) {
   using V = typename A::V;
   constexpr int HX = AsmTile<A>::HX, VX = AsmTile<A>::VX;
   const int HY = ty + 2, VY = ty + 1;
@@ -652,7 +659,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
   static_assert(kRowT < NT, "step 1 layout");
   // the y-faces start at another warp than the x-faces, so that what is left over of each after whole
   // rounds of the block falls on different warps
-  const int tid = threadIdx.x, tid2 = (threadIdx.x + NT / 2) & (NT - 1);
+  const int tid2 = (tid + NT / 2) & (NT - 1);
   const V zero = A::k(0.0);
   const int nx = I.nx, ny = I.ny, P = I.pitch;
   // 32-bit cell indices: every batch holds fewer than 2^31 cells (checked at allocation), and an
@@ -715,7 +722,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
       }
     }
   }
-  __syncthreads();
+  tile_sync<NT>(bar);
   // 2) vertex values (Solver.cc:299-422): corners copy, interior bilinear, boundary edges
   //    linear, then Dirichlet overrides with XMIN < XMAX < YMIN < YMAX precedence. The bilinear
   //    value wB (wL f00 + wR f10) + wT (wL f01 + wR f11) is formed from the two row
@@ -742,7 +749,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
     }
     S.vS[vy][vx] = val;
   }
-  __syncthreads();
+  tile_sync<NT>(bar);
   // 3a) x-faces (vertex column Iv between cells Iv-1 and Iv)
   for (int q = tid; q < ty * VX; q += NT) {
     const int vx = q % VX, ry = q / VX;
@@ -795,7 +802,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
     S.yB[vy][cx] = Jv == 0 ? bm : aB;
     S.yT[vy][cx] = Jv == ny ? bm : aT;
   }
-  __syncthreads();
+  tile_sync<NT>(bar);
   // 4) per cell: diagonal in the reference's triplet order, RHS, scaling, scatter
   float rmax = 0.0f;
 #pragma unroll
@@ -856,7 +863,7 @@ __global__ void __launch_bounds__(kAsmThreads, A::kAsmBlocks) k_assemble(Common 
     // the extrapolated start g the last polish left in the idle y buffer (none before the first
     // step or after the state was replaced: then y0 = D f)
     const float rmax = asm_tile<C, A, kAsmThreads>(S, cm, geo, fl, co, I, (lt % I.ntx) * kTX, (lt / I.ntx) * kTY, kTY,
-                                                   cm.st[b].nhist > 0, cm.st[b].ycur);
+                                                   cm.st[b].nhist > 0, cm.st[b].ycur, threadIdx.x, 0);
     if ((threadIdx.x & 31) == 0 && rmax > 0.0f) atomicMax(&cm.st[b].rmax_bits, __float_as_uint(rmax));
     __syncthreads();
   }

@@ -48,10 +48,10 @@ __device__ __forceinline__ void for_active_chunks(const Common& cm, W&& want, Bo
 // Fills smem[0 .. n) with a 4-aligned stretch [e0, e0 + n) of a vector computed cell-wise by
 // f(k) -> Q4<T> (k a multiple of 4): the chunk plus one row above and below, so that the stencil
 // of every cell in the chunk reads shared memory only.
-template <typename T, typename F>
-__device__ __forceinline__ void stage_rows(T* sm, long long e0, long long n, F&& f) {
-#pragma unroll 2
-  for (long long q = 4LL * threadIdx.x; q < n; q += 4LL * blockDim.x) {
+template <typename T, int U = 2, typename F>
+__device__ __forceinline__ void stage_rows(T* sm, long long e0, int n, F&& f) {
+#pragma unroll U
+  for (int q = 4 * threadIdx.x; q < n; q += 4 * kThreads) {
     const Q4<T> v = f(e0 + q);
     *reinterpret_cast<Q4<T>*>(sm + q) = v;
   }
@@ -310,7 +310,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].outer_active != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
     InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
+    const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const double* yin = sel2(fl.y64, st.ycur);
     double* yout = sel2(fl.y64, st.ycur ^ 1);
     const bool hx = st.has_x != 0;
@@ -322,7 +322,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
     const long long e0 = c0 - P;
     Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
     // y + x (the last Krylov correction, in scaled units) over the chunk and one row each side
-    stage_rows<V>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+    stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
       Q4<V> y = A::ld4(yin + k);
       if (hx) {
         const Q4<T> x = ld4(kr.x + k);
@@ -334,25 +334,22 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
     __syncthreads();
     typename A::Acc q0 = 0, q1 = 0;
     T q2 = (T)0;
-#pragma unroll 1
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
-      if (K < c1) {
-        Q4<V> yc;
-        Q4<T> r;
-        resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
-        A::st4(yout + K, yc);
-        st4(kr.rh + K, r);
-      }
-      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
-        const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
-        sums.put(g, w);
-        q0 = q1 = 0;
-        q2 = (T)0;
-      }
-    }
-    const int sl = (c - I.chunk0) * (CH / Sums::SEG);
-    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
+    for_parts<CH>(I.seg, [&](int g) {
+      const long long K = c0 + 4 * g;
+      if (K >= c1) return;
+      Q4<V> yc;
+      Q4<T> r;
+      resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
+      A::st4(yout + K, yc);
+      st4(kr.rh + K, r);
+    }, [&](int p) {
+      const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
+      sums.put(p, w);
+      q0 = q1 = 0;
+      q2 = (T)0;
+    });
+    const int sl = (c - I.chunk0) * (CH / I.seg);
+    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl, I.seg);
     R tot[3];
     if (chunk_finish<3, R>(st, PH_RESID, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
       if (after_resid<typename RedOf<T>::R, R>(st, tot, tol, inner_tol, max_refine, cm.precond)) {
@@ -365,7 +362,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
   });
 }
 template <typename T, typename C, typename A, int CH>
-__global__ void __launch_bounds__(kThreads, 4) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
                                                         double tol, double inner_tol, int max_refine) {
   count_launch(cm.ctl);
   resid_body<T, C, A, CH>(cm, fl, co, kr, tol, inner_tol, max_refine);
@@ -399,7 +396,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
     InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
+    const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;  // iterations finished; this one is it + 1
     const bool rs = st.restart != 0;
     const T alpha = rhead(num<R>(st.alpha)), beta = rhead(num<R>(st.beta)), omega = rhead(num<R>(st.omega));
@@ -415,9 +412,9 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     const long long e0 = c0 - P;
     Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
     if (it == 0) {
-      stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) { return ld4(kr.rh + k); });
+      stage_rows<T>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) { return ld4(kr.rh + k); });
     } else {
-      stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+      stage_rows<T, 1>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
         const Q4<T> r = ld4(ro + k), v = ld4(vo + k), t = ld4(kr.t + k);
         Q4<T> p = it > 1 ? ld4(po + k) : r;
         const bool mine = k >= c0 && k < c1;
@@ -446,9 +443,8 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     }
     __syncthreads();
     T q0 = (T)0, q1 = (T)0;
-#pragma unroll 2
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+    for_parts<CH>(I.seg, [&](int g) {
+      const long long K = c0 + 4 * g;
       if (K < c1) {
         const int o = (int)(K - e0);
         const Q4<T> cw = ld4(co.cw + K), ce = ld4(co.ce + K);
@@ -460,14 +456,13 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
         q0 = dot4<T>(rh, v, q0);
         if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
       }
-      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
-        const R w[2] = {rfrom<R>(q0), rfrom<R>(q1)};
-        sums.put(g, w);
-        q0 = q1 = (T)0;
-      }
-    }
-    const int sl = (c - I.chunk0) * (CH / Sums::SEG);
-    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
+    }, [&](int p) {
+      const R w[2] = {rfrom<R>(q0), rfrom<R>(q1)};
+      sums.put(p, w);
+      q0 = q1 = (T)0;
+    });
+    const int sl = (c - I.chunk0) * (CH / I.seg);
+    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl, I.seg);
     R tot[2];
     if (chunk_finish<2, R>(st, PH_K1, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0)
       after_v(st, tot);
@@ -491,7 +486,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
     InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
+    const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;
     const T alpha = rhead(num<R>(st.alpha));
     const T* r = it > 0 ? sel2(kr.r, (it + 1) & 1) : kr.rh;
@@ -501,7 +496,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     const long long c1 = min(c0 + (long long)CH, inst_end(I));
     const long long e0 = c0 - P;
     Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
-    stage_rows<T>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+    stage_rows<T>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
       Q4<T> x = ld4(r + k);
       const Q4<T> v = ld4(vv + k);
 #pragma unroll
@@ -510,9 +505,8 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     });
     __syncthreads();
     T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
-#pragma unroll 2
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+    for_parts<CH>(I.seg, [&](int g) {
+      const long long K = c0 + 4 * g;
       if (K < c1) {
         const int o = (int)(K - e0);
         const Q4<T> s = *reinterpret_cast<const Q4<T>*>(sm + o);
@@ -527,15 +521,14 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
         q[3] = dot4<T>(rh, s, q[3]);
         q[4] = dot4<T>(rh, t, q[4]);
       }
-      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
-        const R w[5] = {rfrom<R>(q[0]), rfrom<R>(q[1]), rfrom<R>(q[2]), rfrom<R>(q[3]), rfrom<R>(q[4])};
-        sums.put(g, w);
+    }, [&](int p) {
+      const R w[5] = {rfrom<R>(q[0]), rfrom<R>(q[1]), rfrom<R>(q[2]), rfrom<R>(q[3]), rfrom<R>(q[4])};
+      sums.put(p, w);
 #pragma unroll
-        for (int k = 0; k < 5; ++k) q[k] = (T)0;
-      }
-    }
-    const int sl = (c - I.chunk0) * (CH / Sums::SEG);
-    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl);
+      for (int k = 0; k < 5; ++k) q[k] = (T)0;
+    });
+    const int sl = (c - I.chunk0) * (CH / I.seg);
+    sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl, I.seg);
     R tot[5];
     if (chunk_finish<5, R>(st, PH_K2, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
       if (after_t(st, tot, max_iters)) {
@@ -559,7 +552,7 @@ __device__ __forceinline__ void bicg3_body(const Common& cm, const Kry<T>& kr, u
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].fin_seq == seq; }, [&](int c) {
     const int b = cm.chunk_inst[c];
     const InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
+    const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;  // the solve's last iteration
     using R = typename RedOf<T>::R;
     const T alpha = rhead(num<R>(st.alpha)), omega = rhead(num<R>(st.omega));
@@ -614,7 +607,8 @@ __device__ __forceinline__ PolishAt polish_at(const Fields& fl, int ycur, int nh
   return a;
 }
 // One 4-cell group from the staged max(y, 0) (sm + o); real: cells of the group inside the grid
-template <typename C, typename A>
+// EARLY: every load is issued before the first is used (more registers: for few warps in flight).
+template <typename C, typename A, bool EARLY>
 __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int P, const Coef<C>& co, long long K,
                                              const Fields& fl, const PolishAt& at, int real, typename A::V& mass,
                                              typename A::V& rsum, float& mn) {
@@ -622,7 +616,16 @@ __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int
   // y' = R + sum over the neighbours of the outflow fraction times max(y, 0): every term is
   // >= 0, accumulated one direction at a time so that one coefficient row is live at once
   const Q4<V> R = A::ld4(fl.R + K);
-  Q4<V> yp = R;
+  Q4<V> yp = R, e_inv, e_cols, e_fn, e_h2, e_h3, e_h4, e_r;
+  if (EARLY) {
+    e_inv = A::ld4(fl.invD + K);
+    e_cols = A::ld4(fl.colsum + K);
+    e_fn = A::ld4(fl.f + K);
+    e_h2 = at.nh >= 2 ? A::ld4(at.h2 + K) : e_fn;
+    e_h3 = at.nh >= 3 ? A::ld4(at.h3 + K) : e_h2;
+    e_h4 = at.nh >= 4 ? A::ld4(at.h4 + K) : e_h3;
+    if (fl.decay) e_r = A::ld4(fl.decay + K);
+  }
 #pragma unroll
   for (int dir = 0; dir < 4; ++dir) {
     const Q4<V> c = CoefW<C, A>::row(co, dir, K);
@@ -630,7 +633,7 @@ __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int
 #pragma unroll
     for (int m = 0; m < 4; ++m) yp.a[m] = A::fmap(c.a[m], sm[on + m], yp.a[m]);
   }
-  const Q4<V> inv = A::ld4(fl.invD + K), cols = A::ld4(fl.colsum + K);
+  const Q4<V> inv = EARLY ? e_inv : A::ld4(fl.invD + K), cols = EARLY ? e_cols : A::ld4(fl.colsum + K);
   Q4<V> fo;
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
@@ -640,15 +643,16 @@ __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int
     rsum = A::addp(rsum, R.a[m]);
     if (m < real) mn = fminf(mn, A::f32(fv));
   }
-  const Q4<V> fn = A::ld4(fl.f + K);
+  const Q4<V> fn = EARLY ? e_fn : A::ld4(fl.f + K);
   Q4<V> g;
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     // the states read here (the oldest one included) are read before the slot is replaced
-    const V h2 = at.nh >= 2 ? A::ld(at.h2, K + m) : fn.a[m];
-    const V h3 = at.nh >= 3 ? A::ld(at.h3, K + m) : h2;
-    const V h4 = at.nh >= 4 ? A::ld(at.h4, K + m) : h3;
-    g.a[m] = A::extrap(fo.a[m], fn.a[m], h2, h3, h4, at.nh, fl.decay ? A::ld(fl.decay, K + m) : A::k(1.0));
+    const V h2 = EARLY ? e_h2.a[m] : at.nh >= 2 ? A::ld(at.h2, K + m) : fn.a[m];
+    const V h3 = EARLY ? e_h3.a[m] : at.nh >= 3 ? A::ld(at.h3, K + m) : h2;
+    const V h4 = EARLY ? e_h4.a[m] : at.nh >= 4 ? A::ld(at.h4, K + m) : h3;
+    const V r = !fl.decay ? A::k(1.0) : EARLY ? e_r.a[m] : A::ld(fl.decay, K + m);
+    g.a[m] = A::extrap(fo.a[m], fn.a[m], h2, h3, h4, at.nh, r);
   }
   A::st4(at.gout + K, g);
   A::st4(at.hw + K, fn);  // f^n into the oldest slot
@@ -676,16 +680,16 @@ template <typename C, typename A, int CH>
 __global__ void __launch_bounds__(kThreads, 4) k_polish(Common cm, Fields fl, Coef<C> co, int c0, int c1) {
   using V = typename A::V;
   using R = typename A::R;
-  using Sums = ChunkSums<CH, 3, R>;
+  using Sums = ChunkSums<CH, 2, R>;
   count_launch(cm.ctl);
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ double s_part[3 * Sums::kParts];
-  __shared__ float s_min[kThreads / 32];
+  __shared__ double s_part[2 * Sums::kParts];
+  __shared__ float s_min[kThreads / 32], s_clamp[kThreads / 32];
   V* sm = reinterpret_cast<V*>(smraw);
   for_active_chunks(cm, [&](int b_) { return cm.inst[b_].enabled != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
     InstState& st = cm.st[b];
-    const InstDev I = cm.inst[b];
+    const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const PolishAt at = polish_at(fl, st.ycur, st.nhist, st.hslot, cm.hist_cap);
     const int P = I.pitch;
     const long long c0 = chunk_start<CH>(c, I);
@@ -693,7 +697,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_polish(Common cm, Fields fl, Co
     const long long e0 = c0 - P;
     Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
     float clamp = 0.0f;
-    stage_rows<V>(sm, e0, (c1 - c0) + 2LL * P, [&](long long k) {
+    stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
       Q4<V> v = A::ld4(at.y + k);
       const bool mine = k >= c0 && k < c1;
 #pragma unroll
@@ -706,26 +710,34 @@ __global__ void __launch_bounds__(kThreads, 4) k_polish(Common cm, Fields fl, Co
     __syncthreads();
     V mass = A::k(0.0), rsum = A::k(0.0);
     float mn = 3.0e38f;
-#pragma unroll 1
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
+    for_parts<CH>(I.seg, [&](int g) {
+      const long long K = c0 + 4 * g;
       if (K < c1)
-        polish_group<C, A>(sm, (int)(K - e0), P, co, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
-      if (Sums::SEG != 4096 || g == CH / (4 * kThreads) - 1) {
-        const R w[3] = {mass, rsum, rfrom<R>(clamp)};
-        sums.put(g, w);
-        mass = rsum = A::k(0.0);
-        clamp = 0.0f;
-      }
-    }
+        polish_group<C, A, false>(sm, (int)(K - e0), P, co, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
+    }, [&](int p) {
+      const R w[2] = {mass, rsum};
+      sums.put(p, w);
+      mass = rsum = A::k(0.0);
+    });
+    // clamped cells (whole numbers) and the minimum: the chunk's, with the first of its segments
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = mn;
-    const int sl = (c - I.chunk0) * (CH / Sums::SEG), left = I.nseg - sl;
-    sums.template store<double>(cm.part, cm.pstride, I.seg0 + sl, left);
-    if (threadIdx.x < CH / Sums::SEG && (int)threadIdx.x < left) {  // the chunk's minimum, for each of its segments
-      float m = s_min[0];
-      for (int w = 1; w < kThreads / 32; ++w) m = fminf(m, s_min[w]);
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      clamp += __shfl_xor_sync(0xffffffffu, clamp, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      s_min[threadIdx.x >> 5] = mn;
+      s_clamp[threadIdx.x >> 5] = clamp;
+    }
+    const int sl = (c - I.chunk0) * (CH / I.seg), left = I.nseg - sl;
+    sums.template store<double>(cm.part, cm.pstride, I.seg0 + sl, left, I.seg);
+    if ((int)threadIdx.x < min(CH / I.seg, left)) {
+      float m = s_min[0], cl = s_clamp[0];
+      for (int w = 1; w < kThreads / 32; ++w) {
+        m = fminf(m, s_min[w]);
+        cl += s_clamp[w];
+      }
+      cm.part[2 * (size_t)cm.pstride + I.seg0 + sl + threadIdx.x] = threadIdx.x == 0 ? (double)cl : 0.0;
       cm.part[3 * (size_t)cm.pstride + I.seg0 + sl + threadIdx.x] = (double)m;
     }
     double tot[3];

@@ -71,16 +71,23 @@ __device__ __forceinline__ Q4<double> ld4cg(const double* p) {
   return Q4<double>{{u.x, u.y, w.x, w.y}};
 }
 
-// Warp sums of a share -> segment sums in the global partials. parts[q][k]: the sum over cells
-// [128 k, 128 (k + 1)) of the share.
+// a plain struct of 4-byte words, copied by the block's first threads
+template <typename X>
+__device__ __forceinline__ void copy_words(X& to, const X& from) {
+  static_assert(sizeof(X) % 4 == 0 && sizeof(X) / 4 <= kTeamThreads, "one word per thread");
+  if (threadIdx.x < sizeof(X) / 4)
+    reinterpret_cast<unsigned*>(&to)[threadIdx.x] = reinterpret_cast<const unsigned*>(&from)[threadIdx.x];
+}
+
+// Warp sums of a share -> segment sums in the global partials. parts[q][p]: the sum over part p.
 template <int NQ, typename R, typename S>
 __device__ __forceinline__ void team_store(const R* parts, int np, int seg, int nseg, S* part, long long stride,
                                            int at) {
   __syncthreads();
+  const int pp = seg / part_cells(seg);
   for (int k = threadIdx.x; k < NQ * nseg; k += kTeamThreads) {
     const int q = k / nseg, s = k - q * nseg;
-    const R v = seg == 128 ? parts[q * np + s] : tree8(&parts[q * np + 8 * s]);
-    part[(size_t)q * stride + at + s] = rconv<S>(v);
+    part[(size_t)q * stride + at + s] = rconv<S>(tree(&parts[q * np + pp * s], pp));
   }
 }
 
@@ -99,7 +106,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ InstState S;
   __shared__ InstDev sI;
-  __shared__ double s_tot[2 * kPartQ];
+  __shared__ double s_tot[8 * kPartQ];
   __shared__ float s_w[kTeamThreads / 32];
   __shared__ int s_go;
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -108,21 +115,22 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
   double* const parts = reinterpret_cast<double*>(smraw);
   unsigned char* const mem = smraw + (((size_t)kPartQ * np * 8 + 15) & ~(size_t)15);
 
-  for (int e = ta.first[blockIdx.x]; e < ta.first[blockIdx.x + 1]; ++e) {
+  const int e_end = ta.first ? ta.first[blockIdx.x + 1] : (int)blockIdx.x + 1;
+  for (int e = ta.first ? ta.first[blockIdx.x] : (int)blockIdx.x; e < e_end; ++e) {
     const TeamShare sh = ta.share[e];
     __syncthreads();
-    if (tid == 0) {
-      sI = cm.inst[sh.inst];
-      S = cm.st[sh.inst];
-    }
+    copy_words(sI, cm.inst[sh.inst]);
+    copy_words(S, cm.st[sh.inst]);
     __syncthreads();
     const InstDev& I = sI;
-    const int P = I.pitch, SEG = ta.seg;
+    const int P = I.pitch, SEG = I.seg;
     const long long c0 = I.base + (long long)sh.s0 * SEG;
     const long long c1 = min(I.base + (long long)sh.s1 * SEG, inst_end(I));
-    const int own = (int)(c1 - c0), ext = own + 2 * P;
+    const int own = sh.s1 > sh.s0 ? (int)(c1 - c0) : 0, ext = own > 0 ? own + 2 * P : 0;
     const int nseg = sh.s1 - sh.s0, seg0 = I.seg0 + sh.s0;
-    const int gend = nseg * SEG / 4;  // groups of whole segments: a multiple of a warp
+    // warps take parts in turn; a part is part/128 groups of every lane
+    const int part_c = part_cells(SEG), pend = nseg * (SEG / part_c), lane = tid & 31;
+    const bool two = part_c == 256;
     const long long e0 = c0 - P;
     TeamBar bar{ta.bar + (size_t)sh.inst * kTeamBarStride, 0u, sh.nb};
     float* const tmax = ta.tmax + (blockIdx.x - sh.rank);
@@ -155,14 +163,17 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
     for (int step = 0; ok && step < ta.nsteps; ++step) {
       // ---------------------------------------------------------------- assembly
       if (ta.phases & TEAM_ASSEMBLE) {
-        AsmTile<A>& tile = *reinterpret_cast<AsmTile<A>*>(mem);
+        // a tile's steps are short between its barriers: each quarter of the block has a tile of its own
+        constexpr int QT = kTeamThreads / kTeamParts;
+        const int part_ = tid / QT;
+        AsmTile<A>& tile = reinterpret_cast<AsmTile<A>*>(mem)[part_];
         const int nty = (I.ny + sh.ty - 1) / sh.ty, nt = I.ntx * nty;
         const bool has_g = S.nhist > 0;
         float rmax = 0.0f;
-        for (int t = sh.rank; t < nt; t += sh.nb) {
-          rmax = fmaxf(rmax, asm_tile<C, A, kTeamThreads>(tile, cm, geo, fl, cf, I, (t % I.ntx) * kTX,
-                                                          (t / I.ntx) * sh.ty, sh.ty, has_g, S.ycur));
-          __syncthreads();
+        for (int t = sh.rank + part_ * sh.nb; t < nt; t += sh.nb * kTeamParts) {
+          rmax = fmaxf(rmax, asm_tile<C, A, QT>(tile, cm, geo, fl, cf, I, (t % I.ntx) * kTX, (t / I.ntx) * sh.ty,
+                                                sh.ty, has_g, S.ycur, tid % QT, 1 + part_));
+          tile_sync<QT>(1 + part_);
         }
         if ((tid & 31) == 0) s_w[warp] = rmax;
         __syncthreads();
@@ -182,18 +193,23 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
 #pragma unroll
           for (int w = 1; w < kTeamThreads / 32; ++w) m = fmaxf(m, s_w[w]);
           S.rmax_bits = m > 0.0f ? __float_as_uint(m) : 0u;
-          S.restart = 0;
-          S.has_x = 0;
-          S.iters = 0;
-          S.iters_total = 0;
-          S.refines = 0;
-          S.clamped = 0;
         }
         __syncthreads();
       }
       // ---------------------------------------------------------------- refinement loop
       if (ta.phases & TEAM_SOLVE) {
         const float sc = rhs_scale(S.rmax_bits), isc = 1.0f / sc;
+        __syncthreads();
+        if (tid == 0) {
+          S.restart = 0;
+          S.has_x = 0;
+          S.iters = 0;
+          S.iters_total = 0;
+          S.refines = 0;
+          S.clamped = 0;
+          S.rmax_bits = 0u;  // where a kernel of its own assembles, it collects the next step's maximum here
+        }
+        __syncthreads();
         for (;;) {
           const double* yin = sel2(fl.y64, S.ycur);
           double* yout = sel2(fl.y64, S.ycur ^ 1);
@@ -208,11 +224,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             *reinterpret_cast<Q4<V>*>(sv + l) = y;
           }
           __syncthreads();
-          for (int g = tid; g < gend; g += kTeamThreads) {
+          for (int p = warp; p < pend; p += kTeamThreads / 32) {
             typename A::Acc q0 = 0, q1 = 0;
             T q2 = (T)0;
-            if (4 * g < own) {
-              const int l = 4 * g;
+            for (int k = 0; k < part_c; k += 128) {
+              const int l = p * part_c + k + 4 * lane;
+              if (l >= own) continue;
               Q4<V> yc;
               Q4<T> r;
               resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
@@ -223,7 +240,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
             const R t = warp_totals<3, R>(w);
-            if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + (g >> 5)] = t;
+            if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + p] = t;
           }
           team_store<3, R, R>(reinterpret_cast<const R*>(parts), np, SEG, nseg, reinterpret_cast<R*>(part()),
                               cm.pstride, seg0);
@@ -233,19 +250,24 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
           flip ^= 1;
           if (tid == 0) {
             const R* tt = reinterpret_cast<const R*>(s_tot);
-            const R tot[3] = {radd(tt[0], tt[1]), radd(tt[2], tt[3]), radd(tt[4], tt[5])};
+            const R tot[3] = {tt[0], tt[1], tt[2]};
             s_go = after_resid<RK, R>(S, tot, ta.tol, ta.inner_tol, ta.max_refine, cm.precond);
           }
           __syncthreads();
           if (!s_go) break;
           // -------------------------------------------------------------- Krylov solve
+          // this thread's k-th group: its first cell in the share
+          const auto cell_of = [&](int k) {
+            return two ? (warp + kTeamThreads / 32 * (k >> 1)) * 256 + (k & 1) * 128 + 4 * lane
+                       : (warp + kTeamThreads / 32 * k) * 128 + 4 * lane;
+          };
           Q4<T> cw[GN], ce[GN], cs[GN], cn[GN];
           if (ON) {
 #pragma unroll
             for (int k = 0; k < GN; ++k) {
-              const int g = tid + k * kTeamThreads;
-              if (4 * g < own) {
-                const long long K = c0 + 4 * g;
+              const int l = cell_of(k);
+              if (l < own) {
+                const long long K = c0 + l;
                 cw[k] = ld4(ck.cw + K);
                 ce[k] = ld4(ck.ce + K);
                 cs[k] = ld4(ck.cs + K);
@@ -290,9 +312,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             __syncthreads();
             // v = B^-1 A~ p
-            const auto product_v = [&](int g, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
+            const auto product_v = [&](int l, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
                                        T& q0, T& q1) {
-              const int l = 4 * g;
               Q4<T> v = stencil_sm<T>(sp, P + l, P, w, ea, so, no);
               if (cm.precond) v = line4<T>(v, line_of<T>(w, ea));
               st4(at_v(P + l), v);
@@ -301,29 +322,32 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               q0 = dot4<T>(rh, v, q0);
               if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
             };
-            const auto put2 = [&](int g, T q0, T q1) {
+            const auto put2 = [&](int p, T q0, T q1) {
               const RK w[2] = {rfrom<RK>(q0), rfrom<RK>(q1)};
               const RK t = warp_totals<2, RK>(w);
-              if (red_writes<2>()) reinterpret_cast<RK*>(parts)[red_q<2>() * np + (g >> 5)] = t;
+              if (red_writes<2>()) reinterpret_cast<RK*>(parts)[red_q<2>() * np + p] = t;
             };
             if (ON) {
+              T q0 = (T)0, q1 = (T)0;
 #pragma unroll
               for (int k = 0; k < GN; ++k) {
-                const int g = tid + k * kTeamThreads;
-                if (g < gend) {
-                  T q0 = (T)0, q1 = (T)0;
-                  if (4 * g < own) product_v(g, cw[k], ce[k], cs[k], cn[k], q0, q1);
-                  put2(g, q0, q1);
-                }
+                const int l = cell_of(k), p = warp + kTeamThreads / 32 * (two ? k >> 1 : k);
+                if (p >= pend) break;
+                if (l < own) product_v(l, cw[k], ce[k], cs[k], cn[k], q0, q1);
+                if (two && !(k & 1)) continue;
+                put2(p, q0, q1);
+                q0 = q1 = (T)0;
               }
             } else {
-              for (int g = tid; g < gend; g += kTeamThreads) {
+              for (int p = warp; p < pend; p += kTeamThreads / 32) {
                 T q0 = (T)0, q1 = (T)0;
-                if (4 * g < own) {
-                  const long long K = c0 + 4 * g;
-                  product_v(g, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q0, q1);
+                for (int k = 0; k < part_c; k += 128) {
+                  const int l = p * part_c + k + 4 * lane;
+                  if (l >= own) continue;
+                  const long long K = c0 + l;
+                  product_v(l, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q0, q1);
                 }
-                put2(g, q0, q1);
+                put2(p, q0, q1);
               }
             }
             team_store<2, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
@@ -334,7 +358,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             flip ^= 1;
             if (tid == 0) {
               const RK* tt = reinterpret_cast<const RK*>(s_tot);
-              const RK tot[2] = {radd(tt[0], tt[1]), radd(tt[2], tt[3])};
+              const RK tot[2] = {tt[0], tt[1]};
               after_v(S, tot);
             }
             __syncthreads();
@@ -356,9 +380,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             __syncthreads();
             // t = B^-1 A~ s
-            const auto product_t = [&](int g, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
+            const auto product_t = [&](int l, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
                                        T (&q)[5]) {
-              const int l = 4 * g;
               Q4<T> t = stencil_sm<T>(sr, P + l, P, w, ea, so, no);
               if (cm.precond) t = line4<T>(t, line_of<T>(w, ea));
               if (ON) st4(st_ + l, t);
@@ -370,29 +393,33 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               q[3] = dot4<T>(rh, s, q[3]);
               q[4] = dot4<T>(rh, t, q[4]);
             };
-            const auto put5 = [&](int g, const T (&q)[5]) {
+            const auto put5 = [&](int p, const T (&q)[5]) {
               const RK w[5] = {rfrom<RK>(q[0]), rfrom<RK>(q[1]), rfrom<RK>(q[2]), rfrom<RK>(q[3]), rfrom<RK>(q[4])};
               const RK t = warp_totals<5, RK>(w);
-              if (red_writes<5>()) reinterpret_cast<RK*>(parts)[red_q<5>() * np + (g >> 5)] = t;
+              if (red_writes<5>()) reinterpret_cast<RK*>(parts)[red_q<5>() * np + p] = t;
             };
             if (ON) {
+              T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
 #pragma unroll
               for (int k = 0; k < GN; ++k) {
-                const int g = tid + k * kTeamThreads;
-                if (g < gend) {
-                  T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
-                  if (4 * g < own) product_t(g, cw[k], ce[k], cs[k], cn[k], q);
-                  put5(g, q);
-                }
+                const int l = cell_of(k), p = warp + kTeamThreads / 32 * (two ? k >> 1 : k);
+                if (p >= pend) break;
+                if (l < own) product_t(l, cw[k], ce[k], cs[k], cn[k], q);
+                if (two && !(k & 1)) continue;
+                put5(p, q);
+#pragma unroll
+                for (int m = 0; m < 5; ++m) q[m] = (T)0;
               }
             } else {
-              for (int g = tid; g < gend; g += kTeamThreads) {
+              for (int p = warp; p < pend; p += kTeamThreads / 32) {
                 T q[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
-                if (4 * g < own) {
-                  const long long K = c0 + 4 * g;
-                  product_t(g, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q);
+                for (int k = 0; k < part_c; k += 128) {
+                  const int l = p * part_c + k + 4 * lane;
+                  if (l >= own) continue;
+                  const long long K = c0 + l;
+                  product_t(l, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q);
                 }
-                put5(g, q);
+                put5(p, q);
               }
             }
             team_store<5, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
@@ -405,7 +432,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               const RK* tt = reinterpret_cast<const RK*>(s_tot);
               RK tot[5];
 #pragma unroll
-              for (int k = 0; k < 5; ++k) tot[k] = radd(tt[2 * k], tt[2 * k + 1]);
+              for (int k = 0; k < 5; ++k) tot[k] = tt[k];
               s_go = !after_t(S, tot, ta.max_iters);
             }
             __syncthreads();
@@ -448,15 +475,17 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
         }
         __syncthreads();
         float mn = 3.0e38f;
-        for (int g = tid; g < gend; g += kTeamThreads) {
+        for (int p = warp; p < pend; p += kTeamThreads / 32) {
           V mass = A::k(0.0), rsum = A::k(0.0);
-          if (4 * g < own) {
-            const long long K = c0 + 4 * g;
-            polish_group<C, A>(sv, P + 4 * g, P, cf, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
+          for (int k = 0; k < part_c; k += 128) {
+            const int l = p * part_c + k + 4 * lane;
+            if (l >= own) continue;
+            const long long K = c0 + l;
+            polish_group<C, A, true>(sv, P + l, P, cf, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
           }
           const R w[2] = {mass, rsum};
           const R t = warp_totals<2, R>(w);
-          if (red_writes<2>()) reinterpret_cast<R*>(parts)[red_q<2>() * np + (g >> 5)] = t;
+          if (red_writes<2>()) reinterpret_cast<R*>(parts)[red_q<2>() * np + p] = t;
         }
         team_store<2, R, double>(reinterpret_cast<const R*>(parts), np, SEG, nseg, part(), cm.pstride, seg0);
         // clamped cells (whole numbers) and the minimum: one entry per share, the rest of its segments 0
@@ -496,7 +525,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
           gmin = s_w[0];
           for (int w = 1; w < kTeamThreads / 32; ++w) gmin = fmin(gmin, (double)s_w[w]);
 #pragma unroll
-          for (int k = 0; k < 3; ++k) tot[k] = radd(s_tot[2 * k], s_tot[2 * k + 1]);
+          for (int k = 0; k < 3; ++k) tot[k] = s_tot[k];
         }
         flip ^= 1;
         if (tid == 0) after_polish(S, tot[0], tot[1], tot[2], gmin);
@@ -505,10 +534,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
     }
     // the instance's state goes back once, by the team's first block (the others only read it
     // before their first barrier)
+    if (ok && sh.rank == 0) {
+      if (tid == 0) S.outer_active = S.inner_active = 0;
+      __syncthreads();
+      copy_words(cm.st[sh.inst], S);
+    }
     if (ok && sh.rank == 0 && tid == 0) {
-      S.outer_active = 0;
-      S.inner_active = 0;
-      cm.st[sh.inst] = S;
       if (ta.report && S.status == ST_NEGATIVE) ta.stat[TEAM_NEGATIVE] = 1;
       if (ta.report && S.status == ST_NOT_CONVERGED) ta.stat[TEAM_NOT_CONVERGED] = 1;
     }

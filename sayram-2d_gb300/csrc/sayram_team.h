@@ -7,9 +7,10 @@
 namespace sg {
 
 constexpr int kTeamThreads = 512;
+constexpr int kTeamParts = 4;  // tiles a block assembles at once, by a quarter of its threads each
 
-// One block's share of one instance: reduction segments [s0, s1). The nb blocks of an instance (its
-// team) are neighbours in the grid, rank 0 first.
+// One block's share of one instance: reduction segments [s0, s1), none for a block that only helps
+// with the assembly. The nb blocks of an instance (its team) are neighbours in the grid, rank 0 first.
 struct TeamShare {
   int inst, rank, nb;
   int s0, s1;
@@ -22,7 +23,8 @@ enum { TEAM_GAVE_UP = 0, TEAM_NEGATIVE = 1, TEAM_NOT_CONVERGED = 2, TEAM_FLAGS =
 
 struct TeamArgs {
   const TeamShare* share;
-  const int* first;    // block k has shares [first[k], first[k + 1]); more than one only of teams of one
+  const int* first;    // block k has shares [first[k], first[k + 1]), more than one only of teams of one;
+                       // null: share k
   unsigned* bar;       // kTeamBarStride counters per instance: arrivals, departures
   float* tmax;         // per block: max of the right-hand side over its tiles
   volatile int* stat;  // TEAM_* flags in mapped host memory: what the launch's last step ended with
@@ -30,7 +32,6 @@ struct TeamArgs {
   int max_refine, max_iters;
   int nsteps, phases;
   int report;          // 1: set the flags of the last step
-  int seg;             // cells per reduction segment (128 or 1024)
   int own_cap;         // cells of the largest share, rounded up to whole segments
   int pmax;            // widest row pitch
 };
@@ -42,7 +43,7 @@ inline size_t team_smem(size_t tsize, bool chip, long long own_cap, long long pm
   const size_t ext = (size_t)(own_cap + 2 * pmax), halo = (size_t)(2 * pmax);
   // r, p, v, x with both halos, t and r^ / r, p (or the staged 8-byte solution), v and x halos
   size_t n = chip ? 4 * ext * tsize + 2 * (size_t)own_cap * tsize : ext * tsize + ext * 8 + 2 * halo * tsize;
-  if (n < tile_bytes) n = tile_bytes;
+  if (n < kTeamParts * tile_bytes) n = kTeamParts * tile_bytes;
   return n + (size_t)kPartQ * (own_cap / 128) * 8 + 16;
 }
 
