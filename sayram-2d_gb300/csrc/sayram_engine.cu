@@ -46,6 +46,8 @@ using sg::InstState;
 
 }  // namespace
 
+constexpr int kTeamSteps = 32;  // most steps of one cooperative launch, which so stays well below a second
+
 struct sayram_batch_s {
   sayram_options opt{};
   int dev = 0;
@@ -240,7 +242,6 @@ struct sayram_batch_s {
   unsigned* d_bar = nullptr;
   float* d_tmax = nullptr;
   int* h_stat = nullptr;  // pinned, written by k_team (TEAM_* flags)
-  static constexpr int kTeamSteps = 32;
   static constexpr long long kSplitCells = 2048;
   int plan_team();
   int launch_team(int nsteps, int phases, bool last = true);
@@ -634,6 +635,42 @@ int sayram_batch_s::rebuild_lists() {
   return plan_team();
 }
 
+namespace {
+
+// Tiles of an instance's assembly when they are ty rows high, and the height of k_team's: the least rows
+// (halo included) that one of its nb blocks goes through, four tiles at a time (their steps overlap, so
+// a round of them counts as a few rows more).
+long long tile_count(const InstDev& I, int ty) { return (long long)I.ntx * ((I.ny + ty - 1) / ty); }
+int team_tile_rows(const InstDev& I, int nb) {
+  int best = sg::kTY;
+  long long cost = -1;
+  for (int ty = sg::kTY; ty >= 2; ty /= 2) {
+    const long long per = (tile_count(I, ty) + nb - 1) / nb;
+    const long long c = per * (ty + 2) + (per + sg::kTeamParts - 1) / sg::kTeamParts * 8;
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = ty;
+    }
+  }
+  return best;
+}
+
+// The shares of instance b over nb blocks that own its segments and `help` that only assemble;
+// returns the most segments of one.
+int split_instance(const InstDev& I, int b, int nb, int help, sg::TeamShare* out) {
+  const int all = nb + help, ty = team_tile_rows(I, all);
+  int most = 0;
+  for (int r = 0; r < all; ++r) {
+    const int s0 = r < nb ? (int)((long long)I.nseg * r / nb) : I.nseg;
+    const int s1 = r < nb ? (int)((long long)I.nseg * (r + 1) / nb) : I.nseg;
+    out[r] = sg::TeamShare{b, r, all, s0, s1, ty};
+    most = std::max(most, s1 - s0);
+  }
+  return most;
+}
+
+}  // namespace
+
 // Splits the enabled instances' reduction segments over the blocks of one cooperative launch: the
 // smallest number of segments per block with which the teams fit (whole instances, largest first,
 // when there are more instances than blocks), then the form that fits the shared memory -- on
@@ -659,22 +696,6 @@ int sayram_batch_s::plan_team() {
   std::vector<sg::TeamShare> share;
   std::vector<int> first;
   long long own = 0;  // cells of the largest share
-  // The assembly's tile height: the least rows (halo included) that a block goes through, four tiles
-  // at a time (their steps overlap, so a round of them counts as a few rows more).
-  auto tile_count = [](const InstDev& I, int ty) { return (long long)I.ntx * ((I.ny + ty - 1) / ty); };
-  auto tile_rows = [&](const InstDev& I, int nb) {
-    int best = sg::kTY;
-    long long cost = -1;
-    for (int ty = sg::kTY; ty >= 2; ty /= 2) {
-      const long long per = (tile_count(I, ty) + nb - 1) / nb;
-      const long long c = per * (ty + 2) + (per + sg::kTeamParts - 1) / sg::kTeamParts * 8;
-      if (cost < 0 || c < cost) {
-        cost = c;
-        best = ty;
-      }
-    }
-    return best;
-  };
   if (ni <= blocks) {
     // the fewest cells per block with which the teams fit
     auto need = [&](long long q) {
@@ -699,13 +720,9 @@ int sayram_batch_s::plan_team() {
       const int nb = (int)((I.nseg + s - 1) / s);
       // blocks that are left over help with the assembly, up to one per smallest tile
       const long long help = std::min(left * cells(b) / total, std::max<long long>(0, tile_count(I, 2) - nb));
-      const int all = nb + (int)help, ty = tile_rows(I, all);
-      for (int r = 0; r < all; ++r) {
-        const int s0 = r < nb ? (int)((long long)I.nseg * r / nb) : I.nseg;
-        const int s1 = r < nb ? (int)((long long)I.nseg * (r + 1) / nb) : I.nseg;
-        share.push_back({b, r, all, s0, s1, ty});
-        own = std::max<long long>(own, (long long)(s1 - s0) * I.seg);
-      }
+      const size_t at = share.size();
+      share.resize(at + nb + (size_t)help);
+      own = std::max<long long>(own, (long long)split_instance(I, b, nb, (int)help, share.data() + at) * I.seg);
     }
   } else {
     std::vector<int> order(on);
@@ -721,7 +738,7 @@ int sayram_batch_s::plan_team() {
     }
     for (auto& v : bin) {
       first.push_back((int)share.size());
-      for (int b : v) share.push_back({b, 0, 1, 0, hinst[b].nseg, tile_rows(hinst[b], 1)});
+      for (int b : v) share.push_back({b, 0, 1, 0, hinst[b].nseg, team_tile_rows(hinst[b], 1)});
     }
     first.push_back((int)share.size());
     own = most;
@@ -2219,12 +2236,14 @@ constexpr int kNoAllocMaxSide = 4096;       // nx, ny limit (host tables are on 
 constexpr int kNoAllocChunk = 1024;  // cells per chunk of the streaming kernels on this path
 constexpr int kNoAllocMaxChunks = (int)(kNoAllocCells / kNoAllocChunk) + 2;
 constexpr int kNoAllocMaxTiles = 8192;
+constexpr int kNoAllocMaxBlocks = 256;  // blocks of the cooperative step
 constexpr size_t kNoAllocTableBytes = 1u << 20;
 constexpr size_t kNoAllocBytes = kNoAllocTableBytes + (size_t)kNoAllocCells * 28 * sizeof(double);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 std::mutex g_noalloc_mu;
+size_t g_noalloc_smem[128] = {};  // shared memory a block of k_team may use, per device
 unsigned char* g_noalloc_base[128] = {};  // device address of g_noalloc_scratch, per device
 
 // Per-cell set-up from separate coefficient arrays (alpha-major) in the caller's device memory:
@@ -2265,6 +2284,9 @@ int noalloc_device_base(int dev, unsigned char** out) {
     cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
     if (e != cudaSuccess || !ptr)
       return fail(SAYRAM_ERR_CUDA, std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e));
+    int can = 0;
+    SG_CUDA(cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, dev));
+    g_noalloc_smem[dev] = can ? sg::team_smem_limit_f64(true) : 0;
     g_noalloc_base[dev] = (unsigned char*)ptr;
   }
   *out = g_noalloc_base[dev];
@@ -2342,6 +2364,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   static thread_local double hxe[kNoAllocMaxSide + 1], hye[kNoAllocMaxSide + 1];
   static thread_local double hwx[2 * (kNoAllocMaxSide + 1)], hwy[2 * (kNoAllocMaxSide + 1)];
   static thread_local int hchunk[kNoAllocMaxChunks], htile[kNoAllocMaxTiles];
+  static thread_local TeamShare hshare[kNoAllocMaxBlocks];
 
   // ---- carve the scratch array
   NoAllocLayout lay{base, base + kNoAllocBytes};
@@ -2355,8 +2378,12 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   double* d_dirv = lay.take<double>(doff > 0 ? doff : 1);
   const long long pstride = 8LL * kNoAllocMaxChunks;
   double* d_part = lay.take<double>(kPartSets * kPartQ * pstride);
+  TeamShare* d_share = lay.take<TeamShare>(kNoAllocMaxBlocks);
+  unsigned* d_bar = lay.take<unsigned>(kTeamBarStride);
+  float* d_tmax = lay.take<float>(kNoAllocMaxBlocks);
+  int* d_stat = lay.take<int>(TEAM_FLAGS);
   unsigned char* tables_end = lay.cur;
-  if (!d_part || tables_end > base + kNoAllocTableBytes) return fail(SAYRAM_ERR_ARG, "tables exceed the scratch");
+  if (!d_stat || tables_end > base + kNoAllocTableBytes) return fail(SAYRAM_ERR_ARG, "tables exceed the scratch");
   lay.cur = base + kNoAllocTableBytes;
   Geo geo{};
   Fields fl{};
@@ -2436,8 +2463,37 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   SG_CUDA(cudaFuncSetAttribute(k_resid<double, double, F64A, kNoAllocChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_na));
   SG_CUDA(cudaFuncSetAttribute(k_polish<double, F64A, kNoAllocChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_na));
   SG_CUDA(cudaGetLastError());
+  // whole steps as one cooperative launch where the instance's vectors fit the chip (all but very wide
+  // grids); else pass by pass from here
+  const int blocks = std::min(nsm, kNoAllocMaxBlocks), per = (I.nseg + blocks - 1) / blocks;
+  const int nb = (I.nseg + per - 1) / per;
+  const int help = (int)std::min<long long>(blocks - nb, std::max<long long>(0, tile_count(I, 2) - nb));
+  const long long own = (long long)split_instance(I, 0, nb, help, hshare) * I.seg;
+  const size_t smem_team = team_smem(sizeof(double), true, own, pitch, sizeof(AsmTile<F64A>));
+  const bool team = own <= team_chip_cells(sizeof(double)) && smem_team <= g_noalloc_smem[dev];
+  int hstat[TEAM_FLAGS] = {};
+  if (team && nsteps > 0) {
+    SG_CUDA(cudaMemcpyAsync(d_share, hshare, sizeof(TeamShare) * (nb + help), cudaMemcpyHostToDevice, stream));
+    TeamArgs ta{};
+    ta.share = d_share;
+    ta.bar = d_bar;
+    ta.tmax = d_tmax;
+    ta.stat = d_stat;
+    ta.tol = o.tol;
+    ta.inner_tol = o.inner_tol;
+    ta.max_refine = o.max_refine;
+    ta.max_iters = o.max_iters;
+    ta.phases = TEAM_STEP;
+    ta.own_cap = (int)own;
+    ta.pmax = (int)pitch;
+    for (int s = 0; s < nsteps; s += ta.nsteps) {
+      ta.nsteps = std::min(nsteps - s, kTeamSteps);
+      SG_CUDA(team_launch_f64(TeamLaunch{nb + help, smem_team, true, stream}, cm, geo, fl, co, kr, ta));
+    }
+    SG_CUDA(cudaMemcpyAsync(hstat, d_stat, sizeof(hstat), cudaMemcpyDeviceToHost, stream));
+  }
   Ctl hctl;
-  for (int s = 0; s < nsteps; ++s) {
+  for (int s = 0; !team && s < nsteps; ++s) {
     SG_CUDA(cudaMemsetAsync(d_ctl, 0, 2 * sizeof(int), stream));
     k_begin<<<1, 32, 0, stream>>>(cm);
     k_assemble<double, F64A><<<gt, kAsmThreads, 0, stream>>>(cm, geo, fl, co, 0, -1);
@@ -2468,6 +2524,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   InstState hs;
   SG_CUDA(cudaMemcpyAsync(&hs, d_st, sizeof(hs), cudaMemcpyDeviceToHost, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
+  if (hstat[TEAM_GAVE_UP]) return fail(SAYRAM_ERR_TIMEOUT, "a device barrier of the cooperative step gave up waiting");
   if (stats_out) {
     stats_out->steps = hs.steps;
     stats_out->t = (double)hs.steps * pd->dt;

@@ -130,12 +130,12 @@ __device__ __forceinline__ void count_launch(Ctl* ctl) {
 }
 
 // ------------------------------------------------------------------------------ FP64 reciprocals
-// 1/b and a/b in FP64 by Newton-Raphson from an FP32 reciprocal (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): the
-// seed's error of ~2^-22 squares twice, so the reciprocal is rounded correctly but for ties within
-// 2^-30 of an ulp, and one residual step rounds the quotient. Four (seven) operations on the FP64
-// pipe; the plain operators measured 4478 cycles for one dependent division of one warp, 68 times a
-// multiply-add. Zeros, subnormals, infinities, NaNs and the outermost exponents take the operators.
+// 1/b and a/b in FP64 from an FP32 reciprocal r0 (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): with e = 1 - m r0, at most
+// 2^-21, 1/m = r0 (1 + e + e^2 + ...) and what the first three terms leave, e^3, is 2^-10 of an ulp;
+// one residual step rounds the quotient. Three (six) operations on the FP64 pipe, which takes 19
+// cycles per SM for a warp's operation. Zeros, subnormals, infinities, NaNs and the outermost
+// exponents take the plain operators.
 __device__ __forceinline__ double rcp64(double b) {
   const int hi = __double2hiint(b), lo = __double2loint(b), e = (hi >> 20) & 0x7ff;
   if (e < 3 || e > 2042) return 1.0 / b;
@@ -144,9 +144,9 @@ __device__ __forceinline__ double rcp64(double b) {
   const float f = __uint_as_float(__funnelshift_l((unsigned)lo, (unsigned)((hi & 0x000fffff) | 0x07f00000), 3));
   const unsigned s = __float_as_uint(__fdividef(1.0f, f));
   const double r0 = __hiloint2double((int)((s >> 3) + 0x38000000u), (int)(s << 29));
-  const double r1 = __fma_rn(r0, __fma_rn(-m, r0, 1.0), r0);
-  const double r2 = __fma_rn(r1, __fma_rn(-m, r1, 1.0), r1);
-  return __hiloint2double((__double2hiint(r2) + (1023 - e) * 0x100000) | (hi & 0x80000000), __double2loint(r2));
+  const double d = __fma_rn(-m, r0, 1.0);
+  const double r = __fma_rn(r0, __fma_rn(d, d, d), r0);
+  return __hiloint2double((__double2hiint(r) + (1023 - e) * 0x100000) | (hi & 0x80000000), __double2loint(r));
 }
 __device__ __forceinline__ double div64(double a, double b) {
   const double r = rcp64(b), q = __dmul_rn(a, r);
@@ -285,17 +285,35 @@ __device__ __forceinline__ R tree(const R* a, int n) {
 
 // The totals of NQ quantities over nseg segment sums part[q * stride + seg0 ...]: task (q, h) is one
 // warp adding every eighth run of 32 segments, lane by lane, then its tree; a total is the tree over
-// its eight tasks. In sm[0 .. NQ) for the first warp after the call (sm holds 8 * NQ entries).
-template <int NQ, typename R>
+// its eight tasks. In sm[0 .. NQ) for the first warp after the call (sm holds 8 * NQ entries). NW:
+// warps of the block; a warp issues the loads of all its tasks before it adds.
+template <int NQ, int NW, typename R>
 __device__ __forceinline__ void seg_total(const R* part, long long stride, int seg0, int nseg, R* sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int q = warp >> 3; q < NQ; q += nw >> 3) {
+  constexpr int G = NW / 8, NT = (NQ + G - 1) / G, NL = NW > 8 ? 4 : 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* src = reinterpret_cast<const double*>(part) + seg0;
+  double w[NT][NL];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int q = (warp >> 3) + G * t;
     const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
-    R a = rfrom<R>(0.0f);
+#pragma unroll
+    for (int k = 0; k < NL; ++k) {
+      const int s = h * 32 + lane + 256 * k;
+      w[t][k] = q < NQ && s < nseg ? __ldcg(src + (size_t)q * stride + s) : 0.0;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int q = (warp >> 3) + G * t, h = (warp - q) & 7;
+    if (q >= NQ) break;
+    R a = num<R>(w[t][0]);
     if (h * 32 < nseg) {
-      const double* src = reinterpret_cast<const double*>(part) + (size_t)q * stride + seg0;
-#pragma unroll 4
-      for (int s = h * 32 + lane; s < nseg; s += 256) a = radd(a, num<R>(__ldcg(src + s)));
+#pragma unroll
+      for (int k = 1; k < NL; ++k)
+        if (h * 32 + 256 * k < nseg) a = radd(a, num<R>(w[t][k]));
+      for (int s = h * 32 + lane + 256 * NL; s < nseg; s += 256)
+        a = radd(a, num<R>(__ldcg(src + (size_t)q * stride + s)));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a = radd(a, rshfl(a, o));
     }
@@ -304,7 +322,7 @@ __device__ __forceinline__ void seg_total(const R* part, long long stride, int s
   __syncthreads();
   if (warp == 0) {
     R t = rfrom<R>(0.0f);
-    if (lane < NQ) t = tree(sm + 8 * lane, 8);
+    if (lane < NQ) t = tree(sm + 8 * lane, nseg > 32 ? 8 : 1);
     __syncwarp();
     if (lane < NQ) sm[lane] = t;
     __syncwarp();
@@ -329,7 +347,7 @@ __device__ __forceinline__ bool chunk_finish(InstState& st, int phase, const Ins
   if (!s_last) return false;
   __threadfence();
   R* sm = reinterpret_cast<R*>(s_tot);
-  seg_total<NQ, R>(part, stride, I.seg0, I.nseg, sm);
+  seg_total<NQ, kThreads / 32, R>(part, stride, I.seg0, I.nseg, sm);
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) tot[q] = sm[q];

@@ -273,8 +273,8 @@ struct CoefW<float, A> {
 // ||B^-1 r||^2.
 template <typename T, typename C, typename A>
 __device__ __forceinline__ void resid_group(const typename A::V* sm, int o, int P, const Coef<C>& co, long long K,
-                                            const double* Rp, float sc, int precond, Q4<typename A::V>& yc, Q4<T>& r,
-                                            typename A::Acc& q0, typename A::Acc& q1, T& q2) {
+                                            const double* Rp, float sc, int precond, bool first, Q4<typename A::V>& yc,
+                                            Q4<T>& r, typename A::Acc& q0, typename A::Acc& q1, T& q2) {
   using V = typename A::V;
   const Q4<V> cw = CoefW<C, A>::row(co, 0, K), ce = CoefW<C, A>::row(co, 1, K);
   const Q4<V> cs = CoefW<C, A>::row(co, 2, K), cn = CoefW<C, A>::row(co, 3, K);
@@ -282,13 +282,13 @@ __device__ __forceinline__ void resid_group(const typename A::V* sm, int o, int 
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const V yv = sm[o + m];
-    const V s1 = A::fma(cn.a[m], sm[o + m + P], A::fma(cs.a[m], sm[o + m - P],
-                        A::fma(ce.a[m], sm[o + m + 1], A::mul(cw.a[m], sm[o + m - 1]))));
-    const V rv = A::sub(R.a[m], A::sub(yv, s1));
+    // (R - y) + the neighbours' inflow, one multiply-add each
+    const V rv = A::fma(cn.a[m], sm[o + m + P], A::fma(cs.a[m], sm[o + m - P],
+                        A::fma(ce.a[m], sm[o + m + 1], A::fma(cw.a[m], sm[o + m - 1], A::sub(R.a[m], yv)))));
     yc.a[m] = yv;
     r.a[m] = A::template scaled<T>(rv, sc);
     q0 = A::sq_scaled(rv, sc, q0);
-    q1 = A::sq_scaled(R.a[m], sc, q1);
+    if (first) q1 = A::sq_scaled(R.a[m], sc, q1);  // ||R|| does not change within a step
   }
   if (precond) {  // the Krylov matrix's couplings (the hi parts in the FP32 modes)
     r = line4<T>(r, line_of<T>(ld4(co.cw + K), ld4(co.ce + K)));
@@ -339,7 +339,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       if (K >= c1) return;
       Q4<V> yc;
       Q4<T> r;
-      resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
+      resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, st.refines == 0, yc, r, q0, q1, q2);
       A::st4(yout + K, yc);
       st4(kr.rh + K, r);
     }, [&](int p) {
@@ -362,7 +362,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
   });
 }
 template <typename T, typename C, typename A, int CH>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
+__global__ void __launch_bounds__(kThreads, 3) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
                                                         double tol, double inner_tol, int max_refine) {
   count_launch(cm.ctl);
   resid_body<T, C, A, CH>(cm, fl, co, kr, tol, inner_tol, max_refine);

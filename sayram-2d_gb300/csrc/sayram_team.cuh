@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               if (l >= own) continue;
               Q4<V> yc;
               Q4<T> r;
-              resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, yc, r, q0, q1, q2);
+              resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, S.refines == 0, yc, r, q0, q1, q2);
               A::st4(yout + c0 + l, yc);
               st4(sr + P + l, r);
               if (ON) st4(srh + l, r);
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
           team_store<3, R, R>(reinterpret_cast<const R*>(parts), np, SEG, nseg, reinterpret_cast<R*>(part()),
                               cm.pstride, seg0);
           if (!(ok = team_sync(bar, ta.stat))) break;
-          seg_total<3, R>(reinterpret_cast<const R*>(part()), cm.pstride, I.seg0, I.nseg,
+          seg_total<3, kTeamThreads / 32, R>(reinterpret_cast<const R*>(part()), cm.pstride, I.seg0, I.nseg,
                           reinterpret_cast<R*>(s_tot));
           flip ^= 1;
           if (tid == 0) {
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             team_store<2, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
                                   cm.pstride, seg0);
             if (!(ok = team_sync(bar, ta.stat))) break;
-            seg_total<2, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
+            seg_total<2, kTeamThreads / 32, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
                              reinterpret_cast<RK*>(s_tot));
             flip ^= 1;
             if (tid == 0) {
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             team_store<5, RK, RK>(reinterpret_cast<const RK*>(parts), np, SEG, nseg, reinterpret_cast<RK*>(part()),
                                   cm.pstride, seg0);
             if (!(ok = team_sync(bar, ta.stat))) break;
-            seg_total<5, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
+            seg_total<5, kTeamThreads / 32, RK>(reinterpret_cast<const RK*>(part()), cm.pstride, I.seg0, I.nseg,
                              reinterpret_cast<RK*>(s_tot));
             flip ^= 1;
             if (tid == 0) {
@@ -515,17 +515,21 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
         if (!(ok = team_sync(bar, ta.stat))) break;
         double tot[3] = {0.0, 0.0, 0.0}, gmin = 0.0;
         if (last && sh.rank == 0) {
-          seg_total<3, double>(part(), cm.pstride, I.seg0, I.nseg, s_tot);
-          double m = 1.0e300;
-          for (int k = tid; k < I.nseg; k += kTeamThreads) m = fmin(m, __ldcg(part() + 3 * (size_t)cm.pstride + I.seg0 + k));
+          seg_total<3, kTeamThreads / 32, double>(part(), cm.pstride, I.seg0, I.nseg, s_tot);
+          float m = 3.0e38f;  // the minima are FP32 values
+          for (int k = tid; k < I.nseg; k += kTeamThreads)
+            m = fminf(m, (float)__ldcg(part() + 3 * (size_t)cm.pstride + I.seg0 + k));
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
-          if ((tid & 31) == 0) s_w[warp] = (float)m;  // the minima are FP32 values
+          for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+          if ((tid & 31) == 0) s_w[warp] = m;
           __syncthreads();
-          gmin = s_w[0];
-          for (int w = 1; w < kTeamThreads / 32; ++w) gmin = fmin(gmin, (double)s_w[w]);
+          if (tid == 0) {
 #pragma unroll
-          for (int k = 0; k < 3; ++k) tot[k] = s_tot[k];
+            for (int w = 1; w < kTeamThreads / 32; ++w) m = fminf(m, s_w[w]);
+            gmin = (double)m;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) tot[k] = s_tot[k];
+          }
         }
         flip ^= 1;
         if (tid == 0) after_polish(S, tot[0], tot[1], tot[2], gmin);
