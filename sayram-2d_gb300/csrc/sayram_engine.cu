@@ -203,6 +203,7 @@ struct sayram_batch_s {
   // launch shape of the streaming kernels: cells per chunk (one block iteration) and blocks per SM
   int chunk = 2048;
   int gmult = 16;
+  int grid_inst() const { return std::max(1, std::min(cap_slots, nsm * 8)); }
   int grid_stream() const { return std::max(1, std::min(cap_chunks, nsm * gmult)); }
   int nchunks_of(int nx, int ny) const {
     const long long cells = round_up((long long)ny * round_up(nx, 4), 4);
@@ -925,7 +926,8 @@ int sayram_batch_s::step_once(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, c
   launch("assemble", [&] { k_assemble<C, A><<<gt, kAsmThreads, 0, stream>>>(cm, geo, fl, cfull, 0, -1); });
   for (int o = 0; o < opt.max_refine; ++o) {
     launch("resid", [&] {
-      k_resid<T, C, A, CH><<<gs, kThreads, smem_wide(), stream>>>(cm, fl, cfull, kr, opt.tol, opt.inner_tol, opt.max_refine);
+      k_resid<T, C, A, CH><<<gs, kThreads, smem_wide(), stream>>>(cm, fl, cfull, kr);
+      k_after_resid<T, A><<<grid_inst(), kThreads, 0, stream>>>(cm, opt.tol, opt.inner_tol, opt.max_refine);
     });
     SG_CUDA(cudaGetLastError());
     if (o == opt.max_refine - 1) break;
@@ -945,9 +947,12 @@ int sayram_batch_s::step_once(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, c
         tail = 10LL * h_ctl->n_inner < (long long)n_enabled();
       }
       launch(tail ? "krylov_tail10" : "krylov_rest", [&] {
-        launch("bicg1", [&] { k_bicg1<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr); });
-        launch("bicg2", [&] { k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr, opt.max_iters); });
-        launch("bicg3", [&] { k_bicg3<T, CH><<<gs, kThreads, 0, stream>>>(cm, kr); });
+        launch("bicg1", [&] {
+          k_bicg1<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr);
+          k_after_v<T><<<grid_inst(), kThreads, 0, stream>>>(cm);
+        });
+        launch("bicg2", [&] { k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(cm, ck, kr); });
+        launch("bicg3", [&] { k_after_t<T><<<grid_inst(), kThreads, 0, stream>>>(cm, opt.max_iters); });
       });
       SG_CUDA(cudaGetLastError());
       if (!timing && (it < 4 || (it & 3) == 3)) {
@@ -1015,7 +1020,8 @@ int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck,
   c2.h_inner = hin;
   cudaGraphNode_t rnode;
   SG_CUDA(cudaStreamBeginCaptureToGraph(stream, obody, nullptr, nullptr, 0, mode));
-  k_resid<T, C, A, CH><<<gs, kThreads, smem_wide(), stream>>>(c2, fl, cfull, kr, opt.tol, opt.inner_tol, opt.max_refine);
+  k_resid<T, C, A, CH><<<gs, kThreads, smem_wide(), stream>>>(c2, fl, cfull, kr);
+  k_after_resid<T, A><<<grid_inst(), kThreads, 0, stream>>>(c2, opt.tol, opt.inner_tol, opt.max_refine);
   if ((rc = last_captured(&rnode))) { cudaStreamEndCapture(stream, &obody); return rc; }
   SG_CUDA(cudaStreamEndCapture(stream, &obody));
   // inner WHILE inside the outer body
@@ -1029,8 +1035,9 @@ int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck,
   cudaGraph_t ibody = ip.conditional.phGraph_out[0];
   SG_CUDA(cudaStreamBeginCaptureToGraph(stream, ibody, nullptr, nullptr, 0, mode));
   k_bicg1<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(c2, ck, kr);
-  k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(c2, ck, kr, opt.max_iters);
-  k_bicg3<T, CH><<<gs, kThreads, 0, stream>>>(c2, kr);
+  k_after_v<T><<<grid_inst(), kThreads, 0, stream>>>(c2);
+  k_bicg2<T, CH><<<gs, kThreads, smem_spmv<T>(), stream>>>(c2, ck, kr);
+  k_after_t<T><<<grid_inst(), kThreads, 0, stream>>>(c2, opt.max_iters);
   SG_CUDA(cudaStreamEndCapture(stream, &ibody));
   // suffix (the solve-only graph leaves the polish to its caller)
   if (prefix) {
@@ -1318,6 +1325,18 @@ namespace sg {
 int host_fail(int code, const std::string& msg) { return fail(code, msg); }
 }  // namespace sg
 
+namespace {
+// up to kMost 8-byte values handed to the device with a launch
+struct PutArgs {
+  static constexpr int kMost = 480;
+  int n;
+  double v[kMost];
+};
+__global__ void k_put(double* dst, PutArgs p) {
+  for (int k = threadIdx.x; k < p.n; k += blockDim.x) dst[k] = p.v[k];
+}
+}  // namespace
+
 // ================================================================================== C-ABI
 extern "C" {
 
@@ -1550,10 +1569,14 @@ int sayram_batch_set_dirichlet(sayram_batch b, int idx, int side, const double* 
   const int m = (side <= 1) ? I.ny + 1 : I.nx + 1;
   if (n != m) return fail(SAYRAM_ERR_ARG, "expected " + std::to_string(m) + " vertex values");
   SG_CUDA(cudaSetDevice(b->dev));
-  std::vector<double> wv(m);
-  for (int k = 0; k < m; ++k) wv[k] = b->wide(v[k]);
-  SG_CUDA(cudaMemcpyAsync(b->d_dirv + I.dir[side], wv.data(), sizeof(double) * m, cudaMemcpyHostToDevice, b->stream));
-  SG_CUDA(cudaStreamSynchronize(b->stream));
+  // the values travel as kernel parameters: no copy to wait for, and the caller's buffer is free at once
+  for (int at = 0; at < m; at += PutArgs::kMost) {
+    PutArgs p;
+    p.n = std::min(m - at, PutArgs::kMost);
+    for (int k = 0; k < p.n; ++k) p.v[k] = b->wide(v[at + k]);
+    k_put<<<1, 256, 0, b->stream>>>(b->d_dirv + I.dir[side] + at, p);
+  }
+  SG_CUDA(cudaGetLastError());
   return SAYRAM_OK;
 }
 
@@ -2523,7 +2546,8 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
     k_begin<<<1, 32, 0, stream>>>(cm);
     k_assemble<double, F64A><<<gt, kAsmThreads, 0, stream>>>(cm, geo, fl, co, 0, -1);
     for (int r = 0; r < o.max_refine; ++r) {
-      k_resid<double, double, F64A, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, fl, co, kr, o.tol, o.inner_tol, o.max_refine);
+      k_resid<double, double, F64A, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, fl, co, kr);
+      k_after_resid<double, F64A><<<1, kThreads, 0, stream>>>(cm, o.tol, o.inner_tol, o.max_refine);
       SG_CUDA(cudaGetLastError());
       if (r == o.max_refine - 1) break;
       SG_CUDA(cudaMemcpyAsync(&hctl, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));
@@ -2531,8 +2555,9 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
       if (hctl.n_outer == 0) break;
       for (int it = 0; it < o.max_iters; ++it) {
         k_bicg1<double, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, co, kr);
-        k_bicg2<double, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, co, kr, o.max_iters);
-        k_bicg3<double, kNoAllocChunk><<<gs, kThreads, 0, stream>>>(cm, kr);
+        k_after_v<double><<<1, kThreads, 0, stream>>>(cm);
+        k_bicg2<double, kNoAllocChunk><<<gs, kThreads, smem_na, stream>>>(cm, co, kr);
+        k_after_t<double><<<1, kThreads, 0, stream>>>(cm, o.max_iters);
         SG_CUDA(cudaGetLastError());
         if (it < 4 || (it & 3) == 3) {
           SG_CUDA(cudaMemcpyAsync(&hctl, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream));

@@ -42,7 +42,7 @@ constexpr double kEps = DBL_EPSILON;  // gEPS, source/common.h:38
 enum { XMIN = 0, XMAX = 1, YMIN = 2, YMAX = 3 };
 enum { DIRICHLET = 0, ZEROFLUX = 1 };
 enum { ST_OK = 0, ST_NOT_CONVERGED = 3, ST_NEGATIVE = 4 };
-enum { PH_K1 = 0, PH_K2 = 1, PH_RESID = 3, PH_POLISH = 4, PH_COUNT = 8 };
+enum { PH_POLISH = 0, PH_COUNT = 2 };
 
 // Per-instance constants.
 struct InstDev {
@@ -72,7 +72,7 @@ struct InstState {
   int ycur, outer_active, inner_active;
   int restart, has_x;
   int iters;               // Krylov iterations of this solve finished so far
-  unsigned int fin_seq;    // Ctl::seq of the iteration its last solve converged in (k_bicg3)
+  int pad_i;
   int iters_total, refines, status;
   int nhist;               // earlier states held in the history buffers (extrapolated start)
   int hslot;               // history buffer holding f^(n-1); f^(n-2), ... are in the ones before it
@@ -88,7 +88,6 @@ struct Ctl {
   unsigned int kdone[8];        // blocks finished per kernel (graph-conditional updates)
   unsigned int outer_loops;     // residual evaluations run by the device-side loop this step
   unsigned int inner_loops;     // Krylov iterations run by the device-side loop this solve
-  unsigned int seq;             // Krylov iterations launched on this batch (one per k_bicg2)
 };
 
 template <typename T>

@@ -549,7 +549,6 @@ static __global__ void k_begin(Common cm) {
     s.restart = 0;
     s.has_x = 0;
     s.iters = 0;
-    s.fin_seq = 0u;
     s.iters_total = 0;
     s.refines = 0;
     s.clamped = 0;
@@ -561,7 +560,6 @@ static __global__ void k_begin(Common cm) {
     cm.ctl->inner_loops = 0u;
     cm.ctl->kdone[0] = 0u;
     cm.ctl->kdone[1] = 0u;
-    cm.ctl->seq = 0u;
   }
 }
 

@@ -299,8 +299,7 @@ __device__ __forceinline__ void resid_group(const typename A::V* sm, int o, int 
 // r = R - A~ (y + x) in the wide arithmetic; writes y + x to the other y buffer and the Krylov's
 // right-hand side B^-1 r (T precision, scaled) to rh.
 template <typename T, typename C, typename A, int CH>
-__device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, const Coef<C>& co, const Kry<T>& kr,
-                                           double tol, double inner_tol, int max_refine) {
+__device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, const Coef<C>& co, const Kry<T>& kr) {
   using V = typename A::V;
   using R = typename A::R;
   using Sums = ChunkSums<CH, 3, R>;
@@ -309,7 +308,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
   V* sm = reinterpret_cast<V*>(smraw);
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].outer_active != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
+    const InstState& st = cm.st[b];
     const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const double* yin = sel2(fl.y64, st.ycur);
     double* yout = sel2(fl.y64, st.ycur ^ 1);
@@ -321,16 +320,33 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
     const long long c1 = min(c0 + (long long)CH, inst_end(I));
     const long long e0 = c0 - P;
     Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
-    // y + x (the last Krylov correction, in scaled units) over the chunk and one row each side
-    stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
-      Q4<V> y = A::ld4(yin + k);
-      if (hx) {
-        const Q4<T> x = ld4(kr.x + k);
+    // y, or y + x (the last Krylov correction, in scaled units), over the chunk and one row each side.
+    // The last iteration's part of x is formed here from its vectors: a pass of its own over the
+    // instances that finish in an iteration would move more bytes and take a launch.
+    if (!hx) {
+      stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) { return A::ld4(yin + k); });
+    } else {
+      using RK = typename RedOf<T>::R;
+      const int it = st.iters;
+      const T alpha = rhead(num<RK>(st.alpha)), omega = rhead(num<RK>(st.omega));
+      const T* rr = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
+      const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
+      const T* vv = sel2(kr.v, it & 1);
+      stage_rows<V, 1>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
+        Q4<V> y = A::ld4(yin + k);
+        const Q4<T> r = ld4(rr + k), v = ld4(vv + k);
+        const Q4<T> p = it > 1 ? ld4(pp + k) : r;
+        Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
+        if (it > 1) x = ld4(kr.x + k);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) y.a[m] = A::template add_scaled<T>(y.a[m], x.a[m], isc);
-      }
-      return y;
-    });
+        for (int m = 0; m < 4; ++m) {
+          const T sv = fmaT(-alpha, v.a[m], r.a[m]);
+          const T xv = fmaT(alpha, p.a[m], fmaT(omega, sv, x.a[m]));
+          y.a[m] = A::template add_scaled<T>(y.a[m], xv, isc);
+        }
+        return y;
+      });
+    }
     __syncthreads();
     typename A::Acc q0 = 0, q1 = 0;
     T q2 = (T)0;
@@ -350,23 +366,12 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
     });
     const int sl = (c - I.chunk0) * (CH / I.seg);
     sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl, I.seg);
-    R tot[3];
-    if (chunk_finish<3, R>(st, PH_RESID, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
-      if (after_resid<typename RedOf<T>::R, R>(st, tot, tol, inner_tol, max_refine, cm.precond)) {
-        st.inner_active = 1;
-        atomicAdd(&cm.ctl->n_inner, 1);
-      } else {
-        atomicSub(&cm.ctl->n_outer, 1);
-      }
-    }
   });
 }
 template <typename T, typename C, typename A, int CH>
-__global__ void __launch_bounds__(kThreads, 3) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr,
-                                                        double tol, double inner_tol, int max_refine) {
+__global__ void __launch_bounds__(kThreads, sizeof(typename A::Acc) == 4 ? 4 : 3) k_resid(Common cm, Fields fl, Coef<C> co, Kry<T> kr) {
   count_launch(cm.ctl);
-  resid_body<T, C, A, CH>(cm, fl, co, kr, tol, inner_tol, max_refine);
-  loop_epilogue(cm, 0);
+  resid_body<T, C, A, CH>(cm, fl, co, kr);
 }
 
 // ------------------------------------------------------------------------------ BiCGSTAB
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_resid(Common cm, Fields fl, Coe
 //     computed once per cell into shared memory (chunk plus one row above and below) and the
 //     stencil reads p there. The first iteration of a solve has p = r = r^ and writes only v.
 // k2: s = r - alpha v staged likewise, t = B^-1 A~ s; the five sums of after_t.
-// k3: x += alpha p + omega s of the instances whose solve ended in this iteration.
+// The residual kernel forms x's last part (alpha p + omega s) of a solve that has ended.
 // The residual's own dot products come from k2's sums (after_t), so no third pass over the vectors
 // separates r from p: 88 B per cell and iteration in FP32 (first iteration 52 B) against 100 B (88
 // B) for update, product and update as three passes, and one barrier or launch less. FP64 is bound
@@ -395,7 +400,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
   T* sm = reinterpret_cast<T*>(smraw);
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
+    const InstState& st = cm.st[b];
     const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;  // iterations finished; this one is it + 1
     const bool rs = st.restart != 0;
@@ -463,21 +468,16 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     });
     const int sl = (c - I.chunk0) * (CH / I.seg);
     sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl, I.seg);
-    R tot[2];
-    if (chunk_finish<2, R>(st, PH_K1, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0)
-      after_v(st, tot);
   });
 }
 template <typename T, int CH>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 5 : 4) k_bicg1(Common cm, Coef<T> co, Kry<T> kr) {
+__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg1(Common cm, Coef<T> co, Kry<T> kr) {
   count_launch(cm.ctl);
-  if (blockIdx.x == 0 && threadIdx.x == 0) cm.ctl->seq += 1u;
   bicg1_body<T, CH>(cm, co, kr);
 }
 
 template <typename T, int CH>
-__device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, const Kry<T>& kr, int max_iters,
-                                           unsigned seq) {
+__device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, const Kry<T>& kr) {
   using R = typename RedOf<T>::R;
   using Sums = ChunkSums<CH, 5, R>;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -485,7 +485,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
   T* sm = reinterpret_cast<T*>(smraw);
   for_active_chunks(cm, [&](int b_) { return cm.st[b_].inner_active != 0; }, [&](int c) {
     const int b = cm.chunk_inst[c];
-    InstState& st = cm.st[b];
+    const InstState& st = cm.st[b];
     const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;
     const T alpha = rhead(num<R>(st.alpha));
@@ -529,59 +529,68 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     });
     const int sl = (c - I.chunk0) * (CH / I.seg);
     sums.store(reinterpret_cast<R*>(cm.part), cm.pstride, I.seg0 + sl, I.nseg - sl, I.seg);
-    R tot[5];
-    if (chunk_finish<5, R>(st, PH_K2, I, reinterpret_cast<const R*>(cm.part), cm.pstride, tot) && threadIdx.x == 0) {
-      if (after_t(st, tot, max_iters)) {
-        st.fin_seq = seq;
-        st.inner_active = 0;
-        atomicSub(&cm.ctl->n_inner, 1);
-      }
-    }
   });
 }
 template <typename T, int CH>
-__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg2(Common cm, Coef<T> co, Kry<T> kr,
-                                                                         int max_iters) {
+__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg2(Common cm, Coef<T> co, Kry<T> kr) {
   count_launch(cm.ctl);
-  bicg2_body<T, CH>(cm, co, kr, max_iters, cm.ctl->seq);
-  loop_epilogue(cm, 1);
+  bicg2_body<T, CH>(cm, co, kr);
 }
 
-template <typename T, int CH>
-__device__ __forceinline__ void bicg3_body(const Common& cm, const Kry<T>& kr, unsigned seq) {
-  for_active_chunks(cm, [&](int b_) { return cm.st[b_].fin_seq == seq; }, [&](int c) {
-    const int b = cm.chunk_inst[c];
-    const InstState& st = cm.st[b];
-    const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
-    const int it = st.iters;  // the solve's last iteration
-    using R = typename RedOf<T>::R;
-    const T alpha = rhead(num<R>(st.alpha)), omega = rhead(num<R>(st.omega));
-    const T* rr = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
-    const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
-    const T* vv = sel2(kr.v, it & 1);
-    const long long c0 = chunk_start<CH>(c, I);
-    const long long c1 = min(c0 + (long long)CH, inst_end(I));
-#pragma unroll 2
-    for (int g = 0; g < CH / (4 * kThreads); ++g) {
-      const long long K = c0 + 4 * (threadIdx.x + g * kThreads);
-      if (K >= c1) continue;
-      const Q4<T> r = ld4(rr + K), v = ld4(vv + K);
-      const Q4<T> p = it > 1 ? ld4(pp + K) : r;
-      Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
-      if (it > 1) x = ld4(kr.x + K);
+// The decisions that follow from a pass's sums, in a small kernel of their own after it (one block per
+// instance concerned). The passes' blocks leave right after their sums: counting themselves in (a
+// fence and an atomic per chunk, so that the last could decide) held each of them up for ~2 us
+// of its ~20, and k_bicg2 on 1024 instances took 3.30 ms a call instead of 2.74.
+template <int NQ, typename R, typename W, typename D>
+__device__ __forceinline__ void decide(const Common& cm, W&& want, D&& body) {
+  __shared__ double s_tot[8 * NQ];
+  R* sm = reinterpret_cast<R*>(s_tot);
+  for (int b = blockIdx.x, ni = n_inst(cm); b < ni; b += gridDim.x) {
+    InstState& st = cm.st[b];
+    if (!want(st)) continue;  // uniform in the block
+    const InstDev& I = cm.inst[b];
+    __syncthreads();
+    seg_total<NQ, kThreads / 32, R>(reinterpret_cast<const R*>(cm.part), cm.pstride, I.seg0, I.nseg, sm);
+    if (threadIdx.x == 0) {
+      R tot[NQ];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const T s = fmaT(-alpha, v.a[m], r.a[m]);
-        x.a[m] = fmaT(alpha, p.a[m], fmaT(omega, s, x.a[m]));
-      }
-      st4(kr.x + K, x);
+      for (int q = 0; q < NQ; ++q) tot[q] = sm[q];
+      body(st, tot);
+    }
+  }
+}
+template <typename T, typename A>
+__global__ void __launch_bounds__(kThreads) k_after_resid(Common cm, double tol, double inner_tol, int max_refine) {
+  using R = typename A::R;
+  count_launch(cm.ctl);
+  decide<3, R>(cm, [](const InstState& st) { return st.outer_active != 0; }, [&](InstState& st, const R(&tot)[3]) {
+    if (after_resid<typename RedOf<T>::R, R>(st, tot, tol, inner_tol, max_refine, cm.precond)) {
+      st.inner_active = 1;
+      atomicAdd(&cm.ctl->n_inner, 1);
+    } else {
+      atomicSub(&cm.ctl->n_outer, 1);
     }
   });
+  loop_epilogue(cm, 0);
 }
-template <typename T, int CH>
-__global__ void __launch_bounds__(kThreads, krylov_blocks<T>()) k_bicg3(Common cm, Kry<T> kr) {
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_after_v(Common cm) {
+  using R = typename RedOf<T>::R;
   count_launch(cm.ctl);
-  bicg3_body<T, CH>(cm, kr, cm.ctl->seq);
+  decide<2, R>(cm, [](const InstState& st) { return st.inner_active != 0; },
+               [&](InstState& st, const R(&tot)[2]) { after_v(st, tot); });
+}
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_after_t(Common cm, int max_iters) {
+  using R = typename RedOf<T>::R;
+  count_launch(cm.ctl);
+  decide<5, R>(cm, [](const InstState& st) { return st.inner_active != 0; }, [&](InstState& st, const R(&tot)[5]) {
+    if (after_t(st, tot, max_iters)) {
+      st.inner_active = 0;
+      atomicSub(&cm.ctl->n_inner, 1);
+    }
+  });
+  loop_epilogue(cm, 1);
 }
 
 // ------------------------------------------------------------------------------ polish + checks
