@@ -225,16 +225,27 @@ __host__ __device__ constexpr int red_pow2() { return NQ <= 1 ? 1 : NQ <= 2 ? 2 
 // half of its quantities to its partner and keeps the other half, so NQ = 5 takes 9 additions
 // instead of 25. Quantity q ends in the lanes with lane / (32 / P) = q (P: NQ rounded up to a power
 // of two); the value returned is this lane's.
-template <int NQ, typename R>
-__device__ __forceinline__ R warp_totals(const R (&in)[NQ]) {
+// In: the type of the terms. FP32 terms of double-word sums become double words in the first addition
+// (2Sum is exact; the bits are those of adding them with zero low parts).
+__device__ __forceinline__ float rshfl(float a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ dw radd_up(float a, float b, dw) { return two_sum(a, b); }
+__device__ __forceinline__ dw radd_up(dw a, dw b, dw) { return dw_add_same(a, b); }
+__device__ __forceinline__ double radd_up(double a, double b, double) { return __dadd_rn(a, b); }
+template <int NQ, typename R, typename In>
+__device__ __forceinline__ R warp_totals(const In (&in)[NQ]) {
   constexpr int P = red_pow2<NQ>();
-  R v[P];
-#pragma unroll
-  for (int q = 0; q < P; ++q) v[q] = q < NQ ? in[q] : rfrom<R>(0.0f);
+  static_assert(P >= 2, "at least two quantities");
   const int lane = threadIdx.x & 31;
-  int off = 16;
+  R v[P / 2];
 #pragma unroll
-  for (int n = P; n > 1; n >>= 1) {
+  for (int q = 0; q < P / 2; ++q) {
+    const In lo = in[q], hi = q + P / 2 < NQ ? in[q + P / 2] : In{};
+    const bool up = (lane & 16) != 0;
+    v[q] = radd_up(up ? hi : lo, rshfl(up ? lo : hi, 16), R{});
+  }
+  int off = 8;
+#pragma unroll
+  for (int n = P / 2; n > 1; n >>= 1) {
     const bool up = (lane & off) != 0;
 #pragma unroll
     for (int q = 0; q < n / 2; ++q) {
@@ -362,7 +373,8 @@ struct ChunkSums {
   static constexpr bool kWhole = CH == 4096;              // one segment per chunk
   static constexpr int kParts = kWhole ? 8 : CH / 128;    // most parts of a chunk
   R (*sm)[kParts];  // [NQ][kParts] in shared memory
-  __device__ __forceinline__ void put(int p, const R (&v)[NQ]) {
+  template <typename In>
+  __device__ __forceinline__ void put(int p, const In (&v)[NQ]) {
     const R t = warp_totals<NQ, R>(v);
     if (red_writes<NQ>()) sm[red_q<NQ>()][p] = t;
   }

@@ -64,6 +64,8 @@ __device__ __forceinline__ float fmaT(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mulT(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mulT(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float subT(float a, float b) { return __fadd_rn(a, -b); }
+__device__ __forceinline__ double subT(double a, double b) { return __dadd_rn(a, -b); }
 
 // FP64 <-> FP32 of the preconditioner's factors (non-negative, at most a few units) by moving the
 // fields: conversions run at the FP64 rate, 1/64 of the integer rate. Truncated; below FP32's
@@ -89,13 +91,18 @@ __device__ __forceinline__ double widen<double>(float a) {
 // block Jacobi with 4-cell alpha-line blocks, the direction in which the scaled systems are
 // stiffest (Dxx/dalpha^2 against Dyy/dlogE^2). line4 returns B^-1 q by Thomas elimination
 // without pivoting (B is a column-diagonally-dominant M-matrix: every column of the outflow
-// fractions sums to < 1, so each pivot stays in (0, 1]). The pivots are inverted in FP32 whatever
-// the vector precision (any map close to B^-1 preconditions as well; every kernel applies the
-// same one); padding cells (q = cw = ce = 0) stay 0.
+// fractions sums to < 1, so each pivot stays in (0, 1]). The pivots are inverted in FP32, to a few ulps,
+// whatever the vector precision (any map close to B^-1 preconditions as well; every kernel applies
+// the same one); padding cells (q = cw = ce = 0) stay 0.
 template <typename T>
 struct Line {
   T w1, w2, w3, c0, c1, c2, i1, i2, i3;
 };
+__device__ __forceinline__ float rcp_fast(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
 template <typename T>
 __device__ __forceinline__ Line<T> line_of(const Q4<T>& cw, const Q4<T>& ce) {
   Line<T> L;
@@ -103,11 +110,11 @@ __device__ __forceinline__ Line<T> line_of(const Q4<T>& cw, const Q4<T>& ce) {
   L.w2 = cw.a[2];
   L.w3 = cw.a[3];
   L.c0 = ce.a[0];
-  const float i1 = __frcp_rn(__fmaf_rn(-narrow(cw.a[1]), narrow(ce.a[0]), 1.0f));
+  const float i1 = rcp_fast(__fmaf_rn(-narrow(cw.a[1]), narrow(ce.a[0]), 1.0f));
   const float c1 = __fmul_rn(narrow(ce.a[1]), i1);
-  const float i2 = __frcp_rn(__fmaf_rn(-narrow(cw.a[2]), c1, 1.0f));
+  const float i2 = rcp_fast(__fmaf_rn(-narrow(cw.a[2]), c1, 1.0f));
   const float c2 = __fmul_rn(narrow(ce.a[2]), i2);
-  const float i3 = __frcp_rn(__fmaf_rn(-narrow(cw.a[3]), c2, 1.0f));
+  const float i3 = rcp_fast(__fmaf_rn(-narrow(cw.a[3]), c2, 1.0f));
   L.i1 = widen<T>(i1);
   L.i2 = widen<T>(i2);
   L.i3 = widen<T>(i3);
@@ -130,22 +137,44 @@ __device__ __forceinline__ Q4<T> line4(const Q4<T>& q, const Line<T>& L) {
   return z;
 }
 
-// A~ x over a 4-cell group from a staged vector (sm + o: the group's first cell; rows P apart):
-// four multiply-adds per cell
+// A row of the matrix for one 4-cell group.
 template <typename T>
-__device__ __forceinline__ Q4<T> stencil_sm(const T* sm, int o, int P, const Q4<T>& cw, const Q4<T>& ce,
-                                            const Q4<T>& cs, const Q4<T>& cn) {
+struct Row {
+  Q4<T> cw, ce, cs, cn;
+};
+template <typename T>
+__device__ __forceinline__ Row<T> row_of(const Coef<T>& co, long long K) {
+  return Row<T>{ld4(co.cw + K), ld4(co.ce + K), ld4(co.cs + K), ld4(co.cn + K)};
+}
+// B^-1 A~ x (or A~ x) over a group from a staged vector (sm + o: its first cell; rows P apart).
+// In FP32: A~ = B - (couplings to other groups), so B^-1 A~ x = x - B^-1 q with q the inflow from the rows
+// below and above and, at the group's ends, from its neighbours in the row; the couplings inside the
+// group drop out. That takes B^-1 to the vectors' own precision (with FP64 vectors and FP32 pivots
+// the solve's system would be off by 1e-7 and cost a refinement), so in FP64 it is B^-1 (A~ x).
+template <typename T>
+__device__ __forceinline__ Q4<T> product(const T* sm, int o, int P, const Row<T>& w, int precond) {
   const Q4<T> c = *reinterpret_cast<const Q4<T>*>(sm + o);
   const Q4<T> d = *reinterpret_cast<const Q4<T>*>(sm + o - P);
   const Q4<T> u = *reinterpret_cast<const Q4<T>*>(sm + o + P);
   const T w0 = sm[o - 1], e3 = sm[o + 4];
-  Q4<T> r;
+  Q4<T> q;
+  if (sizeof(T) == 4 && precond) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q.a[k] = fmaT(w.cn.a[k], u.a[k], mulT(w.cs.a[k], d.a[k]));
+    q.a[0] = fmaT(w.cw.a[0], w0, q.a[0]);
+    q.a[3] = fmaT(w.ce.a[3], e3, q.a[3]);
+    q = line4<T>(q, line_of<T>(w.cw, w.ce));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q.a[k] = subT(c.a[k], q.a[k]);
+    return q;
+  }
   const T wv[4] = {w0, c.a[0], c.a[1], c.a[2]};
   const T ev[4] = {c.a[1], c.a[2], c.a[3], e3};
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    r.a[k] = fmaT(-cn.a[k], u.a[k], fmaT(-cs.a[k], d.a[k], fmaT(-ce.a[k], ev[k], fmaT(-cw.a[k], wv[k], c.a[k]))));
-  return r;
+    q.a[k] = fmaT(-w.cn.a[k], u.a[k], fmaT(-w.cs.a[k], d.a[k], fmaT(-w.ce.a[k], ev[k], fmaT(-w.cw.a[k], wv[k], c.a[k]))));
+  if (precond) q = line4<T>(q, line_of<T>(w.cw, w.ce));
+  return q;
 }
 template <typename T>
 __device__ __forceinline__ T dot4(const Q4<T>& a, const Q4<T>& b, T q) {
@@ -359,7 +388,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       A::st4(yout + K, yc);
       st4(kr.rh + K, r);
     }, [&](int p) {
-      const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
+      const typename A::Acc w[3] = {q0, q1, q2};
       sums.put(p, w);
       q0 = q1 = 0;
       q2 = (T)0;
@@ -452,9 +481,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
       const long long K = c0 + 4 * g;
       if (K < c1) {
         const int o = (int)(K - e0);
-        const Q4<T> cw = ld4(co.cw + K), ce = ld4(co.ce + K);
-        Q4<T> v = stencil_sm<T>(sm, o, P, cw, ce, ld4(co.cs + K), ld4(co.cn + K));
-        if (cm.precond) v = line4<T>(v, line_of<T>(cw, ce));  // v = B^-1 A~ p
+        const Q4<T> v = product<T>(sm, o, P, row_of<T>(co, K), cm.precond);  // v = B^-1 A~ p
         st4(vn + K, v);
         // r^ (on a restart it is p itself)
         const Q4<T> rh = rs ? *reinterpret_cast<const Q4<T>*>(sm + o) : ld4(kr.rh + K);
@@ -462,7 +489,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
         if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
       }
     }, [&](int p) {
-      const R w[2] = {rfrom<R>(q0), rfrom<R>(q1)};
+      const T w[2] = {q0, q1};
       sums.put(p, w);
       q0 = q1 = (T)0;
     });
@@ -510,9 +537,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
       if (K < c1) {
         const int o = (int)(K - e0);
         const Q4<T> s = *reinterpret_cast<const Q4<T>*>(sm + o);
-        const Q4<T> cw = ld4(co.cw + K), ce = ld4(co.ce + K);
-        Q4<T> t = stencil_sm<T>(sm, o, P, cw, ce, ld4(co.cs + K), ld4(co.cn + K));
-        if (cm.precond) t = line4<T>(t, line_of<T>(cw, ce));  // t = B^-1 A~ s
+        const Q4<T> t = product<T>(sm, o, P, row_of<T>(co, K), cm.precond);  // t = B^-1 A~ s
         st4(kr.t + K, t);
         const Q4<T> rh = ld4(kr.rh + K);
         q[0] = dot4<T>(t, s, q[0]);
@@ -522,8 +547,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
         q[4] = dot4<T>(rh, t, q[4]);
       }
     }, [&](int p) {
-      const R w[5] = {rfrom<R>(q[0]), rfrom<R>(q[1]), rfrom<R>(q[2]), rfrom<R>(q[3]), rfrom<R>(q[4])};
-      sums.put(p, w);
+      sums.put(p, q);
 #pragma unroll
       for (int k = 0; k < 5; ++k) q[k] = (T)0;
     });

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               if (ON) st4(srh + l, r);
               if (!ON || edge(l)) st4(kr.rh + c0 + l, r);
             }
-            const R w[3] = {rfrom<R>(q0), rfrom<R>(q1), rfrom<R>(q2)};
+            const typename A::Acc w[3] = {q0, q1, q2};
             const R t = warp_totals<3, R>(w);
             if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + p] = t;
           }
@@ -261,18 +261,12 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             return two ? (warp + kTeamThreads / 32 * (k >> 1)) * 256 + (k & 1) * 128 + 4 * lane
                        : (warp + kTeamThreads / 32 * k) * 128 + 4 * lane;
           };
-          Q4<T> cw[GN], ce[GN], cs[GN], cn[GN];
+          Row<T> row[GN];
           if (ON) {
 #pragma unroll
             for (int k = 0; k < GN; ++k) {
               const int l = cell_of(k);
-              if (l < own) {
-                const long long K = c0 + l;
-                cw[k] = ld4(ck.cw + K);
-                ce[k] = ld4(ck.ce + K);
-                cs[k] = ld4(ck.cs + K);
-                cn[k] = ld4(ck.cn + K);
-              }
+              if (l < own) row[k] = row_of<T>(ck, c0 + l);
             }
           }
           // p = r = r^; the neighbours' rows of r
@@ -312,10 +306,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             __syncthreads();
             // v = B^-1 A~ p
-            const auto product_v = [&](int l, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
-                                       T& q0, T& q1) {
-              Q4<T> v = stencil_sm<T>(sp, P + l, P, w, ea, so, no);
-              if (cm.precond) v = line4<T>(v, line_of<T>(w, ea));
+            const auto product_v = [&](int l, const Row<T>& w, T& q0, T& q1) {
+              const Q4<T> v = product<T>(sp, P + l, P, w, cm.precond);
               st4(at_v(P + l), v);
               if (ON && edge(l)) st4(kr.v[0] + c0 + l, v);
               const Q4<T> rh = rs ? ld4(sp + P + l) : ON ? ld4(srh + l) : ld4(kr.rh + c0 + l);
@@ -323,7 +315,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
             };
             const auto put2 = [&](int p, T q0, T q1) {
-              const RK w[2] = {rfrom<RK>(q0), rfrom<RK>(q1)};
+              const T w[2] = {q0, q1};
               const RK t = warp_totals<2, RK>(w);
               if (red_writes<2>()) reinterpret_cast<RK*>(parts)[red_q<2>() * np + p] = t;
             };
@@ -333,7 +325,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               for (int k = 0; k < GN; ++k) {
                 const int l = cell_of(k), p = warp + kTeamThreads / 32 * (two ? k >> 1 : k);
                 if (p >= pend) break;
-                if (l < own) product_v(l, cw[k], ce[k], cs[k], cn[k], q0, q1);
+                if (l < own) product_v(l, row[k], q0, q1);
                 if (two && !(k & 1)) continue;
                 put2(p, q0, q1);
                 q0 = q1 = (T)0;
@@ -344,8 +336,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
                 for (int k = 0; k < part_c; k += 128) {
                   const int l = p * part_c + k + 4 * lane;
                   if (l >= own) continue;
-                  const long long K = c0 + l;
-                  product_v(l, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q0, q1);
+                  product_v(l, row_of<T>(ck, c0 + l), q0, q1);
                 }
                 put2(p, q0, q1);
               }
@@ -380,10 +371,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             }
             __syncthreads();
             // t = B^-1 A~ s
-            const auto product_t = [&](int l, const Q4<T>& w, const Q4<T>& ea, const Q4<T>& so, const Q4<T>& no,
-                                       T (&q)[5]) {
-              Q4<T> t = stencil_sm<T>(sr, P + l, P, w, ea, so, no);
-              if (cm.precond) t = line4<T>(t, line_of<T>(w, ea));
+            const auto product_t = [&](int l, const Row<T>& w, T (&q)[5]) {
+              const Q4<T> t = product<T>(sr, P + l, P, w, cm.precond);
               if (ON) st4(st_ + l, t);
               if (!ON || edge(l)) st4(kr.t + c0 + l, t);
               const Q4<T> s = ld4(sr + P + l), rh = ON ? ld4(srh + l) : ld4(kr.rh + c0 + l);
@@ -394,8 +383,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               q[4] = dot4<T>(rh, t, q[4]);
             };
             const auto put5 = [&](int p, const T (&q)[5]) {
-              const RK w[5] = {rfrom<RK>(q[0]), rfrom<RK>(q[1]), rfrom<RK>(q[2]), rfrom<RK>(q[3]), rfrom<RK>(q[4])};
-              const RK t = warp_totals<5, RK>(w);
+              const RK t = warp_totals<5, RK>(q);
               if (red_writes<5>()) reinterpret_cast<RK*>(parts)[red_q<5>() * np + p] = t;
             };
             if (ON) {
@@ -404,7 +392,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               for (int k = 0; k < GN; ++k) {
                 const int l = cell_of(k), p = warp + kTeamThreads / 32 * (two ? k >> 1 : k);
                 if (p >= pend) break;
-                if (l < own) product_t(l, cw[k], ce[k], cs[k], cn[k], q);
+                if (l < own) product_t(l, row[k], q);
                 if (two && !(k & 1)) continue;
                 put5(p, q);
 #pragma unroll
@@ -416,8 +404,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
                 for (int k = 0; k < part_c; k += 128) {
                   const int l = p * part_c + k + 4 * lane;
                   if (l >= own) continue;
-                  const long long K = c0 + l;
-                  product_t(l, ld4(ck.cw + K), ld4(ck.ce + K), ld4(ck.cs + K), ld4(ck.cn + K), q);
+                  product_t(l, row_of<T>(ck, c0 + l), q);
                 }
                 put5(p, q);
               }
