@@ -299,35 +299,39 @@ __device__ __forceinline__ R tree(const R* a, int n) {
 // warps of the block; a warp issues the loads of all its tasks before it adds.
 template <int NQ, int NW, typename R>
 __device__ __forceinline__ void seg_total(const R* part, long long stride, int seg0, int nseg, R* sm) {
-  constexpr int G = NW / 8, NT = (NQ + G - 1) / G, NL = NW > 8 ? 4 : 1;
+  constexpr int G = NW / 8, NT = (NQ + G - 1) / G, NL = NW > 8 ? 2 : 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double* src = reinterpret_cast<const double*>(part) + seg0;
-  double w[NT][NL];
+  R a[NT];
 #pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    const int q = (warp >> 3) + G * t;
-    const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
+  for (int t = 0; t < NT; ++t) a[t] = rfrom<R>(0.0f);
+#pragma unroll 1
+  for (int s0 = lane; s0 < nseg; s0 += 256 * NL) {
+    double w[NT][NL];
 #pragma unroll
-    for (int k = 0; k < NL; ++k) {
-      const int s = h * 32 + lane + 256 * k;
-      w[t][k] = q < NQ && s < nseg ? __ldcg(src + (size_t)q * stride + s) : 0.0;
+    for (int t = 0; t < NT; ++t) {
+      const int q = (warp >> 3) + G * t;
+      const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
+#pragma unroll
+      for (int k = 0; k < NL; ++k) {
+        const int s = s0 + h * 32 + 256 * k;
+        w[t][k] = q < NQ && s < nseg ? __ldcg(src + (size_t)q * stride + s) : 0.0;
+      }
     }
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int k = 0; k < NL; ++k) a[t] = radd(a[t], num<R>(w[t][k]));
   }
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
     const int q = (warp >> 3) + G * t, h = (warp - q) & 7;
     if (q >= NQ) break;
-    R a = num<R>(w[t][0]);
     if (h * 32 < nseg) {
 #pragma unroll
-      for (int k = 1; k < NL; ++k)
-        if (h * 32 + 256 * k < nseg) a = radd(a, num<R>(w[t][k]));
-      for (int s = h * 32 + lane + 256 * NL; s < nseg; s += 256)
-        a = radd(a, num<R>(__ldcg(src + (size_t)q * stride + s)));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a = radd(a, rshfl(a, o));
+      for (int o = 16; o > 0; o >>= 1) a[t] = radd(a[t], rshfl(a[t], o));
     }
-    if (lane == 0) sm[8 * q + h] = a;
+    if (lane == 0) sm[8 * q + h] = a[t];
   }
   __syncthreads();
   if (warp == 0) {

@@ -274,6 +274,10 @@ template <typename C, typename A>
 struct CoefW;
 template <typename A>
 struct CoefW<double, A> {
+  __device__ static typename A::V cell(const Coef<double>& c, int which, long long K) {
+    const double* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
+    return A::from_d(a[K]);
+  }
   __device__ static Q4<typename A::V> row(const Coef<double>& c, int which, long long K) {
     const double* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
     const Q4<double> q = ld4(a + K);
@@ -285,6 +289,11 @@ struct CoefW<double, A> {
 };
 template <typename A>
 struct CoefW<float, A> {
+  __device__ static typename A::V cell(const Coef<float>& c, int which, long long K) {
+    const float* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
+    const float* l = which == 0 ? c.lw : which == 1 ? c.le : which == 2 ? c.ls : c.ln;
+    return A::hilo(a[K], l[K]);
+  }
   __device__ static Q4<typename A::V> row(const Coef<float>& c, int which, long long K) {
     const float* a = which == 0 ? c.cw : which == 1 ? c.ce : which == 2 ? c.cs : c.cn;
     const float* l = which == 0 ? c.lw : which == 1 ? c.le : which == 2 ? c.ls : c.ln;
@@ -322,6 +331,62 @@ __device__ __forceinline__ void resid_group(const typename A::V* sm, int o, int 
   if (precond) {  // the Krylov matrix's couplings (the hi parts in the FP32 modes)
     r = line4<T>(r, line_of<T>(ld4(co.cw + K), ld4(co.ce + K)));
     q2 = dot4<T>(r, r, q2);
+  }
+}
+
+// ---- one cell per lane. A share of few cells keeps few warps busy with four cells per lane, one after
+// another; with a cell per lane it keeps four times as many. The lanes of a group chain its sums
+// in the order of the 4-cell form, so the bits are the same.
+// acc over the group's cells in order: f(a, x) with this lane's x, a from the lane before; all lanes get
+// the group's result
+template <typename X>
+__device__ __forceinline__ X lane_get(X a, int from) { return __shfl_sync(0xffffffffu, a, from); }
+__device__ __forceinline__ dw lane_get(dw a, int from) {
+  return dw{__shfl_sync(0xffffffffu, a.hi, from), __shfl_sync(0xffffffffu, a.lo, from)};
+}
+template <typename X, typename F>
+__device__ __forceinline__ X group_chain(X zero, F&& f) {
+  const int base = threadIdx.x & 28;
+  X acc = zero;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) acc = lane_get(f(acc), base + j);
+  return acc;
+}
+// resid_group for the cell of this lane (on: the cell is in the share; every lane of a warp comes here);
+// q0, q1, q2: the group's terms, in each of its lanes
+template <typename T, typename C, typename A>
+__device__ __forceinline__ void resid_cell(const typename A::V* sm, int o, int P, const Coef<C>& co, long long K, bool on,
+                                           const double* Rp, float sc, int precond, bool first, typename A::V& yc, T& r,
+                                           typename A::Acc& q0, typename A::Acc& q1, T& q2) {
+  using V = typename A::V;
+  V rv = A::k(0.0), R = A::k(0.0);
+  Q4<T> cwq{}, ceq{};
+  r = (T)0;
+  if (on) {
+    R = A::ld(Rp, K);
+    yc = sm[o];
+    if (precond) {
+      cwq = ld4(co.cw + (K & ~3LL));
+      ceq = ld4(co.ce + (K & ~3LL));
+    }
+    rv = A::fma(CoefW<C, A>::cell(co, 3, K), sm[o + P], A::fma(CoefW<C, A>::cell(co, 2, K), sm[o - P],
+                A::fma(CoefW<C, A>::cell(co, 1, K), sm[o + 1], A::fma(CoefW<C, A>::cell(co, 0, K), sm[o - 1],
+                A::sub(R, yc)))));
+    r = A::template scaled<T>(rv, sc);
+  }
+  using Acc = typename A::Acc;
+  q0 = group_chain<Acc>((Acc)0, [&](Acc a) { return A::sq_scaled(rv, sc, a); });
+  q1 = first ? group_chain<Acc>((Acc)0, [&](Acc a) { return A::sq_scaled(R, sc, a); }) : (Acc)0;
+  q2 = (T)0;
+  if (precond) {
+    const int base = threadIdx.x & 28;
+    Q4<T> g;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) g.a[j] = __shfl_sync(0xffffffffu, r, base + j);
+    g = line4<T>(g, line_of<T>(cwq, ceq));
+    const int c = threadIdx.x & 3;
+    r = c == 0 ? g.a[0] : c == 1 ? g.a[1] : c == 2 ? g.a[2] : g.a[3];
+    q2 = dot4<T>(g, g, (T)0);
   }
 }
 
@@ -690,6 +755,34 @@ __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int
   A::st4(at.gout + K, g);
   A::st4(at.hw + K, fn);  // f^n into the oldest slot
   A::st4(fl.f + K, fo);
+}
+// polish_group for the cell of this lane (see resid_cell); real: the cell is in the grid
+template <typename C, typename A>
+__device__ __forceinline__ void polish_cell(const typename A::V* sm, int o, int P, const Coef<C>& co, long long K, bool on,
+                                            const Fields& fl, const PolishAt& at, bool real, typename A::V& mass,
+                                            typename A::V& rsum, float& mn) {
+  using V = typename A::V;
+  V R = A::k(0.0), fo = A::k(0.0), cols = A::k(0.0);
+  if (on) {
+    R = A::ld(fl.R, K);
+    const V cw = CoefW<C, A>::cell(co, 0, K), ce = CoefW<C, A>::cell(co, 1, K);
+    const V cs = CoefW<C, A>::cell(co, 2, K), cn = CoefW<C, A>::cell(co, 3, K);
+    const V inv = A::ld(fl.invD, K), fn = A::ld(fl.f, K);
+    cols = A::ld(fl.colsum, K);
+    const V h2 = at.nh >= 2 ? A::ld(at.h2, K) : fn;
+    const V h3 = at.nh >= 3 ? A::ld(at.h3, K) : h2;
+    const V h4 = at.nh >= 4 ? A::ld(at.h4, K) : h3;
+    const V r = fl.decay ? A::ld(fl.decay, K) : A::k(1.0);
+    const V yp = A::fmap(cn, sm[o + P], A::fmap(cs, sm[o - P], A::fmap(ce, sm[o + 1], A::fmap(cw, sm[o - 1], R))));
+    fo = A::mul(yp, inv);
+    if (real) mn = fminf(mn, A::f32(fo));
+    const V g = A::extrap(fo, fn, h2, h3, h4, at.nh, r);
+    A::st(at.gout, K, g);
+    A::st(at.hw, K, fn);
+    A::st(fl.f, K, fo);
+  }
+  mass = group_chain<V>(A::k(0.0), [&](V a) { return A::fmap(cols, fo, a); });
+  rsum = group_chain<V>(A::k(0.0), [&](V a) { return A::addp(a, R); });
 }
 // an instance's step is complete: sums of colsum f, R and the clamped count, and the minimum of f
 __device__ __forceinline__ void after_polish(InstState& st, double mass, double rsum, double clamped, double gmin) {

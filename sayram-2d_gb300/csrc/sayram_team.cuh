@@ -23,6 +23,7 @@ namespace sg {
 // barriers around one thread's release and acquire order every thread's accesses. Measured with 512
 // bytes written before and read after it by every block: 1.42 us at 9 to 152 blocks; further
 // fences around the two cost 0.27 us, and a flag per block that every block polls 2.98 us at 152.
+constexpr int kFineParts = 4;  // most parts of a share that takes a cell per lane
 struct TeamBar {
   unsigned* cnt;
   unsigned target;
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
   __shared__ double s_tot[8 * kPartQ];
   __shared__ float s_w[kTeamThreads / 32];
   __shared__ int s_go;
+  __shared__ double s_gs[3 * kFineParts * 32];  // group sums of a share handled cell by cell
   const int tid = threadIdx.x, warp = tid >> 5;
   const int np = ta.own_cap / 128;  // warp sums of the largest share
   const size_t ext_cap = (size_t)ta.own_cap + 2 * (size_t)ta.pmax;
@@ -131,6 +133,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
     // warps take parts in turn; a part is part/128 groups of every lane
     const int part_c = part_cells(SEG), pend = nseg * (SEG / part_c), lane = tid & 31;
     const bool two = part_c == 256;
+    // a cell per lane instead of four (resid_cell, polish_cell) where that leaves no SM sub-partition more
+    // warps than it can hide: FP64 work is bound by the pipe, which a warp's operation holds for 64
+    // cycles, so it only gains while some sub-partitions would have had nothing
+    const bool fine = ON && !two && pend <= (sizeof(typename A::Acc) == 8 ? 2 : kFineParts);
     const long long e0 = c0 - P;
     TeamBar bar{ta.bar + (size_t)sh.inst * kTeamBarStride, 0u, sh.nb};
     float* const tmax = ta.tmax + (blockIdx.x - sh.rank);
@@ -224,23 +230,54 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             *reinterpret_cast<Q4<V>*>(sv + l) = y;
           }
           __syncthreads();
-          for (int p = warp; p < pend; p += kTeamThreads / 32) {
-            typename A::Acc q0 = 0, q1 = 0;
-            T q2 = (T)0;
-            for (int k = 0; k < part_c; k += 128) {
-              const int l = p * part_c + k + 4 * lane;
-              if (l >= own) continue;
-              Q4<V> yc;
-              Q4<T> r;
-              resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, S.refines == 0, yc, r, q0, q1, q2);
-              A::st4(yout + c0 + l, yc);
-              st4(sr + P + l, r);
-              if (ON) st4(srh + l, r);
-              if (!ON || edge(l)) st4(kr.rh + c0 + l, r);
+          if (fine) {
+            const int p = warp >> 2, l = 4 * 8 * warp + lane;  // part and cell
+            if (p < pend) {
+              V yc;
+              T r;
+              typename A::Acc q0, q1;
+              T q2;
+              resid_cell<T, C, A>(sv, P + l, P, cf, c0 + l, l < own, fl.R, sc, cm.precond, S.refines == 0, yc, r, q0,
+                                  q1, q2);
+              if (l < own) {
+                A::st(yout, c0 + l, yc);
+                sr[P + l] = r;
+                if (ON) srh[l] = r;
+                if (!ON || edge(l)) kr.rh[c0 + l] = r;
+              }
+              if ((lane & 3) == 0) {
+                typename A::Acc* gs = reinterpret_cast<typename A::Acc*>(s_gs) + 3 * (l >> 2);
+                gs[0] = q0;
+                gs[1] = q1;
+                gs[2] = q2;
+              }
             }
-            const typename A::Acc w[3] = {q0, q1, q2};
-            const R t = warp_totals<3, R>(w);
-            if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + p] = t;
+            __syncthreads();
+            if (warp < pend) {
+              const typename A::Acc* gs = reinterpret_cast<const typename A::Acc*>(s_gs) + 3 * (32 * warp + lane);
+              const typename A::Acc w[3] = {gs[0], gs[1], gs[2]};
+              const R t = warp_totals<3, R>(w);
+              if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + warp] = t;
+            }
+          } else {
+            for (int p = warp; p < pend; p += kTeamThreads / 32) {
+              typename A::Acc q0 = 0, q1 = 0;
+              T q2 = (T)0;
+              for (int k = 0; k < part_c; k += 128) {
+                const int l = p * part_c + k + 4 * lane;
+                if (l >= own) continue;
+                Q4<V> yc;
+                Q4<T> r;
+                resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, S.refines == 0, yc, r, q0, q1, q2);
+                A::st4(yout + c0 + l, yc);
+                st4(sr + P + l, r);
+                if (ON) st4(srh + l, r);
+                if (!ON || edge(l)) st4(kr.rh + c0 + l, r);
+              }
+              const typename A::Acc w[3] = {q0, q1, q2};
+              const R t = warp_totals<3, R>(w);
+              if (red_writes<3>()) reinterpret_cast<R*>(parts)[red_q<3>() * np + p] = t;
+            }
           }
           team_store<3, R, R>(reinterpret_cast<const R*>(parts), np, SEG, nseg, reinterpret_cast<R*>(part()),
                               cm.pstride, seg0);
@@ -462,17 +499,38 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
         }
         __syncthreads();
         float mn = 3.0e38f;
-        for (int p = warp; p < pend; p += kTeamThreads / 32) {
-          V mass = A::k(0.0), rsum = A::k(0.0);
-          for (int k = 0; k < part_c; k += 128) {
-            const int l = p * part_c + k + 4 * lane;
-            if (l >= own) continue;
+        if (fine) {
+          const int p = warp >> 2, l = 4 * 8 * warp + lane;
+          if (p < pend) {
             const long long K = c0 + l;
-            polish_group<C, A, true>(sv, P + l, P, cf, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
+            V mass, rsum;
+            polish_cell<C, A>(sv, P + l, P, cf, K, l < own, fl, at, (int)(K - I.base) % P < I.nx, mass, rsum, mn);
+            if ((lane & 3) == 0) {
+              V* gs = reinterpret_cast<V*>(s_gs) + 2 * (l >> 2);
+              gs[0] = mass;
+              gs[1] = rsum;
+            }
           }
-          const R w[2] = {mass, rsum};
-          const R t = warp_totals<2, R>(w);
-          if (red_writes<2>()) reinterpret_cast<R*>(parts)[red_q<2>() * np + p] = t;
+          __syncthreads();
+          if (warp < pend) {
+            const V* gs = reinterpret_cast<const V*>(s_gs) + 2 * (32 * warp + lane);
+            const R w[2] = {gs[0], gs[1]};
+            const R t = warp_totals<2, R>(w);
+            if (red_writes<2>()) reinterpret_cast<R*>(parts)[red_q<2>() * np + warp] = t;
+          }
+        } else {
+          for (int p = warp; p < pend; p += kTeamThreads / 32) {
+            V mass = A::k(0.0), rsum = A::k(0.0);
+            for (int k = 0; k < part_c; k += 128) {
+              const int l = p * part_c + k + 4 * lane;
+              if (l >= own) continue;
+              const long long K = c0 + l;
+              polish_group<C, A, true>(sv, P + l, P, cf, K, fl, at, I.nx - (int)(K - I.base) % P, mass, rsum, mn);
+            }
+            const R w[2] = {mass, rsum};
+            const R t = warp_totals<2, R>(w);
+            if (red_writes<2>()) reinterpret_cast<R*>(parts)[red_q<2>() * np + p] = t;
+          }
         }
         team_store<2, R, double>(reinterpret_cast<const R*>(parts), np, SEG, nseg, part(), cm.pstride, seg0);
         // clamped cells (whole numbers) and the minimum: one entry per share, the rest of its segments 0
@@ -502,10 +560,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
         if (!(ok = team_sync(bar, ta.stat))) break;
         double tot[3] = {0.0, 0.0, 0.0}, gmin = 0.0;
         if (last && sh.rank == 0) {
-          seg_total<3, kTeamThreads / 32, double>(part(), cm.pstride, I.seg0, I.nseg, s_tot);
           float m = 3.0e38f;  // the minima are FP32 values
           for (int k = tid; k < I.nseg; k += kTeamThreads)
             m = fminf(m, (float)__ldcg(part() + 3 * (size_t)cm.pstride + I.seg0 + k));
+          seg_total<3, kTeamThreads / 32, double>(part(), cm.pstride, I.seg0, I.nseg, s_tot);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
           if ((tid & 31) == 0) s_w[warp] = m;
