@@ -148,16 +148,16 @@ SG_HD dw dw_mul(dw x, dw y) {
   return fast2sum(c.hi, cl3);
 }
 
-// 1/y: approximate FP32 reciprocal t (a few ulps), then r = t + t*(1 - y*t) with y*t formed in
-// double-word; the Newton step squares the relative error of t.
+// 1/y: approximate FP32 reciprocal t (a few ulps), then r = t + t*(1 - y*t); the Newton step squares the
+// relative error of t. 1 - y.hi*t is exact as one FMA (the product is within 2^-22 of 1 and its last
+// bit is 2^-47), so e is 1 - y*t to 2^-47.
 SG_HD dw dw_rcp(dw y) {
 #ifdef __CUDA_ARCH__
   const float t = __fdividef(1.0f, y.hi);
 #else
   const float t = 1.0f / y.hi;
 #endif
-  const dw p = dw_mul_f(y, t);               // y*t ~ 1
-  const float e = DW_SUB(DW_SUB(1.0f, p.hi), p.lo);  // 1 - p.hi is exact (Sterbenz)
+  const float e = DW_FMA(-y.lo, t, DW_FMA(-y.hi, t, 1.0f));
   return fast2sum(t, DW_MUL(t, e));
 }
 

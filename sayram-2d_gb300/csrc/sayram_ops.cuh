@@ -241,27 +241,24 @@ struct DWA {
   __device__ static V div(V a, V b) { return dw_div(a, b); }
   __device__ static V abs(V a) { return dw_abs(a); }
   __device__ static V neg(V a) { return dw_neg(a); }
-  // as F64A::extrap, in double-word: with loss rates up to 10 per day an increment is ~10 % of f,
-  // so FP32 increments would leave ~1e-8 of f in the start, above what the extrapolation achieves; the
-  // starting point only steers the iteration, the converged answer does not depend on it
+  // as F64A::extrap, in double-word: with loss rates up to 10 per day an increment is ~10 % of f, so
+  // FP32 increments would leave ~1e-8 of f in the start, above what the extrapolation achieves. (The
+  // closed forms leave up to 31 u^2 ~ 1e-13 of f, a hundredth of the residual target; the starting
+  // point only steers the iteration, the converged answer does not depend on it.)
   __device__ static V extrap(V f, V h1, V h2, V h3, V h4, int n, V r) {
-    const dw c1 = dw_mul(h1, r);
-    const dw d1 = sub(f, c1);
-    dw c = d1;
-    if (n >= 2) {
-      const dw r2 = dw_mul(r, r), c2 = dw_mul(h2, r2);
-      const dw d2 = sub(c1, c2);
-      if (n == 2) {
-        c = sub(dw{2.0f * d1.hi, 2.0f * d1.lo}, d2);
-      } else {
-        const dw r3 = dw_mul(r2, r), c3 = dw_mul(h3, r3);
-        const dw d3 = sub(c2, c3);
-        c = n == 3 ? add(dw_mul_f(sub(d1, d2), 3.0f), d3)
-                   : sub(sub(dw_mul_f(add(d1, d3), 4.0f), dw_mul_f(d2, 6.0f)), sub(c3, dw_mul(h4, dw_mul(r3, r))));
-      }
-    }
-    return dw_mul(r, add(f, c));
+    dw a;
+    if (n >= 4)
+      a = dw_fma(r, dw_fma(r, dw_fma(r, dw_fma(r, h4, dw_mul_f(h3, -5.0f)), dw_mul_f(h2, 10.0f)),
+                           dw_mul_f(h1, -10.0f)), dw_mul_f(f, 5.0f));
+    else if (n == 3)
+      a = dw_fma(r, dw_fma(r, dw_fma(dw_neg(r), h3, times4(h2)), dw_mul_f(h1, -6.0f)), times4(f));
+    else if (n == 2)
+      a = dw_fma(r, dw_fma(r, h2, dw_mul_f(h1, -3.0f)), dw_mul_f(f, 3.0f));
+    else
+      a = dw_fma(dw_neg(r), h1, dw{2.0f * f.hi, 2.0f * f.lo});
+    return dw_mul(r, a);
   }
+  __device__ static V times4(V a) { return dw{4.0f * a.hi, 4.0f * a.lo}; }
   __device__ static V rsub1(V a) { return dw_add_f(dw_neg(a), 1.0f); }  // 1 - a (DWPlusFP)
   __device__ static V max0(V a) { return dw_max0(a); }
   __device__ static V k(double c) { return dw_from_double(c); }
@@ -595,16 +592,15 @@ __device__ __forceinline__ void inner_face(typename A::V aK, typename A::V SK, t
                                            typename A::V* AK, typename A::V* AL) {
   using V = typename A::V;
   const V absK = A::abs(aK), absL = A::abs(aL);
-  const V denom = A::addp(A::addp(absK, absL), A::k(2 * kEps));
-  const V muK = A::div(A::addp(absL, A::k(kEps)), denom);
+  const V denom = A::addf(A::addp(absK, absL), (float)(2 * kEps));  // both constants are powers of two
+  const V muK = A::div(A::addf(absL, (float)kEps), denom);
   const V muL = A::rsub1(muK);
   const V B = A::dot2s(muL, aL, muK, aK);
   // B+ = (|B| + B)/2 goes to K's coefficient, B- = (|B| - B)/2 to L's; at most one is nonzero,
   // so only that one is multiplied by its 1/(f + eps) and added (all terms >= 0)
   const V mK = A::mul(muK, SK), mL = A::mul(muL, SL);
   const bool pos = A::gt0(B);
-  const V T = A::mul(pos ? B : A::pos_part(A::neg(B)), pos ? invK : invL);
-  const V X = A::addp(pos ? mK : mL, T);
+  const V X = A::fmap(pos ? B : A::pos_part(A::neg(B)), pos ? invK : invL, pos ? mK : mL);
   *AK = pos ? X : mK;
   *AL = pos ? mL : X;
 }
@@ -696,10 +692,10 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
           V fb = zero;
           if (Iv > 0) {
             fa = A::ld(fl.f, K - 1);
-            ia = A::rcp(A::addp(fa, A::k(kEps)));
+            ia = A::rcp(A::addf(fa, (float)kEps));
           }
           if (Iv < nx) fb = A::ld(fl.f, K);
-          r = xin ? A::fmap(wL, fa, A::mul(wR, fb)) : (Iv == 0 ? fb : fa);
+          r = xin ? A::dot2(wL, fa, wR, fb) : (Iv == 0 ? fb : fa);
         }
         S.fS[hy][vx] = fa;
         S.iS[hy][vx] = ia;
@@ -711,7 +707,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
       V fv = zero, iv = zero;
       if (i < nx && j >= 0 && j < ny) {
         fv = A::ld(fl.f, K0 + (tid2 - 1) * P + w);
-        iv = A::rcp(A::addp(fv, A::k(kEps)));
+        iv = A::rcp(A::addf(fv, (float)kEps));
       }
       S.fS[tid2][W1] = fv;
       S.iS[tid2][W1] = iv;
@@ -741,7 +737,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
       const V r0 = rS[Jv > 0 ? vy : vy + 1][vx];
       if (Jv > 0 && Jv < ny) {  // interior and vertical boundary edges: linear in y
         const V r1 = rS[vy + 1][vx];
-        val = A::fmap(S.hS[vy][0], r0, A::mul(S.hS[vy][1], r1));
+        val = A::dot2(S.hS[vy][0], r0, S.hS[vy][1], r1);
       } else {
         val = r0;  // horizontal boundary edges (linear in x) and corners
       }
