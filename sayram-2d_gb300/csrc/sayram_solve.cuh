@@ -192,7 +192,7 @@ __device__ __forceinline__ T dot4(const Q4<T>& a, const Q4<T>& b, T q) {
 template <typename RK, typename R>
 __device__ __forceinline__ int after_resid(InstState& st, const R (&tot)[3], double tol, double inner_tol,
                                            int max_refine, int precond) {
-  st.ycur ^= 1;
+  if (st.has_x) st.ycur ^= 1;  // the pass has written y + x to the other buffer
   st.has_x = 0;
   if (st.refines == 0) st.bb = stored(tot[1]);
   st.refines += 1;
@@ -390,8 +390,8 @@ __device__ __forceinline__ void resid_cell(const typename A::V* sm, int o, int P
   }
 }
 
-// r = R - A~ (y + x) in the wide arithmetic; writes y + x to the other y buffer and the Krylov's
-// right-hand side B^-1 r (T precision, scaled) to rh.
+// r = R - A~ (y + x) in the wide arithmetic; writes y + x to the other y buffer (where there is an x)
+// and the Krylov's right-hand side B^-1 r (T precision, scaled) to rh.
 template <typename T, typename C, typename A, int CH>
 __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, const Coef<C>& co, const Kry<T>& kr) {
   using V = typename A::V;
@@ -450,7 +450,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       Q4<V> yc;
       Q4<T> r;
       resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, st.refines == 0, yc, r, q0, q1, q2);
-      A::st4(yout + K, yc);
+      if (hx) A::st4(yout + K, yc);
       st4(kr.rh + K, r);
     }, [&](int p) {
       const typename A::Acc w[3] = {q0, q1, q2};

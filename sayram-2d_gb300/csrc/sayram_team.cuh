@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
               resid_cell<T, C, A>(sv, P + l, P, cf, c0 + l, l < own, fl.R, sc, cm.precond, S.refines == 0, yc, r, q0,
                                   q1, q2);
               if (l < own) {
-                A::st(yout, c0 + l, yc);
+                if (hx) A::st(yout, c0 + l, yc);
                 sr[P + l] = r;
                 if (ON) srh[l] = r;
                 if (!ON || edge(l)) kr.rh[c0 + l] = r;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
                 Q4<V> yc;
                 Q4<T> r;
                 resid_group<T, C, A>(sv, P + l, P, cf, c0 + l, fl.R, sc, cm.precond, S.refines == 0, yc, r, q0, q1, q2);
-                A::st4(yout + c0 + l, yc);
+                if (hx) A::st4(yout + c0 + l, yc);
                 st4(sr + P + l, r);
                 if (ON) st4(srh + l, r);
                 if (!ON || edge(l)) st4(kr.rh + c0 + l, r);
