@@ -202,7 +202,7 @@ struct sayram_batch_s {
 
   // launch shape of the streaming kernels: cells per chunk (one block iteration) and blocks per SM
   int chunk = 2048;
-  int gmult = 16;
+  int gmult = 32;
   int grid_inst() const { return std::max(1, std::min(cap_slots, nsm * 8)); }
   int grid_stream() const { return std::max(1, std::min(cap_chunks, nsm * gmult)); }
   int nchunks_of(int nx, int ny) const {
@@ -870,17 +870,22 @@ int sayram_batch_s::build(const sayram_problem* probs, int count, const sayram_o
       break;
     }
   }
-  // a batch that k_team can still step is stepped faster by it than by the 4096-cell kernels: FP32
-  // modes up to 13,000 cells per SM (1300 x 1300: 680 against 1013 us a step, 40 uneven instances of
-  // 1.98 M cells: 661 against 716), FP64 up to 8,800 (1150 x 1150: 2.49 against 3.62 ms; 28 uneven
-  // instances of 1.39 M cells: 1.95 against 1.89)
-  if (chunk == 4096 && coop && cursor <= (long long)nsm * (mixed ? 13000 : 8800)) chunk = 2048;
+  // a batch that k_team can still step is stepped faster by it than by the 4096-cell kernels: in the FP32
+  // modes as long as it fits (1450 x 1450: 862 against 1265 us a step, 40 uneven instances of 1.98 M
+  // cells: 614 against 630), in FP64 up to 8,800 cells per SM (1150 x 1150: 2.47 against 3.50 ms; 28
+  // uneven instances of 1.39 M cells: 1.93 against 1.80)
+  const bool try_team = chunk == 4096 && coop && cursor <= (long long)nsm * (mixed ? 16000 : 8800);
+  if (try_team) chunk = 2048;
   if ((rc = alloc_storage(cursor + 64, count, chunks, tiles, xoff, yoff, doff, std::max(6 * maxcells, nreal))))
     return rc;
   n = count;
   for (int b = 0; b < count; ++b)
     if ((rc = place(b, probs[b], base[b], xoffv[b], yoffv[b], &doffv[4 * b], hoff[b]))) return rc;
   if ((rc = rebuild_lists())) return rc;
+  if (try_team && !team_grid) {
+    chunk = 4096;
+    if ((rc = rebuild_lists())) return rc;
+  }
   SG_CUDA(cudaStreamSynchronize(stream));
   return SAYRAM_OK;
 }

@@ -426,7 +426,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       const T* rr = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
       const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
       const T* vv = sel2(kr.v, it & 1);
-      stage_rows<V, 1>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
+      stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
         Q4<V> y = A::ld4(yin + k);
         const Q4<T> r = ld4(rr + k), v = ld4(vv + k);
         const Q4<T> p = it > 1 ? ld4(pp + k) : r;

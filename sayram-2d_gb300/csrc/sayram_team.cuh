@@ -141,12 +141,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
     TeamBar bar{ta.bar + (size_t)sh.inst * kTeamBarStride, 0u, sh.nb};
     float* const tmax = ta.tmax + (blockIdx.x - sh.rank);
     // shared memory: r and p with halos, then (on chip) v and x with halos, t and the shadow residual; the
-    // staged 8-byte solution lies over p (and v). In the other form the halos of v and x only.
+    // staged 8-byte solution lies over p (and v). In the other form the halos of v and x only; in FP32
+    // v has the room that the staged solution needs beyond p.
     T* const sr = reinterpret_cast<T*>(mem);
     T* const sp = sr + ext_cap;
     V* const sv = reinterpret_cast<V*>(sp);
-    T* const sv_ = ON ? sp + ext_cap : reinterpret_cast<T*>(sv + ext_cap);  // v: on chip own + halo, else halo
-    T* const sx = ON ? sv_ + ext_cap : sv_ + 2 * ta.pmax;
+    constexpr bool VON = ON || sizeof(T) == 4;
+    T* const sv_ = VON ? sp + ext_cap : reinterpret_cast<T*>(sv + ext_cap);  // v: own + halo, else halo
+    T* const sx = VON ? sv_ + ext_cap : sv_ + 2 * ta.pmax;
     T* const st_ = sx + ext_cap;               // t of the share (on chip)
     T* const srh = st_ + ta.own_cap;           // shadow residual of the share (on chip)
     // a cell of the share that a neighbouring share reads
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
       return l < P ? sx + l : l < P + own ? kr.x + e0 + l : sx + (l - own);
     };
     const auto at_v = [&](int l) -> T* {
-      if (ON) return sv_ + l;
+      if (VON) return sv_ + l;
       return l < P ? sv_ + l : l < P + own ? kr.v[0] + e0 + l : sv_ + (l - own);
     };
 
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
             const auto product_v = [&](int l, const Row<T>& w, T& q0, T& q1) {
               const Q4<T> v = product<T>(sp, P + l, P, w, cm.precond);
               st4(at_v(P + l), v);
-              if (ON && edge(l)) st4(kr.v[0] + c0 + l, v);
+              if (VON && edge(l)) st4(kr.v[0] + c0 + l, v);
               const Q4<T> rh = rs ? ld4(sp + P + l) : ON ? ld4(srh + l) : ld4(kr.rh + c0 + l);
               q0 = dot4<T>(rh, v, q0);
               if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);

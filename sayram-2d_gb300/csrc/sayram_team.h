@@ -41,8 +41,10 @@ constexpr int kTeamBarStride = 16;  // 64 bytes: one team's counters do not shar
 // stay in shared memory; otherwise x, t, v and the shadow residual stay in global memory.
 inline size_t team_smem(size_t tsize, bool chip, long long own_cap, long long pmax, size_t tile_bytes) {
   const size_t ext = (size_t)(own_cap + 2 * pmax), halo = (size_t)(2 * pmax);
-  // r, p, v, x with both halos, t and r^ / r, p (or the staged 8-byte solution), v and x halos
-  size_t n = chip ? 4 * ext * tsize + 2 * (size_t)own_cap * tsize : ext * tsize + ext * 8 + 2 * halo * tsize;
+  // r, p, v, x with both halos, t and r^ / r, the staged 8-byte solution (p, and in FP32 v), the halos of
+  // x and in FP64 v
+  size_t n = chip ? 4 * ext * tsize + 2 * (size_t)own_cap * tsize
+                  : ext * tsize + ext * 8 + (tsize == 4 ? 1 : 2) * halo * tsize;
   if (n < kTeamParts * tile_bytes) n = kTeamParts * tile_bytes;
   return n + (size_t)kPartQ * (own_cap / 128) * 8 + 16;
 }
