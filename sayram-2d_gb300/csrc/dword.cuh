@@ -266,6 +266,21 @@ SG_HD double dw_to_double_int(dw x) {
 #endif
 }
 
+// hi + lo for a pair that dw_from_double made, in integers: lo is a whole number d of units 2^(eh-52),
+// |d| <= 2^28, so the sum's bits are those of hi as a double plus or minus d, with carry and borrow
+// through the exponent. Only below a power of two is the unit halved; that case, hi below 2^-63 (where lo
+// could be subnormal) and specials take the addition.
+SG_HD double dw_join_int(dw x) {
+  const unsigned int h = dw_fbits(x.hi), l = dw_fbits(x.lo);
+  const unsigned int eh = (h >> 23) & 0xFFu;
+  const bool opp = ((h ^ l) >> 31) != 0u;
+  if (eh < 64u || eh == 0xFFu || (opp && (h & 0x7FFFFFu) == 0u)) return (double)x.hi + (double)x.lo;
+  const unsigned int sh = eh - 24u - ((l >> 23) & 0xFFu);
+  const unsigned int d = (((l & 0x7FFFFFu) | 0x800000u) << 5) >> (sh < 31u ? sh : 31u);
+  const unsigned long long m = ((unsigned long long)(h & 0x7FFFFFFFu) << 29) + (896ull << 52);
+  return dw_bitsd(((unsigned long long)(h >> 31) << 63) | (opp ? m - d : m + d));
+}
+
 #undef SG_HD
 #undef DW_ADD
 #undef DW_SUB
