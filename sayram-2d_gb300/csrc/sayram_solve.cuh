@@ -317,13 +317,15 @@ __device__ __forceinline__ void resid_group(const typename A::V* sm, int o, int 
   const Q4<V> cw = CoefW<C, A>::row(co, 0, K), ce = CoefW<C, A>::row(co, 1, K);
   const Q4<V> cs = CoefW<C, A>::row(co, 2, K), cn = CoefW<C, A>::row(co, 3, K);
   const Q4<V> R = A::ld4(Rp + K);
+  yc = *reinterpret_cast<const Q4<V>*>(sm + o);
+  const Q4<V> d = *reinterpret_cast<const Q4<V>*>(sm + o - P), u = *reinterpret_cast<const Q4<V>*>(sm + o + P);
+  const V w0 = sm[o - 1], e3 = sm[o + 4];
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
-    const V yv = sm[o + m];
     // (R - y) + the neighbours' inflow, one multiply-add each
-    const V rv = A::fma(cn.a[m], sm[o + m + P], A::fma(cs.a[m], sm[o + m - P],
-                        A::fma(ce.a[m], sm[o + m + 1], A::fma(cw.a[m], sm[o + m - 1], A::sub(R.a[m], yv)))));
-    yc.a[m] = yv;
+    const V rv = A::fma(cn.a[m], u.a[m], A::fma(cs.a[m], d.a[m],
+                        A::fma(ce.a[m], m < 3 ? yc.a[(m + 1) & 3] : e3,
+                               A::fma(cw.a[m], m > 0 ? yc.a[(m + 3) & 3] : w0, A::sub(R.a[m], yc.a[m])))));
     r.a[m] = A::template scaled<T>(rv, sc);
     q0 = A::sq_scaled(rv, sc, q0);
     if (first) q1 = A::sq_scaled(R.a[m], sc, q1);  // ||R|| does not change within a step
@@ -727,9 +729,21 @@ __device__ __forceinline__ void polish_group(const typename A::V* sm, int o, int
 #pragma unroll
   for (int dir = 0; dir < 4; ++dir) {
     const Q4<V> c = CoefW<C, A>::row(co, dir, K);
-    const int on = o + (dir == 0 ? -1 : dir == 1 ? 1 : dir == 2 ? -P : P);
+    // the neighbours' values: the group's own shifted by one cell, or the group in the row below or above
+    Q4<V> y = *reinterpret_cast<const Q4<V>*>(sm + o + (dir == 2 ? -P : dir == 3 ? P : 0));
+    if (dir == 0) {
+      y.a[3] = y.a[2];
+      y.a[2] = y.a[1];
+      y.a[1] = y.a[0];
+      y.a[0] = sm[o - 1];
+    } else if (dir == 1) {
+      y.a[0] = y.a[1];
+      y.a[1] = y.a[2];
+      y.a[2] = y.a[3];
+      y.a[3] = sm[o + 4];
+    }
 #pragma unroll
-    for (int m = 0; m < 4; ++m) yp.a[m] = A::fmap(c.a[m], sm[on + m], yp.a[m]);
+    for (int m = 0; m < 4; ++m) yp.a[m] = A::fmap(c.a[m], y.a[m], yp.a[m]);
   }
   const Q4<V> inv = EARLY ? e_inv : A::ld4(fl.invD + K), cols = EARLY ? e_cols : A::ld4(fl.colsum + K);
   Q4<V> fo;
