@@ -301,42 +301,68 @@ __device__ __forceinline__ R tree(const R* a, int n) {
 // The totals of NQ quantities over nseg segment sums part[q * stride + seg0 ...]: task (q, h) is one
 // warp adding every eighth run of 32 segments, lane by lane, then its tree; a total is the tree over
 // its eight tasks. In sm[0 .. NQ) for the first warp after the call (sm holds 8 * NQ entries). NW:
-// warps of the block; a warp issues the loads of all its tasks before it adds.
+// warps of the block; a warp issues the loads of all its tasks before it adds. Bound by latency: L2's
+// and the additions'. Steps of a 33 x 32 FP64 instance 1135 -> 1070 us (twenty), of a 90 x 90 one 863 ->
+// 835 us with the short form for up to 256 segments (in double-word it gains nothing there, and its
+// code costs larger instances 1 %), of a 1024 x 1024 double-word one 4173 -> 4142 us with trees side by
+// side.
 template <int NQ, int NW, typename R>
 __device__ __forceinline__ void seg_total(const R* part, long long stride, int seg0, int nseg, R* sm) {
   constexpr int G = NW / 8, NT = (NQ + G - 1) / G, NL = NW > 8 ? 2 : 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double* src = reinterpret_cast<const double*>(part) + seg0;
   R a[NT];
-#pragma unroll
-  for (int t = 0; t < NT; ++t) a[t] = rfrom<R>(0.0f);
-#pragma unroll 1
-  for (int s0 = lane; s0 < nseg; s0 += 256 * NL) {
-    double w[NT][NL];
+  constexpr bool DW = sizeof(rhead(R{})) == 4;
+  if (!DW && nseg <= 256) {  // one run each, as it is: spares two additions on the FP64 pipe
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      const int q = (warp >> 3) + G * t;
-      const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
+      const int q = (warp >> 3) + G * t, s = ((warp - q) & 7) * 32 + lane;
+      a[t] = q < NQ && s < nseg ? num<R>(__ldcg(src + (size_t)q * stride + s)) : rfrom<R>(0.0f);
+    }
+  } else {
 #pragma unroll
-      for (int k = 0; k < NL; ++k) {
-        const int s = s0 + h * 32 + 256 * k;
-        w[t][k] = q < NQ && s < nseg ? __ldcg(src + (size_t)q * stride + s) : 0.0;
+    for (int t = 0; t < NT; ++t) a[t] = rfrom<R>(0.0f);
+#pragma unroll 1
+    for (int s0 = lane; s0 < nseg; s0 += 256 * NL) {
+      double w[NT][NL];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int q = (warp >> 3) + G * t;
+        const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
+#pragma unroll
+        for (int k = 0; k < NL; ++k) {
+          const int s = s0 + h * 32 + 256 * k;
+          w[t][k] = q < NQ && s < nseg ? __ldcg(src + (size_t)q * stride + s) : 0.0;
+        }
       }
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int k = 0; k < NL; ++k) a[t] = radd(a[t], num<R>(w[t][k]));
     }
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-#pragma unroll
-      for (int k = 0; k < NL; ++k) a[t] = radd(a[t], num<R>(w[t][k]));
   }
+  if constexpr (DW) {
+    // the trees of a warp's tasks side by side
 #pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    const int q = (warp >> 3) + G * t, h = (warp - q) & 7;
-    if (q >= NQ) break;
-    if (h * 32 < nseg) {
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a[t] = radd(a[t], rshfl(a[t], o));
+      for (int t = 0; t < NT; ++t) a[t] = radd(a[t], rshfl(a[t], o));
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int q = (warp >> 3) + G * t, h = (warp - q) & 7;
+      if (q < NQ && lane == 0) sm[8 * q + h] = a[t];
     }
-    if (lane == 0) sm[8 * q + h] = a[t];
+  } else {  // one after another where there is something to add: the FP64 pipe is what they wait for
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int q = (warp >> 3) + G * t, h = (warp - q) & 7;
+      if (q >= NQ) break;
+      if (h * 32 < nseg) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a[t] = radd(a[t], rshfl(a[t], o));
+      }
+      if (lane == 0) sm[8 * q + h] = a[t];
+    }
   }
   __syncthreads();
   if (warp == 0) {
