@@ -1,0 +1,171 @@
+"""The cooperative step (whole steps in one launch, a team of blocks per instance) against the separate
+kernels of the same step: the two share their formulas, reduction segments and orders of summation, so
+states and statistics must agree bit for bit at every split of the work. Also the other paths that
+hand work to it, at the sizes where they change form."""
+import ctypes
+import dataclasses
+
+import numpy as np
+import pytest
+
+from sayram2d_gb300 import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(capi, probs, prec, precond, coop, calls):
+    b = capi.Batch(probs, precision=prec, precond=precond)
+    b.set_coop(coop)
+    l0 = b.launches()
+    for n in calls:
+        b.step(n)
+    used = b.launches() - l0
+    out = [b.f(k) for k in range(len(probs))]
+    stats = [b.stats(k) for k in range(len(probs))]
+    b.close()
+    return out, stats, used
+
+
+def _same(a, b):
+    for k, (x, y) in enumerate(zip(a[0], b[0])):
+        assert np.array_equal(x, y), (k, x.shape, float(np.abs(x - y).max()))
+    for k, (x, y) in enumerate(zip(a[1], b[1])):
+        assert x == y, (k, x, y)
+
+
+# cells per reduction segment: 128 up to 65,536 cells (rows padded to 4), 256 up to 131,072, 512 up to
+# 262,144, then 1024; a cell per lane in the smallest shares; a separate assembly launch from 2048 cells
+# per block; the vectors leave the chip above 4096 (FP64) or 8192 cells per block
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("nx,ny,precond", [
+    (1, 1, 1), (33, 32, 1), (33, 32, 0), (1, 513, 1), (5, 700, 0), (700, 5, 1), (2500, 40, 1),
+    (260, 252, 1), (260, 253, 0), (389, 517, 1), (640, 410, 1), (700, 620, 0), (900, 880, 1)])
+def test_one_instance(capi, nx, ny, precond, prec):
+    p = cases.synthetic_problem(nx, ny, 1e-2, seed=nx + ny, tau=0.7)
+    team = _run(capi, [p], prec, precond, True, (2, 1))
+    _same(team, _run(capi, [p], prec, precond, False, (2, 1)))
+    assert all(s["status"] == 0 for s in team[1])
+    # a few launches of it, not one per pass
+    assert team[2] <= 4 * 3, team[2]
+
+
+@pytest.mark.parametrize("prec", [1, 2])
+def test_one_instance_between_two_and_eight_thousand_cells_a_block(capi, prec):
+    """1.3 million cells: by their number they would take chunks of 4096, but the step still fits the
+    cooperative form, with vectors in global memory."""
+    p = cases.synthetic_problem(1180, 1100, 1e-2, seed=5, tau=0.7)
+    b = capi.Batch([p], precision=prec)
+    assert b.launch_shape()[0] == 2048
+    b.close()
+    team = _run(capi, [p], prec, 1, True, (2,))
+    _same(team, _run(capi, [p], prec, 1, False, (2,)))
+    assert team[2] <= 4 * 2, team[2]
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("n,lo,hi", [(24, 20, 220), (152, 8, 60), (153, 8, 60), (400, 1, 48)])
+def test_many_instances(capi, n, lo, hi, prec):
+    """Teams of several blocks, one block each, and (more instances than SMs) several per block."""
+    probs = cases.batch_problems(n, 7, 1e-2, lo, hi)
+    team = _run(capi, probs, prec, 1, True, (2,))
+    _same(team, _run(capi, probs, prec, 1, False, (2,)))
+    assert team[2] <= 4 * 2, team[2]
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_steps_of_one_call_equal_single_calls(capi, prec):
+    """More steps than one launch takes."""
+    p = [cases.synthetic_problem(48, 40, 1e-2, seed=3, tau=0.7)]
+    a = _run(capi, p, prec, 1, True, (70,))
+    b = _run(capi, p, prec, 1, True, (1,) * 70)
+    _same(a, b)
+
+
+@pytest.mark.parametrize("prec", [0, 2])
+@pytest.mark.parametrize("nx", [479, 480, 960])
+def test_dirichlet_values_of_any_number(capi, nx, prec):
+    """A side's values travel 480 to a launch: 480, 481 and 961 of them, as if set at creation."""
+    p = cases.synthetic_problem(nx, 6, 1e-2, seed=nx, tau=0.7)
+    side = next(s for s in (2, 3) if p.dirichlet[s] is not None)
+    v = np.linspace(0.25, 1.75, nx + 1) * np.asarray(p.dirichlet[side]).max()
+    q = dataclasses.replace(p, dirichlet=[v if s == side else d for s, d in enumerate(p.dirichlet)])
+    a, b = capi.Solver(p, precision=prec), capi.Solver(q, precision=prec)
+    a.set_dirichlet(side, v)
+    a.step(2)
+    b.step(2)
+    fa, fb = a.f(), b.f()
+    a.close()
+    b.close()
+    assert np.array_equal(fa, fb)
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (3, 70), (33, 29), (129, 65)])
+def test_state_in_and_out(capi, nx, ny, prec):
+    """set_f then f: FP64 as it is, double-word rounded to hi + lo."""
+    p = cases.synthetic_problem(nx, ny, 1e-2, seed=9, tau=0.7)
+    f = np.random.default_rng(nx).uniform(0.0, 1.0, (nx, ny)) * 10.0 ** np.random.default_rng(ny).uniform(-30, 30, (nx, ny))
+    s = capi.Solver(p, precision=prec)
+    s.set_f(f)
+    got = s.f()
+    s.close()
+    hi = f.astype(np.float32)
+    want = f if prec != 2 else hi.astype(np.float64) + (f - hi).astype(np.float32).astype(np.float64)
+    assert np.array_equal(got, want)
+
+
+def test_noalloc_grid_too_wide_for_the_chip(capi, oracle):
+    """Rows so long that a block's vectors with both halo rows do not fit: pass by pass, to the same
+    tolerance as the other forms (1e-10 in relative L2)."""
+    torch = pytest.importorskip("torch")
+    nx, ny = 4000, 16
+    p = cases.synthetic_problem(nx, ny, 1e-2, seed=31, tau=0.7)
+    keep = {}
+
+    def dev(a):
+        keep[len(keep)] = torch.tensor(np.ascontiguousarray(a, dtype=np.float64), device="cuda")
+        return ctypes.cast(keep[len(keep) - 1].data_ptr(), capi._dp)
+
+    s = capi.sayram_problem()
+    s.nx, s.ny, s.dt = nx, ny, p.dt
+    for name in ("x_edges", "y_edges", "G", "Dxx", "Dxy", "Dyy", "inv_tau"):
+        setattr(s, name, dev(getattr(p, name)))
+    s.f0 = capi._dp()
+    for side in range(4):
+        s.bc[side] = p.bc[side]
+        s.dirichlet[side] = capi._dp() if p.dirichlet[side] is None else dev(p.dirichlet[side])
+    f = torch.tensor(p.f0, device="cuda")
+    out = torch.empty_like(f)
+    st = capi.sayram_stats()
+    rc = capi.load().sayram_step_noalloc(ctypes.byref(s), None, 2, f.data_ptr(), out.data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream, ctypes.byref(st))
+    assert rc == capi.OK, capi.last_error()
+    got, ref = out.cpu().numpy(), oracle.step(p, None, 2, solver="splu")
+    assert np.linalg.norm(got - ref) <= 1e-10 * np.linalg.norm(ref)
+    assert st.steps == 2 and got.min() >= 0.0
+
+
+@pytest.mark.parametrize("lanes", [1, 2])
+def test_server_regions_taken_again(capi, lanes):
+    """Requests served from regions that held others give the bits of a fresh server's."""
+    def requests(seed, sizes):
+        return [(cases.synthetic_problem(a, e, 1e-2, seed=seed + k, tau=0.5), 3 + k) for k, (a, e) in enumerate(sizes)]
+
+    def serve(srv, reqs):
+        ids = [srv.submit(*r) for r in reqs]
+        for _ in range(100):
+            srv.tick()
+            if srv.info()["resident"] == 0 and srv.info()["waiting"] == 0:
+                break
+        return [srv.poll(i)[0] for i in ids]
+
+    first = requests(1, [(120, 90), (33, 20), (64, 64), (20, 130)])
+    second = requests(50, [(70, 111), (128, 128), (9, 14), (40, 41)])
+    kw = dict(max_slots=8, max_side=160, precision=2, lanes=lanes, split_side=64)
+    a, b = capi.Server(5e8, **kw), capi.Server(5e8, **kw)
+    serve(a, first)
+    got, want = serve(a, second), serve(b, second)
+    a.close()
+    b.close()
+    for x, y in zip(got, want):
+        assert np.array_equal(x, y)
