@@ -23,6 +23,8 @@
 // scalars; no block waits on another.
 #pragma once
 
+#include <type_traits>
+
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -305,10 +307,11 @@ __device__ __forceinline__ R tree(const R* a, int n) {
 // and the additions'. Steps of a 33 x 32 FP64 instance 1135 -> 1070 us (twenty), of a 90 x 90 one 863 ->
 // 835 us with the short form for up to 256 segments (in double-word it gains nothing there, and its
 // code costs larger instances 1 %), of a 1024 x 1024 double-word one 4173 -> 4142 us with trees side by
-// side.
+// side, -> 4080 us with four runs on their way at a time above 512 segments (below, where two hold
+// all, four cost 4 % of a 389 x 517 instance's steps: additions of zero).
 template <int NQ, int NW, typename R>
 __device__ __forceinline__ void seg_total(const R* part, long long stride, int seg0, int nseg, R* sm) {
-  constexpr int G = NW / 8, NT = (NQ + G - 1) / G, NL = NW > 8 ? 2 : 1;
+  constexpr int G = NW / 8, NT = (NQ + G - 1) / G;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double* src = reinterpret_cast<const double*>(part) + seg0;
   R a[NT];
@@ -322,8 +325,9 @@ __device__ __forceinline__ void seg_total(const R* part, long long stride, int s
   } else {
 #pragma unroll
     for (int t = 0; t < NT; ++t) a[t] = rfrom<R>(0.0f);
-#pragma unroll 1
-    for (int s0 = lane; s0 < nseg; s0 += 256 * NL) {
+    // one round of the segments from r0 on: NL runs of each task
+    const auto round = [&](int r0, auto nl) {
+      constexpr int NL = decltype(nl)::value;
       double w[NT][NL];
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
@@ -331,7 +335,7 @@ __device__ __forceinline__ void seg_total(const R* part, long long stride, int s
         const int h = (warp - q) & 7;  // the first tasks of different quantities fall on different warps
 #pragma unroll
         for (int k = 0; k < NL; ++k) {
-          const int s = s0 + h * 32 + 256 * k;
+          const int s = r0 + lane + h * 32 + 256 * k;
           w[t][k] = q < NQ && s < nseg ? __ldcg(src + (size_t)q * stride + s) : 0.0;
         }
       }
@@ -339,6 +343,18 @@ __device__ __forceinline__ void seg_total(const R* part, long long stride, int s
       for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int k = 0; k < NL; ++k) a[t] = radd(a[t], num<R>(w[t][k]));
+    };
+    int r0 = 0;
+    if (NW > 8) {
+      if (__builtin_expect(nseg > 512, 0)) {
+#pragma unroll 1
+        for (; r0 < nseg; r0 += 1024) round(r0, std::integral_constant<int, 4>{});
+      } else {
+        round(0, std::integral_constant<int, 2>{});
+      }
+    } else {
+#pragma unroll 1
+      for (; r0 < nseg; r0 += 256) round(r0, std::integral_constant<int, 1>{});
     }
   }
   if constexpr (DW) {
