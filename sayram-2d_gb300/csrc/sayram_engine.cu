@@ -539,7 +539,8 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
 }
 
 // Zeroes cells [begin, end) of every per-cell array (a reused region must start at zero), in one
-// launch: block row y takes array y. Regions begin and end at multiples of 32 cells.
+// launch: block row y takes array y. Regions begin and end at multiples of 32 cells. (Admitting 48
+// requests to a server took 12.7 ms with a memset per array, 6.1 ms so.)
 struct ZeroList {
   float4* p[40];
   int quads[40];  // 16-byte words per 4 cells: 1 for 4-byte elements, 2 for 8-byte ones
@@ -716,6 +717,7 @@ int sayram_batch_s::plan_team() {
   std::vector<sg::TeamShare> share;
   std::vector<int> first;
   long long own = 0;  // cells of the largest share
+  double asm_most = 0.0;  // cells the busiest block would assemble
   if (ni <= blocks) {
     // the fewest cells per block with which the teams fit
     auto need = [&](long long q) {
@@ -743,6 +745,7 @@ int sayram_batch_s::plan_team() {
       const size_t at = share.size();
       share.resize(at + nb + (size_t)help);
       own = std::max<long long>(own, (long long)split_instance(I, b, nb, (int)help, share.data() + at) * I.seg);
+      asm_most = std::max(asm_most, (double)cells(b) / (nb + (int)help));
     }
   } else {
     std::vector<int> order(on);
@@ -788,9 +791,15 @@ int sayram_batch_s::plan_team() {
   SG_CUDA(cudaStreamSynchronize(stream));
   team_grid = first.empty() ? (int)share.size() : (int)first.size() - 1;
   team_bins = !first.empty();
-  // a block of k_team has 16 warps for its tiles, k_assemble up to 48 per SM: with many cells per block
-  // the launch it costs is less than it gains
-  team_split = own >= kSplitCells;
+  // a block of k_team has 16 warps for its tiles and its instance's alone, k_assemble up to 48 per SM and
+  // any tile: with many cells per block the launch it costs is less than it gains. Microseconds a step
+  // with and without a launch of its own, double-word: 512 x 512 (2048 cells a block) 74 / 64, 560 x 560
+  // (3072) 84 / 88, 800 x 800 158 / 180, 40 uneven instances 153 / 187; several instances to a block:
+  // up to 60 x 60 114 / 109, up to 100 x 100 258 / 288. In FP64 both are bound by the pipe, and only
+  // the balance counts: 620 x 620 293 / 284, 900 x 900 562 / 552, 24 instances 352 / 346, 40 instances
+  // (blocks up to 1.3 times the mean) 519 / 547, several to a block 280 / 259.
+  if (team_bins) team_split = dwm && own > 2 * kSplitCells;
+  else team_split = own > kSplitCells && (mixed || asm_most > 1.15 * (double)total / blocks);
   team_chip = chip;
   team_own = own;
   team_pmax = pm;
@@ -982,8 +991,8 @@ int sayram_batch_s::last_captured(cudaGraphNode_t* node) {
   return SAYRAM_OK;
 }
 
-// One step as a graph: memset + begin + assemble, WHILE(outer){ resid, WHILE(inner){ k1 k2 k3 } },
-// polish. The WHILE conditions are set on the device by the residual and Krylov kernels.
+// One step as a graph: memset + begin + assemble, WHILE(outer){ resid, its decisions, WHILE(inner){ k1, v's
+// decisions, k2, t's } }, polish. The WHILE conditions are set on the device by the deciding kernels.
 template <typename T, typename C, typename A, int CH>
 int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck, const sg::Kry<T>& kr, bool prefix) {
   using namespace sg;
@@ -1081,7 +1090,11 @@ int sayram_batch_s::launch_steps(int nsteps) {
             {"assemble", sg::TEAM_ASSEMBLE}, {"solve_coop", sg::TEAM_SOLVE}, {"polish", sg::TEAM_POLISH}};
         for (auto& p : ph) {
           int r2 = SAYRAM_OK;
-          launch(p.first, [&] { r2 = launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH); });
+          launch(p.first, [&] {
+            r2 = team_split && p.second == sg::TEAM_ASSEMBLE
+                     ? launch_assemble(0, -1)
+                     : launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH);
+          });
           if (r2) rc = r2;
         }
         if (rc) return rc;
@@ -1575,6 +1588,7 @@ int sayram_batch_set_dirichlet(sayram_batch b, int idx, int side, const double* 
   if (n != m) return fail(SAYRAM_ERR_ARG, "expected " + std::to_string(m) + " vertex values");
   SG_CUDA(cudaSetDevice(b->dev));
   // the values travel as kernel parameters: no copy to wait for, and the caller's buffer is free at once
+  // (81 values: 11.4 us a call with a copy and a wait, 5.4 so)
   for (int at = 0; at < m; at += PutArgs::kMost) {
     PutArgs p;
     p.n = std::min(m - at, PutArgs::kMost);

@@ -63,7 +63,7 @@ def test_one_instance_between_two_and_eight_thousand_cells_a_block(capi, prec):
 
 
 @pytest.mark.parametrize("prec", [0, 1, 2])
-@pytest.mark.parametrize("n,lo,hi", [(24, 20, 220), (152, 8, 60), (153, 8, 60), (400, 1, 48)])
+@pytest.mark.parametrize("n,lo,hi", [(24, 20, 220), (40, 100, 200), (152, 8, 60), (153, 8, 60), (400, 1, 48)])
 def test_many_instances(capi, n, lo, hi, prec):
     """Teams of several blocks, one block each, and (more instances than SMs) several per block."""
     probs = cases.batch_problems(n, 7, 1e-2, lo, hi)
