@@ -322,10 +322,9 @@ def run_reference(a):
 # each kernel must touch once (neighbour re-reads served by cache are not counted).
 BYTES32 = {
     "assemble": 2 * 8 + 8 * 8 + 4 * (4 + 4) + 4 * 8,  # f, start g, 8 factors -> 4 hi+lo coefs, invD/R/colsum/y
-    "resid": 8 + 4 + 8 + 4 * (4 + 4) + 8 + 4,     # y, x, R, hi+lo coefs -> y', r
-    "bicg1": 4 * 4 + 4 * 4 + 2 * 4,               # r, p, v, r^, 4 coefs -> p', v'
-    "bicg2": 2 * 4 + 4 * 4 + 4,                   # r, v, 4 coefs -> t
-    "bicg3": 6 * 4 + 2 * 4,                       # r, v, p, t, r^, x -> x, r
+    "resid": 8 + 4 * 4 + 8 + 4 * (4 + 4) + 8 + 4,  # y, r, v, p, x, R, hi+lo coefs -> y', r
+    "bicg1": 6 * 4 + 4 * 4 + 4 * 4,               # r, v, t, p, x, r^, 4 coefs -> r, p, x, v
+    "bicg2": 3 * 4 + 4 * 4 + 4,                   # r, v, r^, 4 coefs -> t
     "polish": 8 + 4 * (4 + 4) + 3 * 8 + 8 + 3 * 8 + 8 + 3 * 8,  # y, hi+lo coefs, R, invD, colsum, f, 3 earlier
                                                             # states, loss factor -> f, history slot, start g
 }
@@ -334,12 +333,19 @@ BYTES32 = {
 # The same for the FP64 drop-in (mode 0): FP64 Krylov vectors and coefficients.
 BYTES64 = {
     "assemble": BYTES32["assemble"],              # 8-byte coefficients either way (FP64 or hi+lo)
-    "resid": 8 + 8 + 8 + 4 * 8 + 8 + 8,           # y, x, R, coefs -> y', r
-    "bicg1": 4 * 8 + 4 * 8 + 2 * 8,               # r, p, v, r^, 4 coefs -> p', v'
-    "bicg2": 2 * 8 + 4 * 8 + 8,                   # r, v, 4 coefs -> t
-    "bicg3": 6 * 8 + 2 * 8,                       # r, v, p, t, r^, x -> x, r
+    "resid": 8 + 4 * 8 + 8 + 4 * 8 + 8 + 8,       # y, r, v, p, x, R, coefs -> y', r
+    "bicg1": 6 * 8 + 4 * 8 + 4 * 8,               # r, v, t, p, x, r^, 4 coefs -> r, p, x, v
+    "bicg2": 3 * 8 + 4 * 8 + 8,                   # r, v, r^, 4 coefs -> t
     "polish": BYTES32["polish"],
 }
+
+
+def first_bytes(model):
+    """The first pass of its kind moves less: a step's first residual has no correction to add (y, R,
+    coefficients -> r), a solve's first iteration has p = r = r^ and no x (r^, 4 coefs -> v; r^, v, 4
+    coefs -> t)."""
+    t = 4 if model is BYTES32 else 8
+    return {"resid": 8 + 8 + 32 + t, "bicg1": 6 * t, "bicg2": 7 * t}
 
 
 # The algorithmic bytes per cell of the hot-path analysis, for the assembly: read f, Lxx, Lxy,
@@ -351,7 +357,7 @@ ANALYSIS_BYTES = {"assemble": 96}
 # DRAM bytes per processed cell measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum) on the
 # 256-instance case of the same kernels (one ncu capture per kernel); traffic grows with the
 # cells processed, so a launch's traffic is this figure times the cells it processed.
-TRAFFIC32 = {"assemble": 142.5, "bicg1": 27.5, "bicg2": 26.5, "bicg3": 23.2, "resid": 58.1, "polish": 131.5}
+TRAFFIC32 = {"assemble": 142.0, "polish": 126.5}
 
 
 def kernel_roofline(b, probs, peak, steps=2, model=None):
@@ -367,16 +373,22 @@ def kernel_roofline(b, probs, peak, steps=2, model=None):
     after = [b.stats(k) for k in range(len(probs))]
     it = np.array([a["total_iterations"] - c["total_iterations"] for a, c in zip(after, before)], dtype=np.float64)
     rf = np.array([a["total_refinements"] - c["total_refinements"] for a, c in zip(after, before)], dtype=np.float64)
-    proc = {"assemble": cells.sum() * steps, "polish": cells.sum() * steps, "resid": (cells * rf).sum(),
-            "bicg1": (cells * it).sum(), "bicg2": (cells * it).sum(), "bicg3": (cells * it).sum()}
+    # refinement passes end in a Krylov solve but for each step's last
+    solves = np.minimum(np.maximum(rf - steps, 0.0), it)
+    later, first = (cells * (it - solves)).sum(), (cells * solves).sum()
+    fb = first_bytes(model)
+    moved = {"assemble": model["assemble"] * cells.sum() * steps, "polish": model["polish"] * cells.sum() * steps,
+             "resid": model["resid"] * first + fb["resid"] * cells.sum() * steps,
+             "bicg1": model["bicg1"] * later + fb["bicg1"] * first,
+             "bicg2": model["bicg2"] * later + fb["bicg2"] * first}
     out = {}
     for name, (ms, n) in kt.items():
-        if name == "solve_coop" and n > 0:  # the refinement loop as one cooperative kernel
-            byts = sum(model[k] * proc[k] for k in ("resid", "bicg1", "bicg2", "bicg3"))
+        if name == "solve_coop" and n > 0:  # the refinement loop within the cooperative step
+            byts = sum(moved[k] for k in ("resid", "bicg1", "bicg2"))
             out[name] = {"ms": ms, "launches": int(n), "bytes": byts, "GBps": byts / (ms * 1e-3) / 1e9,
                          "share": 0.0}
         elif name in model and n > 0:
-            byts = model[name] * proc[name]
+            byts = moved[name]
             out[name] = {"ms": ms, "launches": int(n), "bytes": byts, "GBps": byts / (ms * 1e-3) / 1e9,
                          "share": 0.0}
         else:

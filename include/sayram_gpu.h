@@ -212,7 +212,7 @@ int sayram_batch_elapsed_ms(sayram_batch b, int slot0, int slot1, double* ms);
 /* Per-kernel timing: when enabled, every launch is bracketed by CUDA events on the batch's
  * stream (steps then run without graphs). sayram_batch_kernel_times fills up to cap entries of
  * names/total milliseconds/launch counts and returns the number of entries: one per kernel, plus
- * "krylov_tail10" and "krylov_rest", the time of whole BiCGSTAB iterations (their three kernels)
+ * "krylov_tail10" and "krylov_rest", the time of whole BiCGSTAB iterations (bicg1, bicg2, bicg3)
  * in which fewer than 10 % / at least 10 % of the enabled instances were still iterating. */
 int sayram_batch_enable_timing(sayram_batch b, int enable);
 int sayram_batch_kernel_times(sayram_batch b, const char** names, double* total_ms,
@@ -222,10 +222,11 @@ int sayram_batch_kernel_times(sayram_batch b, const char** names, double* total_
  * fastest. The instances' state is restored afterwards, so tuning does not advance the
  * simulation. Writes the choice if the pointers are not NULL. */
 int sayram_batch_autotune(sayram_batch b, int steps, int* chunk_out, int* blocks_per_sm_out);
-/* The refinement loop of a step runs as one cooperative kernel (grid-wide barriers between its
- * passes) when every chunk of the batch gets a block in one wave of co-resident blocks -- a
- * single large instance or a few -- and as the graph's loops of separate kernels otherwise.
- * on = 0 always uses the separate kernels (the results are the same bit for bit). Default: 1. */
+/* A batch that fits the chip (in the FP32 modes about two million cells, in FP64 about 1.3 million
+ * by default) takes whole steps in one cooperative launch: a team of blocks per instance, with a
+ * barrier between its passes, or, with more instances than SMs, blocks with several instances
+ * each; larger batches run as the graph's loops of separate kernels. on = 0 always uses the
+ * separate kernels (the results are the same bit for bit). Default: 1. */
 int sayram_batch_set_coop(sayram_batch b, int on);
 /* Sets the launch shape directly (chunk 1024, 2048 or 4096 cells; 1..64 blocks per SM), or reads
  * it back. The default is chosen from the batch size; results do not depend on it beyond the
@@ -320,7 +321,9 @@ void sayram_server_destroy(sayram_server s);
  * The first call on a device looks up the array's device address (cudaGetSymbolAddress) and
  * keeps it for later calls; make that first call before any stream capture begins. The kept
  * address does not survive cudaDeviceReset: calls after a reset are not supported. Every call
- * waits for its stream between launches (it reads the loops' control words back to the host).
+ * waits for its stream before it returns; on grids whose rows are too long for the cooperative form
+ * (a block keeps its share and a row above and below in shared memory: up to about 3000 cells a row
+ * fit) also between launches, to read the loops' control words back to the host.
  * All calls share the array: each call clears it at its start and the array keeps the last
  * call's contents afterwards. Calls that overlap on the GPU (several host threads or streams at
  * once) race on it and must be serialized by the caller. */

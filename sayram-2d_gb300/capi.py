@@ -341,8 +341,8 @@ class Batch:
         check(self._L.sayram_batch_set_dtable(self.h, int(idx), ctypes.byref(t)), "sayram_batch_set_dtable")
 
     def set_coop(self, on: bool) -> None:
-        """Run each step's refinement loop as one cooperative kernel when the batch's chunks fit in
-        one wave of co-resident blocks (default), or always as the loops of separate kernels."""
+        """Take whole steps in one cooperative launch when the batch fits the chip (default), or always
+        as separate kernels."""
         check(self._L.sayram_batch_set_coop(self.h, 1 if on else 0), "sayram_batch_set_coop")
 
     def set_launch_shape(self, chunk: int, blocks_per_sm: int) -> None:

@@ -18,9 +18,10 @@
 // Reductions are deterministic and have one order, whichever kernel runs them: the cells of an
 // instance are cut into segments (seg_cells: 128 to 4096, by its size and the batch's chunk size),
 // every segment's sum is a fixed tree over its cells, and an instance's total is a fixed tree over
-// its segments (seg_total). In the per-pass kernels the last block to finish an instance's
-// chunks (counted with one atomic per chunk) forms the totals and updates that instance's Krylov
-// scalars; no block waits on another.
+// its segments (seg_total). After a pass of the per-pass kernels a small kernel with a block per
+// instance forms the totals and updates the instance's scalars (k_after_*; for the polish the last
+// block to finish the instance's chunks); no block waits on another. In k_team every block of an
+// instance's team forms them, after the team's barrier.
 #pragma once
 
 #include <type_traits>

@@ -5,9 +5,12 @@
 //   k_begin      per step: resets the per-instance solver state
 //   k_assemble   fused vertex interpolation + PPFV face fluxes + diagonal/RHS + Jacobi scaling
 //   k_resid      outer residual r = R - A~ y (adds the last Krylov correction first)
-//   k_bicg1/2/3  one BiCGSTAB iteration in T precision (FP64 or FP32) with fused SpMV + dots
+//   k_bicg1/2    one BiCGSTAB iteration in T precision (FP64 or FP32) with fused SpMV + dots
+//   k_after_*    the decisions after each of these passes, a block per instance
 //   k_polish     positivity polish y' = R + (I - A~) y+, f = y'/D, min / clamp / mass checks
-//                (these four in sayram_solve.cuh)
+//                (these in sayram_solve.cuh)
+//   k_team       all of a step but the set-up in one launch, for batches that fit the chip
+//                (sayram_team.cuh)
 //   k_field_*    alpha-major FP64 <-> padded system order transposes for the host-buffer step
 //
 // The assembly, residual, polish and state are written once over an arithmetic policy A:
@@ -60,7 +63,7 @@ __device__ __forceinline__ int n_chunks(const Common& cm) { return cm.dyn ? cm.d
 __device__ __forceinline__ int n_tiles(const Common& cm) { return cm.dyn ? cm.dyn[1] : cm.ntiles; }
 __device__ __forceinline__ int n_inst(const Common& cm) { return cm.dyn ? cm.dyn[2] : cm.ninst; }
 
-// The last block of a loop-deciding kernel sets the graph's WHILE conditions from the number of
+// The last block of a deciding kernel (k_after_resid, k_after_t) sets the graph's WHILE conditions from the number of
 // instances still active. The trip counters make both loops terminate after guard_refine
 // residual evaluations and guard_iters Krylov iterations even if the counts were inconsistent.
 // which = 0: after the residual (decides both loops); which = 1: after a Krylov iteration.
