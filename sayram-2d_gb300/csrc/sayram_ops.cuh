@@ -635,25 +635,24 @@ struct AsmTile {
   V hS[VY][2];  // the tile's vertex rows: bilinear weights (wB, wT), Solver.cc:333-336
 };
 
-// Barrier among the NT threads that share a tile: the whole block, or (bar > 0) one of its parts.
-template <int NT>
-__device__ __forceinline__ void tile_sync(int bar) {
+// Barrier among the threads that share a tile: the whole block, or (bar > 0) n of them.
+__device__ __forceinline__ void tile_sync(int bar, int n) {
   if (bar == 0) __syncthreads();
-  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NT) : "memory");
+  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory");
 }
 
-// Assembles the tile of up to kTX x ty cells at (i0, j0) of instance I by NT threads (tid: 0 .. NT);
-// returns this warp's max of the right-hand side. yc: the current y buffer; has_g: the idle one holds
-// the extrapolated start. The cells, vertices and faces of a tile at the grid's right or upper edge
+// Assembles the tile of up to kTX x ty cells at (i0, j0) of instance I by NT threads (tid: 0 .. NT; a
+// power of two); returns this warp's max of the right-hand side. yc: the current y buffer; has_g: the idle
+// one holds the extrapolated start. The cells, vertices and faces of a tile at the grid's right or upper edge
 // are dealt to the threads without gaps: an idle lane takes as long as a busy one (both policies
 // are bound by their arithmetic), and on grids of 64 to 256 a side a tenth of the lanes were idle.
 // Measured with it (and, in FP64, the shorter reciprocal and the sign tests on bits), per 4-step call:
 // double-word, 1024 uneven instances, 4.26 -> 4.05 ms; FP64, 192 instances, 3.46 -> 2.98 ms; mixed
 // 4.07 -> 3.54 ms.
-template <typename C, typename A, int NT>
+template <typename C, typename A>
 __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const Geo& geo, const Fields& fl,
                                           const Coef<C>& co, const InstDev& I, int i0, int j0, const int ty,
-                                          bool has_g, int yc, const int tid, const int bar) {
+                                          bool has_g, int yc, const int tid, const int NT, const int bar) {
   using V = typename A::V;
   constexpr int VX = AsmTile<A>::VX;
   const int nx = I.nx, ny = I.ny, P = I.pitch;
@@ -725,7 +724,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
       S.hS[vy][1] = in ? A::ld(cm.wy, 2 * (I.ye + Jv) + 1) : zero;
     }
   }
-  tile_sync<NT>(bar);
+  tile_sync(bar, NT);
   // 2) vertex values (Solver.cc:299-422): corners copy, interior bilinear, boundary edges
   //    linear, then Dirichlet overrides with XMIN < XMAX < YMIN < YMAX precedence. The bilinear
   //    value wB (wL f00 + wR f10) + wT (wL f01 + wR f11) is formed from the two row
@@ -750,7 +749,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
     }
     S.vS[vy][vx] = val;
   }
-  tile_sync<NT>(bar);
+  tile_sync(bar, NT);
   // 3a) x-faces (vertex column Iv between cells Iv-1 and Iv)
   for (int q = tid; q < W1 * h; q += NT) {
     const int ry = (q * rW1) >> 16, vx = q - ry * W1;
@@ -793,7 +792,7 @@ __device__ __forceinline__ float asm_tile(AsmTile<A>& S, const Common& cm, const
     S.yB[vy][cx] = Jv == 0 ? bm : aB;
     S.yT[vy][cx] = Jv == ny ? bm : aT;
   }
-  tile_sync<NT>(bar);
+  tile_sync(bar, NT);
   // 4) per cell: diagonal in the reference's triplet order, RHS, scaling, scatter
   float rmax = 0.0f;
 #pragma unroll 1
@@ -851,8 +850,8 @@ __global__ void __launch_bounds__(kAsmThreads, A::kAsmBlocks) k_assemble(Common 
     const int lt = t - I.tile0;
     // the extrapolated start g the last polish left in the idle y buffer (none before the first
     // step or after the state was replaced: then y0 = D f)
-    const float rmax = asm_tile<C, A, kAsmThreads>(S, cm, geo, fl, co, I, (lt % I.ntx) * kTX, (lt / I.ntx) * kTY, kTY,
-                                                   cm.st[b].nhist > 0, cm.st[b].ycur, threadIdx.x, 0);
+    const float rmax = asm_tile<C, A>(S, cm, geo, fl, co, I, (lt % I.ntx) * kTX, (lt / I.ntx) * kTY, kTY,
+                                      cm.st[b].nhist > 0, cm.st[b].ycur, threadIdx.x, kAsmThreads, 0);
     if ((threadIdx.x & 31) == 0 && rmax > 0.0f) atomicMax(&cm.st[b].rmax_bits, __float_as_uint(rmax));
     __syncthreads();
   }

@@ -171,17 +171,24 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_team(Common cm, Geo geo, Fi
     for (int step = 0; ok && step < ta.nsteps; ++step) {
       // ---------------------------------------------------------------- assembly
       if (ta.phases & TEAM_ASSEMBLE) {
-        // a tile's steps are short between its barriers: each quarter of the block has a tile of its own
-        constexpr int QT = kTeamThreads / kTeamParts;
-        const int part_ = tid / QT;
-        AsmTile<A>& tile = reinterpret_cast<AsmTile<A>*>(mem)[part_];
+        // a tile's steps are short between its barriers: four tiles at a time, by a quarter of the block each.
+        // A block with one or two of them gives all its threads to those, as far as a tile has faces for
+        // them (33 cells across need 99 to 1089 threads). Microseconds a step before and after: 33 x 32
+        // FP64 22.2 / 21.4, 90 x 90 FP64 37.6 / 36.8, 256 x 256 double-word 42.4 / 34.5 (FP64 78.4 / 70.3),
+        // 24 instances of up to 64 x 64 39 / 32; with more tiles the number of threads as a variable
+        // costs a little, 400 x 400 57.2 / 58.0.
         const int nty = (I.ny + sh.ty - 1) / sh.ty, nt = I.ntx * nty;
+        const int tiles = (nt + sh.nb - 1) / sh.nb, faces = (min(kTX, I.nx) + 1) * (2 * sh.ty + 1);
+        int QT = kTeamThreads / (tiles > 2 ? kTeamParts : tiles);
+        while (QT > kTeamThreads / kTeamParts && QT >= 2 * faces) QT /= 2;
+        const int parts_ = kTeamThreads / QT, part_ = tid / QT;
+        AsmTile<A>& tile = reinterpret_cast<AsmTile<A>*>(mem)[part_];
         const bool has_g = S.nhist > 0;
         float rmax = 0.0f;
-        for (int t = sh.rank + part_ * sh.nb; t < nt; t += sh.nb * kTeamParts) {
-          rmax = fmaxf(rmax, asm_tile<C, A, QT>(tile, cm, geo, fl, cf, I, (t % I.ntx) * kTX, (t / I.ntx) * sh.ty,
-                                                sh.ty, has_g, S.ycur, tid % QT, 1 + part_));
-          tile_sync<QT>(1 + part_);
+        for (int t = sh.rank + part_ * sh.nb; t < nt; t += sh.nb * parts_) {
+          rmax = fmaxf(rmax, asm_tile<C, A>(tile, cm, geo, fl, cf, I, (t % I.ntx) * kTX, (t / I.ntx) * sh.ty, sh.ty,
+                                            has_g, S.ycur, tid % QT, QT, 1 + part_));
+          tile_sync(1 + part_, QT);
         }
         if ((tid & 31) == 0) s_w[warp] = rmax;
         __syncthreads();
