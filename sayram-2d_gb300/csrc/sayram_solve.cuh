@@ -199,8 +199,8 @@ __device__ __forceinline__ int after_resid(InstState& st, const R (&tot)[3], dou
   st.cum_refines += 1;
   st.rr64 = stored(tot[0]);
   const R bb = num<R>(st.bb);
-  const R bound = rmul(rfrom<R>(tol * tol), bb);  // ||r|| <= tol ||R||
-  if (!rgt(tot[0], bound)) {
+  const R bound = rmul(rfrom<R>(tol * tol), bb);  // ||r|| <= tol ||R||, or R = 0
+  if (!rgt(tot[0], bound) || !rgt(bb, rfrom<R>(0.0f))) {
     st.outer_active = 0;
     st.status = ST_OK;
     return 0;
