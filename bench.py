@@ -333,9 +333,9 @@ BYTES32 = {
 # The same for the FP64 drop-in (mode 0): FP64 Krylov vectors and coefficients.
 BYTES64 = {
     "assemble": BYTES32["assemble"],              # 8-byte coefficients either way (FP64 or hi+lo)
-    "resid": 8 + 4 * 8 + 8 + 4 * 8 + 8 + 8,       # y, r, v, p, x, R, coefs -> y', r
-    "bicg1": 6 * 8 + 4 * 8 + 4 * 8,               # r, v, t, p, x, r^, 4 coefs -> r, p, x, v
-    "bicg2": 3 * 8 + 4 * 8 + 8,                   # r, v, r^, 4 coefs -> t
+    "resid": 8 + 3 * 8 + 8 + 4 * 8 + 8 + 8,       # y, s, p, x, R, coefs -> y', r
+    "bicg1": 6 * 8 + 4 * 8 + 4 * 8,               # s, v, t, p, x, r^, 4 coefs -> r, p, x, v
+    "bicg2": 3 * 8 + 4 * 8 + 2 * 8,               # r, v, r^, 4 coefs -> t, s
     "polish": BYTES32["polish"],
 }
 
@@ -345,7 +345,7 @@ def first_bytes(model):
     coefficients -> r), a solve's first iteration has p = r = r^ and no x (r^, 4 coefs -> v; r^, v, 4
     coefs -> t)."""
     t = 4 if model is BYTES32 else 8
-    return {"resid": 8 + 8 + 32 + t, "bicg1": 6 * t, "bicg2": 7 * t}
+    return {"resid": 8 + 8 + 32 + t, "bicg1": 6 * t, "bicg2": (7 if t == 4 else 8) * t}
 
 
 # The algorithmic bytes per cell of the hot-path analysis, for the assembly: read f, Lxx, Lxy,

@@ -305,6 +305,9 @@ struct CoefW<float, A> {
   }
 };
 
+template <typename T>
+constexpr bool kStoreS = sizeof(T) == 8;  // s of an iteration is stored (see k_bicg1)
+
 // ------------------------------------------------------------------------------ outer residual
 // One 4-cell group of r = R - A~ y in the wide arithmetic from the staged y (sm + o): y itself, the
 // scaled residual with the preconditioner applied, and the group's terms of ||r||^2, ||R||^2 and
@@ -425,18 +428,19 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       using RK = typename RedOf<T>::R;
       const int it = st.iters;
       const T alpha = rhead(num<RK>(st.alpha)), omega = rhead(num<RK>(st.omega));
-      const T* rr = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
+      const T* rr = kStoreS<T> ? kr.r[1] : it > 1 ? sel2(kr.r, it & 1) : kr.rh;  // s, or r
       const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
       const T* vv = sel2(kr.v, it & 1);
       stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
         Q4<V> y = A::ld4(yin + k);
-        const Q4<T> r = ld4(rr + k), v = ld4(vv + k);
-        const Q4<T> p = it > 1 ? ld4(pp + k) : r;
+        Q4<T> s = ld4(rr + k), v;
+        if (!kStoreS<T>) v = ld4(vv + k);
+        const Q4<T> p = kStoreS<T> || it > 1 ? ld4(pp + k) : s;
         Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
         if (it > 1) x = ld4(kr.x + k);
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-          const T sv = fmaT(-alpha, v.a[m], r.a[m]);
+          const T sv = kStoreS<T> ? s.a[m] : fmaT(-alpha, v.a[m], s.a[m]);
           const T xv = fmaT(alpha, p.a[m], fmaT(omega, sv, x.a[m]));
           y.a[m] = A::template add_scaled<T>(y.a[m], xv, isc);
         }
@@ -487,6 +491,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(typename A::Acc) == 4 ? 4 : 3
 // four multiply-adds and no FP64-rate conversions in the preconditioner. Measured, whole calls: 192
 // uneven FP64 instances, 4 steps, 19.2 -> 15.8 ms; 1024 in double-word 22.5 -> 20.2 ms; 24 in
 // double-word, 6 steps, 2.94 -> 2.47 ms; 192 mixed with Jacobi scaling 14.7 -> 14.0 ms.
+// FP64 is bound by its pipe, not by HBM: there k2 stores s (in r[1]; r stays in r[0]), and neither the
+// next k1 nor the residual kernel forms it again (192 uneven instances, 4 steps: k1 4.15 -> 3.95, k2
+// 3.47 -> 3.52, residuals 1.24 -> 1.21 ms).
 template <typename T, int CH>
 __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, const Kry<T>& kr) {
   using R = typename RedOf<T>::R;
@@ -501,10 +508,10 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     const int it = st.iters;  // iterations finished; this one is it + 1
     const bool rs = st.restart != 0;
     const T alpha = rhead(num<R>(st.alpha)), beta = rhead(num<R>(st.beta)), omega = rhead(num<R>(st.omega));
-    const T* ro = it > 1 ? sel2(kr.r, it & 1) : kr.rh;
+    const T* ro = kStoreS<T> ? kr.r[1] : it > 1 ? sel2(kr.r, it & 1) : kr.rh;  // s, or r
     const T* po = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
     const T* vo = sel2(kr.v, it & 1);
-    T* rn = sel2(kr.r, (it + 1) & 1);
+    T* rn = kStoreS<T> ? kr.r[0] : sel2(kr.r, (it + 1) & 1);
     T* pn = sel2(kr.p, (it + 1) & 1);
     T* vn = sel2(kr.v, (it + 1) & 1);
     const int P = I.pitch;
@@ -517,12 +524,12 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     } else {
       stage_rows<T, 1>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
         const Q4<T> r = ld4(ro + k), v = ld4(vo + k), t = ld4(kr.t + k);
-        Q4<T> p = it > 1 ? ld4(po + k) : r;
+        Q4<T> p = kStoreS<T> || it > 1 ? ld4(po + k) : r;
         const bool mine = k >= c0 && k < c1;
         Q4<T> s, q;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-          s.a[m] = fmaT(-alpha, v.a[m], r.a[m]);
+          s.a[m] = kStoreS<T> ? r.a[m] : fmaT(-alpha, v.a[m], r.a[m]);
           q.a[m] = fmaT(-omega, t.a[m], s.a[m]);
         }
         if (mine) {
@@ -583,7 +590,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;
     const T alpha = rhead(num<R>(st.alpha));
-    const T* r = it > 0 ? sel2(kr.r, (it + 1) & 1) : kr.rh;
+    const T* r = it == 0 ? kr.rh : kStoreS<T> ? kr.r[0] : sel2(kr.r, (it + 1) & 1);
     const T* vv = sel2(kr.v, (it + 1) & 1);
     const int P = I.pitch;
     const long long c0 = chunk_start<CH>(c, I);
@@ -595,6 +602,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
       const Q4<T> v = ld4(vv + k);
 #pragma unroll
       for (int m = 0; m < 4; ++m) x.a[m] = fmaT(-alpha, v.a[m], x.a[m]);
+      if (kStoreS<T> && k >= c0 && k < c1) st4(kr.r[1] + k, x);
       return x;
     });
     __syncthreads();
