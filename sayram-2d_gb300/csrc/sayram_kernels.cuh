@@ -75,7 +75,7 @@ struct InstState {
   int ycur, outer_active, inner_active;
   int restart, has_x;
   int iters;               // Krylov iterations of this solve finished so far
-  int pad_i;
+  int swapped;             // rh and x of the per-pass kernels have changed places (rh_of)
   int iters_total, refines, status;
   int nhist;               // earlier states held in the history buffers (extrapolated start)
   int hslot;               // history buffer holding f^(n-1); f^(n-2), ... are in the ones before it

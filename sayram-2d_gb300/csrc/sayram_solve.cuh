@@ -192,7 +192,10 @@ __device__ __forceinline__ T dot4(const Q4<T>& a, const Q4<T>& b, T q) {
 template <typename RK, typename R>
 __device__ __forceinline__ int after_resid(InstState& st, const R (&tot)[3], double tol, double inner_tol,
                                            int max_refine, int precond) {
-  if (st.has_x) st.ycur ^= 1;  // the pass has written y + x to the other buffer
+  if (st.has_x) {
+    st.ycur ^= 1;  // the pass has written y + x to the other buffer
+    if (st.iters == 1) st.swapped ^= 1;  // and r to x's place (resid_body)
+  }
   st.has_x = 0;
   if (st.refines == 0) st.bb = stored(tot[1]);
   st.refines += 1;
@@ -266,6 +269,12 @@ __device__ __forceinline__ int after_t(InstState& st, const R (&tot)[5], int max
   } else {
     st.beta = stored(beta);
   }
+  // A restart writes r^, which the second iteration's first pass still reads as r and p, also where a
+  // neighbouring block writes: the next residual is the restart there.
+  if (st.restart && st.iters == 1) {
+    st.has_x = 1;
+    return 1;
+  }
   return 0;
 }
 
@@ -307,6 +316,13 @@ struct CoefW<float, A> {
 
 template <typename T>
 constexpr bool kStoreS = sizeof(T) == 8;  // s of an iteration is stored (see k_bicg1)
+// The shadow residual and the solution of an instance's solve. A solve's first iteration has p = r =
+// r^ and no x, so the residual after a solve of one iteration reads r^ in its neighbours' rows too:
+// it writes the next solve's into x's array, and the two change places.
+template <typename T>
+__device__ __forceinline__ T* rh_of(const Kry<T>& kr, const InstState& st) { return st.swapped ? kr.x : kr.rh; }
+template <typename T>
+__device__ __forceinline__ T* x_of(const Kry<T>& kr, const InstState& st) { return st.swapped ? kr.rh : kr.x; }
 
 // ------------------------------------------------------------------------------ outer residual
 // One 4-cell group of r = R - A~ y in the wide arithmetic from the staged y (sm + o): y itself, the
@@ -412,6 +428,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
     const double* yin = sel2(fl.y64, st.ycur);
     double* yout = sel2(fl.y64, st.ycur ^ 1);
     const bool hx = st.has_x != 0;
+    T* const rout = hx && st.iters == 1 ? x_of(kr, st) : rh_of(kr, st);
     const float sc = rhs_scale(st.rmax_bits);  // r is handed over as r * sc
     const float isc = 1.0f / sc;                // exact: sc is a power of two
     const int P = I.pitch;
@@ -428,8 +445,9 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       using RK = typename RedOf<T>::R;
       const int it = st.iters;
       const T alpha = rhead(num<RK>(st.alpha)), omega = rhead(num<RK>(st.omega));
-      const T* rr = kStoreS<T> ? kr.r[1] : it > 1 ? sel2(kr.r, it & 1) : kr.rh;  // s, or r
-      const T* pp = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
+      const T* rr = kStoreS<T> ? kr.r[1] : it > 1 ? sel2(kr.r, it & 1) : rh_of(kr, st);  // s, or r
+      const T* pp = it > 1 ? sel2(kr.p, it & 1) : rh_of(kr, st);
+      const T* xx = x_of(kr, st);
       const T* vv = sel2(kr.v, it & 1);
       stage_rows<V>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
         Q4<V> y = A::ld4(yin + k);
@@ -437,7 +455,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
         if (!kStoreS<T>) v = ld4(vv + k);
         const Q4<T> p = kStoreS<T> || it > 1 ? ld4(pp + k) : s;
         Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
-        if (it > 1) x = ld4(kr.x + k);
+        if (it > 1) x = ld4(xx + k);
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
           const T sv = kStoreS<T> ? s.a[m] : fmaT(-alpha, v.a[m], s.a[m]);
@@ -457,7 +475,7 @@ __device__ __forceinline__ void resid_body(const Common& cm, const Fields& fl, c
       Q4<T> r;
       resid_group<T, C, A>(sm, (int)(K - e0), P, co, K, fl.R, sc, cm.precond, st.refines == 0, yc, r, q0, q1, q2);
       if (hx) A::st4(yout + K, yc);
-      st4(kr.rh + K, r);
+      st4(rout + K, r);
     }, [&](int p) {
       const typename A::Acc w[3] = {q0, q1, q2};
       sums.put(p, w);
@@ -508,8 +526,10 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     const int it = st.iters;  // iterations finished; this one is it + 1
     const bool rs = st.restart != 0;
     const T alpha = rhead(num<R>(st.alpha)), beta = rhead(num<R>(st.beta)), omega = rhead(num<R>(st.omega));
-    const T* ro = kStoreS<T> ? kr.r[1] : it > 1 ? sel2(kr.r, it & 1) : kr.rh;  // s, or r
-    const T* po = it > 1 ? sel2(kr.p, it & 1) : kr.rh;
+    T* const rhat = rh_of(kr, st);
+    T* const xx = x_of(kr, st);
+    const T* ro = kStoreS<T> ? kr.r[1] : it > 1 ? sel2(kr.r, it & 1) : rhat;  // s, or r
+    const T* po = it > 1 ? sel2(kr.p, it & 1) : rhat;
     const T* vo = sel2(kr.v, it & 1);
     T* rn = kStoreS<T> ? kr.r[0] : sel2(kr.r, (it + 1) & 1);
     T* pn = sel2(kr.p, (it + 1) & 1);
@@ -520,7 +540,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
     const long long e0 = c0 - P;
     Sums sums{reinterpret_cast<R(*)[Sums::kParts]>(s_part)};
     if (it == 0) {
-      stage_rows<T>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) { return ld4(kr.rh + k); });
+      stage_rows<T>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) { return ld4(rhat + k); });
     } else {
       stage_rows<T, 1>(sm, e0, (int)(c1 - c0) + 2 * P, [&](long long k) {
         const Q4<T> r = ld4(ro + k), v = ld4(vo + k), t = ld4(kr.t + k);
@@ -534,17 +554,17 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
         }
         if (mine) {
           Q4<T> x{{(T)0, (T)0, (T)0, (T)0}};
-          if (it > 1) x = ld4(kr.x + k);
+          if (it > 1) x = ld4(xx + k);
 #pragma unroll
           for (int m = 0; m < 4; ++m) x.a[m] = fmaT(alpha, p.a[m], fmaT(omega, s.a[m], x.a[m]));
-          st4(kr.x + k, x);
+          st4(xx + k, x);
         }
 #pragma unroll
         for (int m = 0; m < 4; ++m) p.a[m] = rs ? q.a[m] : fmaT(beta, fmaT(-omega, v.a[m], p.a[m]), q.a[m]);
         if (mine) {
           st4(rn + k, q);
           st4(pn + k, p);
-          if (rs) st4(kr.rh + k, q);
+          if (rs) st4(rhat + k, q);
         }
         return p;
       });
@@ -558,7 +578,7 @@ __device__ __forceinline__ void bicg1_body(const Common& cm, const Coef<T>& co, 
         const Q4<T> v = product<T>(sm, o, P, row_of<T>(co, K), cm.precond);  // v = B^-1 A~ p
         st4(vn + K, v);
         // r^ (on a restart it is p itself)
-        const Q4<T> rh = rs ? *reinterpret_cast<const Q4<T>*>(sm + o) : ld4(kr.rh + K);
+        const Q4<T> rh = rs ? *reinterpret_cast<const Q4<T>*>(sm + o) : ld4(rhat + K);
         q0 = dot4<T>(rh, v, q0);
         if (rs && it > 0) q1 = dot4<T>(rh, rh, q1);
       }
@@ -590,7 +610,8 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
     const InstDev& I = cm.inst[b];  // fields are read where they are needed: registers are short
     const int it = st.iters;
     const T alpha = rhead(num<R>(st.alpha));
-    const T* r = it == 0 ? kr.rh : kStoreS<T> ? kr.r[0] : sel2(kr.r, (it + 1) & 1);
+    const T* const rhat = rh_of(kr, st);
+    const T* r = it == 0 ? rhat : kStoreS<T> ? kr.r[0] : sel2(kr.r, (it + 1) & 1);
     const T* vv = sel2(kr.v, (it + 1) & 1);
     const int P = I.pitch;
     const long long c0 = chunk_start<CH>(c, I);
@@ -614,7 +635,7 @@ __device__ __forceinline__ void bicg2_body(const Common& cm, const Coef<T>& co, 
         const Q4<T> s = *reinterpret_cast<const Q4<T>*>(sm + o);
         const Q4<T> t = product<T>(sm, o, P, row_of<T>(co, K), cm.precond);  // t = B^-1 A~ s
         st4(kr.t + K, t);
-        const Q4<T> rh = ld4(kr.rh + K);
+        const Q4<T> rh = ld4(rhat + K);
         q[0] = dot4<T>(t, s, q[0]);
         q[1] = dot4<T>(t, t, q[1]);
         q[2] = dot4<T>(s, s, q[2]);

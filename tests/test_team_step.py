@@ -49,6 +49,29 @@ def test_one_instance(capi, nx, ny, precond, prec):
     assert team[2] <= 4 * 3, team[2]
 
 
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("nx,ny,dt", [(900, 880, 1e-5), (389, 517, 1e-4), (700, 620, 1e-3)])
+def test_solves_of_one_iteration_with_chunks_in_turn(capi, nx, ny, dt, prec):
+    """Short time steps end a solve after one iteration, whose residual pass reads the shadow residual in
+    the neighbouring chunks' rows while it writes the next one: with one block per SM a chunk's
+    neighbours are written long before or after it reads them."""
+    p = cases.synthetic_problem(nx, ny, dt, seed=nx, tau=0.7)
+    got = []
+    for coop in (True, False, False):
+        b = capi.Batch([p], precision=prec, inner_tol=1e-2, max_refine=40)
+        b.set_launch_shape(1024, 1)
+        b.set_coop(coop)
+        b.step(3)
+        got.append(([b.f(0)], [b.stats(0)]))
+        b.close()
+    _same(got[0], got[1])
+    _same(got[1], got[2])
+    s = got[0][1][0]
+    assert s["status"] == 0
+    if dt == 1e-5:  # some solves took one iteration
+        assert s["total_iterations"] < 2 * (s["total_refinements"] - s["steps"]), s
+
+
 @pytest.mark.parametrize("prec", [1, 2])
 def test_one_instance_between_two_and_eight_thousand_cells_a_block(capi, prec):
     """1.3 million cells: by their number they would take chunks of 4096, but the step still fits the
