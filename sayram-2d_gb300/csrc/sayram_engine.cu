@@ -1314,6 +1314,7 @@ int sayram_batch_s::check_team() {
   SG_CUDA(cudaStreamSynchronize(stream));
   if (!*(volatile int*)(h_stat + sg::TEAM_GAVE_UP)) return SAYRAM_OK;
   h_stat[sg::TEAM_GAVE_UP] = 0;
+  rmax_clear = false;  // the lost step has not written its states back
   SG_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(unsigned) * (size_t)cap_slots * sg::kTeamBarStride, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
   return fail(SAYRAM_ERR_TIMEOUT, "a device barrier of the cooperative step gave up waiting");
