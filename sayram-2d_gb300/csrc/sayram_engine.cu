@@ -46,6 +46,12 @@ using sg::InstState;
 
 }  // namespace
 
+// ||r|| / ||R|| from their squares; infinite where a square was out of range
+static double relative_residual(double rr, double bb) {
+  if (!std::isfinite(rr) || !std::isfinite(bb)) return INFINITY;
+  return bb > 0 ? std::sqrt(rr / bb) : 0.0;
+}
+
 constexpr int kTeamSteps = 32;  // most steps of one cooperative launch, which so stays well below a second
 
 struct sayram_batch_s {
@@ -383,10 +389,7 @@ struct sayram_batch_s {
     return out;
   }
   // the relative residual the last step's solve ended at
-  double rel_of(const InstState& s) const {
-    const double bb = unwide(s.bb), rr = unwide(s.rr64);
-    return bb > 0 ? std::sqrt(rr / bb) : 0.0;
-  }
+  double rel_of(const InstState& s) const { return relative_residual(unwide(s.rr64), unwide(s.bb)); }
   double unwide(double w) const {
     if (!dwm) return w;
     float pr[2];
@@ -2603,7 +2606,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
                         : hs.status == ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED : SAYRAM_OK;
     stats_out->refinements = hs.refines;
     stats_out->iterations = hs.iters_total;
-    stats_out->rel_residual = hs.bb > 0 ? std::sqrt(hs.rr64 / hs.bb) : 0.0;
+    stats_out->rel_residual = relative_residual(hs.rr64, hs.bb);
     stats_out->min_f = hs.min_f;
     stats_out->clamped = hs.clamped;
     stats_out->mass_drift = hs.mass_drift;

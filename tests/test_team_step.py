@@ -192,3 +192,26 @@ def test_server_regions_taken_again(capi, lanes):
     b.close()
     for x, y in zip(got, want):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("coop", [True, False])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("state", ["residual", "inf", "nan"])
+def test_a_residual_out_of_range_is_not_converged(capi, state, prec, coop):
+    """The sum of squares of a residual far above the right-hand side overflows FP32 (time step 1e25,
+    boundary values 0: R is about 1e-28, R - M f about 1e-3), and a state that is not finite has no
+    residual: no step may report either as solved. FP64 holds the first one's squares and solves it."""
+    p = cases.synthetic_problem(24, 20, 1e25 if state == "residual" else 1e-2, seed=1, tau=1e30)
+    p = dataclasses.replace(p, dirichlet=[None if d is None else 0.0 * np.asarray(d) for d in p.dirichlet])
+    s = capi.Solver(p, precision=prec)
+    s.set_coop(coop)
+    f = np.array(p.f0)
+    if state != "residual":
+        f[5, 7] = float(state)
+    s.set_f(f)
+    rc = capi.load().sayram_update(s.h)
+    st = s.stats(0)
+    s.close()
+    want = capi.OK if state == "residual" and prec == 0 else capi.ERR_NOT_CONVERGED
+    assert rc == want and st["status"] == want, (rc, st)
+    assert (st["rel_residual"] < 1e-10) == (want == capi.OK)
