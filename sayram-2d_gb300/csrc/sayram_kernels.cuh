@@ -141,8 +141,9 @@ __device__ __forceinline__ void count_launch(Ctl* ctl) {
 // the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): with e = 1 - m r0, at most
 // 2^-21, 1/m = r0 (1 + e + e^2 + ...) and what the first three terms leave, e^3, is 2^-10 of an ulp;
 // one residual step rounds the quotient. Three (six) operations on the FP64 pipe, which takes 19
-// cycles per SM for a warp's operation. Zeros, subnormals, infinities, NaNs and the outermost
-// exponents take the plain operators.
+// cycles per SM for a warp's operation. Divisors that are zeros, subnormals, infinities, NaNs or of the
+// outermost exponents take the plain operators, against which the results are otherwise within one unit in
+// the last place.
 __device__ __forceinline__ double rcp64(double b) {
   const int hi = __double2hiint(b), lo = __double2loint(b), e = (hi >> 20) & 0x7ff;
   if (e < 3 || e > 2042) return 1.0 / b;
@@ -156,6 +157,8 @@ __device__ __forceinline__ double rcp64(double b) {
   return __hiloint2double((__double2hiint(r) + (1023 - e) * 0x100000) | (hi & 0x80000000), __double2loint(r));
 }
 __device__ __forceinline__ double div64(double a, double b) {
+  const int e = (__double2hiint(b) >> 20) & 0x7ff;
+  if (e < 3 || e > 2042) return a / b;
   const double r = rcp64(b), q = __dmul_rn(a, r);
   const double t = __fma_rn(__fma_rn(-b, q, a), r, q);
   return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : t;

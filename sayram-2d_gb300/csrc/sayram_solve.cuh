@@ -241,7 +241,7 @@ __device__ __forceinline__ void after_v(InstState& st, const R (&tot)[2]) {
     st.restart = 0;
   }
   const R rho = num<R>(st.rho), alpha = rdiv(rho, tot[0]);
-  if (rhead(tot[0]) != 0 && isfinite(rhead(alpha)) && rhead(rho) != 0) {
+  if (rhead(tot[0]) != 0 && isfinite(rhead(tot[0])) && isfinite(rhead(alpha)) && rhead(rho) != 0) {
     st.alpha = stored(alpha);
   } else {
     st.alpha = 0.0;  // breakdown: this iteration degenerates to a minimal-residual step
