@@ -53,6 +53,7 @@ static double relative_residual(double rr, double bb) {
 }
 
 constexpr int kTeamSteps = 32;  // most steps of one cooperative launch, which so stays well below a second
+constexpr int kRefused = -1;    // launch_team: the device did not take the cooperative launch (not an error of a call)
 
 struct sayram_batch_s {
   sayram_options opt{};
@@ -252,6 +253,7 @@ struct sayram_batch_s {
   static constexpr long long kSplitCells = 2048;
   int plan_team();
   int launch_team(int nsteps, int phases, bool last = true);
+  int launch_team_steps(int nsteps, int* queued);
   // dispatch of the per-step sequence on precision and chunk size (graph: build it; else: run it)
   template <typename T, typename C, typename A>
   int run_chunked(const sg::Coef<C>& cf, const sg::Coef<T>& ck, const sg::Kry<T>& kr, bool as_graph, bool prefix) {
@@ -810,6 +812,8 @@ int sayram_batch_s::plan_team() {
   return SAYRAM_OK;
 }
 
+// One cooperative launch. A device or context that does not take it (one with fewer SMs to give than
+// the plan has blocks, for instance) is not asked again: the batch goes on as separate kernels.
 int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   sg::TeamArgs ta{};
   ta.share = d_share;
@@ -827,13 +831,14 @@ int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   ta.own_cap = (int)team_own;
   ta.pmax = team_pmax;
   sg::TeamLaunch l{team_grid, team_smem, team_chip, stream};
-  if (dwm)
-    SG_CUDA(sg::team_launch_dw(l, cm, geo, fl, c32, k32, ta));
-  else if (mixed)
-    SG_CUDA(sg::team_launch_mixed(l, cm, geo, fl, c32, k32, ta));
-  else
-    SG_CUDA(sg::team_launch_f64(l, cm, geo, fl, c64, k64, ta));
-  return SAYRAM_OK;
+  const cudaError_t e = dwm     ? sg::team_launch_dw(l, cm, geo, fl, c32, k32, ta)
+                        : mixed ? sg::team_launch_mixed(l, cm, geo, fl, c32, k32, ta)
+                                : sg::team_launch_f64(l, cm, geo, fl, c64, k64, ta);
+  if (e == cudaSuccess) return SAYRAM_OK;
+  cudaGetLastError();
+  coop = 0;
+  team_grid = 0;
+  return kRefused;
 }
 
 int sayram_batch_s::build(const sayram_problem* probs, int count, const sayram_options* o) {
@@ -1080,47 +1085,53 @@ int sayram_batch_s::run_steps(int nsteps) {
   return finish_status();
 }
 
+// Queues steps as cooperative launches; *queued: how many, all of them unless one was refused (kRefused).
+int sayram_batch_s::launch_team_steps(int nsteps, int* queued) {
+  int& s = *queued;
+  if (timing) {  // the phases of a step one by one
+    for (; s < nsteps; ++s) {
+      launch("begin", [&] { sg::k_begin<<<(n + 255) / 256, 256, 0, stream>>>(cm); });
+      const std::pair<const char*, int> ph[3] = {
+          {"assemble", sg::TEAM_ASSEMBLE}, {"solve_coop", sg::TEAM_SOLVE}, {"polish", sg::TEAM_POLISH}};
+      for (auto& p : ph) {
+        int rc = SAYRAM_OK;
+        launch(p.first, [&] {
+          rc = team_split && p.second == sg::TEAM_ASSEMBLE
+                   ? launch_assemble(0, -1)
+                   : launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH);
+        });
+        if (rc) return rc;
+      }
+    }
+    return SAYRAM_OK;
+  }
+  if (team_split) {
+    for (; s < nsteps; ++s) {
+      int rc = rmax_clear ? SAYRAM_OK : launch_begin();
+      rmax_clear = true;
+      if (!rc) rc = launch_assemble(0, -1);
+      if (!rc) rc = launch_team(1, sg::TEAM_SOLVE | sg::TEAM_POLISH, s == nsteps - 1);
+      if (rc) return rc;
+    }
+    return SAYRAM_OK;
+  }
+  while (s < nsteps) {  // a launch stays well below a second
+    const int k = std::min(nsteps - s, kTeamSteps);
+    int rc = launch_team(k, sg::TEAM_STEP, s + k == nsteps);
+    if (rc) return rc;
+    s += k;
+  }
+  return SAYRAM_OK;
+}
+
 int sayram_batch_s::launch_steps(int nsteps) {
   if (nsteps < 0) return fail(SAYRAM_ERR_ARG, "nsteps must be >= 0");
   SG_CUDA(cudaSetDevice(dev));
+  int s = 0;  // steps queued
   if (team_grid > 0) {
     h_stat[sg::TEAM_NEGATIVE] = h_stat[sg::TEAM_NOT_CONVERGED] = 0;  // nothing of this batch is running
-    if (timing) {  // the phases of a step one by one
-      for (int s = 0; s < nsteps; ++s) {
-        int rc = SAYRAM_OK;
-        launch("begin", [&] { sg::k_begin<<<(n + 255) / 256, 256, 0, stream>>>(cm); });
-        const std::pair<const char*, int> ph[3] = {
-            {"assemble", sg::TEAM_ASSEMBLE}, {"solve_coop", sg::TEAM_SOLVE}, {"polish", sg::TEAM_POLISH}};
-        for (auto& p : ph) {
-          int r2 = SAYRAM_OK;
-          launch(p.first, [&] {
-            r2 = team_split && p.second == sg::TEAM_ASSEMBLE
-                     ? launch_assemble(0, -1)
-                     : launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH);
-          });
-          if (r2) rc = r2;
-        }
-        if (rc) return rc;
-      }
-      return SAYRAM_OK;
-    }
-    if (team_split) {
-      for (int s = 0; s < nsteps; ++s) {
-        int rc = rmax_clear ? SAYRAM_OK : launch_begin();
-        rmax_clear = true;
-        if (!rc) rc = launch_assemble(0, -1);
-        if (!rc) rc = launch_team(1, sg::TEAM_SOLVE | sg::TEAM_POLISH, s == nsteps - 1);
-        if (rc) return rc;
-      }
-      return SAYRAM_OK;
-    }
-    for (int s = 0; s < nsteps;) {  // a launch stays well below a second
-      const int k = std::min(nsteps - s, kTeamSteps);
-      int rc = launch_team(k, sg::TEAM_STEP, s + k == nsteps);
-      if (rc) return rc;
-      s += k;
-    }
-    return SAYRAM_OK;
+    int rc = launch_team_steps(nsteps, &s);
+    if (rc != kRefused) return rc;
   }
   const bool use_graph = opt.use_graph && !timing;
   if (use_graph && !gexec) {
@@ -1130,7 +1141,7 @@ int sayram_batch_s::launch_steps(int nsteps) {
       return rc;
     }
   }
-  for (int s = 0; s < nsteps; ++s) {
+  for (; s < nsteps; ++s) {
     if (use_graph) {
       SG_CUDA(cudaGraphLaunch(gexec, stream));
       continue;
@@ -2535,7 +2546,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   SG_CUDA(cudaFuncSetAttribute(k_polish<double, F64A, kNoAllocChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_na));
   SG_CUDA(cudaGetLastError());
   // whole steps as one cooperative launch where the instance's vectors fit the chip (all but very wide
-  // grids); else pass by pass from here
+  // grids) and the caller's stream takes it; else pass by pass from here
   const int blocks = std::min(nsm, kNoAllocMaxBlocks), per = (I.nseg + blocks - 1) / blocks;
   const int nb = (I.nseg + per - 1) / per;
   const int help = (int)std::min<long long>(blocks - nb, std::max<long long>(0, tile_count(I, 2) - nb));
@@ -2543,6 +2554,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   const size_t smem_team = team_smem(sizeof(double), true, own, pitch, sizeof(AsmTile<F64A>));
   const bool team = own <= team_chip_cells(sizeof(double)) && smem_team <= g_noalloc_smem[dev];
   int hstat[TEAM_FLAGS] = {};
+  int queued = 0;  // steps queued as cooperative launches: all, unless one is refused
   if (team && nsteps > 0) {
     SG_CUDA(cudaMemcpyAsync(d_share, hshare, sizeof(TeamShare) * (nb + help), cudaMemcpyHostToDevice, stream));
     TeamArgs ta{};
@@ -2557,14 +2569,17 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
     ta.phases = TEAM_STEP;
     ta.own_cap = (int)own;
     ta.pmax = (int)pitch;
-    for (int s = 0; s < nsteps; s += ta.nsteps) {
-      ta.nsteps = std::min(nsteps - s, kTeamSteps);
-      SG_CUDA(team_launch_f64(TeamLaunch{nb + help, smem_team, true, stream}, cm, geo, fl, co, kr, ta));
+    for (; queued < nsteps; queued += ta.nsteps) {
+      ta.nsteps = std::min(nsteps - queued, kTeamSteps);
+      if (team_launch_f64(TeamLaunch{nb + help, smem_team, true, stream}, cm, geo, fl, co, kr, ta) != cudaSuccess) {
+        cudaGetLastError();
+        break;
+      }
     }
     SG_CUDA(cudaMemcpyAsync(hstat, d_stat, sizeof(hstat), cudaMemcpyDeviceToHost, stream));
   }
   Ctl hctl;
-  for (int s = 0; !team && s < nsteps; ++s) {
+  for (int s = queued; s < nsteps; ++s) {
     SG_CUDA(cudaMemsetAsync(d_ctl, 0, 2 * sizeof(int), stream));
     k_begin<<<1, 32, 0, stream>>>(cm);
     k_assemble<double, F64A><<<gt, kAsmThreads, 0, stream>>>(cm, geo, fl, co, 0, -1);
