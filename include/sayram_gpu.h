@@ -176,7 +176,10 @@ int sayram_batch_create(const sayram_problem* probs, int n, const sayram_options
                         sayram_batch* out);
 int sayram_batch_size(sayram_batch b);
 /* Advances every instance by nsteps. Returns NOT_CONVERGED / NEGATIVE if any instance's last
- * step did (per-instance detail in sayram_batch_stats). */
+ * step did (per-instance detail in sayram_batch_stats). SAYRAM_ERR_TIMEOUT: a wait of the cooperative
+ * step ran out (its blocks wait for one another at most about a second at a time) and the instances'
+ * states are lost; until each has a new one (sayram_batch_set_f, or f_in of sayram_batch_step_host) steps
+ * and reads of a lost f return SAYRAM_ERR_STATE, and its stats the status SAYRAM_ERR_TIMEOUT. */
 int sayram_batch_step(sayram_batch b, int nsteps);
 /* The end-to-end form: if f_in is not NULL it first replaces every instance's f from the packed
  * host array (instances concatenated, each alpha-major), then steps, then, if f_out is not
@@ -290,7 +293,9 @@ int sayram_server_submit(sayram_server s, const sayram_problem* p, int nsteps, l
 /* One scheduling round: every idle lane admits waiting requests and launches one step of its
  * resident instances; the call returns when at least one lane's step has finished, after copying
  * out the instances of the finished lanes that reached their step count. With one lane: admission,
- * one step of every resident instance, completions. */
+ * one step of every resident instance, completions. SAYRAM_ERR_TIMEOUT with completions: a lane's
+ * cooperative step gave up (see sayram_batch_step); all of the lane's resident requests have ended, with
+ * that status in their stats and an f of NaN. */
 int sayram_server_tick(sayram_server s, int* n_completed);
 /* SAYRAM_OK and the result (f alpha-major, stats, submit/done times in seconds of the steady
  * clock) when request id has completed -- the result is then released; SAYRAM_ERR_STATE if not
@@ -326,7 +331,8 @@ void sayram_server_destroy(sayram_server s);
  * (a block keeps its share and a row above and below in shared memory: up to about 3000 cells a row
  * fit) also between launches, to read the loops' control words back to the host.
  * All calls share the array: each call clears it at its start and the array keeps the last
- * call's contents afterwards. Calls that overlap on the GPU (several host threads or streams at
+ * call's contents afterwards. After SAYRAM_ERR_TIMEOUT (a wait of the cooperative form ran out) f_out
+ * holds no state; a later call is not concerned. Calls that overlap on the GPU (several host threads or streams at
  * once) race on it and must be serialized by the caller. */
 int sayram_step_noalloc(const sayram_problem* p, const sayram_options* opt, int nsteps,
                         const double* f_in, double* f_out, void* stream, sayram_stats* stats);

@@ -374,6 +374,16 @@ struct sayram_batch_s {
   int launch_steps(int nsteps);  // queue steps on the stream (no status read-back)
   int read_ctl();
   int check_team();
+  // Instances whose state a lost step has left between two steps (check_team): they have no state until
+  // the caller gives them one.
+  std::vector<char> lost;
+  int whole(int idx = -1) const {  // instance idx (all when idx < 0) has a state
+    for (int b = idx < 0 ? 0 : idx; b < (idx < 0 ? (int)lost.size() : std::min(idx + 1, (int)lost.size())); ++b)
+      if (lost[b])
+        return fail(SAYRAM_ERR_STATE, "instance " + std::to_string(b) +
+                                          " lost its state in a step that gave up: set its f first");
+    return SAYRAM_OK;
+  }
   int status_of(bool negative, bool not_converged);
   int finish_status();
   template <typename T, typename C, typename A, int CH>
@@ -584,6 +594,7 @@ int sayram_batch_s::place(int b, const sayram_problem& p, long long base, int xe
     pmax = I.pitch;
   }
   I.enabled = 1;
+  if (b < (int)lost.size()) lost[b] = 0;
   for (int s = 0; s < 4; ++s) I.bc[s] = p.bc[s];
   I.base = base;
   I.hoff = hoff;
@@ -828,6 +839,7 @@ int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   ta.max_iters = opt.max_iters;
   ta.nsteps = nsteps;
   ta.phases = phases;
+  ta.polls = sg::kTeamPolls;
   ta.own_cap = (int)team_own;
   ta.pmax = team_pmax;
   sg::TeamLaunch l{team_grid, team_smem, team_chip, stream};
@@ -1253,6 +1265,8 @@ int sayram_batch_s::set_dtable(int idx, const sayram_dtable* t) {
 // simulation.
 int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
   if (steps < 1) steps = 1;
+  int rc = whole();
+  if (rc) return rc;
   SG_CUDA(cudaSetDevice(dev));
   constexpr int kSnap = 3 + sg::kHist;
   double* snap = nullptr;  // f, the history states and both y buffers
@@ -1282,7 +1296,7 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
   const bool timing_was = timing;
   timing = false;  // per-kernel events would split the graph into a host loop
   double best = 1e300;
-  int bc = chunk, bg = gmult, rc = SAYRAM_OK;
+  int bc = chunk, bg = gmult;
   tune_log.clear();
   for (int ci = 0; ci < 3 && rc == SAYRAM_OK; ++ci)
     for (int gi = 0; gi < 4 && rc == SAYRAM_OK; ++gi) {
@@ -1291,6 +1305,7 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
       drop_graph();
       if ((rc = rebuild_lists())) break;
       if ((rc = launch_steps(1))) break;  // builds the graph, warms up
+      if ((rc = check_team())) break;
       if ((rc = restore())) break;
       cudaEventRecord(e0, stream);
       if ((rc = launch_steps(steps))) break;
@@ -1298,6 +1313,7 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
       cudaEventSynchronize(e1);
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
+      if ((rc = check_team())) break;
       tune_log.push_back({chunk, gmult, (double)ms / steps});
       if (ms < best) {
         best = ms;
@@ -1311,6 +1327,7 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
   drop_graph();
   int rc2 = rebuild_lists();
   if (!rc2) rc2 = restore();
+  if (!rc2) lost.clear();  // a step that gave up in between is undone
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(snap);
@@ -1322,14 +1339,20 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
   return SAYRAM_OK;
 }
 
-// Waits for the stream; an error when a barrier of k_team gave up (its counters are cleared, so the
-// batch stays usable, but the step is lost).
+// Waits for the stream; an error when a barrier of k_team gave up. The blocks have left f, the earlier
+// states and y between two steps, and which steps is not known (a launch takes up to kTeamSteps of them
+// and writes the instances' scalars at its end), so every instance is without a state until it gets a
+// new one. What the next launches need is put right here: barriers, flags, and no history to start from.
 int sayram_batch_s::check_team() {
   SG_CUDA(cudaStreamSynchronize(stream));
   if (!*(volatile int*)(h_stat + sg::TEAM_GAVE_UP)) return SAYRAM_OK;
   h_stat[sg::TEAM_GAVE_UP] = 0;
   rmax_clear = false;  // the lost step has not written its states back
+  lost.assign(cap_slots, 0);
+  for (int b = 0; b < cap_slots; ++b) lost[b] = hinst[b].enabled ? 1 : 0;
   SG_CUDA(cudaMemsetAsync(d_bar, 0, sizeof(unsigned) * (size_t)cap_slots * sg::kTeamBarStride, stream));
+  static_assert(offsetof(InstState, lost) == offsetof(InstState, nhist) + sizeof(int), "cleared together");
+  SG_CUDA(cudaMemset2DAsync((char*)d_st + offsetof(InstState, nhist), sizeof(InstState), 0, 2 * sizeof(int), cap_slots, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
   return fail(SAYRAM_ERR_TIMEOUT, "a device barrier of the cooperative step gave up waiting");
 }
@@ -1426,7 +1449,8 @@ int sayram_batch_size(sayram_batch b) { return b ? b->n : 0; }
 
 int sayram_batch_step(sayram_batch b, int nsteps) {
   if (!b) return fail(SAYRAM_ERR_ARG, "null handle");
-  return b->run_steps(nsteps);
+  int rc = b->whole();
+  return rc ? rc : b->run_steps(nsteps);
 }
 
 // The instances are split into about kPieces runs at instance boundaries (a small first run);
@@ -1436,6 +1460,8 @@ int sayram_batch_step(sayram_batch b, int nsteps) {
 int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, double* f_out) {
   if (!b) return fail(SAYRAM_ERR_ARG, "null handle");
   if (nsteps < 0) return fail(SAYRAM_ERR_ARG, "nsteps must be >= 0");
+  if (f_in) b->lost.clear();  // every instance gets a state
+  if (int rc0 = b->whole()) return rc0;
   SG_CUDA(cudaSetDevice(b->dev));
   constexpr int kPieces = 16;  // per call, 8 / 12 / 16 runs: 17.3 / 17.0 / 17.0 ms (4096 instances)
   struct Piece {
@@ -1571,6 +1597,7 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
 
 int sayram_batch_get_f(sayram_batch b, int idx, double* f_out) {
   if (!b || !f_out || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
+  if (int rc = b->whole(idx)) return rc;
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
   const int t0 = I.tile0, t1 = I.tile0 + I.ntx * I.nty;
@@ -1591,6 +1618,7 @@ int sayram_batch_set_f(sayram_batch b, int idx, const double* f) {
   SG_CUDA(cudaGetLastError());
   SG_CUDA(cudaMemsetAsync((char*)(b->d_st + idx) + offsetof(InstState, nhist), 0, sizeof(int), b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
+  if (idx < (int)b->lost.size()) b->lost[idx] = 0;
   return SAYRAM_OK;
 }
 
@@ -1647,6 +1675,7 @@ int sayram_batch_stats(sayram_batch b, int idx, sayram_stats* out) {
   out->status = s.steps == 0 ? SAYRAM_OK
                 : s.status == sg::ST_NEGATIVE ? SAYRAM_ERR_NEGATIVE
                 : s.status == sg::ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED : SAYRAM_OK;
+  if (idx < (int)b->lost.size() && b->lost[idx]) out->status = SAYRAM_ERR_TIMEOUT;
   out->refinements = s.refines;
   out->iterations = s.iters_total;
   out->rel_residual = b->rel_of(s);
@@ -1660,11 +1689,12 @@ int sayram_batch_stats(sayram_batch b, int idx, sayram_stats* out) {
 
 int sayram_batch_export_system(sayram_batch b, int idx, double* M5, double* R) {
   if (!b || !M5 || !R || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
+  int rc = b->whole(idx);
+  if (rc) return rc;
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
   b->rmax_clear = false;
-  int rc = b->launch_assemble(0, -1);
-  if (rc) return rc;
+  if ((rc = b->launch_assemble(0, -1))) return rc;
   const size_t rows = (size_t)I.ny * I.pitch;
   std::vector<double> invD(rows), Rr(rows), c[4];
   SG_CUDA(cudaMemcpyAsync(invD.data(), b->fl.invD + I.base, rows * 8, cudaMemcpyDeviceToHost, b->stream));
@@ -2051,8 +2081,14 @@ struct ServerLane {
                               cudaMemcpyDeviceToHost, eng.stream));
       SG_CUDA(cudaMemcpyAsync(&sts[q], eng.d_st + fin[q], sizeof(InstState), cudaMemcpyDeviceToHost, eng.stream));
     }
-    int trc = eng.check_team();  // waits for the copies too
-    if (trc) return trc;
+    const int trc = eng.check_team();  // waits for the copies too
+    if (trc && trc != SAYRAM_ERR_TIMEOUT) return trc;
+    if (trc) {  // the step is lost, and every resident instance's state with it: all end here
+      info.instance_steps -= info.resident;
+      fin.clear();
+      for (int k = 0; k < cfg.max_slots; ++k)
+        if (slots[k].used) fin.push_back(k);
+    }
     const double t1 = now_seconds();
     info.busy_seconds += t1 - t_begin;
     info.collect_seconds += t1 - ts;
@@ -2060,14 +2096,16 @@ struct ServerLane {
       Slot& S = slots[fin[q]];
       InstDev& I = eng.hinst[fin[q]];
       Result& R = results[S.id];
-      R.f.resize((size_t)S.nx * S.ny);
-      for (int i = 0; i < S.nx; ++i)
+      R.f.assign((size_t)S.nx * S.ny, NAN);
+      for (int i = 0; !trc && i < S.nx; ++i)
         for (int j = 0; j < S.ny; ++j) R.f[(size_t)i * S.ny + j] = eng.unwide(rows[q][(size_t)j * I.pitch + i]);
-      const InstState& hs = sts[q];
+      const InstState hs = trc ? InstState{} : sts[q];
       R.st.steps = hs.steps;
       R.st.t = (double)hs.steps * I.dt;
-      R.st.status = hs.status == sg::ST_NEGATIVE ? SAYRAM_ERR_NEGATIVE
-                    : hs.status == sg::ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED : SAYRAM_OK;
+      R.st.status = trc                                   ? trc
+                    : hs.status == sg::ST_NEGATIVE      ? SAYRAM_ERR_NEGATIVE
+                    : hs.status == sg::ST_NOT_CONVERGED ? SAYRAM_ERR_NOT_CONVERGED
+                                                        : SAYRAM_OK;
       R.st.refinements = hs.refines;
       R.st.iterations = hs.iters_total;
       R.st.rel_residual = eng.rel_of(hs);
@@ -2087,7 +2125,7 @@ struct ServerLane {
       dirty = true;
     }
     if (ncomp) *ncomp = (int)fin.size();
-    return SAYRAM_OK;
+    return trc;
   }
 
   // sizes the lane's arrays from its share of the budget (tables, staging, lists, cell arena)
@@ -2170,8 +2208,10 @@ struct sayram_server_s {
         if (r < 0) return SAYRAM_ERR_CUDA;
         if (r == 0) continue;
         int n = 0;
-        if ((rc = L->finish(results, &n))) return rc;
+        rc = L->finish(results, &n);
         total += n;
+        if (ncomp) *ncomp = total;
+        if (rc) return rc;
         done = true;
       }
       if (done) break;
@@ -2567,6 +2607,7 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
     ta.max_refine = o.max_refine;
     ta.max_iters = o.max_iters;
     ta.phases = TEAM_STEP;
+    ta.polls = kTeamPolls;
     ta.own_cap = (int)own;
     ta.pmax = (int)pitch;
     for (; queued < nsteps; queued += ta.nsteps) {

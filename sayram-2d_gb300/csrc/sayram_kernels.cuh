@@ -78,6 +78,7 @@ struct InstState {
   int swapped;             // rh and x of the per-pass kernels have changed places (rh_of)
   int iters_total, refines, status;
   int nhist;               // earlier states held in the history buffers (extrapolated start)
+  int lost;                // a barrier of k_team gave up: launches queued behind it leave the instance alone
   int hslot;               // history buffer holding f^(n-1); f^(n-2), ... are in the ones before it
   unsigned int rmax_bits;  // bits of max |R| over the instance (non-negative float; atomicMax order)
   unsigned int cnt[PH_COUNT];

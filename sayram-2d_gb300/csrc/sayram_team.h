@@ -31,10 +31,12 @@ struct TeamArgs {
   double tol, inner_tol;
   int max_refine, max_iters;
   int nsteps, phases;
+  int polls;           // most polls of one barrier (kTeamPolls; 0: the first barrier gives up)
   int report;          // 1: set the flags of the last step
   int own_cap;         // cells of the largest share, rounded up to whole segments
   int pmax;            // widest row pitch
 };
+constexpr int kTeamPolls = 1 << 20;  // ~0.7 us each; blocks of a launch run together, milliseconds apart at most
 constexpr int kTeamBarStride = 16;  // 64 bytes: one team's counters do not share a line with another's
 
 // Bytes of dynamic shared memory (sayram_team.cuh lays it out). chip: the Krylov vectors of a share

@@ -18,8 +18,8 @@ LIB = capi.lib_path().encode()
 FOREVER = 1 << 30
 
 
-def shim_set(passed, refused):
-    assert shim.shim_set(LIB, passed, refused) == 0
+def shim_set(passed, odd, give_up=0):
+    assert shim.shim_set(LIB, passed, odd, give_up) == 0
 
 
 def one(nx, ny, seed=3):
@@ -61,7 +61,8 @@ def refused(passed, probs, steps, timing=False):
         same(got, want)
 
 
-def refused_noalloc(passed):
+def noalloc_run(nsteps):
+    """A call of the allocation-free step on one problem, as a function of nothing."""
     import torch
 
     p = one(64, 60)[0]
@@ -83,11 +84,16 @@ def refused_noalloc(passed):
 
     def run():
         out = torch.empty_like(f)
-        rc = capi.load().sayram_step_noalloc(ctypes.byref(s), None, 40, f.data_ptr(), out.data_ptr(),
+        rc = capi.load().sayram_step_noalloc(ctypes.byref(s), None, nsteps, f.data_ptr(), out.data_ptr(),
                                              torch.cuda.current_stream().cuda_stream, ctypes.byref(st))
-        assert rc == capi.OK, capi.last_error()
-        return out.cpu().numpy(), st.as_dict()
+        return rc, out.cpu().numpy(), st.as_dict()
 
+    run.keep = keep
+    return run
+
+
+def refused_noalloc(passed):
+    run = noalloc_run(40)
     capi.load()
     shim_set(FOREVER, 0)
     want = run()
@@ -95,7 +101,8 @@ def refused_noalloc(passed):
     shim_set(passed, FOREVER)
     got = run()
     assert shim.shim_calls() == passed + 1
-    assert np.array_equal(got[0], want[0]) and got[1] == want[1] and want[1]["steps"] == 40
+    assert got[0] == want[0] == capi.OK and np.array_equal(got[1], want[1])
+    assert got[2] == want[2] and want[2]["steps"] == 40
 
 
 def refused_server():
@@ -121,7 +128,144 @@ def refused_server():
     same(got, want)
 
 
+def fresh(probs, fs, prec, steps):
+    """The batch's f after steps from the given states, by a batch that has seen nothing else."""
+    b = capi.Batch(probs, precision=prec)
+    for k, f in enumerate(fs):
+        b.set_f(k, f)
+    b.step(steps)
+    out = result(b)[0]
+    b.close()
+    return out
+
+
+def gave_up():
+    """A wait that runs out loses the state of the batch: nothing is stepped on from it or read from it until
+    every instance has a new one, launches queued behind it leave a lost instance alone, and then all is as in a
+    new batch."""
+    L = capi.load()
+    probs = one(90, 70) + one(1, 1)  # a team of many blocks, and one of a single block, which waits for nobody
+    fs = [np.array(p.f0) * 0.5 for p in probs]
+    packed = np.concatenate([f.ravel() for f in fs])
+    out = np.empty_like(packed)
+    for prec in (0, 1, 2):
+        shim_set(FOREVER, 0)
+        want = fresh(probs, fs, prec, 3)
+        b = capi.Batch(probs, precision=prec)
+        b.step(2)
+        its = b.stats(0)["total_iterations"]
+        shim_set(0, 1, 1)
+        assert L.sayram_batch_step(b.h, 70) == capi.ERR_TIMEOUT
+        assert shim.shim_calls() == 3
+        st = [b.stats(k) for k in range(2)]
+        assert [s["status"] for s in st] == [capi.ERR_TIMEOUT] * 2
+        assert st[0]["steps"] == 2 and st[0]["total_iterations"] == its, st
+        m5, r = np.empty((5, 6300)), np.empty(6300)
+
+        def refusals():
+            return (L.sayram_batch_step(b.h, 1), L.sayram_batch_step_host(b.h, 1, None, out.ctypes.data),
+                    L.sayram_batch_autotune(b.h, 1, None, None))
+
+        assert refusals() == (capi.ERR_STATE,) * 3
+        assert L.sayram_batch_get_f(b.h, 0, capi._ptr(out)) == capi.ERR_STATE
+        assert L.sayram_batch_export_system(b.h, 0, capi._ptr(m5), capi._ptr(r)) == capi.ERR_STATE
+        b.set_f(0, fs[0])
+        assert np.allclose(b.f(0), fs[0], rtol=1e-14, atol=0) and refusals() == (capi.ERR_STATE,) * 3
+        b.set_f(1, fs[1])
+        assert b.stats(1)["status"] == capi.OK
+        b.step(3)
+        got = result(b)
+        assert all(np.array_equal(x, y) for x, y in zip(got[0], want))
+        assert all(s["status"] == capi.OK for s in got[1])
+        # again, with the new states in the packed form
+        shim_set(0, 1, 1)
+        assert L.sayram_batch_step_host(b.h, 1, packed.ctypes.data, out.ctypes.data) == capi.ERR_TIMEOUT
+        b.step_host(3, packed.ctypes.data, out.ctypes.data)
+        assert np.array_equal(out, np.concatenate([f.ravel() for f in want]))
+        b.close()
+
+
+def gave_up_split():
+    L = capi.load()
+    probs = one(700, 620)
+    for prec in (1, 2):
+        shim_set(FOREVER, 0)
+        want = fresh(probs, [probs[0].f0], prec, 2)
+        b = capi.Batch(probs, precision=prec)
+        b.step(2)
+        shim_set(1, 1, 1)
+        assert L.sayram_batch_step(b.h, 4) == capi.ERR_TIMEOUT
+        assert b.stats(0)["steps"] == 3  # the first of the four
+        b.set_f(0, probs[0].f0)
+        b.step(2)
+        assert np.array_equal(b.f(0), want[0])
+        b.close()
+
+
+def gave_up_autotune():
+    """Tuning restores the state, whatever its steps came to."""
+    L = capi.load()
+    a, b = capi.Batch(one(90, 70), precision=2), capi.Batch(one(90, 70), precision=2)
+    shim_set(FOREVER, 0)
+    for x in (a, b):
+        x.step(3)
+    for passed in (0, 1):
+        shim_set(passed, 1, 1)
+        assert L.sayram_batch_autotune(a.h, 2, None, None) == capi.ERR_TIMEOUT
+    for x in (a, b):
+        x.step(3)
+    assert np.array_equal(a.f(0), b.f(0))
+    a.close()
+    b.close()
+
+
+def gave_up_noalloc():
+    run = noalloc_run(40)
+    capi.load()
+    shim_set(FOREVER, 0)
+    want = run()
+    shim_set(0, 1, 1)
+    assert run()[0] == capi.ERR_TIMEOUT
+    got = run()
+    assert got[0] == capi.OK and np.array_equal(got[1], want[1]) and got[2] == want[2]
+
+
+def gave_up_server():
+    L = capi.load()
+    reqs = [(one(a, e, seed=a)[0], n) for a, e, n in ((40, 33, 7), (96, 80, 3), (17, 23, 5))]
+    shim_set(FOREVER, 0)
+    srv = capi.Server(2e9, max_slots=8, max_side=128, precision=2)
+
+    def serve():
+        ids = [srv.submit(*r) for r in reqs]
+        for _ in range(7):
+            srv.tick()
+        return [srv.poll(i)[:2] for i in ids]
+
+    want = serve()
+    ids = [srv.submit(*r) for r in reqs]
+    shim_set(2, 1, 1)
+    srv.tick()
+    srv.tick()
+    n = ctypes.c_int()
+    assert L.sayram_server_tick(srv.h, ctypes.byref(n)) == capi.ERR_TIMEOUT and n.value == 3
+    info = srv.info()
+    assert info["resident"] == 0 and info["arena_cells_used"] == 0 and info["completed"] == 6
+    for i in ids:
+        f, st = srv.poll(i)[:2]
+        assert st["status"] == capi.ERR_TIMEOUT and np.isnan(f).all()
+    got = serve()
+    srv.close()
+    for x, y in zip(got, want):
+        assert np.array_equal(x[0], y[0]) and x[1] == y[1]
+
+
 SCENARIOS = {
+    "gave up": gave_up,
+    "gave up split": gave_up_split,
+    "gave up autotune": gave_up_autotune,
+    "gave up noalloc": gave_up_noalloc,
+    "gave up server": gave_up_server,
     "first": lambda: refused(0, one(90, 70), (2, 1)),
     "second": lambda: refused(1, one(90, 70), (40, 1)),
     "bins": lambda: refused(0, cases.batch_problems(160, 7, 1e-2, 8, 40), (2,)),

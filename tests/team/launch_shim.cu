@@ -1,42 +1,46 @@
 // Stands in for the launchers of the cooperative step (sayram_team.h) in a test's process: loaded with
 // its symbols global before the library, it is what the library's own calls reach. It refuses launches
-// as a device without room for them does, or hands them on.
+// as a device without room for them does, hands them on without any polls for their barriers (the first
+// barrier of a team of several blocks gives up), or hands them on as they are.
 #include <dlfcn.h>
 
 #include "sayram_team.h"
 
-static int g_pass = 0, g_refuse = 0, g_calls = 0;
+static int g_pass = 0, g_odd = 0, g_give_up = 0, g_calls = 0;
 static void* g_lib = nullptr;
 
-// lib: the library's path; the next `pass` launches are handed on, the `refuse` after them refused
-extern "C" int shim_set(const char* lib, int pass, int refuse) {
+// lib: the library's path; the next `pass` launches are handed on, the `odd` after them refused (or, with
+// give_up, handed on without polls)
+extern "C" int shim_set(const char* lib, int pass, int odd, int give_up) {
   if (!g_lib) g_lib = dlopen(lib, RTLD_LAZY | RTLD_LOCAL);
   g_pass = pass;
-  g_refuse = refuse;
+  g_odd = odd;
+  g_give_up = give_up;
   g_calls = 0;
   return g_lib ? 0 : 1;
 }
 extern "C" int shim_calls() { return g_calls; }
 
 template <typename F, typename... X>
-static cudaError_t on(F* self, const X&... x) {
+static cudaError_t on(F* self, sg::TeamArgs ta, const X&... x) {
   ++g_calls;
   if (g_pass > 0) {
     --g_pass;
-  } else if (g_refuse > 0) {
-    --g_refuse;
-    return cudaErrorCooperativeLaunchTooLarge;
+  } else if (g_odd > 0) {
+    --g_odd;
+    if (!g_give_up) return cudaErrorCooperativeLaunchTooLarge;
+    ta.polls = 0;
   }
   Dl_info info;
   F* f = dladdr(reinterpret_cast<void*>(self), &info) ? reinterpret_cast<F*>(dlsym(g_lib, info.dli_sname)) : nullptr;
-  return f && f != self ? f(x...) : cudaErrorSymbolNotFound;
+  return f && f != self ? f(x..., ta) : cudaErrorSymbolNotFound;
 }
 
 namespace sg {
 #define SHIM(name, T)                                                                                          \
   cudaError_t name(const TeamLaunch& l, const Common& cm, const Geo& geo, const Fields& fl, const Coef<T>& co, \
                    const Kry<T>& kr, const TeamArgs& ta) {                                                     \
-    return on(&name, l, cm, geo, fl, co, kr, ta);                                                              \
+    return on(&name, ta, l, cm, geo, fl, co, kr);                                                              \
   }
 SHIM(team_launch_f64, double)
 SHIM(team_launch_mixed, float)

@@ -31,3 +31,10 @@ def _child(shim, scenario):
                                       "server"])
 def test_a_refused_launch_goes_on_as_separate_kernels(shim, scenario):
     _child(shim, scenario)
+
+
+@pytest.mark.parametrize("scenario", ["gave up", "gave up split", "gave up autotune", "gave up noalloc",
+                                      "gave up server"])
+def test_a_wait_that_runs_out(shim, scenario):
+    """The barriers of one launch get no polls: its blocks leave, and the host is told."""
+    _child(shim, scenario)
