@@ -202,18 +202,12 @@ __device__ __forceinline__ int after_resid(InstState& st, const R (&tot)[3], dou
   st.cum_refines += 1;
   st.rr64 = stored(tot[0]);
   const R bb = num<R>(st.bb);
-  // A residual too large for its sum's range, or not a number, is not below any tolerance, and a solve
-  // from it cannot make progress. The comparisons below would let it pass: a double-word sum that
-  // overflows becomes NaN (2Sum subtracts infinities), and infinity is not above an infinite bound.
-  if (!isfinite(rhead(tot[0])) || !isfinite(rhead(bb))) {
-    st.outer_active = 0;
-    st.status = ST_NOT_CONVERGED;
-    return 0;
-  }
   const R bound = rmul(rfrom<R>(tol * tol), bb);  // ||r|| <= tol ||R||, or R = 0
   if (!rgt(tot[0], bound) || !rgt(bb, rfrom<R>(0.0f))) {
+    // A residual that is not a number, or that an infinite bound lets pass, is not below any tolerance (a
+    // double-word sum that overflows becomes NaN: 2Sum subtracts infinities), and no solve starts from it
     st.outer_active = 0;
-    st.status = ST_OK;
+    st.status = isfinite(rhead(tot[0])) && isfinite(rhead(bb)) ? ST_OK : ST_NOT_CONVERGED;
     return 0;
   }
   if (st.refines >= max_refine) {
