@@ -229,7 +229,9 @@ int sayram_batch_autotune(sayram_batch b, int steps, int* chunk_out, int* blocks
  * by default) takes whole steps in one cooperative launch: a team of blocks per instance, with a
  * barrier between its passes, or, with more instances than SMs, blocks with several instances
  * each; larger batches run as the graph's loops of separate kernels, and so does a batch whose
- * cooperative launch the device has refused. on = 0 always uses the separate kernels (the results are
+ * cooperative launch the device has refused. Handles and servers that several threads step on one GPU at
+ * the same time share its SMs: a launch takes a half, a quarter, ... of them by the number of calls in
+ * flight. on = 0 always uses the separate kernels (the results are
  * the same bit for bit). Default: 1. */
 int sayram_batch_set_coop(sayram_batch b, int on);
 /* Sets the launch shape directly (chunk 1024, 2048 or 4096 cells; 1..64 blocks per SM), or reads

@@ -52,6 +52,56 @@ static double relative_residual(double rr, double bb) {
   return bb > 0 ? std::sqrt(rr / bb) : 0.0;
 }
 
+// Callers that step something on one GPU at the same time share its SMs: the cooperative step's blocks fill
+// the SMs they are on, so launches over the whole chip would take turns, and the barriers, which are most
+// of a small instance's step, leave the chip idle in each turn. Counts the calls in flight per device; a
+// launch takes 1 / 2^level of the SMs, 2^level at least the most calls seen in flight over the last
+// windows. What a launch computes does not depend on the level.
+class DeviceUse {
+ public:
+  static DeviceUse& of(int dev) {
+    static DeviceUse use[128];
+    return use[dev & 127];
+  }
+  void enter() {
+    std::lock_guard<std::mutex> g(mu);
+    ++inflight;
+    roll();
+  }
+  void leave() {
+    std::lock_guard<std::mutex> g(mu);
+    --inflight;
+  }
+  int level(int most) {
+    std::lock_guard<std::mutex> g(mu);
+    roll();
+    int l = 0;
+    while (l < most && (1 << l) < std::max(peak, last)) ++l;
+    return l;
+  }
+
+ private:
+  static constexpr double kWindow = 0.005;  // seconds; longer than the host's part of a loop of short calls
+  std::mutex mu;
+  int inflight = 0, peak = 0, last = 0;  // now; the most in this window and in the one before
+  double since = 0.0;
+  void roll() {
+    const double t = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
+    if (t - since > kWindow) {
+      last = t - since > 2 * kWindow ? 0 : peak;
+      peak = 0;
+      since = t;
+    }
+    peak = std::max(peak, inflight);
+  }
+};
+struct DeviceCall {  // one call in flight
+  DeviceUse& use;
+  explicit DeviceCall(int dev) : use(DeviceUse::of(dev)) { use.enter(); }
+  ~DeviceCall() { use.leave(); }
+  DeviceCall(const DeviceCall&) = delete;
+};
+
 constexpr int kTeamSteps = 32;  // most steps of one cooperative launch, which so stays well below a second
 constexpr int kRefused = -1;    // launch_team: the device did not take the cooperative launch (not an error of a call)
 
@@ -135,6 +185,10 @@ struct sayram_batch_s {
     h_ctl = nullptr;
     if (h_stat) cudaFreeHost(h_stat);
     h_stat = nullptr;
+    for (auto& e : team_ev) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
     for (auto e : evpool) cudaEventDestroy(e);
     evpool.clear();
     for (auto& e : slots)
@@ -233,27 +287,39 @@ struct sayram_batch_s {
   }
   // Whole steps as one cooperative launch (k_team), for batches that fit the chip: every instance gets
   // a team of blocks, or, with more instances than SMs, every block whole instances. Re-planned
-  // whenever the lists change; team_grid 0: the batch runs as separate kernels.
+  // whenever the lists change; no grid: the batch runs as separate kernels.
   int coop = 1;
   int team_sms = 0;    // blocks the plan may use (0: one per SM)
-  int team_grid = 0;
-  bool team_chip = false;
+  struct TeamPlan {
+    bool made = false;
+    int grid = 0;
+    bool chip = false;
+    bool split = false;  // the assembly as a kernel of its own before each step's launch
+    bool bins = false;   // blocks with several whole instances each
+    size_t smem = 0;
+    long long own = 0;
+  };
+  static constexpr int kTeamLevels = 8;  // plans for 1 / 2^k of the SMs (DeviceUse), made when first wanted
+  TeamPlan plans[kTeamLevels];
+  int team_grid() const { return plans[0].grid; }  // 0: not stepped by k_team
   bool rmax_clear = false;  // every instance's rmax_bits is 0 (k_team leaves it so)
-  bool team_split = false;  // the assembly as a kernel of its own before each step's launch
-  bool team_bins = false;  // blocks with several whole instances each
-  size_t team_smem = 0;
-  int team_pmax = 4;
-  long long team_own = 0;
   size_t team_limit[2] = {0, 0};  // shared memory a block may use: streaming, on chip (0: not asked yet)
-  sg::TeamShare* d_share = nullptr;
-  int* d_first = nullptr;
+  int team_pmax = 4;
+  int shares_cap = 0;
+  sg::TeamShare* d_share = nullptr;  // shares_cap of them for every plan
+  int* d_first = nullptr;            // nsm + 1 of them for every plan
   unsigned* d_bar = nullptr;
   float* d_tmax = nullptr;
   int* h_stat = nullptr;  // pinned, written by k_team (TEAM_* flags)
   static constexpr long long kSplitCells = 2048;
+  cudaEvent_t team_ev[2] = {nullptr, nullptr};  // ends of a call's last two runs of steps
   int plan_team();
-  int launch_team(int nsteps, int phases, bool last = true);
+  int make_plan(int level);
+  int plan_now(const TeamPlan** out);
+  int launch_team(const TeamPlan& plan, int nsteps, int phases, bool last = true);
   int launch_team_steps(int nsteps, int* queued);
+  int launch_separate(int nsteps);
+  bool by_flags = false;  // the last step queued was k_team's, which leaves its outcome in h_stat
   // dispatch of the per-step sequence on precision and chunk size (graph: build it; else: run it)
   template <typename T, typename C, typename A>
   int run_chunked(const sg::Coef<C>& cf, const sg::Coef<T>& ck, const sg::Kry<T>& kr, bool as_graph, bool prefix) {
@@ -489,8 +555,9 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
   SG_ALLOC(d_dirv, std::max<long long>(dcap, 1));
   pstride = 8LL * chunks_cap;  // a chunk of 1024 cells holds 8 segments, the most of any chunk size
   SG_ALLOC(d_part, (long long)sg::kPartSets * sg::kPartQ * pstride);
-  SG_ALLOC(d_share, std::max(slots, nsm));
-  SG_ALLOC(d_first, nsm + 1);
+  shares_cap = std::max(slots, nsm);
+  SG_ALLOC(d_share, (long long)kTeamLevels * shares_cap);
+  SG_ALLOC(d_first, (long long)kTeamLevels * (nsm + 1));
   SG_ALLOC(d_bar, (long long)slots * sg::kTeamBarStride);
   SG_ALLOC(d_tmax, nsm);
   SG_CUDA(cudaMallocHost(&h_stat, sizeof(int) * sg::TEAM_FLAGS));
@@ -711,11 +778,34 @@ int split_instance(const InstDev& I, int b, int nb, int help, sg::TeamShare* out
 // Splits the enabled instances' reduction segments over the blocks of one cooperative launch: the
 // smallest number of segments per block with which the teams fit (whole instances, largest first,
 // when there are more instances than blocks), then the form that fits the shared memory -- on
-// chip, or with the vectors in global memory. No plan (team_grid = 0) when neither fits, or for
+// chip, or with the vectors in global memory. No plan (grid 0) when neither fits, or for
 // chunks of 4096 cells, whose segments are too coarse to split.
 int sayram_batch_s::plan_team() {
-  team_grid = 0;
+  for (auto& p : plans) p = TeamPlan{};
   rmax_clear = false;
+  return make_plan(0);
+}
+// The plan for this moment: the least share of the SMs, down to this level's, that a plan exists for. A batch
+// that only the whole chip holds: in the FP32 modes the chip is free for others between its launches, a step
+// each (under 1 ms), and as separate kernels two such would take half as long again (1100 x 1100 in
+// double-word, us a step of both: 881 / 1353); an FP64 step is a millisecond or more, and separate kernels
+// cost little where the pipe is the bound (1024 x 1024: 3627 / 3939), while a call of a small instance beside
+// it takes 56 us instead of waiting for launches to end: no plan (null).
+int sayram_batch_s::plan_now(const TeamPlan** out) {
+  const int level = timing ? 0 : DeviceUse::of(dev).level(kTeamLevels - 1);
+  for (int l = level; l > 0; --l) {
+    int rc = plans[l].made ? SAYRAM_OK : make_plan(l);
+    if (rc) return rc;
+    *out = &plans[l];
+    if (plans[l].grid > 0) return SAYRAM_OK;
+  }
+  *out = level > 0 && !mixed ? nullptr : &plans[0];
+  return SAYRAM_OK;
+}
+int sayram_batch_s::make_plan(int level) {
+  TeamPlan plan;
+  plan.made = true;
+  plans[level] = plan;
   if (!coop || chunk == 4096) return SAYRAM_OK;
   std::vector<int> on;
   long long total = 0, most = 0;
@@ -728,7 +818,7 @@ int sayram_batch_s::plan_team() {
       most = std::max(most, cells(b));
       pm = std::max(pm, hinst[b].pitch);
     }
-  const int blocks = team_sms > 0 ? std::min(team_sms, nsm) : nsm, ni = (int)on.size();
+  const int blocks = std::max(1, (team_sms > 0 ? std::min(team_sms, nsm) : nsm) >> level), ni = (int)on.size();
   if (ni == 0) return SAYRAM_OK;
   std::vector<sg::TeamShare> share;
   std::vector<int> first;
@@ -801,12 +891,14 @@ int sayram_batch_s::plan_team() {
   }
   bool chip = own <= sg::team_chip_cells(ts) && sg::team_smem(ts, true, own, pm, tile) <= team_limit[1];
   if (!chip && sg::team_smem(ts, false, own, pm, tile) > team_limit[0]) return SAYRAM_OK;
-  SG_CUDA(cudaMemcpyAsync(d_share, share.data(), sizeof(sg::TeamShare) * share.size(), cudaMemcpyHostToDevice, stream));
+  SG_CUDA(cudaMemcpyAsync(d_share + (long long)level * shares_cap, share.data(), sizeof(sg::TeamShare) * share.size(),
+                          cudaMemcpyHostToDevice, stream));
   if (!first.empty())
-    SG_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, stream));
+    SG_CUDA(cudaMemcpyAsync(d_first + (long long)level * (nsm + 1), first.data(), sizeof(int) * first.size(),
+                            cudaMemcpyHostToDevice, stream));
   SG_CUDA(cudaStreamSynchronize(stream));
-  team_grid = first.empty() ? (int)share.size() : (int)first.size() - 1;
-  team_bins = !first.empty();
+  plan.grid = first.empty() ? (int)share.size() : (int)first.size() - 1;
+  plan.bins = !first.empty();
   // a block of k_team has 16 warps for its tiles and its instance's alone, k_assemble up to 48 per SM and
   // any tile: with many cells per block the launch it costs is less than it gains. Microseconds a step
   // with and without a launch of its own, double-word: 512 x 512 (2048 cells a block) 74 / 64, 560 x 560
@@ -814,21 +906,23 @@ int sayram_batch_s::plan_team() {
   // up to 60 x 60 114 / 109, up to 100 x 100 258 / 288. In FP64 both are bound by the pipe, and only
   // the balance counts: 620 x 620 293 / 284, 900 x 900 562 / 552, 24 instances 352 / 346, 40 instances
   // (blocks up to 1.3 times the mean) 519 / 547, several to a block 280 / 259.
-  if (team_bins) team_split = dwm && own > 2 * kSplitCells;
-  else team_split = own > kSplitCells && (mixed || asm_most > 1.15 * (double)total / blocks);
-  team_chip = chip;
-  team_own = own;
+  if (plan.bins) plan.split = dwm && own > 2 * kSplitCells;
+  else plan.split = own > kSplitCells && (mixed || asm_most > 1.15 * (double)total / blocks);
+  plan.chip = chip;
+  plan.own = own;
   team_pmax = pm;
-  team_smem = sg::team_smem(ts, chip, own, pm, tile);
+  plan.smem = sg::team_smem(ts, chip, own, pm, tile);
+  plans[level] = plan;
   return SAYRAM_OK;
 }
 
 // One cooperative launch. A device or context that does not take it (one with fewer SMs to give than
 // the plan has blocks, for instance) is not asked again: the batch goes on as separate kernels.
-int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
+int sayram_batch_s::launch_team(const TeamPlan& plan, int nsteps, int phases, bool last) {
+  const long long level = &plan - plans;
   sg::TeamArgs ta{};
-  ta.share = d_share;
-  ta.first = team_bins ? d_first : nullptr;
+  ta.share = d_share + level * shares_cap;
+  ta.first = plan.bins ? d_first + level * (nsm + 1) : nullptr;
   ta.bar = d_bar;
   ta.tmax = d_tmax;
   ta.stat = h_stat;
@@ -840,16 +934,16 @@ int sayram_batch_s::launch_team(int nsteps, int phases, bool last) {
   ta.nsteps = nsteps;
   ta.phases = phases;
   ta.polls = sg::kTeamPolls;
-  ta.own_cap = (int)team_own;
+  ta.own_cap = (int)plan.own;
   ta.pmax = team_pmax;
-  sg::TeamLaunch l{team_grid, team_smem, team_chip, stream};
+  sg::TeamLaunch l{plan.grid, plan.smem, plan.chip, stream};
   const cudaError_t e = dwm     ? sg::team_launch_dw(l, cm, geo, fl, c32, k32, ta)
                         : mixed ? sg::team_launch_mixed(l, cm, geo, fl, c32, k32, ta)
                                 : sg::team_launch_f64(l, cm, geo, fl, c64, k64, ta);
   if (e == cudaSuccess) return SAYRAM_OK;
   cudaGetLastError();
   coop = 0;
-  team_grid = 0;
+  for (auto& p : plans) p = TeamPlan{};
   return kRefused;
 }
 
@@ -911,7 +1005,7 @@ int sayram_batch_s::build(const sayram_problem* probs, int count, const sayram_o
   for (int b = 0; b < count; ++b)
     if ((rc = place(b, probs[b], base[b], xoffv[b], yoffv[b], &doffv[4 * b], hoff[b]))) return rc;
   if ((rc = rebuild_lists())) return rc;
-  if (try_team && !team_grid) {
+  if (try_team && !team_grid()) {
     chunk = 4096;
     if ((rc = rebuild_lists())) return rc;
   }
@@ -1084,9 +1178,10 @@ int sayram_batch_s::build_graph(const sg::Coef<C>& cfull, const sg::Coef<T>& ck,
 }
 
 int sayram_batch_s::run_steps(int nsteps) {
+  DeviceCall call(dev);
   int rc = launch_steps(nsteps);
   if (rc) return rc;
-  if (team_grid > 0 && nsteps > 0) {  // k_team has left the outcome in host memory
+  if (by_flags && nsteps > 0) {  // k_team has left the outcome in host memory
     if ((rc = check_team())) return rc;
     if (timing) collect_timing();
     volatile int* f = h_stat;
@@ -1098,40 +1193,57 @@ int sayram_batch_s::run_steps(int nsteps) {
 }
 
 // Queues steps as cooperative launches; *queued: how many, all of them unless one was refused (kRefused).
+// At most two runs of a few milliseconds are on their way at a time, so that a long call goes on with fewer
+// SMs soon after another call has begun (90 x 90 FP64, 4000 steps: a 33 x 32 instance's calls beside it take
+// 50 us; with every launch over the whole chip they took 1.6 ms each).
 int sayram_batch_s::launch_team_steps(int nsteps, int* queued) {
   int& s = *queued;
+  const TeamPlan* plan = nullptr;
+  by_flags = true;
   if (timing) {  // the phases of a step one by one
     for (; s < nsteps; ++s) {
+      int rc = plan_now(&plan);
+      if (rc) return rc;
       launch("begin", [&] { sg::k_begin<<<(n + 255) / 256, 256, 0, stream>>>(cm); });
       const std::pair<const char*, int> ph[3] = {
           {"assemble", sg::TEAM_ASSEMBLE}, {"solve_coop", sg::TEAM_SOLVE}, {"polish", sg::TEAM_POLISH}};
       for (auto& p : ph) {
-        int rc = SAYRAM_OK;
         launch(p.first, [&] {
-          rc = team_split && p.second == sg::TEAM_ASSEMBLE
+          rc = plan->split && p.second == sg::TEAM_ASSEMBLE
                    ? launch_assemble(0, -1)
-                   : launch_team(1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH);
+                   : launch_team(*plan, 1, p.second, s == nsteps - 1 && p.second == sg::TEAM_POLISH);
         });
         if (rc) return rc;
       }
     }
     return SAYRAM_OK;
   }
-  if (team_split) {
-    for (; s < nsteps; ++s) {
-      int rc = rmax_clear ? SAYRAM_OK : launch_begin();
+  for (int run = 0; s < nsteps; ++run) {
+    if (run >= 2 && team_ev[run & 1]) SG_CUDA(cudaEventSynchronize(team_ev[run & 1]));
+    int rc = plan_now(&plan);
+    if (rc) return rc;
+    const int most = mixed || !plan ? kTeamSteps : (int)std::max(1LL, std::min((long long)kTeamSteps, 16384 / plan->own));
+    const int end = s + std::min(nsteps - s, most);
+    by_flags = plan != nullptr;
+    if (!plan) {
+      if ((rc = launch_separate(end - s))) return rc;
+      s = end;
+    } else if (!plan->split) {
+      if ((rc = launch_team(*plan, end - s, sg::TEAM_STEP, end == nsteps))) return rc;
+      s = end;
+    }
+    for (; s < end; ++s) {
+      rc = rmax_clear ? SAYRAM_OK : launch_begin();
       rmax_clear = true;
       if (!rc) rc = launch_assemble(0, -1);
-      if (!rc) rc = launch_team(1, sg::TEAM_SOLVE | sg::TEAM_POLISH, s == nsteps - 1);
+      if (!rc) rc = launch_team(*plan, 1, sg::TEAM_SOLVE | sg::TEAM_POLISH, s == nsteps - 1);
       if (rc) return rc;
     }
-    return SAYRAM_OK;
-  }
-  while (s < nsteps) {  // a launch stays well below a second
-    const int k = std::min(nsteps - s, kTeamSteps);
-    int rc = launch_team(k, sg::TEAM_STEP, s + k == nsteps);
-    if (rc) return rc;
-    s += k;
+    if (s + most < nsteps) {  // the run after the next waits for this one
+      cudaEvent_t& e = team_ev[run & 1];
+      if (!e) SG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      SG_CUDA(cudaEventRecord(e, stream));
+    }
   }
   return SAYRAM_OK;
 }
@@ -1140,11 +1252,17 @@ int sayram_batch_s::launch_steps(int nsteps) {
   if (nsteps < 0) return fail(SAYRAM_ERR_ARG, "nsteps must be >= 0");
   SG_CUDA(cudaSetDevice(dev));
   int s = 0;  // steps queued
-  if (team_grid > 0) {
+  if (team_grid() > 0) {
     h_stat[sg::TEAM_NEGATIVE] = h_stat[sg::TEAM_NOT_CONVERGED] = 0;  // nothing of this batch is running
     int rc = launch_team_steps(nsteps, &s);
     if (rc != kRefused) return rc;
   }
+  return launch_separate(nsteps - s);
+}
+// steps as separate kernels: each step's graph, or launched from here
+int sayram_batch_s::launch_separate(int nsteps) {
+  by_flags = false;
+  rmax_clear = false;
   const bool use_graph = opt.use_graph && !timing;
   if (use_graph && !gexec) {
     int rc = run_mode(true);
@@ -1153,7 +1271,7 @@ int sayram_batch_s::launch_steps(int nsteps) {
       return rc;
     }
   }
-  for (; s < nsteps; ++s) {
+  for (int s = 0; s < nsteps; ++s) {
     if (use_graph) {
       SG_CUDA(cudaGraphLaunch(gexec, stream));
       continue;
@@ -1474,7 +1592,7 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
     // the first run is small (a quarter of the others): its copy in is what the first assembly
     // waits for, and its polish is what the first copy out waits for; the rest are about equal
     // (a batch stepped by k_team copies around whole steps: runs of at least 4 MB, which take 20 us)
-    const long long least = b->team_grid > 0 ? 1LL << 19 : 1;
+    const long long least = b->team_grid() > 0 ? 1LL << 19 : 1;
     const long long target = std::max(least, (b->nreal + kPieces - 1) / kPieces);
     const long long first = std::max(least, (b->nreal + 4 * kPieces - 1) / (4 * kPieces));
     int a = 0;
@@ -1522,7 +1640,7 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
   // An instance whose state changed restarts its extrapolation history; one given back its own
   // current state (a host round trip) keeps it (k_field_in compares bit for bit).
   int rc = SAYRAM_OK;
-  const bool split = b->team_grid == 0 && b->opt.use_graph && !b->timing && nsteps >= 1 && np >= 2 && (f_in || f_out);
+  const bool split = b->team_grid() == 0 && b->opt.use_graph && !b->timing && nsteps >= 1 && np >= 2 && (f_in || f_out);
   if (split) {
     // Graph stepping with host buffers: the first step's assembly runs piece by piece behind the
     // copies in (each piece's tiles as soon as its cells have landed), and the last step's
@@ -1920,6 +2038,17 @@ long long region_cells(int nx, int ny) { return round_up((long long)(ny + 2) * r
 
 }  // namespace
 
+// A server counts as one call in flight, however many of its lanes are stepping: they have SMs of their own.
+struct ServerUse {
+  int dev = 0, stepping = 0;
+  void enter() {
+    if (stepping++ == 0) DeviceUse::of(dev).enter();
+  }
+  void leave() {
+    if (--stepping == 0) DeviceUse::of(dev).leave();
+  }
+};
+
 // One lane of the server: an engine with its own stream, arena, slots and queue. A lane runs one
 // step at a time; the server launches every idle lane that has work and collects each lane when
 // its step has finished, so lanes of small and of large instances advance at their own pace.
@@ -1939,11 +2068,13 @@ struct ServerLane {
   sayram_server_info info{};
   bool dirty = false;
   bool inflight = false;         // a step has been launched and not yet collected
+  ServerUse* use = nullptr;
   cudaEvent_t done_ev = nullptr;  // recorded after the step's launches
   double t_launch = 0.0, t_begin = 0.0;
 
   ~ServerLane() {
     if (inflight && done_ev) cudaEventSynchronize(done_ev);  // the engine's arrays outlive its step
+    if (inflight) use->leave();
     for (Request* r : waiting) delete r;
     if (done_ev) cudaEventDestroy(done_ev);
   }
@@ -2043,8 +2174,13 @@ struct ServerLane {
     const double tl = now_seconds();
     info.lists_seconds += tl - ta;
     if (info.resident == 0) return SAYRAM_OK;
-    if ((rc = eng.launch_steps(1))) return rc;
-    SG_CUDA(cudaEventRecord(done_ev, eng.stream));
+    use->enter();
+    rc = eng.launch_steps(1);
+    const cudaError_t e = rc ? cudaSuccess : cudaEventRecord(done_ev, eng.stream);
+    if (rc || e != cudaSuccess) {
+      use->leave();
+      return rc ? rc : fail(SAYRAM_ERR_CUDA, std::string("server step: ") + cudaGetErrorString(e));
+    }
     inflight = true;
     t_begin = t0;
     t_launch = tl;
@@ -2065,6 +2201,7 @@ struct ServerLane {
     if (ncomp) *ncomp = 0;
     SG_CUDA(cudaSetDevice(eng.dev));
     inflight = false;
+    use->leave();
     const double ts = now_seconds();
     info.step_seconds += ts - t_launch;
     info.ticks++;
@@ -2175,6 +2312,7 @@ struct ServerLane {
 // The server: one lane, or two -- instances with max(nx, ny) <= split in the first (its own
 // share of the budget and of the tables), the rest in the second.
 struct sayram_server_s {
+  ServerUse use;  // outlives the lanes
   std::vector<std::unique_ptr<ServerLane>> lanes;
   int split = 0;
   double wait_seconds = 600.0;  // longest host wait of one tick for a lane's step
@@ -2263,6 +2401,8 @@ int sayram_server_create(const sayram_server_config* cfg, const sayram_options* 
       const int small = std::min(L->eng.nsm - 1, std::max(1, (int)std::lround(0.5 * frac * L->eng.nsm)));
       L->eng.team_sms = k == 0 ? small : L->eng.nsm - small;
     }
+    L->use = &s->use;
+    s->use.dev = L->eng.dev;
     s->lanes.push_back(std::move(L));
   }
   *out = s.release();
@@ -2587,12 +2727,19 @@ extern "C" int sayram_step_noalloc(const sayram_problem* pd, const sayram_option
   SG_CUDA(cudaGetLastError());
   // whole steps as one cooperative launch where the instance's vectors fit the chip (all but very wide
   // grids) and the caller's stream takes it; else pass by pass from here
-  const int blocks = std::min(nsm, kNoAllocMaxBlocks), per = (I.nseg + blocks - 1) / blocks;
-  const int nb = (I.nseg + per - 1) / per;
-  const int help = (int)std::min<long long>(blocks - nb, std::max<long long>(0, tile_count(I, 2) - nb));
-  const long long own = (long long)split_instance(I, 0, nb, help, hshare) * I.seg;
-  const size_t smem_team = team_smem(sizeof(double), true, own, pitch, sizeof(AsmTile<F64A>));
-  const bool team = own <= team_chip_cells(sizeof(double)) && smem_team <= g_noalloc_smem[dev];
+  DeviceCall call(dev);
+  int nb = 0, help = 0;
+  long long own = 0;
+  size_t smem_team = 0;
+  bool team = false;
+  for (int level = DeviceUse::of(dev).level(7); !team && level >= 0; --level) {
+    const int blocks = std::max(1, std::min(nsm, kNoAllocMaxBlocks) >> level), per = (I.nseg + blocks - 1) / blocks;
+    nb = (I.nseg + per - 1) / per;
+    help = (int)std::min<long long>(blocks - nb, std::max<long long>(0, tile_count(I, 2) - nb));
+    own = (long long)split_instance(I, 0, nb, help, hshare) * I.seg;
+    smem_team = team_smem(sizeof(double), true, own, pitch, sizeof(AsmTile<F64A>));
+    team = own <= team_chip_cells(sizeof(double)) && smem_team <= g_noalloc_smem[dev];
+  }
   int hstat[TEAM_FLAGS] = {};
   int queued = 0;  // steps queued as cooperative launches: all, unless one is refused
   if (team && nsteps > 0) {

@@ -3,6 +3,8 @@ The shim stands before the library's own launchers of the cooperative step."""
 import ctypes
 import os
 import sys
+import threading
+import time
 
 import numpy as np
 
@@ -260,7 +262,39 @@ def gave_up_server():
         assert np.array_equal(x[0], y[0]) and x[1] == y[1]
 
 
+def side_by_side():
+    """While another thread's call is in flight a launch takes at most half the SMs, and all of them again
+    after it, with the same bits; a call in flight goes on with fewer when another begins."""
+    import torch
+
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    for prec in (0, 1, 2):
+        for probs in (one(200, 180), cases.batch_problems(nsm + 8, 7, 1e-2, 8, 40)):
+            shim_set(FOREVER, 0)
+            other, alone, b = capi.Batch(one(33, 32), precision=prec), capi.Batch(probs, precision=prec), None
+            alone.step(2)
+            alone.step(2)
+            whole = shim.shim_grid()
+            assert nsm // 2 < whole <= nsm
+            b = capi.Batch(probs, precision=prec)
+            shim.shim_hold(400)
+            t = threading.Thread(target=other.step, args=(1,))
+            t.start()
+            while not shim.shim_held():
+                time.sleep(0.001)
+            b.step(2)
+            assert 0 < shim.shim_grid() <= nsm // 2, shim.shim_grid()
+            t.join()
+            time.sleep(0.05)
+            b.step(2)
+            assert shim.shim_grid() == whole
+            same(result(b), result(alone))
+            for x in (other, alone, b):
+                x.close()
+
+
 SCENARIOS = {
+    "side by side": side_by_side,
     "gave up": gave_up,
     "gave up split": gave_up_split,
     "gave up autotune": gave_up_autotune,

@@ -4,6 +4,10 @@
 // barrier of a team of several blocks gives up), or hands them on as they are.
 #include <dlfcn.h>
 
+#include <atomic>
+#include <chrono>
+#include <thread>
+
 #include "sayram_team.h"
 
 static int g_pass = 0, g_odd = 0, g_give_up = 0, g_calls = 0;
@@ -21,9 +25,23 @@ extern "C" int shim_set(const char* lib, int pass, int odd, int give_up) {
 }
 extern "C" int shim_calls() { return g_calls; }
 
+static std::atomic<int> g_hold{0}, g_held{0}, g_grid{0};
+// the next launch waits on the host for ms milliseconds first; shim_held: it is waiting or has waited
+extern "C" void shim_hold(int ms) {
+  g_held = 0;
+  g_hold = ms;
+}
+extern "C" int shim_held() { return g_held; }
+extern "C" int shim_grid() { return g_grid; }  // blocks of the last launch
+
 template <typename F, typename... X>
-static cudaError_t on(F* self, sg::TeamArgs ta, const X&... x) {
+static cudaError_t on(F* self, sg::TeamArgs ta, const sg::TeamLaunch& l, const X&... x) {
   ++g_calls;
+  g_grid = l.grid;
+  if (const int ms = g_hold.exchange(0)) {
+    g_held = 1;
+    std::this_thread::sleep_for(std::chrono::milliseconds(ms));
+  }
   if (g_pass > 0) {
     --g_pass;
   } else if (g_odd > 0) {
@@ -33,7 +51,7 @@ static cudaError_t on(F* self, sg::TeamArgs ta, const X&... x) {
   }
   Dl_info info;
   F* f = dladdr(reinterpret_cast<void*>(self), &info) ? reinterpret_cast<F*>(dlsym(g_lib, info.dli_sname)) : nullptr;
-  return f && f != self ? f(x..., ta) : cudaErrorSymbolNotFound;
+  return f && f != self ? f(l, x..., ta) : cudaErrorSymbolNotFound;
 }
 
 namespace sg {

@@ -38,3 +38,7 @@ def test_a_refused_launch_goes_on_as_separate_kernels(shim, scenario):
 def test_a_wait_that_runs_out(shim, scenario):
     """The barriers of one launch get no polls: its blocks leave, and the host is told."""
     _child(shim, scenario)
+
+
+def test_calls_side_by_side_share_the_chip(shim):
+    _child(shim, "side by side")

@@ -215,3 +215,54 @@ def test_a_residual_out_of_range_is_not_converged(capi, state, prec, coop):
     want = capi.OK if state == "residual" and prec == 0 else capi.ERR_NOT_CONVERGED
     assert rc == want and st["status"] == want, (rc, st)
     assert (st["rel_residual"] < 1e-10) == (want == capi.OK)
+
+
+def test_handles_stepped_side_by_side(capi):
+    """Handles of all kinds stepped from eight threads, in calls of one step and of many, with a server
+    beside them: each gives the bits it gives alone, whatever share of the chip its launches had."""
+    import threading
+
+    kinds = [([cases.synthetic_problem(33, 32, 1e-2, seed=1, tau=0.7)], 0, (1,) * 40),
+             ([cases.synthetic_problem(90, 90, 1e-2, seed=2, tau=0.7)], 0, (100,)),
+             ([cases.synthetic_problem(80, 80, 1e-2, seed=3, tau=0.7)], 2, (1,) * 60),
+             ([cases.synthetic_problem(389, 517, 1e-2, seed=4, tau=0.7)], 2, (40, 1, 1)),
+             ([cases.synthetic_problem(700, 620, 1e-2, seed=5, tau=0.7)], 1, (3,) * 10),
+             ([cases.synthetic_problem(256, 256, 1e-2, seed=6, tau=0.7)], 0, (1,) * 20),
+             (cases.batch_problems(24, 7, 1e-2, 20, 120), 2, (1,) * 20),
+             (cases.batch_problems(170, 7, 1e-2, 8, 40), 1, (70,))]
+
+    def run(kind, out, start):
+        probs, prec, calls = kind
+        b = capi.Batch(probs, precision=prec)
+        if start:
+            start.wait()
+        for n in calls:
+            b.step(n)
+        out.append(([b.f(k) for k in range(len(probs))], [b.stats(k) for k in range(len(probs))]))
+        b.close()
+
+    def serve(out, start):
+        srv = capi.Server(5e8, max_slots=8, max_side=128, precision=2, lanes=2, split_side=64)
+        if start:
+            start.wait()
+        ids = [srv.submit(cases.synthetic_problem(a, a + 7, 1e-2, seed=a, tau=0.5), 30) for a in (20, 40, 64, 100)]
+        while srv.info()["completed"] < len(ids):
+            srv.tick()
+        got = [srv.poll(i) for i in ids]
+        srv.close()
+        out.append(([g[0] for g in got], [g[1] for g in got]))
+
+    alone, mixed = [[] for _ in range(9)], [[] for _ in range(9)]
+    for kind, out in zip(kinds, alone):
+        run(kind, out, None)
+    serve(alone[8], None)
+    start = threading.Barrier(9)
+    ts = [threading.Thread(target=run, args=(k, o, start)) for k, o in zip(kinds, mixed)]
+    ts.append(threading.Thread(target=serve, args=(mixed[8], start)))
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for a, m in zip(alone, mixed):
+        assert len(m) == 1
+        _same(a[0], m[0])
