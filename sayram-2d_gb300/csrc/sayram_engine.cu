@@ -183,7 +183,6 @@ struct sayram_batch_s {
     tab_cap = 0;
     if (h_ctl) cudaFreeHost(h_ctl);
     h_ctl = nullptr;
-    if (h_stat) cudaFreeHost(h_stat);
     h_stat = nullptr;
     for (auto& e : team_ev) {
       if (e) cudaEventDestroy(e);
@@ -310,7 +309,7 @@ struct sayram_batch_s {
   int* d_first = nullptr;            // nsm + 1 of them for every plan
   unsigned* d_bar = nullptr;
   float* d_tmax = nullptr;
-  int* h_stat = nullptr;  // pinned, written by k_team (TEAM_* flags)
+  int* h_stat = nullptr;  // behind h_ctl, written by k_team (TEAM_* flags)
   static constexpr long long kSplitCells = 2048;
   cudaEvent_t team_ev[2] = {nullptr, nullptr};  // ends of a call's last two runs of steps
   int plan_team();
@@ -556,12 +555,16 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
   pstride = 8LL * chunks_cap;  // a chunk of 1024 cells holds 8 segments, the most of any chunk size
   SG_ALLOC(d_part, (long long)sg::kPartSets * sg::kPartQ * pstride);
   shares_cap = std::max(slots, nsm);
-  SG_ALLOC(d_share, (long long)kTeamLevels * shares_cap);
-  SG_ALLOC(d_first, (long long)kTeamLevels * (nsm + 1));
-  SG_ALLOC(d_bar, (long long)slots * sg::kTeamBarStride);
-  SG_ALLOC(d_tmax, nsm);
-  SG_CUDA(cudaMallocHost(&h_stat, sizeof(int) * sg::TEAM_FLAGS));
-  std::memset(h_stat, 0, sizeof(int) * sg::TEAM_FLAGS);
+  {  // the tables of the cooperative step, all of 4-byte entries, in one allocation (an allocation takes 8 us)
+    static_assert(sizeof(sg::TeamShare) % sizeof(int) == 0 && alignof(sg::TeamShare) == alignof(int), "an int array");
+    const long long nbar = (long long)slots * sg::kTeamBarStride, nfirst = (long long)kTeamLevels * (nsm + 1);
+    int* t = nullptr;
+    SG_ALLOC(t, nbar + nsm + nfirst + (long long)kTeamLevels * shares_cap * (long long)(sizeof(sg::TeamShare) / sizeof(int)));
+    d_bar = (unsigned*)t;
+    d_tmax = (float*)(t + nbar);
+    d_first = t + nbar + nsm;
+    d_share = (sg::TeamShare*)(d_first + nfirst);
+  }
   SG_ALLOC(d_stage, stage_cap);
   cell_arrays.clear();
   double** geos[10] = {&geo.aAx, &geo.aBx, &geo.Sx, &geo.aAy, &geo.aBy, &geo.Sy, &geo.ukk, &geo.sdiag, &geo.G,
@@ -599,8 +602,10 @@ int sayram_batch_s::alloc_storage(long long cells, int slots, int chunks_cap, in
     }
   }
 #undef SG_ALLOC
-  SG_CUDA(cudaMallocHost(&h_ctl, sizeof(Ctl)));
-  std::memset(h_ctl, 0, sizeof(Ctl));
+  const size_t pinned = sizeof(Ctl) + sizeof(int) * sg::TEAM_FLAGS;
+  SG_CUDA(cudaMallocHost(&h_ctl, pinned));
+  std::memset((void*)h_ctl, 0, pinned);
+  h_stat = (int*)(h_ctl + 1);
   hinst.assign(slots, InstDev{});
   cm = sg::Common{};
   cm.inst = d_inst;
@@ -1713,11 +1718,25 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
   return rc;
 }
 
+// Cells up to which a state is transposed on the host: there the launch costs more than the cells. set_f and
+// get_f in us, on the host / on the device: 16 x 16 FP64 12 / 16 and 12 / 18, 64 x 64 16 / 18 and 16 / 19, 80 x
+// 80 in double-word 25 / 20 and 20 / 19, 256 x 256 FP64 105 / 28 and 100 / 22.
+constexpr size_t kHostTranspose = 4096;
+
 int sayram_batch_get_f(sayram_batch b, int idx, double* f_out) {
   if (!b || !f_out || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
   if (int rc = b->whole(idx)) return rc;
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
+  const size_t nr = (size_t)I.ny * I.pitch;
+  if (nr <= kHostTranspose) {
+    std::vector<double> rows(nr);
+    SG_CUDA(cudaMemcpyAsync(rows.data(), b->fl.f + I.base, sizeof(double) * nr, cudaMemcpyDeviceToHost, b->stream));
+    SG_CUDA(cudaStreamSynchronize(b->stream));
+    for (int i = 0; i < I.nx; ++i)
+      for (int j = 0; j < I.ny; ++j) f_out[(size_t)i * I.ny + j] = b->unwide(rows[(size_t)j * I.pitch + i]);
+    return SAYRAM_OK;
+  }
   const int t0 = I.tile0, t1 = I.tile0 + I.ntx * I.nty;
   // transposed (and, in double-word mode, converted) on the device into the staging buffer
   b->layout_out(t0, t1, b->d_stage - I.hoff, b->stream);
@@ -1731,9 +1750,17 @@ int sayram_batch_set_f(sayram_batch b, int idx, const double* f) {
   if (!b || !f || idx < 0 || idx >= b->n) return fail(SAYRAM_ERR_ARG, "bad handle, index or buffer");
   SG_CUDA(cudaSetDevice(b->dev));
   const InstDev& I = b->hinst[idx];
-  SG_CUDA(cudaMemcpyAsync(b->d_stage, f, sizeof(double) * (size_t)I.nx * I.ny, cudaMemcpyHostToDevice, b->stream));
-  b->layout_in(I.tile0, I.tile0 + I.ntx * I.nty, b->d_stage - I.hoff, 0, b->stream);
-  SG_CUDA(cudaGetLastError());
+  const size_t nr = (size_t)I.ny * I.pitch;
+  std::vector<double> rows(nr <= kHostTranspose ? nr : 0, 0.0);
+  if (!rows.empty()) {
+    for (int i = 0; i < I.nx; ++i)
+      for (int j = 0; j < I.ny; ++j) rows[(size_t)j * I.pitch + i] = b->wide(f[(size_t)i * I.ny + j]);
+    SG_CUDA(cudaMemcpyAsync(b->fl.f + I.base, rows.data(), sizeof(double) * nr, cudaMemcpyHostToDevice, b->stream));
+  } else {
+    SG_CUDA(cudaMemcpyAsync(b->d_stage, f, sizeof(double) * (size_t)I.nx * I.ny, cudaMemcpyHostToDevice, b->stream));
+    b->layout_in(I.tile0, I.tile0 + I.ntx * I.nty, b->d_stage - I.hoff, 0, b->stream);
+    SG_CUDA(cudaGetLastError());
+  }
   SG_CUDA(cudaMemsetAsync((char*)(b->d_st + idx) + offsetof(InstState, nhist), 0, sizeof(int), b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
   if (idx < (int)b->lost.size()) b->lost[idx] = 0;
@@ -1748,8 +1775,16 @@ int sayram_batch_set_dirichlet(sayram_batch b, int idx, int side, const double* 
   const int m = (side <= 1) ? I.ny + 1 : I.nx + 1;
   if (n != m) return fail(SAYRAM_ERR_ARG, "expected " + std::to_string(m) + " vertex values");
   SG_CUDA(cudaSetDevice(b->dev));
-  // the values travel as kernel parameters: no copy to wait for, and the caller's buffer is free at once
-  // (81 values: 11.4 us a call with a copy and a wait, 5.4 so)
+  // up to three launches' worth of values travel as kernel parameters: no copy to wait for, and the caller's
+  // buffer is free at once (81 values: 11.4 us a call with a copy and a wait, 5.4 so; 1025: 14.1 / 12.6; 4097:
+  // 20 / 38)
+  if (m > 3 * PutArgs::kMost) {
+    std::vector<double> wv(m);
+    for (int k = 0; k < m; ++k) wv[k] = b->wide(v[k]);
+    SG_CUDA(cudaMemcpyAsync(b->d_dirv + I.dir[side], wv.data(), sizeof(double) * m, cudaMemcpyHostToDevice, b->stream));
+    SG_CUDA(cudaStreamSynchronize(b->stream));
+    return SAYRAM_OK;
+  }
   for (int at = 0; at < m; at += PutArgs::kMost) {
     PutArgs p;
     p.n = std::min(m - at, PutArgs::kMost);

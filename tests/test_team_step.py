@@ -266,3 +266,28 @@ def test_handles_stepped_side_by_side(capi):
     for a, m in zip(alone, mixed):
         assert len(m) == 1
         _same(a[0], m[0])
+
+
+@pytest.mark.parametrize("prec", [0, 2])
+@pytest.mark.parametrize("ny", [1024, 1025])
+def test_state_transposed_on_either_side(capi, ny, prec):
+    """4096 cells go through the host, more through the device, in a batch whose instances are of both kinds:
+    the states come back as they went in, to the other instances' none."""
+    probs = [cases.synthetic_problem(a, b, 1e-2, seed=k, tau=0.7) for k, (a, b) in enumerate([(9, 7), (3, ny), (70, 66)])]
+    b = capi.Batch(probs, precision=prec)
+    before = [b.f(k) for k in range(3)]
+    f = np.random.default_rng(ny).uniform(0.0, 1.0, (3, ny)) * 10.0 ** np.random.default_rng(1).uniform(-30, 30, (3, ny))
+    b.set_f(1, f)
+    got = [b.f(k) for k in range(3)]
+    b.close()
+    hi = f.astype(np.float32)
+    want = f if prec == 0 else hi.astype(np.float64) + (f - hi).astype(np.float32).astype(np.float64)
+    assert np.array_equal(got[1], want)
+    assert np.array_equal(got[0], before[0]) and np.array_equal(got[2], before[2])
+
+
+@pytest.mark.parametrize("prec", [0, 2])
+@pytest.mark.parametrize("nx", [1439, 1440])
+def test_dirichlet_values_at_the_last_launch(capi, nx, prec):
+    """1440 values are the most that travel with launches; 1441 are copied."""
+    test_dirichlet_values_of_any_number(capi, nx, prec)
