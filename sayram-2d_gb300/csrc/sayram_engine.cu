@@ -1390,6 +1390,7 @@ int sayram_batch_s::autotune(int steps, int* best_chunk, int* best_grid) {
   if (steps < 1) steps = 1;
   int rc = whole();
   if (rc) return rc;
+  DeviceCall call(dev);
   SG_CUDA(cudaSetDevice(dev));
   constexpr int kSnap = 3 + sg::kHist;
   double* snap = nullptr;  // f, the history states and both y buffers
@@ -1651,6 +1652,7 @@ int sayram_batch_step_host(sayram_batch b, int nsteps, const double* f_in, doubl
     // copies in (each piece's tiles as soon as its cells have landed), and the last step's
     // polish runs piece by piece ahead of the copies out; in between, graphs. Every piece holds
     // whole instances, so the per-instance reductions stay inside one launch.
+    DeviceCall call(b->dev);
     if ((rc = b->ensure_solve_graph())) return rc;
     if (nsteps > 2 && (rc = b->launch_steps(0))) return rc;  // builds the full step's graph up front
     for (int s = 0; s < nsteps; ++s) {

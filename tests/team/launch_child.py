@@ -293,8 +293,37 @@ def side_by_side():
                 x.close()
 
 
+def beside_separate_kernels():
+    """A call that runs as separate kernels is in flight like any other, in each of its forms."""
+    import torch
+
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    shim_set(FOREVER, 0)
+    b = capi.Batch(one(200, 180), precision=2)
+    b.step(1)
+    whole = shim.shim_grid()
+    a = capi.Batch(cases.batch_problems(24, 7, 1e-2, 64, 200), precision=2)
+    a.set_launch_shape(4096, 32)  # segments too coarse for teams
+    packed = np.concatenate([np.array(p.f0).ravel() for p in a.problems])
+    out = np.empty_like(packed)
+    for call in (lambda: a.step(2000), lambda: a.step_host(2000, packed.ctypes.data, out.ctypes.data),
+                 lambda: a.autotune(200)):
+        t = threading.Thread(target=call)
+        t.start()
+        time.sleep(0.1)
+        b.step(1)
+        grid = shim.shim_grid()
+        assert t.is_alive()
+        assert 0 < grid <= nsm // 2 < whole, (grid, whole)
+        t.join()
+        a.set_launch_shape(4096, 32)
+    a.close()
+    b.close()
+
+
 SCENARIOS = {
     "side by side": side_by_side,
+    "beside separate kernels": beside_separate_kernels,
     "gave up": gave_up,
     "gave up split": gave_up_split,
     "gave up autotune": gave_up_autotune,

@@ -40,5 +40,6 @@ def test_a_wait_that_runs_out(shim, scenario):
     _child(shim, scenario)
 
 
-def test_calls_side_by_side_share_the_chip(shim):
-    _child(shim, "side by side")
+@pytest.mark.parametrize("scenario", ["side by side", "beside separate kernels"])
+def test_calls_side_by_side_share_the_chip(shim, scenario):
+    _child(shim, scenario)
