@@ -4,6 +4,7 @@
 // layout, the chunk/tile work lists, the per-step launch sequence and the optional CUDA graph.
 // Every public function returns a status code and records a message for sayram_last_error().
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <deque>
 #include <map>
@@ -63,37 +64,29 @@ class DeviceUse {
     static DeviceUse use[128];
     return use[dev & 127];
   }
-  void enter() {
-    std::lock_guard<std::mutex> g(mu);
-    ++inflight;
-    roll();
-  }
-  void leave() {
-    std::lock_guard<std::mutex> g(mu);
-    --inflight;
-  }
+  void enter() { inflight.fetch_add(1); }
+  void leave() { inflight.fetch_sub(1); }
+  // the level for a launch of a call that has entered
   int level(int most) {
     std::lock_guard<std::mutex> g(mu);
-    roll();
+    const auto t = std::chrono::steady_clock::now();
+    if (t - since > kWindow) {
+      last = t - since > 2 * kWindow ? 0 : peak;
+      peak = 0;
+      since = t;
+    }
+    peak = std::max(peak, inflight.load());
     int l = 0;
     while (l < most && (1 << l) < std::max(peak, last)) ++l;
     return l;
   }
 
  private:
-  static constexpr double kWindow = 0.005;  // seconds; longer than the host's part of a loop of short calls
+  static constexpr std::chrono::milliseconds kWindow{5};  // longer than the host's part of a loop of short calls
+  std::atomic<int> inflight{0};
   std::mutex mu;
-  int inflight = 0, peak = 0, last = 0;  // now; the most in this window and in the one before
-  double since = 0.0;
-  void roll() {
-    const double t = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
-    if (t - since > kWindow) {
-      last = t - since > 2 * kWindow ? 0 : peak;
-      peak = 0;
-      since = t;
-    }
-    peak = std::max(peak, inflight);
-  }
+  int peak = 0, last = 0;  // the most calls in flight in this window and in the one before
+  std::chrono::steady_clock::time_point since{};
 };
 struct DeviceCall {  // one call in flight
   DeviceUse& use;
