@@ -215,8 +215,10 @@ int sayram_batch_elapsed_ms(sayram_batch b, int slot0, int slot1, double* ms);
 /* Per-kernel timing: when enabled, every launch is bracketed by CUDA events on the batch's
  * stream (steps then run without graphs). sayram_batch_kernel_times fills up to cap entries of
  * names/total milliseconds/launch counts and returns the number of entries: one per kernel, plus
- * "krylov_tail10" and "krylov_rest", the time of whole BiCGSTAB iterations (bicg1, bicg2, bicg3)
- * in which fewer than 10 % / at least 10 % of the enabled instances were still iterating. */
+ * "krylov_tail10" and "krylov_rest", the time of whole BiCGSTAB iterations in which fewer than 10 % / at
+ * least 10 % of the enabled instances were still iterating. "bicg1" is an iteration's first pass with the
+ * decisions after it, "bicg2" its second pass, "bicg3" the decisions after that one; a batch stepped by
+ * cooperative launches has "solve_coop", the whole refinement loop, in place of these. */
 int sayram_batch_enable_timing(sayram_batch b, int enable);
 int sayram_batch_kernel_times(sayram_batch b, const char** names, double* total_ms,
                               long long* launches, int cap);
@@ -231,8 +233,7 @@ int sayram_batch_autotune(sayram_batch b, int steps, int* chunk_out, int* blocks
  * each; larger batches run as the graph's loops of separate kernels, and so does a batch whose
  * cooperative launch the device has refused. Handles and servers that several threads step on one GPU at
  * the same time share its SMs: a launch takes a half, a quarter, ... of them by the number of calls in
- * flight. on = 0 always uses the separate kernels (the results are
- * the same bit for bit). Default: 1. */
+ * flight. on = 0 always uses the separate kernels (the results are the same bit for bit). Default: 1. */
 int sayram_batch_set_coop(sayram_batch b, int on);
 /* Sets the launch shape directly (chunk 1024, 2048 or 4096 cells; 1..64 blocks per SM), or reads
  * it back. The default is chosen from the batch size; results do not depend on it beyond the

@@ -246,8 +246,8 @@ __device__ __forceinline__ void after_v(InstState& st, const R (&tot)[2]) {
 // omega t, so (r, r) and (r^, r) follow from these sums and the pass that would form them is not
 // needed. (r^, s) is zero by the choice of alpha, but for rounding, and is summed all the same: without
 // it the error of rho stays from one iteration to the next, and long solves stall (four sums were 3 % faster
-// on most double-word cases, but a burst of 48 server requests took 378 instead of 39 ms and four
-// FP64 steps of 1024 x 1024 23.6 instead of 12.7). Returns 1 when this Krylov solve ends.
+// on most double-word cases, but a burst of 48 server requests took 378 instead of 39 ms and, from the same
+// fields, four FP64 steps of 1024 x 1024 23.6 instead of 12.7). Returns 1 when this Krylov solve ends.
 template <typename R>
 __device__ __forceinline__ int after_t(InstState& st, const R (&tot)[5], int max_iters) {
   const R ts = tot[0], tt = tot[1];
