@@ -291,3 +291,20 @@ def test_state_transposed_on_either_side(capi, ny, prec):
 def test_dirichlet_values_at_the_last_launch(capi, nx, prec):
     """1440 values are the most that travel with launches; 1441 are copied."""
     test_dirichlet_values_of_any_number(capi, nx, prec)
+
+
+@pytest.mark.parametrize("coop", [True, False])
+@pytest.mark.parametrize("prec,tol", [(0, 1e-10), (1, 1e-8), (2, 1e-8)])
+@pytest.mark.parametrize("precond", [0, 1])
+def test_long_solves(capi, oracle, precond, prec, tol, coop):
+    """A time step that leaves almost no diagonal: hundreds of iterations in one step, in FP64 in a single
+    solve to the final tolerance, in which the residual's dot products only come from earlier sums."""
+    p = cases.synthetic_problem(40, 36, 1e6, seed=11, tau=1e30)
+    s = capi.Solver(p, precision=prec, precond=precond)
+    s.set_coop(coop)
+    s.update()
+    f, st = s.f(), s.stats(0)
+    s.close()
+    ref = oracle.step(p, None, 1, solver="splu")
+    assert st["status"] == capi.OK and st["iterations"] >= 150, st
+    assert np.linalg.norm(f - ref) <= tol * np.linalg.norm(ref)
